@@ -123,7 +123,8 @@ typedef struct {
     double pair_slack;  /* pair capacity = slack * pairs of the first list; 0 = 1.6 and at least
                            the reference's own n_sub * BranchLmtLen/2 as far as 30% of free memory allows */
     int search_lanes;   /* lanes per subsphere in the neighbour search: 8, 16 or 32 (0 = 8) */
-    int clump_batch;    /* members each lane of the clump pass loads at a time: 1, 2 or 4 (0 = 1) */
+    int clump_batch;    /* kept for callers and reported back (1, 2 or 4; 0 = 1): the clump pass gives each
+                           member a lane of its own */
     int pair_blocks;    /* blocks per SM of the pair kernel's grid: 2 .. 16 (0 = 12) */
 } nbc_options;
 
@@ -308,9 +309,8 @@ nbc_status nbc_server_set_cohort(nbc_server* s, int max_requests);
 
 /* Autotuner (no reference counterpart): times trial_steps steps (after a
  * short warm-up) of engines made from these scenes with candidate launch
- * shapes -- lanes per subsphere of the neighbour search, members per lane
- * of the clump pass, blocks per SM of the pair kernel -- by coordinate
- * descent from the defaults, a candidate replacing the incumbent only when
+ * shapes -- lanes per subsphere of the neighbour search, blocks per SM of
+ * the pair kernel -- by coordinate descent from the defaults, a candidate replacing the incumbent only when
  * it is at least 3% faster, and writes the fastest into opt (other fields
  * untouched).  The shapes change no result: every candidate computes the
  * same lists and forces bit for bit.  The choice is cached in the process

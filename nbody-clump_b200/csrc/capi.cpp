@@ -499,16 +499,10 @@ nbc_status nbc_autotune(const nbc_scene_desc* const* scenes, int n, nbc_options*
         best.pair_blocks = 12;
         best.use_graph = 1;
         double tb = trial(best);
-        const int lanes[] = {16, 32}, batch[] = {2, 4}, blocks[] = {4, 8, 16};
+        const int lanes[] = {16, 32}, blocks[] = {4, 8, 16};
         for (int x : lanes) {
             nbc_options o = best;
             o.search_lanes = x;
-            const double t = trial(o);
-            if (t < 0.97 * tb) { best = o; tb = t; }
-        }
-        for (int x : batch) {
-            nbc_options o = best;
-            o.clump_batch = x;
             const double t = trial(o);
             if (t < 0.97 * tb) { best = o; tb = t; }
         }

@@ -314,8 +314,9 @@ class EngineT final : public EngineBase {
             copy_(fix, h_.part_fix + o, n * sizeof(int), cudaMemcpyDeviceToHost);
         }
         if (cid) {
-            copy_(cid, h_.clump_id + o, n * sizeof(int), cudaMemcpyDeviceToHost);
-            for (int i = 0; i < n; i++) cid[i] -= P.clump_off;
+            std::vector<int2> cm(n);
+            copy_(cm.data(), h_.cm + o, n * sizeof(int2), cudaMemcpyDeviceToHost);
+            for (int i = 0; i < n; i++) cid[i] = cold_[cm[i].x];
         }
         if (pos || rad) {
             std::vector<double4> tmp(n);
@@ -330,41 +331,37 @@ class EngineT final : public EngineBase {
         refresh_dev();
         const ScenePar& P = hpar_[s];
         std::vector<double4> tmp(P.nsub);
+        std::vector<int2> cm(P.nsub);
         copy_(tmp.data(), h_.lom + P.sub_off, P.nsub * sizeof(double4), cudaMemcpyDeviceToHost);
+        copy_(cm.data(), h_.cm + P.sub_off, P.nsub * sizeof(int2), cudaMemcpyDeviceToHost);
         for (int i = 0; i < P.nsub; i++) {
-            if (local) { local[3 * i] = tmp[i].x; local[3 * i + 1] = tmp[i].y; local[3 * i + 2] = tmp[i].z; }
-            if (mass) mass[i] = tmp[i].w;
+            const double4& t = tmp[cm[i].y - P.sub_off];   // a scene's member slots are its subsphere range
+            if (local) { local[3 * i] = t.x; local[3 * i + 1] = t.y; local[3 * i + 2] = t.z; }
+            if (mass) mass[i] = t.w;
         }
     }
     void get_clump_prop(int s, double* prop) override {
         const ScenePar& P = hpar_[s];
-        std::vector<double4> tmp(P.nclump);
-        copy_(tmp.data(), h_.cprop + P.clump_off, P.nclump * sizeof(double4), cudaMemcpyDeviceToHost);
-        for (int i = 0; i < P.nclump; i++) {
-            prop[4 * i] = tmp[i].x; prop[4 * i + 1] = tmp[i].y; prop[4 * i + 2] = tmp[i].z; prop[4 * i + 3] = tmp[i].w;
-        }
+        clumps_out<4>(h_.cprop, P, prop);
+    }
+    // clump records of one scene in the caller's order, W doubles each
+    template <int W>
+    void clumps_out(const double4* src, const ScenePar& P, double* dst) {
+        const int n = P.nclump;
+        k_clumps_out<W><<<std::min(cdiv(n, 256), sm_count_ * 8), 256, 0, stream_>>>(src, h_.cold, P.clump_off, n,
+                                                                                   (double*)h_.stage);
+        CK(cudaGetLastError());
+        copy_(dst, h_.stage, (size_t)n * W * sizeof(double), cudaMemcpyDeviceToHost);
     }
     void get_clumps(int s, double* pos, double* vel, double* quat, double* w, double* f, double* t) override {
         refresh_dev();
         const ScenePar& P = hpar_[s];
-        int n = P.nclump, o = P.clump_off;
-        std::vector<double4> tmp(n);
-        auto pull3 = [&](double4* src, double* dst) {
-            if (!dst) return;
-            copy_(tmp.data(), src + o, n * sizeof(double4), cudaMemcpyDeviceToHost);
-            for (int i = 0; i < n; i++) { dst[3 * i] = tmp[i].x; dst[3 * i + 1] = tmp[i].y; dst[3 * i + 2] = tmp[i].z; }
-        };
-        pull3(h_.cpos, pos);
-        pull3(h_.cvel, vel);
-        pull3(h_.cw, w);
-        pull3(h_.cF, f);
-        pull3(h_.cT, t);
-        if (quat) {
-            copy_(tmp.data(), h_.cq + o, n * sizeof(double4), cudaMemcpyDeviceToHost);
-            for (int i = 0; i < n; i++) {
-                quat[4 * i] = tmp[i].x; quat[4 * i + 1] = tmp[i].y; quat[4 * i + 2] = tmp[i].z; quat[4 * i + 3] = tmp[i].w;
-            }
-        }
+        if (pos) clumps_out<3>(h_.cpos, P, pos);
+        if (vel) clumps_out<3>(h_.cvel, P, vel);
+        if (w) clumps_out<3>(h_.cw, P, w);
+        if (f) clumps_out<3>(h_.cF, P, f);
+        if (t) clumps_out<3>(h_.cT, P, t);
+        if (quat) clumps_out<4>(h_.cq, P, quat);
     }
     void get_sub_forces(int s, double* f, double* t) override {
         refresh_dev();
@@ -600,7 +597,9 @@ class EngineT final : public EngineBase {
         CK(cudaStreamSynchronize(stream_));
     }
     // Writes (src == nullptr: appends to out) or reads (from src at offset
-    // off) the checkpoint's blocks in one fixed order.
+    // off) the checkpoint's blocks in one fixed order.  The file holds clumps
+    // in the caller's order and what the engine keeps per member slot in
+    // subsphere order, so it does not depend on the engine's own order.
     void ck_blocks(std::vector<char>& out, const std::vector<char>* src, size_t off, const CkHeader& hd) {
         const size_t N = N_;
         auto blk = [&](void* dev, size_t n) {
@@ -613,6 +612,36 @@ class EngineT final : public EngineBase {
                 if (off + n > src->size()) throw ArgError("checkpoint truncated");
                 copy_(dev, src->data() + off, n, cudaMemcpyHostToDevice);
                 off += n;
+            }
+        };
+        // the same for a block that the host holds
+        auto hblk = [&](void* host, size_t n) {
+            if (!n) return;
+            if (!src) {
+                const size_t at = out.size();
+                out.resize(at + n);
+                memcpy(out.data() + at, host, n);
+            } else {
+                if (off + n > src->size()) throw ArgError("checkpoint truncated");
+                memcpy(host, src->data() + off, n);
+                off += n;
+            }
+        };
+        // an array of the clumps, in the caller's order in the file
+        auto cblk = [&](double4* dev) {
+            std::vector<double4> own(K_), file(K_);
+            if (!src) {
+                copy_(own.data(), dev, K_ * sizeof(double4), cudaMemcpyDeviceToHost);
+                for (int s = 0; s < S_; s++)
+                    for (int c = hpar_[s].clump_off; c < hpar_[s].clump_off + hpar_[s].nclump; c++)
+                        file[hpar_[s].clump_off + cold_[c]] = own[c];
+            }
+            hblk(file.data(), K_ * sizeof(double4));
+            if (src) {
+                for (int s = 0; s < S_; s++)
+                    for (int c = hpar_[s].clump_off; c < hpar_[s].clump_off + hpar_[s].nclump; c++)
+                        own[c] = file[hpar_[s].clump_off + cold_[c]];
+                copy_(dev, own.data(), K_ * sizeof(double4), cudaMemcpyHostToDevice);
             }
         };
         // scene bookkeeping first (its pair regions size the rest)
@@ -641,30 +670,70 @@ class EngineT final : public EngineBase {
         }
         // subspheres, current sort order
         blk(h_.posr, N * sizeof(double4));
-        blk(h_.lom, N * sizeof(double4));
-        blk(h_.cum, N * sizeof(double4));
-        blk(h_.clump_id, N * sizeof(int));
-        blk(h_.part_fix, N * sizeof(int));
+        std::vector<int2> cm(N);
+        std::vector<double4> slot[3], file[3];   // lom, cum, kin by member slot and by subsphere
+        std::vector<int> cid(N), fix(N);
+        double4* slot_dev[3] = {h_.lom, h_.cum, h_.kin};
+        for (int a = 0; a < 3; a++) { slot[a].resize(N); file[a].resize(N); }
+        if (!src) {
+            copy_(cm.data(), h_.cm, N * sizeof(int2), cudaMemcpyDeviceToHost);
+            copy_(fix.data(), h_.part_fix, N * sizeof(int), cudaMemcpyDeviceToHost);
+            for (int a = 0; a < 3; a++) copy_(slot[a].data(), slot_dev[a], N * sizeof(double4), cudaMemcpyDeviceToHost);
+            for (int s = 0; s < S_; s++)
+                for (int i = hpar_[s].sub_off; i < hpar_[s].sub_off + hpar_[s].nsub; i++) {
+                    cid[i] = hpar_[s].clump_off + cold_[cm[i].x];
+                    for (int a = 0; a < 3; a++) file[a][i] = slot[a][cm[i].y];
+                }
+        }
+        hblk(file[0].data(), N * sizeof(double4));
+        hblk(file[1].data(), N * sizeof(double4));
+        hblk(cid.data(), N * sizeof(int));
+        hblk(fix.data(), N * sizeof(int));
         blk(h_.level, N * sizeof(int));
         blk(h_.key, N * sizeof(int));
-        blk(h_.kin, N * sizeof(double4));
+        hblk(file[2].data(), N * sizeof(double4));
+        if (src) {
+            for (int s = 0; s < S_; s++)
+                for (int i = hpar_[s].sub_off; i < hpar_[s].sub_off + hpar_[s].nsub; i++) {
+                    if (fix[i] < 0 || fix[i] >= hpar_[s].nsub) throw ArgError("checkpoint of different scenes");
+                    const int m = mrow_[hpar_[s].sub_off + fix[i]];
+                    cm[i] = make_int2(mcl_[m], m);
+                    cid[i] = hpar_[s].clump_off + cold_[mcl_[m]];
+                    for (int a = 0; a < 3; a++) slot[a][m] = file[a][i];
+                }
+            copy_(h_.cm, cm.data(), N * sizeof(int2), cudaMemcpyHostToDevice);
+            copy_(h_.part_fix, fix.data(), N * sizeof(int), cudaMemcpyHostToDevice);
+            for (int a = 0; a < 3; a++) copy_(slot_dev[a], slot[a].data(), N * sizeof(double4), cudaMemcpyHostToDevice);
+        }
         blk(h_.bhist, (size_t)NB_SLOTS * 3 * N * sizeof(R4<R>));
         blk(h_.bbits, N * sizeof(uint16_t));
         blk(h_.fbnd, 2 * N * sizeof(R4<R>));
         if (h_.fint) blk(h_.fint, 2 * N * sizeof(R4<R>));
         blk(h_.bidx, N * sizeof(int));
         // clumps
-        blk(h_.cpos, K_ * sizeof(double4));
-        blk(h_.cvel, K_ * sizeof(double4));
-        blk(h_.cw, K_ * sizeof(double4));
-        blk(h_.cq, K_ * sizeof(double4));
-        blk(h_.cprop, K_ * sizeof(double4));
-        blk(h_.cinv, K_ * sizeof(double4));
-        blk(h_.mem_cl, N * sizeof(int));
-        blk(h_.cF, K_ * sizeof(double4));
-        blk(h_.cT, K_ * sizeof(double4));
-        blk(h_.mem_start, (K_ + 1) * sizeof(int));
-        blk(h_.mem_idx, N * sizeof(int));
+        for (double4* a : {h_.cpos, h_.cvel, h_.cw, h_.cq, h_.cprop, h_.cinv}) cblk(a);
+        // the member lists, by the caller's clump number (follow from the
+        // subspheres' clumps, so a load makes them from those)
+        std::vector<int> fcl(N), fst(K_ + 1, 0), fidx(N);
+        for (size_t i = 0; i < N; i++) fst[cid[i] + 1]++;
+        for (int k = 0; k < K_; k++) fst[k + 1] += fst[k];
+        {
+            std::vector<int> cur(fst.begin(), fst.end() - 1);
+            for (size_t i = 0; i < N; i++) fidx[cur[cid[i]]++] = (int)i;
+        }
+        for (int k = 0; k < K_; k++)
+            for (int m = fst[k]; m < fst[k + 1]; m++) fcl[m] = k;
+        hblk(fcl.data(), N * sizeof(int));
+        cblk(h_.cF);
+        cblk(h_.cT);
+        hblk(fst.data(), (K_ + 1) * sizeof(int));
+        hblk(fidx.data(), N * sizeof(int));
+        if (src) {
+            std::vector<int> cur(mstart_.begin(), mstart_.end() - 1);
+            std::vector<int2> mo(N);
+            for (size_t i = 0; i < N; i++) mo[cur[cm[i].x]++] = make_int2((int)i, cm[i].y);
+            copy_(h_.mo, mo.data(), N * sizeof(int2), cudaMemcpyHostToDevice);
+        }
         // rows and work-item prefixes
         blk(h_.L[0].row, (N + S_) * sizeof(int));
         blk(h_.L[0].brow, (N + S_) * sizeof(int));
@@ -729,12 +798,16 @@ class EngineT final : public EngineBase {
     bool has_kinds_ = false;    // some scene has split-driver body kinds (Dev::kind)
     bool first_list_ = true;
     int search_lanes_ = 8;
-    int clump_batch_ = 1;    // members per lane per load batch of the clump pass
+    int clump_batch_ = 1;    // as given; the clump pass has one member per lane whatever it says
     int pair_bps_ = 12;      // blocks per SM of the pair kernel's grid
     int sm_count_ = 148;
     int ring_len_ = 1;
     std::vector<ScenePar> hpar_;
     std::vector<int> start_step_;
+    // the engine's clump order (see clump_order): the caller's number within
+    // its scene of each clump, the first member slot and the clump of each
+    // member slot, and the member slot of each of the caller's subspheres
+    std::vector<int> cold_, mstart_, mcl_, mrow_;
     int* hflag_ = nullptr;  // pinned
     int steps_done_ = 0;
     int pend_ = 0, pend_eager_ = 0, pend_before_ = 0;  // steps enqueued and not yet waited for
@@ -824,6 +897,40 @@ class EngineT final : public EngineBase {
     struct RowData { std::vector<int> row, brow, nbr, bnbr, bpair; };
 
     // ---- setup --------------------------------------------------------------
+    // The order in which the engine keeps a scene's clumps: by the grid cell
+    // of the clump's first member (grid level, then z, y, x: the order of the
+    // subspheres), ties in the caller's order.  Clumps that lie side by side
+    // then share cache lines in the clump pass (its members' positions) and
+    // in the pair kernel (velocities, lever arms).  It is kept for the
+    // engine's life: a packed bed mixes slowly.  No result depends on it.
+    static std::vector<int> clump_order(const nbc_scene_desc& D, const ScenePar& P) {
+        std::vector<int> first(D.n_clump, -1);
+        for (int i = D.n_sub - 1; i >= 0; i--) first[D.clump_id[i]] = i;
+        std::vector<uint32_t> key(D.n_clump);
+        for (int k = 0; k < D.n_clump; k++) {
+            const int i = first[k];
+            if (i < 0) { key[k] = 0xffffffffu; continue; }   // a clump without members
+            const int lv = P.levels > 1 ? D.level[i] : 0;
+            const int* dim = P.levels > 1 ? P.ldim[lv] : P.gdim;
+            uint32_t c = 0;
+            for (int a = 2; a >= 0; a--) {
+                const double x = (D.pos[3 * i + a] - P.origin[a]) / (P.levels > 1 ? P.lcell[lv] : P.cell[a]);
+                c = c * (uint32_t)dim[a] + (uint32_t)std::min(std::max(x, 0.0), (double)(dim[a] - 1));
+            }
+            key[k] = (P.levels > 1 ? (uint32_t)P.loff[lv] : 0u) + c;
+        }
+        // stable radix sort, 11 bits a pass
+        std::vector<int> ord(D.n_clump), tmp(D.n_clump);
+        for (int k = 0; k < D.n_clump; k++) ord[k] = k;
+        for (int shift = 0; shift < 33; shift += 11) {
+            int at[2049] = {0};
+            for (int k = 0; k < D.n_clump; k++) at[((key[k] >> shift) & 2047) + 1]++;
+            for (int b = 0; b < 2048; b++) at[b + 1] += at[b];
+            for (int k : ord) tmp[at[(key[k] >> shift) & 2047]++] = k;
+            ord.swap(tmp);
+        }
+        return ord;
+    }
     void setup(const std::vector<const nbc_scene_desc*>& sc) {
         for (size_t s = 0; s < sc.size(); s++) validate_scene(*sc[s], (int)s);
         int ndev = 0;
@@ -838,13 +945,6 @@ class EngineT final : public EngineBase {
         DevMem::keep_pool(opt_.device);
         search_lanes_ = opt_.search_lanes == 16 || opt_.search_lanes == 32 ? opt_.search_lanes : 8;
         clump_batch_ = opt_.clump_batch == 2 || opt_.clump_batch == 4 ? opt_.clump_batch : 1;
-        // the clump pass's staged contact records (dynamic shared memory past the 48 KB default)
-        CK(cudaFuncSetAttribute(k_clump<R, 1, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)clump_dyn_smem<R, 1>()));
-        CK(cudaFuncSetAttribute(k_clump<R, 2, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)clump_dyn_smem<R, 2>()));
-        CK(cudaFuncSetAttribute(k_clump<R, 4, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)clump_dyn_smem<R, 4>()));
-        CK(cudaFuncSetAttribute(k_clump<R, 1, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)clump_dyn_smem<R, 1>()));
-        CK(cudaFuncSetAttribute(k_clump<R, 2, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)clump_dyn_smem<R, 2>()));
-        CK(cudaFuncSetAttribute(k_clump<R, 4, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)clump_dyn_smem<R, 4>()));
         pair_bps_ = opt_.pair_blocks >= 2 && opt_.pair_blocks <= 16 ? opt_.pair_blocks : 12;
         CK(cudaDeviceGetAttribute(&sm_count_, cudaDevAttrMultiProcessorCount, opt_.device));
         S_ = (int)sc.size();
@@ -975,49 +1075,83 @@ class EngineT final : public EngineBase {
         h_.S = S_; h_.N = N_; h_.K = K_;
         h_.cells = cells;
 
-        // host arrays in the input order
+        // host arrays: subspheres in the input order, clumps in the engine's
         std::vector<double4> posr(N_), lom(N_);
-        std::vector<int> cid(N_), fix(N_), lev(N_, 0), sid(N_), csid(K_), mstart(K_ + 1, 0), midx(N_);
+        std::vector<int> fix(N_), lev(N_, 0), sid(N_), csid(K_);
+        std::vector<int2> cm(N_), mo(N_);
         std::vector<double4> cpos(K_), cvel(K_), cw(K_), cq(K_), cprop(K_);
         std::vector<int> kind(has_kinds_ ? K_ : 0, 0);
+        cold_.resize(K_);
+        mstart_.assign(K_ + 1, 0);
+        mcl_.resize(N_);
+        mrow_.resize(N_);
         for (int s = 0; s < S_; s++) {
             const nbc_scene_desc& D = *sc[s];
             const ScenePar& P = hpar_[s];
-            for (int i = 0; i < D.n_sub; i++) {
-                int g = P.sub_off + i;
-                if (D.clump_id[i] < 0 || D.clump_id[i] >= D.n_clump)
-                    throw ArgError("scene " + std::to_string(s) + ": clump id out of range at row " + std::to_string(i));
-                posr[g] = make_double4(D.pos[3 * i], D.pos[3 * i + 1], D.pos[3 * i + 2], D.radius[i]);
-                lom[g] = make_double4(D.local[3 * i], D.local[3 * i + 1], D.local[3 * i + 2], D.mass[i]);
-                cid[g] = P.clump_off + D.clump_id[i];
-                fix[g] = i;
-                sid[g] = s;
-                if (P.levels > 1) {
-                    if (D.level[i] < 0 || D.level[i] >= P.levels)
-                        throw ArgError("scene " + std::to_string(s) + ": grid level out of range at row " + std::to_string(i));
-                    lev[g] = D.level[i];
-                }
-                mstart[cid[g] + 1]++;
-            }
-            for (int k = 0; k < D.n_clump; k++) {
-                int g = P.clump_off + k;
+            const std::vector<int> old = clump_order(D, P);
+            std::vector<int> now(D.n_clump);
+            for (int c = 0; c < D.n_clump; c++) {
+                const int g = P.clump_off + c, k = old[c];
+                now[k] = g;
+                cold_[g] = k;
                 csid[g] = s;
-                cpos[g] = make_double4(D.clump_pos[3 * k], D.clump_pos[3 * k + 1], D.clump_pos[3 * k + 2], 0);
-                cvel[g] = make_double4(D.clump_vel[3 * k], D.clump_vel[3 * k + 1], D.clump_vel[3 * k + 2], 0);
-                cw[g] = make_double4(D.clump_angvel[3 * k], D.clump_angvel[3 * k + 1], D.clump_angvel[3 * k + 2], 0);
-                cq[g] = make_double4(D.clump_quat[4 * k], D.clump_quat[4 * k + 1], D.clump_quat[4 * k + 2], D.clump_quat[4 * k + 3]);
-                cprop[g] = make_double4(D.clump_prop[4 * k], D.clump_prop[4 * k + 1], D.clump_prop[4 * k + 2], D.clump_prop[4 * k + 3]);
                 // bits 0-1: Type; bits 2-3: the kind the split driver's first
                 // half-kick sees, the body's original index (0, 1, 2, or 3 for
                 // any larger index; see k_clump)
                 if (has_kinds_ && D.body_kind) kind[g] = D.body_kind[k] | (std::min(k, 3) << 2);
             }
+            // clump records and body offsets go up in the caller's order and are
+            // put in place on the device
+            for (int k = 0; k < D.n_clump; k++) {
+                const int g = P.clump_off + k;
+                cpos[g] = make_double4(D.clump_pos[3 * k], D.clump_pos[3 * k + 1], D.clump_pos[3 * k + 2], 0);
+                cvel[g] = make_double4(D.clump_vel[3 * k], D.clump_vel[3 * k + 1], D.clump_vel[3 * k + 2], 0);
+                cw[g] = make_double4(D.clump_angvel[3 * k], D.clump_angvel[3 * k + 1], D.clump_angvel[3 * k + 2], 0);
+                cq[g] = make_double4(D.clump_quat[4 * k], D.clump_quat[4 * k + 1], D.clump_quat[4 * k + 2], D.clump_quat[4 * k + 3]);
+                cprop[g] = make_double4(D.clump_prop[4 * k], D.clump_prop[4 * k + 1], D.clump_prop[4 * k + 2], D.clump_prop[4 * k + 3]);
+            }
+            for (int i = 0; i < D.n_sub; i++) {
+                int g = P.sub_off + i;
+                lom[g] = make_double4(D.local[3 * i], D.local[3 * i + 1], D.local[3 * i + 2], D.mass[i]);
+                posr[g] = make_double4(D.pos[3 * i], D.pos[3 * i + 1], D.pos[3 * i + 2], D.radius[i]);
+                cm[g].x = now[D.clump_id[i]];
+                fix[g] = i;
+                sid[g] = s;
+                if (P.levels > 1) lev[g] = D.level[i];
+                mstart_[cm[g].x + 1]++;
+            }
         }
-        for (int k = 0; k < K_; k++) mstart[k + 1] += mstart[k];
+        for (int k = 0; k < K_; k++) mstart_[k + 1] += mstart_[k];
         {
-            std::vector<int> cur(mstart.begin(), mstart.end() - 1);
-            for (int i = 0; i < N_; i++) midx[cur[cid[i]]++] = i;
+            std::vector<int> cur(mstart_.begin(), mstart_.end() - 1);
+            for (int s = 0; s < S_; s++) {
+                const nbc_scene_desc& D = *sc[s];
+                for (int i = 0; i < D.n_sub; i++) {
+                    const int g = hpar_[s].sub_off + i, k = cm[g].x, m = cur[k]++;
+                    cm[g].y = m;
+                    mo[m] = make_int2(g, m);
+                    mcl_[m] = k;
+                    mrow_[g] = m;
+                }
+            }
         }
+
+        // the clump pass's lanes: whole clumps packed into warps, a lane per
+        // member (a clump of more than 32 has a warp of its own, one without
+        // members a lane)
+        std::vector<int4> ltab;
+        ltab.reserve((size_t)N_ + N_ / 4 + 32);
+        for (int s = 0; s < S_; s++)
+            for (int k = hpar_[s].clump_off; k < hpar_[s].clump_off + hpar_[s].nclump; k++) {
+                const int nm = mstart_[k + 1] - mstart_[k], lanes = std::min(std::max(nm, 1), 32);
+                while (ltab.size() % 32 + lanes > 32) ltab.push_back(make_int4(-1, -1, 0, 0));
+                const int head = (int)(ltab.size() % 32);
+                for (int q = 0; q < lanes; q++)
+                    ltab.push_back(make_int4(nm ? mstart_[k] + q : -1, k, nm << 5 | head, s));
+                while (nm > 32 && ltab.size() % 32) ltab.push_back(make_int4(-1, -1, 0, 0));
+            }
+        while (ltab.size() % 32) ltab.push_back(make_int4(-1, -1, 0, 0));
+        h_.W = (int)(ltab.size() / 32);
 
         // device allocation: the per-subsphere and per-clump buffers in one
         // slab, the pair buffers (which grow) in another
@@ -1028,16 +1162,11 @@ class EngineT final : public EngineBase {
             h_.sid = m.take<int>(N);
             h_.csid = m.take<int>(K_);
             h_.posr = m.take<double4>(N); h_.posr2 = m.take<double4>(N);
-            h_.lom = m.take<double4>(N); h_.lom2 = m.take<double4>(N);
-            h_.cum = m.take<double4>(N); h_.cum2 = m.take<double4>(N);
-            h_.clump_id = m.take<int>(N); h_.clump_id2 = m.take<int>(N);
+            h_.cm = m.take<int2>(N); h_.cm2 = m.take<int2>(N);
             h_.part_fix = m.take<int>(N); h_.part_fix2 = m.take<int>(N);
             h_.level = m.take<int>(N); h_.level2 = m.take<int>(N);
             h_.key = m.take<int>(N); h_.key2 = m.take<int>(N);
-            // contact kinematics: world lever arm and mass, one FP64 double4 per
-            // subsphere (the velocities are read from the clump's records)
-            h_.kin = m.take<char>(N * sizeof(double4));
-            h_.kin2 = m.take<char>(N * sizeof(double4));
+            h_.lom = m.take<double4>(N); h_.cum = m.take<double4>(N); h_.kin = m.take<double4>(N);
             h_.bhist = m.take<R4<R>>((size_t)NB_SLOTS * 3 * N); h_.bhist2 = m.take<R4<R>>((size_t)NB_SLOTS * 3 * N);
             h_.bbits = m.take<uint16_t>(N); h_.bbits2 = m.take<uint16_t>(N);
             h_.fsum = m.take<R4<R>>(2 * N);
@@ -1047,10 +1176,11 @@ class EngineT final : public EngineBase {
             h_.cpos = m.take<double4>(K_); h_.cvel = m.take<double4>(K_); h_.cw = m.take<double4>(K_);
             h_.cq = m.take<double4>(K_); h_.cprop = m.take<double4>(K_);
             h_.cinv = m.take<double4>(K_);
-            h_.mem_cl = m.take<int>(N);
+            h_.ltab = m.take<int4>(ltab.size());
+            h_.cold = m.take<int>(K_); h_.stage = m.take<double4>(K_);
             h_.cF = m.take<double4>(K_); h_.cT = m.take<double4>(K_);
             h_.mem_start = m.take<int>(K_ + 1);
-            h_.mem_idx = m.take<int>(N);
+            h_.mo = m.take<int2>(N);
             int* flags = m.take<int>(16);
             h_.post_pending = flags + 0;
             h_.any_rebuild = flags + 1;
@@ -1111,29 +1241,39 @@ class EngineT final : public EngineBase {
         copy_(h_.sid, sid.data(), N * sizeof(int), cudaMemcpyHostToDevice);
         copy_(h_.csid, csid.data(), K_ * sizeof(int), cudaMemcpyHostToDevice);
         copy_(h_.posr, posr.data(), N * sizeof(double4), cudaMemcpyHostToDevice);
-        copy_(h_.lom, lom.data(), N * sizeof(double4), cudaMemcpyHostToDevice);
-        copy_(h_.clump_id, cid.data(), N * sizeof(int), cudaMemcpyHostToDevice);
+        copy_(h_.cm, cm.data(), N * sizeof(int2), cudaMemcpyHostToDevice);
         copy_(h_.part_fix, fix.data(), N * sizeof(int), cudaMemcpyHostToDevice);
         copy_(h_.level, lev.data(), N * sizeof(int), cudaMemcpyHostToDevice);
-        copy_(h_.cpos, cpos.data(), K_ * sizeof(double4), cudaMemcpyHostToDevice);
-        copy_(h_.cvel, cvel.data(), K_ * sizeof(double4), cudaMemcpyHostToDevice);
-        copy_(h_.cw, cw.data(), K_ * sizeof(double4), cudaMemcpyHostToDevice);
-        copy_(h_.cq, cq.data(), K_ * sizeof(double4), cudaMemcpyHostToDevice);
-        copy_(h_.cprop, cprop.data(), K_ * sizeof(double4), cudaMemcpyHostToDevice);
+        copy_(h_.posr2, lom.data(), N * sizeof(double4), cudaMemcpyHostToDevice);
+        k_members_in<<<std::min(cdiv(N_, 256), sm_count_ * 8), 256, 0, stream_>>>(h_.posr2, h_.cm, N_, h_.lom);
+        {
+            std::vector<int> abs(K_);
+            for (int s = 0; s < S_; s++)
+                for (int c = hpar_[s].clump_off; c < hpar_[s].clump_off + hpar_[s].nclump; c++)
+                    abs[c] = hpar_[s].clump_off + cold_[c];
+            copy_(h_.cold, abs.data(), K_ * sizeof(int), cudaMemcpyHostToDevice);
+        }
+        auto clumps_in = [&](const std::vector<double4>& src, double4* dst) {
+            copy_(h_.stage, src.data(), K_ * sizeof(double4), cudaMemcpyHostToDevice);
+            k_clumps_in<<<std::min(cdiv(K_, 256), sm_count_ * 8), 256, 0, stream_>>>(h_.stage, h_.cold, K_, dst);
+            CK(cudaGetLastError());
+        };
+        clumps_in(cpos, h_.cpos);
+        clumps_in(cvel, h_.cvel);
+        clumps_in(cw, h_.cw);
+        clumps_in(cq, h_.cq);
+        clumps_in(cprop, h_.cprop);
         if (h_.kind) copy_(h_.kind, kind.data(), K_ * sizeof(int), cudaMemcpyHostToDevice);
         {
             // the clump pass's reciprocals: IEEE divisions, bitwise those it formed each step
             std::vector<double4> cinv(K_);
             for (int k = 0; k < K_; k++)
                 cinv[k] = make_double4(1.0 / cprop[k].x, 1.0 / cprop[k].y, 1.0 / cprop[k].z, 1.0 / cprop[k].w);
-            copy_(h_.cinv, cinv.data(), K_ * sizeof(double4), cudaMemcpyHostToDevice);
-            std::vector<int> mcl(N);
-            for (int k = 0; k < K_; k++)
-                for (int m = mstart[k]; m < mstart[k + 1]; m++) mcl[m] = k;
-            copy_(h_.mem_cl, mcl.data(), N * sizeof(int), cudaMemcpyHostToDevice);
+            clumps_in(cinv, h_.cinv);
+            copy_(h_.ltab, ltab.data(), ltab.size() * sizeof(int4), cudaMemcpyHostToDevice);
         }
-        copy_(h_.mem_start, mstart.data(), (K_ + 1) * sizeof(int), cudaMemcpyHostToDevice);
-        copy_(h_.mem_idx, midx.data(), N * sizeof(int), cudaMemcpyHostToDevice);
+        copy_(h_.mem_start, mstart_.data(), (K_ + 1) * sizeof(int), cudaMemcpyHostToDevice);
+        copy_(h_.mo, mo.data(), N * sizeof(int2), cudaMemcpyHostToDevice);
         // the first list is empty: rows of zeros (the slab is zeroed)
         int one = 1;
         copy_(h_.any_rebuild, &one, sizeof(int), cudaMemcpyHostToDevice);
@@ -1330,20 +1470,9 @@ class EngineT final : public EngineBase {
     // ---- launches -------------------------------------------------------------
     void launch_clump(int do_pre, cudaGraphConditionalHandle cond = 0, int use_cond = 0,
                       cudaGraphConditionalHandle loop = 0, int use_loop = 0) {
-        const int g = cdiv(K_ + S_, CL_THREADS);
-        if (sphere_any_) {
-            if (clump_batch_ == 1)
-                k_clump<R, 1, true><<<g, CL_THREADS, clump_dyn_smem<R, 1>(), stream_>>>(d_, do_pre, cond, use_cond, loop, use_loop);
-            else if (clump_batch_ == 4)
-                k_clump<R, 4, true><<<g, CL_THREADS, clump_dyn_smem<R, 4>(), stream_>>>(d_, do_pre, cond, use_cond, loop, use_loop);
-            else
-                k_clump<R, 2, true><<<g, CL_THREADS, clump_dyn_smem<R, 2>(), stream_>>>(d_, do_pre, cond, use_cond, loop, use_loop);
-        } else if (clump_batch_ == 1)
-            k_clump<R, 1, false><<<g, CL_THREADS, clump_dyn_smem<R, 1>(), stream_>>>(d_, do_pre, cond, use_cond, loop, use_loop);
-        else if (clump_batch_ == 4)
-            k_clump<R, 4, false><<<g, CL_THREADS, clump_dyn_smem<R, 4>(), stream_>>>(d_, do_pre, cond, use_cond, loop, use_loop);
-        else
-            k_clump<R, 2, false><<<g, CL_THREADS, clump_dyn_smem<R, 2>(), stream_>>>(d_, do_pre, cond, use_cond, loop, use_loop);
+        const int g = cdiv(h_.W + cdiv(S_, 32), CL_WARPS);
+        if (sphere_any_) k_clump<R, true><<<g, CL_THREADS, 0, stream_>>>(d_, do_pre, cond, use_cond, loop, use_loop);
+        else k_clump<R, false><<<g, CL_THREADS, 0, stream_>>>(d_, do_pre, cond, use_cond, loop, use_loop);
         CK(cudaGetLastError());
         if (!capturing_) launches_ += 1;
     }

@@ -28,53 +28,9 @@ constexpr double FIX_T = 17592186044416.0;   // 2^44: fixed-point scale of intru
 constexpr int IDX_MASK = 0x7fffffff;
 constexpr int INTRA = (int)0x80000000u;
 
-// The contact slots of one subsphere (its near front entries, then its near
-// back entries, in row order; SumContForce_clump, src/dem_force_clump.cu:
-// 165-191, sums a subsphere's front entries, then its back entries).
-template <typename R>
-__device__ __forceinline__ void slot_sum(const R4<R>* __restrict__ fs, const R4<R>* __restrict__ bs, size_t cap,
-                                         int rs, int re, int bs0, int be, V3<R>& F, V3<R>& T) {
-    F = v3<R>(0, 0, 0);
-    T = F;
-    // not unrolled: a subsphere has a few near entries at most, and unrolled
-    // copies cost the clump pass registers (and warps per SM)
-#pragma unroll 1
-    for (int e = rs; e < re; e++) {
-        F = F + xyz<R>(fs[2 * (size_t)e]);
-        T = T + xyz<R>(fs[2 * (size_t)e + 1]);
-    }
-#pragma unroll 1
-    for (int e = bs0; e < be; e++) {
-        F = F + xyz<R>(bs[2 * (size_t)e]);
-        T = T + xyz<R>(bs[2 * (size_t)e + 1]);
-    }
-}
-
 // ===========================================================================
 // clump pass
 // ===========================================================================
-
-// 16-byte asynchronous copy global -> shared (no register holds the data in
-// flight, so one thread can have many outstanding), and the wait for all of
-// the calling thread's copies.
-__device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
-    const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(s), "l"(gmem) : "memory");
-}
-__device__ __forceinline__ void cp_async_wait_all() {
-    asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;\n" ::: "memory");
-}
-// a contact record staged for the clump pass: force and torque (two Real4)
-template <typename R> struct SlotRec {
-    R4<R> f, t;
-};
-template <typename R>
-__device__ __forceinline__ void stage_rec(SlotRec<R>* dst, const R4<R>* f, const R4<R>* t) {
-    for (int k = 0; k < (int)sizeof(R4<R>) / 16; k++) {
-        cp_async16((char*)&dst->f + 16 * k, (const char*)f + 16 * k);
-        cp_async16((char*)&dst->t + 16 * k, (const char*)t + 16 * k);
-    }
-}
 
 // Integrate_Before_clump_cuk / Attitude_clump_cuk / Integrate_After_clump_cuk
 // (src/dem_integrate_clumpsphere.cu:3-141), UpdatePos_cuk (src/dem_clump.cu:
@@ -82,15 +38,24 @@ __device__ __forceinline__ void stage_rec(SlotRec<R>* dst, const R4<R>* f, const
 // (src/dem_clumpsphere.cu:86-151), IntegratePene_Before_cuk and
 // Integrate_After_cuk (src/dem_integrate_penetrator.cu:3-113).
 //
-// One clump per lane, 32 clumps per warp.  The member work is spread over
-// the warp instead: the members of the warp's clumps are one contiguous range
-// of the member list, the lanes load all member indices of a chunk and then
-// all member records (every load of the chunk in flight at once), each
-// member's force and lever-arm torque go to shared memory, and each lane then
-// sums its own clump's members in ascending order (the reduce_by_key order)
-// and integrates its clump once.  The new poses are shared the same way and
-// the lanes pose the members 32 at a time.  The lanes after the last clump
-// hold one thread per scene for the intruder.
+// One member per lane.  The host packs whole clumps into warps (Dev::ltab, a
+// record per lane; members of a clump are consecutive lanes, a clump of more
+// than 32 members has a warp of its own that walks them 32 at a time, a clump
+// without members one lane).  A lane sums its member's contact slots, forms
+// the lever-arm torque, and the lanes of a clump add up their members in
+// ascending order through shuffles (the reduce_by_key order); every lane then
+// integrates its clump (a warp instruction costs the same for one lane as for
+// 32), poses its own member from registers, and the clump's first lane writes
+// the clump.  The warps after the last one of the table hold one thread per
+// scene for the intruder.
+//
+// Bound by latency: a chain of four dependent loads (lane record, member
+// index, row offsets and member records, slots), the FP64 integration, the
+// stores.  One lane per clump, with the members of a warp's 32 clumps walked
+// through shared memory in four or more chunks, put that chain in series four
+// times and left 391 blocks of work for 50,000 clumps (events around the pass,
+// one lane per clump -> one per member: 500 clumps 20.6 -> 12.4 us, 13,331 in
+// FP64 27.2 -> 15.8, 50,000 32.8 -> 34.2, 250,000 141 -> 151).
 //
 // A step (do_pre) also advances the spring-history generation so the next
 // contact pass reads what the previous one wrote, and counts itself; the last
@@ -107,65 +72,287 @@ __device__ __forceinline__ bool scene_post(const SceneDyn& y, int post, int L) {
 }
 constexpr int CL_THREADS = 128;
 constexpr int CL_WARPS = CL_THREADS / 32;
-// staged contact records per warp: cl_stage<J>() per member of a chunk on
-// average; a lane whose members would overflow the warp's records sums from
-// global memory directly (same order, same result).  Dynamic shared memory.
-// Four records per member at J <= 2 (a shallower stage at J = 2 sends more
-// lanes to the unstaged sums: 46.6 against 35.9 µs per cfg1 step); two at
-// J = 4, whose 168 registers allow 3 blocks per SM that four records' 104 KB
-// per block would cut to 2.
-template <int J>
-__host__ __device__ constexpr int cl_stage() {
-    return J == 4 ? 2 : 4;
-}
-template <typename R, int J>
-constexpr size_t clump_dyn_smem() {
-    return (size_t)CL_WARPS * cl_stage<J>() * 32 * J * sizeof(SlotRec<R>);
-}
-// J: members each lane keeps in flight per batch of loads (a launch shape
-// the autotuner picks; results do not depend on it); a warp stages 32 J
-// members in shared memory at a time.  J <= 2 fits 128 registers (4 blocks,
-// 16 warps per SM, of which J = 2's 60 KB of shared memory leaves 3) with a
-// few bytes of spill; J = 4 keeps 3 blocks per SM.  J = 1 is the default
-// (the fastest on the cfg1 and cfg3 states).
-// One attitude step (Attitude_clump_cuk, src/dem_integrate_clumpsphere.cu:
-// 45-90, the expressions of k_clump's own update): the split driver's bodies
-// that turn without their first half-kick use it.
+#ifndef NBC_CLUMP_MINB
+#define NBC_CLUMP_MINB 4
+#endif
+// One attitude step (Attitude_clump_cuk, src/dem_integrate_clumpsphere.cu:45-90).
 __device__ __forceinline__ double4 quat_step(double4 q, V3<double> w, V3<double> al, double Dt) {
     const V3<double> Wb = rot_w2b(q, w), Wdb = rot_w2b(q, al);
-    double4 qd, qdd;
-    qd.x = 0.50 * (Wb.x * q.w - Wb.y * q.z + Wb.z * q.y);
-    qd.y = 0.50 * (Wb.x * q.z + Wb.y * q.w - Wb.z * q.x);
-    qd.z = 0.50 * (-Wb.x * q.y + Wb.y * q.x + Wb.z * q.w);
-    qd.w = 0.50 * (-Wb.x * q.x - Wb.y * q.y - Wb.z * q.z);
-    qdd.x = (Wdb.x * q.w - Wdb.y * q.z + Wdb.z * q.y) * 0.50 + (Wb.x * qd.w - Wb.y * qd.z + Wb.z * qd.y) * 0.50;
-    qdd.y = (Wdb.x * q.z + Wdb.y * q.w - Wdb.z * q.x) * 0.50 + (Wb.x * qd.z + Wb.y * qd.w - Wb.z * qd.x) * 0.50;
-    qdd.z = (-Wdb.x * q.y + Wdb.y * q.x + Wdb.z * q.w) * 0.50 + (-Wb.x * qd.y + Wb.y * qd.x + Wb.z * qd.w) * 0.50;
-    qdd.w = (-Wdb.x * q.x - Wdb.y * q.y - Wdb.z * q.z) * 0.50 + (-Wb.x * qd.x - Wb.y * qd.y - Wb.z * qd.z) * 0.50;
+    double4 qd, qdd, r;
+    qd.x = 0.50 * fma3(Wb.x, q.w, -Wb.y, q.z, Wb.z, q.y);
+    qd.y = 0.50 * fma3(Wb.x, q.z, Wb.y, q.w, -Wb.z, q.x);
+    qd.z = 0.50 * fma3(Wb.y, q.x, -Wb.x, q.y, Wb.z, q.w);
+    qd.w = 0.50 * fma3(-Wb.x, q.x, -Wb.y, q.y, -Wb.z, q.z);
+    qdd.x = fma2(0.50, fma3(Wdb.x, q.w, -Wdb.y, q.z, Wdb.z, q.y), 0.50, fma3(Wb.x, qd.w, -Wb.y, qd.z, Wb.z, qd.y));
+    qdd.y = fma2(0.50, fma3(Wdb.x, q.z, Wdb.y, q.w, -Wdb.z, q.x), 0.50, fma3(Wb.x, qd.z, Wb.y, qd.w, -Wb.z, qd.x));
+    qdd.z = fma2(0.50, fma3(Wdb.y, q.x, -Wdb.x, q.y, Wdb.z, q.w), 0.50, fma3(Wb.y, qd.x, -Wb.x, qd.y, Wb.z, qd.w));
+    qdd.w = fma2(0.50, fma3(-Wdb.x, q.x, -Wdb.y, q.y, -Wdb.z, q.z), 0.50, fma3(-Wb.x, qd.x, -Wb.y, qd.y, -Wb.z, qd.z));
     const double h2 = 0.5 * Dt * Dt;
-    double4 r;
-    r.x = (q.x + Dt * qd.x) + h2 * qdd.x;
-    r.y = (q.y + Dt * qd.y) + h2 * qdd.y;
-    r.z = (q.z + Dt * qd.z) + h2 * qdd.z;
-    r.w = (q.w + Dt * qd.w) + h2 * qdd.w;
-    const double inv = 1.0 / sqrt(r.x * r.x + r.y * r.y + r.z * r.z + r.w * r.w);
+    r.x = __fma_rn(h2, qdd.x, __fma_rn(Dt, qd.x, q.x));
+    r.y = __fma_rn(h2, qdd.y, __fma_rn(Dt, qd.y, q.y));
+    r.z = __fma_rn(h2, qdd.z, __fma_rn(Dt, qd.z, q.z));
+    r.w = __fma_rn(h2, qdd.w, __fma_rn(Dt, qd.w, q.w));
+    const double inv = 1.0 / sqrt(__fma_rn(r.w, r.w, fma3(r.x, r.x, r.y, r.y, r.z, r.z)));
     r.x *= inv; r.y *= inv; r.z *= inv; r.w *= inv;
     return r;
 }
 
-// SPH: the build for batches with a sphere-driver scene (ScenePar::sphere);
-// the clump path's build carries none of that code.
-template <typename R, int J, bool SPH>
-__global__ void __launch_bounds__(CL_THREADS, J <= 2 ? 4 : 3) k_clump(const Dev* __restrict__ dp, int do_pre,
-                                                      cudaGraphConditionalHandle cond, int use_cond,
-                                                      cudaGraphConditionalHandle loop, int use_loop) {
-    constexpr int CL_CHUNK = 32 * J;
-    __shared__ double s_mf[CL_WARPS][6][CL_CHUNK];   // member force xyz, torque xyz
-    __shared__ double s_cl[CL_WARPS][13][32];        // clump position, velocity, angular velocity, quaternion
-    __shared__ int s_ms[CL_WARPS][33];               // member-list offsets of the warp's clumps
-    __shared__ int s_sc[CL_WARPS][32];               // scene of each of the warp's clumps
-    __shared__ int s_pre[CL_WARPS][32];              // the clump's scene takes this step
-    extern __shared__ __align__(16) unsigned char cl_dsm[];   // staged contact records
+// The contact slots of one subsphere: its near front entries [r0, r1), then
+// its near back entries [q0, q1), in row order (SumContForce_clump,
+// src/dem_force_clump.cu:165-191, sums a subsphere's front entries, then its
+// back entries); the loads of a few slots are in flight together.
+template <typename R>
+__device__ __forceinline__ void slot_sum(const R4<R>* __restrict__ fs, const R4<R>* __restrict__ bs, int r0, int r1,
+                                         int q0, int q1, V3<R>& F, V3<R>& T) {
+    constexpr int U = sizeof(R) == 4 ? 4 : 2;
+    F = v3<R>(0, 0, 0);
+    T = F;
+    const int nf = r1 - r0, n = nf + (q1 - q0);
+#pragma unroll 1
+    for (int e0 = 0; e0 < n; e0 += U) {
+        R4<R> f[U], t[U];
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            const int e = e0 + u;
+            if (e < n) {
+                const R4<R>* p = e < nf ? fs + 2 * (size_t)(r0 + e) : bs + 2 * (size_t)(q0 + (e - nf));
+                ld_pair(p, f[u], t[u]);
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < U; u++)
+            if (e0 + u < n) {
+                F = F + xyz<R>(f[u]);
+                T = T + xyz<R>(t[u]);
+            }
+    }
+}
+
+// F / M + gravity and the half-kick v + h a
+__device__ __forceinline__ V3<double> linear_acc(V3<double> F, double invM, double grav) {
+    return v3(__dmul_rn(invM, F.x), __dmul_rn(invM, F.y), __fma_rn(invM, F.z, grav));
+}
+__device__ __forceinline__ V3<double> kick(V3<double> v, double h, V3<double> a) {
+    return v3(__fma_rn(h, a.x, v.x), __fma_rn(h, a.y, v.y), __fma_rn(h, a.z, v.z));
+}
+__device__ __forceinline__ V3<double> shfl3(V3<double> v, int src) {
+    return v3(__shfl_sync(0xffffffffu, v.x, src), __shfl_sync(0xffffffffu, v.y, src), __shfl_sync(0xffffffffu, v.z, src));
+}
+
+// The work of warp w of the lane table (see above); every lane of the warp
+// calls it.  SPH: the build for batches with a sphere-driver scene
+// (ScenePar::sphere); the clump path's build carries none of that code.
+template <typename R, bool SPH>
+__device__ __forceinline__ void clump_warp(const Dev& d, int w, int do_pre, int post, int L) {
+    const int lane = threadIdx.x & 31;
+    const int4 tb = d.ltab[w * 32 + lane];   // entry of mo, clump, members << 5 | first lane, scene
+    const bool isc = tb.y >= 0;
+    const int k = isc ? tb.y : 0, sc = isc ? tb.w : 0;
+    const int head = tb.z & 31, nm = tb.z >> 5;
+    const bool stops = d.has_stops;
+    const bool pre_k = isc && (stops ? scene_pre(d.dyn[sc], do_pre, L) : do_pre != 0);
+    const bool post_k = isc && (stops ? scene_post(d.dyn[sc], post, L) : post != 0);
+    // a warp whose clumps all belong to scenes standing still has no work
+    if (stops && !__any_sync(0xffffffffu, pre_k || post_k)) return;
+    const int2* __restrict__ mo = d.mo;
+    int e = tb.x;
+    int2 im = e >= 0 ? mo[e] : make_int2(-1, 0);   // subsphere, member slot
+    double4 cp = ld32(d.cpos + k), cv = ld32(d.cvel + k), cw = ld32(d.cw + k), cq = ld32(d.cq + k);
+    const double4 pr = ld32(d.cinv + k);            // the reciprocals 1/I, 1/M
+    const ScenePar& P = d.par[sc];
+    const double Dt = P.dt, grav = P.gravity;
+    const int most = __reduce_max_sync(0xffffffffu, nm);   // members of the warp's largest clump
+    double4 ps = make_double4(0, 0, 0, 0);
+    V3<double> F = v3(0.0, 0.0, 0.0), T = F;
+    if (post) {
+        const int2* __restrict__ nrb = d.nrb;
+        for (int c0 = 0;; c0 += 32) {
+            V3<double> f = v3(0.0, 0.0, 0.0), t = f;
+            const int i = im.x;
+            if (i >= 0) {
+                const int2 ra = nrb[i + sc], rb = nrb[i + sc + 1];
+                const uint16_t bb = d.bbits[i];
+                ps = ld32(d.posr + i);
+                V3<R> fr, tr;
+                slot_sum<R>((const R4<R>*)d.nfs, (const R4<R>*)d.nbs, ra.x, rb.x, ra.y, rb.y, fr, tr);
+                if (bb) {
+                    const R4<R>* __restrict__ fbd = (const R4<R>*)d.fbnd;
+                    fr = fr + xyz<R>(fbd[i]);
+                    tr = tr + xyz<R>(fbd[(size_t)d.N + i]);
+                }
+                const V3<double> r = v3(ps.x - cp.x, ps.y - cp.y, ps.z - cp.z);
+                f = v3((double)fr.x, (double)fr.y, (double)fr.z);
+                t.x = __dadd_rn((double)tr.x, fma2(r.y, f.z, -r.z, f.y));
+                t.y = __dadd_rn((double)tr.y, fma2(r.z, f.x, -r.x, f.z));
+                t.z = __dadd_rn((double)tr.z, fma2(r.x, f.y, -r.y, f.x));
+            }
+            const int mq = min(most - c0, 32);
+            for (int q = 0; q < mq; q++) {
+                const V3<double> fq = shfl3(f, head + q), tq = shfl3(t, head + q);
+                if (c0 + q < nm) {
+                    if (c0 + q == 0) { F = fq; T = tq; }
+                    else { F = F + fq; T = T + tq; }
+                }
+            }
+            if (c0 + 32 >= most) break;
+            e += 32;
+            im = c0 + 32 + lane < nm ? mo[e] : make_int2(-1, 0);
+        }
+        if (post_k) {
+            if (nm > 0) {
+                if (lane == head) {
+                    if (!(isfinite(F.x) && isfinite(F.y) && isfinite(F.z) && isfinite(T.x) && isfinite(T.y) &&
+                          isfinite(T.z)))
+                        atomicOr(&d.dyn[sc].err, ERR_NONFINITE);
+                    st32(d.cF + k, make_double4(F.x, F.y, F.z, 0.0));
+                    st32(d.cT + k, make_double4(T.x, T.y, T.z, 0.0));
+                }
+            } else {
+                F = xyzd(d.cF[k]);
+                T = xyzd(d.cT[k]);
+            }
+        }
+        // split driver: only Type 0 takes the closing half-kick
+        // (src/dem_integrate_withglue.cu:140)
+        if (post_k && !(SPH && (P.sphere & SPH_KINDS) && (d.kind[k] & 3) != 0)) {
+            const V3<double> v = kick(xyzd(cv), 0.5 * Dt, linear_acc(F, pr.w, grav));
+            const V3<double> o = kick(xyzd(cw), 0.5 * Dt, v3(__dmul_rn(pr.x, T.x), __dmul_rn(pr.y, T.y), __dmul_rn(pr.z, T.z)));
+            cv.x = v.x; cv.y = v.y; cv.z = v.z;
+            cw.x = o.x; cw.y = o.y; cw.z = o.z;
+        }
+    } else {
+        F = xyzd(d.cF[k]);
+        T = xyzd(d.cT[k]);
+        if (im.x >= 0) ps = ld32(d.posr + im.x);
+    }
+    if (post_k && !pre_k && lane == head) {   // closing half-kick only (sync, or the scene's last step)
+        st32(d.cvel + k, cv);
+        st32(d.cw + k, cw);
+    }
+    if (!pre_k) return;
+    if (SPH && (P.sphere & SPH_KIN) && nm > 0) {
+        // the sphere drivers' first half-kick and attitude leave the
+        // intruder out (src/dem_integrate.cu:20-21,72); one member
+        const int i = im.x;
+        if ((d.bbits[i] >> SLOT_INTR) & 1) {
+            const R4<R>* __restrict__ fi = (const R4<R>*)d.fint;
+            const R4<R> a = fi[i], b = fi[(size_t)d.N + i];
+            F = F - v3((double)a.x, (double)a.y, (double)a.z);
+            T = T - v3((double)b.x, (double)b.y, (double)b.z);
+        }
+    }
+    const double4 cp_old = cp;
+    const V3<double> ac = linear_acc(F, pr.w, grav);
+    const V3<double> al = v3(__dmul_rn(pr.x, T.x), __dmul_rn(pr.y, T.y), __dmul_rn(pr.z, T.z));
+    const double h2 = 0.5 * Dt * Dt;
+    // (the sphere drivers' scenes fuse the other product)
+    const bool sph = SPH && P.sphere;
+    cp.x = __dadd_rn(cp.x, sph ? fma2(Dt, cv.x, h2, ac.x) : fma2(h2, ac.x, Dt, cv.x));
+    cp.y = __dadd_rn(cp.y, sph ? fma2(Dt, cv.y, h2, ac.y) : fma2(h2, ac.y, Dt, cv.y));
+    cp.z = __dadd_rn(cp.z, fma2(Dt, cv.z, h2, ac.z));
+    V3<double> v = kick(xyzd(cv), 0.5 * Dt, ac), wv = kick(xyzd(cw), 0.5 * Dt, al);
+    // attitude with the half-kicked angular velocity
+    double4 q = quat_step(cq, wv, al, Dt);
+    if (SPH && (P.sphere & SPH_KINDS)) {
+        // split driver (src/dem_integrate_withglue.cu:3-110).  Its call
+        // passes the original index where the first half-kick expects
+        // Type (src/dem_simulation_split.cu:84-85 against
+        // src/dem_integrate_withglue.cu:113-114), so the kick and the
+        // move go by the body's original index (bits 2-3: 0 free, 1
+        // driven at (-0.2 y, -0.2 x, 0), 2 or more still) and the
+        // attitude by its Type (bits 0-1: turns only for Type 0)
+        const int kd = d.kind[k], ka = kd & 3, kb = (kd >> 2) & 3;
+        if (kb != 0) {
+            cp = cp_old;
+            wv = xyzd(cw);
+            v = xyzd(cv);
+            if (kb == 1) {
+                v = v3(-0.2 * cp_old.y, -0.2 * cp_old.x, 0.0);
+                cp.x += Dt * v.x; cp.y += Dt * v.y; cp.z += Dt * v.z;
+            }
+            if (ka == 0) q = quat_step(cq, wv, al, Dt);
+        }
+        if (ka != 0) q = cq;
+    }
+    if (lane == head) {
+        st32(d.cpos + k, cp);
+        st32(d.cvel + k, make_double4(v.x, v.y, v.z, 0.0));
+        st32(d.cw + k, make_double4(wv.x, wv.y, wv.z, 0.0));
+        st32(d.cq + k, q);
+    }
+    // ---- the member's pose
+    double thr = P.thresh;
+    for (int c0 = 0; c0 < nm; c0 += 32) {
+        if (nm > 32) {   // a warp of its own: the members once more
+            if (c0 + lane >= nm) break;
+            im = mo[d.mem_start[k] + c0 + lane];
+            ps = ld32(d.posr + im.x);
+        }
+        const double4 lo = ld32(d.lom + im.y), c = ld32(d.cum + im.y);
+        const V3<double> arm = rot_b2w(q, v3(lo.x, lo.y, lo.z));
+        const V3<double> p = v3(__dadd_rn(cp.x, arm.x), __dadd_rn(cp.y, arm.y), __dadd_rn(cp.z, arm.z));
+        const V3<double> cn = v3((c.x + p.x) - ps.x, (c.y + p.y) - ps.y, (c.z + p.z) - ps.z);
+        st32(d.cum + im.y, make_double4(cn.x, cn.y, cn.z, 0.0));
+        st32(d.posr + im.x, make_double4(p.x, p.y, p.z, ps.w));
+        st32(d.kin + im.y, make_double4(arm.x, arm.y, arm.z, lo.w));   // world arm, mass
+        if (SPH && (P.sphere & SPH_KINDS))   // split driver: the free body of the first half-kick at 0.1 r
+            thr = ((d.kind[k] >> 2) & 3) == 0 ? 0.10 * ps.w : INFINITY;   // (src/dem_integrate_withglue.cu:41)
+        if (len_floor(cn) > thr) {
+            SceneDyn& y = d.dyn[sc];
+            if (!*(volatile int*)&y.rebuild) atomicExch(&y.rebuild, 1);
+            if (!*(volatile int*)d.any_rebuild) atomicExch(d.any_rebuild, 1);
+        }
+    }
+}
+
+// the intruder and the step count of scene s (one thread)
+__device__ __forceinline__ void scene_step(const Dev& d, int s, int do_pre, int post, int L) {
+    const ScenePar& P = d.par[s];
+    SceneDyn& y = d.dyn[s];
+    const double Dt = P.dt;
+    const bool pre_s = scene_pre(y, do_pre, L), post_s = scene_post(y, post, L);
+    if (post_s) {
+        long long* fx = (long long*)&y.ifix[0];
+        V3<double> tf = v3(fx[0] / FIX_F, fx[1] / FIX_F, fx[2] / FIX_F);
+        V3<double> tt = v3(fx[3] / FIX_T, fx[4] / FIX_T, fx[5] / FIX_T);
+        for (int c = 0; c < 6; c++) fx[c] = 0;
+        y.totF[0] = tf.x; y.totF[1] = tf.y; y.totF[2] = tf.z;
+        y.totT[0] = tt.x; y.totT[1] = tt.y; y.totT[2] = tt.z;
+        if (P.has_intr) {
+            if (P.intr_wait && y.intr_state == 1) y.intr_state = 2;
+            V3<double> reac = v3(-tf.x, -tf.y, -tf.z);
+            if (P.intr_motion == 1 && (!P.intr_wait || y.intr_state != 0)) {
+                V3<double> a = (1.0 / P.intr_mass) * reac;
+                a.z = a.z + P.gravity;
+                for (int c = 0; c < 3; c++) y.intr_v[c] += (0.5 * Dt) * (&a.x)[c];
+            }
+            y.reaction[0] = reac.x; y.reaction[1] = reac.y; y.reaction[2] = reac.z;
+            y.reaction_t[0] = tt.x; y.reaction_t[1] = tt.y; y.reaction_t[2] = tt.z;
+            double* ring = d.ring + ((size_t)s * d.ring_len + (y.step % d.ring_len)) * 6;
+            ring[0] = reac.x; ring[1] = reac.y; ring[2] = reac.z;
+            ring[3] = tt.x; ring[4] = tt.y; ring[5] = tt.z;
+        }
+        y.step += 1;
+    }
+    if (do_pre) y.frozen = !pre_s;
+    if (pre_s && P.has_intr) {
+        if (P.intr_motion == 1 && (!P.intr_wait || y.intr_state != 0)) {
+            V3<double> a = (-1.0 / P.intr_mass) * v3(y.totF[0], y.totF[1], y.totF[2]);
+            a.z = a.z + P.gravity;
+            for (int c = 0; c < 3; c++) {
+                y.intr_p[c] = (y.intr_p[c] + Dt * y.intr_v[c]) + (0.5 * Dt * Dt) * (&a.x)[c];
+                y.intr_v[c] = y.intr_v[c] + (0.5 * Dt) * (&a.x)[c];
+            }
+        } else {
+            for (int c = 0; c < 3; c++) y.intr_p[c] = y.intr_p[c] + Dt * y.intr_v[c];
+        }
+    }
+}
+
+template <typename R, bool SPH>
+__global__ void __launch_bounds__(CL_THREADS, NBC_CLUMP_MINB) k_clump(const Dev* __restrict__ dp, int do_pre,
+                                                                      cudaGraphConditionalHandle cond, int use_cond,
+                                                                      cudaGraphConditionalHandle loop, int use_loop) {
     const Dev& d = *dp;
     if (*d.halt) {
         // a rebuild ran out of pair capacity: the host finishes that step, so
@@ -173,369 +360,18 @@ __global__ void __launch_bounds__(CL_THREADS, J <= 2 ? 4 : 3) k_clump(const Dev*
         if (use_loop && blockIdx.x == 0 && threadIdx.x == 0) cudaGraphSetConditional(loop, 0u);
         return;
     }
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int k0 = (blockIdx.x * CL_WARPS + warp) * 32;
-    const int t = k0 + lane;
     const int post = *d.post_pending;
     const int L = *d.lstep;   // written only by the last block, after every block has read it
     if (do_pre && blockIdx.x == 0 && threadIdx.x == 0) {
         *d.hgen += 1;
         *d.gstep += 1;
     }
-    // warp-uniform: this warp holds clumps of a scene that moves (a warp whose
-    // clumps all belong to scenes standing still skips its work)
-    const bool stops = d.has_stops;
-    bool warp_live = k0 < d.K && !stops;
-    if (k0 < d.K && stops) {
-        const int nq = min(32, d.K - k0);
-        const SceneDyn& yq = d.dyn[d.csid[lane < nq ? t : k0 + nq - 1]];
-        warp_live = __any_sync(0xffffffffu, lane < nq && (scene_pre(yq, do_pre, L) || scene_post(yq, post, L)));
-    }
-    if (warp_live) {
-        const int* __restrict__ mem_start = d.mem_start;
-        const int* __restrict__ mem_idx = d.mem_idx;
-        const double4* __restrict__ posr = d.posr;
-        const int nk = min(32, d.K - k0);
-        const bool isc = lane < nk;
-        const int k = isc ? t : k0 + nk - 1;
-        s_ms[warp][lane] = mem_start[k0 + min(lane, nk)];
-        if (lane == 0) s_ms[warp][32] = mem_start[k0 + nk];
-        const int sc = d.csid[k];
-        double4 cp = d.cpos[k], cv = d.cvel[k], cw = d.cw[k], cq = d.cq[k], pr = d.cinv[k];
-        const bool pre_k = stops ? scene_pre(d.dyn[sc], do_pre, L) : do_pre != 0;
-        const bool post_k = stops ? scene_post(d.dyn[sc], post, L) : post != 0;
-        s_sc[warp][lane] = sc;
-        s_pre[warp][lane] = isc && pre_k;
-        s_cl[warp][0][lane] = cp.x; s_cl[warp][1][lane] = cp.y; s_cl[warp][2][lane] = cp.z;
-        __syncwarp();
-        const int M0 = s_ms[warp][0], M1 = s_ms[warp][nk];
-        const int mb = s_ms[warp][isc ? lane : nk - 1], me = s_ms[warp][isc ? lane + 1 : nk];
-        // the warp-local clump of member slot m: mem_cl[m] - k0
-        const int* __restrict__ mem_cl = d.mem_cl;
-        const ScenePar& P = d.par[sc];
-        const double Dt = P.dt;
-        V3<double> F, T;
-        if (post) {
-            // ---- member sums, CL_CHUNK members of the warp's range at a time:
-            // each member's contact slots (the contact pass of the last step),
-            // its wall and intruder force, and its lever-arm torque
-            const R4<R>* __restrict__ fsl = (const R4<R>*)d.nfs;
-            const R4<R>* __restrict__ bsl = (const R4<R>*)d.nbs;
-            const R4<R>* __restrict__ fbd = (const R4<R>*)d.fbnd;
-            const int2* __restrict__ nrb = d.nrb;
-            const uint16_t* __restrict__ bbits = d.bbits;
-            const size_t N = (size_t)d.N, cap = (size_t)d.cap;
-            SlotRec<R>* stage = (SlotRec<R>*)cl_dsm + (size_t)warp * cl_stage<J>() * CL_CHUNK;
-            F = v3(0.0, 0.0, 0.0);
-            T = F;
-            for (int c0 = M0; c0 < M1; c0 += CL_CHUNK) {
-                int idx[J], own[J];
-#pragma unroll
-                for (int j = 0; j < J; j++) {
-                    const int m = c0 + 32 * j + lane;
-                    idx[j] = m < M1 ? mem_idx[m] : -1;
-                    own[j] = m < M1 ? mem_cl[m] - k0 : 0;
-                }
-                double4 ps[J];
-                int r0[J], r1[J], q0[J], q1[J];
-                uint16_t bb[J];
-#pragma unroll
-                for (int j = 0; j < J; j++) {
-                    const int i = idx[j] < 0 ? 0 : idx[j];
-                    const int ro = i + s_sc[warp][own[j]];
-                    ps[j] = posr[i];
-                    const int2 ra = nrb[ro], rb = nrb[ro + 1];
-                    r0[j] = ra.x;
-                    r1[j] = rb.x;
-                    q0[j] = ra.y;
-                    q1[j] = rb.y;
-                    bb[j] = bbits[i];
-                }
-                // stage every contact record of the lane's members (front
-                // slots, back slots, the boundary force) with asynchronous
-                // copies: one wait for all of them instead of one per slot
-                int nrec = 0;
-#pragma unroll
-                for (int j = 0; j < J; j++)
-                    if (idx[j] >= 0) nrec += (r1[j] - r0[j]) + (q1[j] - q0[j]) + (bb[j] ? 1 : 0);
-                int rbase = nrec;
-#pragma unroll
-                for (int o = 1; o < 32; o <<= 1) {
-                    const int y = __shfl_up_sync(0xffffffffu, rbase, o);
-                    if (lane >= o) rbase += y;
-                }
-                rbase -= nrec;
-                const bool staged = rbase + nrec <= cl_stage<J>() * CL_CHUNK;
-                SlotRec<R>* st = stage + rbase;
-                if (staged) {
-                    int o = 0;
-#pragma unroll
-                    for (int j = 0; j < J; j++) {
-                        if (idx[j] < 0) continue;
-                        for (int e = r0[j]; e < r1[j]; e++, o++) stage_rec<R>(st + o, fsl + 2 * (size_t)e, fsl + 2 * (size_t)e + 1);
-                        for (int e = q0[j]; e < q1[j]; e++, o++) stage_rec<R>(st + o, bsl + 2 * (size_t)e, bsl + 2 * (size_t)e + 1);
-                        if (bb[j]) { stage_rec<R>(st + o, fbd + idx[j], fbd + N + idx[j]); o++; }
-                    }
-                    cp_async_wait_all();
-                }
-                int o = 0;
-#pragma unroll
-                for (int j = 0; j < J; j++) {
-                    if (idx[j] < 0) continue;
-                    const int kk = own[j];
-                    V3<R> fr, tr;
-                    if (staged) {
-                        // the order of slot_sum: front slots, back slots, then the boundary force
-                        fr = v3<R>(0, 0, 0);
-                        tr = fr;
-                        const int ns = (r1[j] - r0[j]) + (q1[j] - q0[j]);
-#pragma unroll 1
-                        for (int e = 0; e < ns; e++, o++) {
-                            fr = fr + xyz<R>(st[o].f);
-                            tr = tr + xyz<R>(st[o].t);
-                        }
-                        if (bb[j]) {
-                            fr = fr + xyz<R>(st[o].f);
-                            tr = tr + xyz<R>(st[o].t);
-                            o++;
-                        }
-                    } else {
-                        slot_sum<R>(fsl, bsl, cap, r0[j], r1[j], q0[j], q1[j], fr, tr);
-                        if (bb[j]) {
-                            fr = fr + xyz<R>(fbd[idx[j]]);
-                            tr = tr + xyz<R>(fbd[N + idx[j]]);
-                        }
-                    }
-                    const V3<double> r = v3(ps[j].x - s_cl[warp][0][kk], ps[j].y - s_cl[warp][1][kk],
-                                            ps[j].z - s_cl[warp][2][kk]);
-                    const V3<double> f = v3((double)fr.x, (double)fr.y, (double)fr.z);
-                    const int q = 32 * j + lane;
-                    s_mf[warp][0][q] = f.x;
-                    s_mf[warp][1][q] = f.y;
-                    s_mf[warp][2][q] = f.z;
-                    s_mf[warp][3][q] = (double)tr.x + (r.y * f.z - r.z * f.y);
-                    s_mf[warp][4][q] = (double)tr.y + (r.z * f.x - r.x * f.z);
-                    s_mf[warp][5][q] = (double)tr.z + (r.x * f.y - r.y * f.x);
-                }
-                __syncwarp();
-                if (isc) {
-                    const int lo = max(mb, c0), hi = min(me, c0 + CL_CHUNK);
-                    for (int m = lo; m < hi; m++) {
-                        const int q = m - c0;
-                        const V3<double> f = v3(s_mf[warp][0][q], s_mf[warp][1][q], s_mf[warp][2][q]);
-                        const V3<double> tc = v3(s_mf[warp][3][q], s_mf[warp][4][q], s_mf[warp][5][q]);
-                        if (m == mb) { F = f; T = tc; }
-                        else { F = F + f; T = T + tc; }
-                    }
-                }
-                __syncwarp();
-            }
-            if (isc && post_k) {
-                if (mb < me) {
-                    if (!(isfinite(F.x) && isfinite(F.y) && isfinite(F.z) && isfinite(T.x) && isfinite(T.y) &&
-                          isfinite(T.z)))
-                        atomicOr(&d.dyn[sc].err, ERR_NONFINITE);
-                    d.cF[k] = make_double4(F.x, F.y, F.z, 0.0);
-                    d.cT[k] = make_double4(T.x, T.y, T.z, 0.0);
-                } else {
-                    F = xyzd(d.cF[k]);
-                    T = xyzd(d.cT[k]);
-                }
-            }
-            // split driver: only Type 0 takes the closing half-kick
-            // (src/dem_integrate_withglue.cu:140)
-            if (post_k && !(SPH && (P.sphere & SPH_KINDS) && (d.kind[k] & 3) != 0)) {
-                V3<double> ac = pr.w * F;   // pr: the reciprocals 1/I, 1/M
-                ac.z = ac.z + P.gravity;
-                V3<double> al = v3(pr.x * T.x, pr.y * T.y, pr.z * T.z);
-                cv.x += (0.5 * Dt) * ac.x; cv.y += (0.5 * Dt) * ac.y; cv.z += (0.5 * Dt) * ac.z;
-                cw.x += (0.5 * Dt) * al.x; cw.y += (0.5 * Dt) * al.y; cw.z += (0.5 * Dt) * al.z;
-            }
-        } else {
-            F = xyzd(d.cF[k]);
-            T = xyzd(d.cT[k]);
-        }
-        if (do_pre) {
-            const double4 cp_old = cp;
-            if (SPH && (P.sphere & SPH_KIN) && mb < me) {
-                // the sphere drivers' first half-kick and attitude leave the
-                // intruder out (src/dem_integrate.cu:20-21,72); one member
-                const int i0 = mem_idx[mb];
-                if ((d.bbits[i0] >> SLOT_INTR) & 1) {
-                    const R4<R>* __restrict__ fi = (const R4<R>*)d.fint;
-                    const R4<R> a = fi[i0], b = fi[(size_t)d.N + i0];
-                    F = F - v3((double)a.x, (double)a.y, (double)a.z);
-                    T = T - v3((double)b.x, (double)b.y, (double)b.z);
-                }
-            }
-            V3<double> ac = pr.w * F;   // pr: the reciprocals 1/I, 1/M
-            ac.z = ac.z + P.gravity;
-            V3<double> al = v3(pr.x * T.x, pr.y * T.y, pr.z * T.z);
-            V3<double> v = xyzd(cv), w = xyzd(cw);
-            V3<double> dist = Dt * v + (0.5 * Dt * Dt) * ac;
-            cp.x += dist.x; cp.y += dist.y; cp.z += dist.z;
-            v = v + (0.5 * Dt) * ac;
-            w = w + (0.5 * Dt) * al;
-            // attitude with the half-kicked angular velocity
-            V3<double> Wb = rot_w2b(cq, w), Wdb = rot_w2b(cq, al);
-            double4 q = cq, qd, qdd;
-            qd.x = 0.50 * (Wb.x * q.w - Wb.y * q.z + Wb.z * q.y);
-            qd.y = 0.50 * (Wb.x * q.z + Wb.y * q.w - Wb.z * q.x);
-            qd.z = 0.50 * (-Wb.x * q.y + Wb.y * q.x + Wb.z * q.w);
-            qd.w = 0.50 * (-Wb.x * q.x - Wb.y * q.y - Wb.z * q.z);
-            qdd.x = (Wdb.x * q.w - Wdb.y * q.z + Wdb.z * q.y) * 0.50 + (Wb.x * qd.w - Wb.y * qd.z + Wb.z * qd.y) * 0.50;
-            qdd.y = (Wdb.x * q.z + Wdb.y * q.w - Wdb.z * q.x) * 0.50 + (Wb.x * qd.z + Wb.y * qd.w - Wb.z * qd.x) * 0.50;
-            qdd.z = (-Wdb.x * q.y + Wdb.y * q.x + Wdb.z * q.w) * 0.50 + (-Wb.x * qd.y + Wb.y * qd.x + Wb.z * qd.w) * 0.50;
-            qdd.w = (-Wdb.x * q.x - Wdb.y * q.y - Wdb.z * q.z) * 0.50 + (-Wb.x * qd.x - Wb.y * qd.y - Wb.z * qd.z) * 0.50;
-            const double h2 = 0.5 * Dt * Dt;
-            q.x = (q.x + Dt * qd.x) + h2 * qdd.x;
-            q.y = (q.y + Dt * qd.y) + h2 * qdd.y;
-            q.z = (q.z + Dt * qd.z) + h2 * qdd.z;
-            q.w = (q.w + Dt * qd.w) + h2 * qdd.w;
-            const double inv = 1.0 / sqrt(q.x * q.x + q.y * q.y + q.z * q.z + q.w * q.w);
-            q.x *= inv; q.y *= inv; q.z *= inv; q.w *= inv;
-            if (SPH && (P.sphere & SPH_KINDS)) {
-                // split driver (src/dem_integrate_withglue.cu:3-110).  Its call
-                // passes the original index where the first half-kick expects
-                // Type (src/dem_simulation_split.cu:84-85 against
-                // src/dem_integrate_withglue.cu:113-114), so the kick and the
-                // move go by the body's original index (bits 2-3: 0 free, 1
-                // driven at (-0.2 y, -0.2 x, 0), 2 or more still) and the
-                // attitude by its Type (bits 0-1: turns only for Type 0)
-                const int kd = d.kind[k], ka = kd & 3, kb = (kd >> 2) & 3;
-                if (kb != 0) {
-                    cp = cp_old;
-                    w = xyzd(cw);
-                    v = xyzd(cv);
-                    if (kb == 1) {
-                        v = v3(-0.2 * cp_old.y, -0.2 * cp_old.x, 0.0);
-                        cp.x += Dt * v.x; cp.y += Dt * v.y; cp.z += Dt * v.z;
-                    }
-                    if (ka == 0) q = quat_step(cq, w, al, Dt);
-                }
-                if (ka != 0) q = cq;
-            }
-            if (!pre_k) {   // the scene stands still: keep the clump as it is
-                cp = cp_old;
-                v = xyzd(cv);
-                w = xyzd(cw);
-                q = cq;
-            }
-            if (isc && pre_k) {
-                d.cpos[k] = cp;
-                d.cvel[k] = make_double4(v.x, v.y, v.z, 0.0);
-                d.cw[k] = make_double4(w.x, w.y, w.z, 0.0);
-                d.cq[k] = q;
-            }
-            __syncwarp();   // the old positions in s_cl are no longer read
-            s_cl[warp][0][lane] = cp.x; s_cl[warp][1][lane] = cp.y; s_cl[warp][2][lane] = cp.z;
-            s_cl[warp][3][lane] = v.x; s_cl[warp][4][lane] = v.y; s_cl[warp][5][lane] = v.z;
-            s_cl[warp][6][lane] = w.x; s_cl[warp][7][lane] = w.y; s_cl[warp][8][lane] = w.z;
-            s_cl[warp][9][lane] = q.x; s_cl[warp][10][lane] = q.y; s_cl[warp][11][lane] = q.z;
-            s_cl[warp][12][lane] = q.w;
-            __syncwarp();
-            // ---- poses of the members, 32 at a time
-            double4* __restrict__ kv = (double4*)d.kin;   // per member: world arm, mass
-            const double4* __restrict__ lom = d.lom;
-            double4* __restrict__ cum = d.cum;
-            double4* __restrict__ posw = d.posr;
-            // J members per lane at a time: all indices, then all member
-            // records, in flight together
-            constexpr int JP = J;
-            for (int c0 = M0; c0 < M1; c0 += 32 * JP) {
-                int idx[JP], own[JP];
-#pragma unroll
-                for (int j = 0; j < JP; j++) {
-                    const int m = c0 + 32 * j + lane;
-                    idx[j] = m < M1 ? mem_idx[m] : -1;
-                    own[j] = m < M1 ? mem_cl[m] - k0 : 0;
-                }
-                double4 lo[JP], old[JP], cu[JP];
-#pragma unroll
-                for (int j = 0; j < JP; j++) {
-                    const int i = idx[j] < 0 ? 0 : idx[j];
-                    lo[j] = lom[i];
-                    old[j] = posw[i];
-                    cu[j] = cum[i];
-                }
-#pragma unroll
-                for (int j = 0; j < JP; j++) {
-                    if (idx[j] < 0) continue;
-                    const int i = idx[j];
-                    const int kk = own[j];
-                    if (!s_pre[warp][kk]) continue;
-                    const double4 qk = make_double4(s_cl[warp][9][kk], s_cl[warp][10][kk], s_cl[warp][11][kk],
-                                                    s_cl[warp][12][kk]);
-                    const V3<double> arm = rot_b2w(qk, v3(lo[j].x, lo[j].y, lo[j].z));
-                    const V3<double> p = v3(s_cl[warp][0][kk] + arm.x, s_cl[warp][1][kk] + arm.y,
-                                            s_cl[warp][2][kk] + arm.z);
-                    const double4 c = cu[j], o = old[j];
-                    const V3<double> cn = v3((c.x + p.x) - o.x, (c.y + p.y) - o.y, (c.z + p.z) - o.z);
-                    const V3<double> vk = v3(s_cl[warp][3][kk], s_cl[warp][4][kk], s_cl[warp][5][kk]);
-                    const V3<double> wk = v3(s_cl[warp][6][kk], s_cl[warp][7][kk], s_cl[warp][8][kk]);
-                    cum[i] = make_double4(cn.x, cn.y, cn.z, 0.0);
-                    posw[i] = make_double4(p.x, p.y, p.z, o.w);
-                    kv[i] = make_double4(arm.x, arm.y, arm.z, lo[j].w);
-                    const int sk = s_sc[warp][kk];
-                    double thr = d.par[sk].thresh;
-                    if (SPH && (d.par[sk].sphere & SPH_KINDS))   // split driver: the free body of the first
-                        thr = ((d.kind[k0 + kk] >> 2) & 3) == 0 ? 0.10 * o.w : INFINITY;   // half-kick at 0.1 r
-                                                                  // (src/dem_integrate_withglue.cu:41)
-                    if (len_floor(cn) > thr) {
-                        SceneDyn& y = d.dyn[sk];
-                        if (!*(volatile int*)&y.rebuild) atomicExch(&y.rebuild, 1);
-                        if (!*(volatile int*)d.any_rebuild) atomicExch(d.any_rebuild, 1);
-                    }
-                }
-            }
-        }
-        if (isc && post_k && !pre_k) {   // closing half-kick only (sync, or the scene's last step)
-            d.cvel[k] = cv;
-            d.cw[k] = cw;
-        }
-    }
-    if (t >= d.K && t < d.K + d.S) {
-        const int s = t - d.K;
-        const ScenePar& P = d.par[s];
-        SceneDyn& y = d.dyn[s];
-        const double Dt = P.dt;
-        const bool pre_s = scene_pre(y, do_pre, L), post_s = scene_post(y, post, L);
-        if (post_s) {
-            long long* fx = (long long*)&y.ifix[0];
-            V3<double> tf = v3(fx[0] / FIX_F, fx[1] / FIX_F, fx[2] / FIX_F);
-            V3<double> tt = v3(fx[3] / FIX_T, fx[4] / FIX_T, fx[5] / FIX_T);
-            for (int c = 0; c < 6; c++) fx[c] = 0;
-            y.totF[0] = tf.x; y.totF[1] = tf.y; y.totF[2] = tf.z;
-            y.totT[0] = tt.x; y.totT[1] = tt.y; y.totT[2] = tt.z;
-            if (P.has_intr) {
-                if (P.intr_wait && y.intr_state == 1) y.intr_state = 2;
-                V3<double> reac = v3(-tf.x, -tf.y, -tf.z);
-                if (P.intr_motion == 1 && (!P.intr_wait || y.intr_state != 0)) {
-                    V3<double> a = (1.0 / P.intr_mass) * reac;
-                    a.z = a.z + P.gravity;
-                    for (int c = 0; c < 3; c++) y.intr_v[c] += (0.5 * Dt) * (&a.x)[c];
-                }
-                y.reaction[0] = reac.x; y.reaction[1] = reac.y; y.reaction[2] = reac.z;
-                y.reaction_t[0] = tt.x; y.reaction_t[1] = tt.y; y.reaction_t[2] = tt.z;
-                double* ring = d.ring + ((size_t)s * d.ring_len + (y.step % d.ring_len)) * 6;
-                ring[0] = reac.x; ring[1] = reac.y; ring[2] = reac.z;
-                ring[3] = tt.x; ring[4] = tt.y; ring[5] = tt.z;
-            }
-            y.step += 1;
-        }
-        if (do_pre) y.frozen = !pre_s;
-        if (pre_s && P.has_intr) {
-            if (P.intr_motion == 1 && (!P.intr_wait || y.intr_state != 0)) {
-                V3<double> a = (-1.0 / P.intr_mass) * v3(y.totF[0], y.totF[1], y.totF[2]);
-                a.z = a.z + P.gravity;
-                for (int c = 0; c < 3; c++) {
-                    y.intr_p[c] = (y.intr_p[c] + Dt * y.intr_v[c]) + (0.5 * Dt * Dt) * (&a.x)[c];
-                    y.intr_v[c] = y.intr_v[c] + (0.5 * Dt) * (&a.x)[c];
-                }
-            } else {
-                for (int c = 0; c < 3; c++) y.intr_p[c] = y.intr_p[c] + Dt * y.intr_v[c];
-            }
-        }
+    const int w = blockIdx.x * CL_WARPS + (threadIdx.x >> 5);
+    if (w < d.W) {
+        clump_warp<R, SPH>(d, w, do_pre, post, L);
+    } else {
+        const int s = (w - d.W) * 32 + (threadIdx.x & 31);
+        if (s < d.S) scene_step(d, s, do_pre, post, L);
     }
     __syncthreads();
     if (threadIdx.x == 0) {
@@ -551,6 +387,32 @@ __global__ void __launch_bounds__(CL_THREADS, J <= 2 ? 4 : 3) k_clump(const Dev*
             }
         }
     }
+}
+
+// Clump records between the engine's order and the caller's (old: the
+// caller's number of each): the n clumps from `first` on, a scene's, out of the
+// engine as W packed doubles per clump, ready to be copied to the caller's
+// array; all of them into it as whole records.
+template <int W>
+static __global__ void k_clumps_out(const double4* __restrict__ src, const int* __restrict__ old, int first, int n,
+                                    double* __restrict__ dst) {
+    for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < n; c += gridDim.x * blockDim.x) {
+        const double4 v = ld32(src + first + c);
+        double* o = dst + (size_t)W * (old[first + c] - first);
+        o[0] = v.x; o[1] = v.y; o[2] = v.z;
+        if (W == 4) o[3] = v.w;
+    }
+}
+static __global__ void k_clumps_in(const double4* __restrict__ src, const int* __restrict__ old, int n,
+                                   double4* __restrict__ dst) {
+    for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < n; c += gridDim.x * blockDim.x)
+        st32(dst + c, ld32(src + old[c]));
+}
+// member records from the caller's subsphere order into their slots
+static __global__ void k_members_in(const double4* __restrict__ src, const int2* __restrict__ cm, int n,
+                                    double4* __restrict__ dst) {
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+        st32(dst + cm[i].y, ld32(src + i));
 }
 
 // The steps a graph launch with a device-side step loop takes (the first
@@ -1002,7 +864,6 @@ static __global__ void __launch_bounds__(RS_THREADS) k_rs_scatter(const int* __r
 // --- reorder and cell table ---------------------------------------------
 // SortArray_*_cuk (src/dem_grid.cu:336-437) for every persistent per-subsphere
 // array at once, into the alternate buffers (written back by k_writeback).
-// The displacement accumulator restarts at zero (src/dem_simulation_clump.cu:172).
 template <typename R>
 __global__ void k_reorder(const Dev* __restrict__ dp) {
     const Dev& d = *dp;
@@ -1023,14 +884,11 @@ __global__ void k_reorder(const Dev* __restrict__ dp) {
         const int k = plan_find(d.psub, ns, t);
         const int i = d.par[d.pscene[k]].sub_off + (t - d.psub[k]);
         const int o = d.perm[i];
-        d.posr2[i] = d.posr[o];
-        d.lom2[i] = d.lom[o];
-        d.cum2[i] = make_double4(0, 0, 0, 0);
-        d.clump_id2[i] = d.clump_id[o];
+        st32(d.posr2 + i, ld32(d.posr + o));
+        d.cm2[i] = d.cm[o];
         d.part_fix2[i] = d.part_fix[o];
         d.level2[i] = d.level[o];
         d.bbits2[i] = d.bbits[o];
-        ((double4*)d.kin2)[i] = ((const double4*)d.kin)[o];
         const R4<R>* b1 = (const R4<R>*)d.bhist;
         R4<R>* b2 = (R4<R>*)d.bhist2;
         const uint16_t bits = d.bbits[o];
@@ -1088,7 +946,7 @@ __device__ __forceinline__ void group_search(const Dev& d, const ScenePar& P, co
     // buffer pointers in registers: the stores below could otherwise alias
     // the pointer table and force it to be re-read on every candidate
     const double4* __restrict__ posr = d.posr2;
-    const int* __restrict__ cid = d.clump_id2;
+    const int2* __restrict__ cm = d.cm2;
     const int* __restrict__ cstart = d.cstart;
     int* __restrict__ cnt_f = d.cnt_f;
     int* __restrict__ xcnt = d.xcnt;
@@ -1100,7 +958,7 @@ __device__ __forceinline__ void group_search(const Dev& d, const ScenePar& P, co
     const int gshift = (threadIdx.x & 31) & ~(SL - 1);
     __syncwarp(gm);  // the group's previous subsphere is done with rs / pre
     const double4 pi = posr[i];
-    const int ci = cid[i];
+    const int ci = cm[i].x;
     const int my = P.levels > 1 ? d.level2[i] : 0;
     const int nrows = 9 * (my + 1);
     // ---- ranges of the stencil rows: lane k resolves rows [k C, k C + C)
@@ -1190,7 +1048,7 @@ __device__ __forceinline__ void group_search(const Dev& d, const ScenePar& P, co
         jn = rs[r] + (lane - pre[r]);
         rn = r;
         pn = posr[jn];
-        cn = cid[jn];
+        cn = cm[jn].x;
     }
     for (int b0 = 0; b0 < total; b0 += SL) {
         const int j = jn, rj = rn, cj = cn;
@@ -1202,7 +1060,7 @@ __device__ __forceinline__ void group_search(const Dev& d, const ScenePar& P, co
             jn = rs[r] + (f - pre[r]);
             rn = r;
             pn = posr[jn];
-            cn = cid[jn];
+            cn = cm[jn].x;
         }
         const double dx = pi.x - pj.x, dy = pi.y - pj.y, dz = pi.z - pj.z;
         const double d2 = dx * dx + dy * dy + dz * dz;
@@ -1552,8 +1410,8 @@ __global__ void k_writeback(Dev* __restrict__ dp) {
         if (blockIdx.x == 0 && threadIdx.x == 0) {
             Dev& w = *dp;
 #define NBC_SWAP(a, b) { auto tmp_ = w.a; w.a = w.b; w.b = tmp_; }
-            NBC_SWAP(posr, posr2) NBC_SWAP(lom, lom2) NBC_SWAP(cum, cum2) NBC_SWAP(clump_id, clump_id2)
-            NBC_SWAP(part_fix, part_fix2) NBC_SWAP(level, level2) NBC_SWAP(key, key2) NBC_SWAP(kin, kin2)
+            NBC_SWAP(posr, posr2) NBC_SWAP(cm, cm2)
+            NBC_SWAP(part_fix, part_fix2) NBC_SWAP(level, level2) NBC_SWAP(key, key2)
             NBC_SWAP(bhist, bhist2) NBC_SWAP(bbits, bbits2)
             NBC_SWAP(L[0], L[1]) NBC_SWAP(H[0], H[1]) NBC_SWAP(touch[0], touch[1])
 #undef NBC_SWAP
@@ -1568,13 +1426,10 @@ __global__ void k_writeback(Dev* __restrict__ dp) {
         const PlanItem it = plan_item(d, ns, t);
         const int i = it.i, s = it.s;
         d.posr[i] = d.posr2[i];
-        d.lom[i] = d.lom2[i];
-        d.cum[i] = d.cum2[i];
-        d.clump_id[i] = d.clump_id2[i];
+        d.cm[i] = d.cm2[i];
         d.part_fix[i] = d.part_fix2[i];
         d.level[i] = d.level2[i];
         d.key[i] = d.key2[i];
-        ((double4*)d.kin)[i] = ((const double4*)d.kin2)[i];
         const uint16_t bits = d.bbits2[i];
         d.bbits[i] = bits;
         const R4<R>* b2 = (const R4<R>*)d.bhist2;
@@ -1735,11 +1590,16 @@ __global__ void __launch_bounds__(SEARCH_THREADS) k_near(const Dev* __restrict__
                 const int k = plan_find(d.pclump, ns, u);
                 const int c = d.par[d.pscene[k]].clump_off + (u - d.pclump[k]);
                 const int mb = d.mem_start[c], me = d.mem_start[c + 1];
-                for (int m = mb; m < me; m++) d.mem_idx[m] = d.inv[d.mem_idx[m]];
+                for (int m = mb; m < me; m++) {
+                    // the displacement restarts at zero (src/dem_simulation_clump.cu:172)
+                    st32(d.cum + m, make_double4(0, 0, 0, 0));
+                    d.mo[m].x = d.inv[d.mo[m].x];
+                }
                 for (int m = mb + 1; m < me; m++) {
-                    int v = d.mem_idx[m], q = m - 1;
-                    while (q >= mb && d.mem_idx[q] > v) { d.mem_idx[q + 1] = d.mem_idx[q]; q--; }
-                    d.mem_idx[q + 1] = v;
+                    const int2 v = d.mo[m];
+                    int q = m - 1;
+                    while (q >= mb && d.mo[q].x > v.x) { d.mo[q + 1] = d.mo[q]; q--; }
+                    d.mo[q + 1] = v;
                 }
             } else if (u < TK + ns) {
                 const int k = u - TK;
@@ -1959,8 +1819,8 @@ template <typename R> struct Body {
 };
 
 template <typename R>
-__device__ __forceinline__ void load_kin(const Dev& d, int i, int c, Body<R>& b) {
-    const double4 r = ((const double4*)d.kin)[i], v = d.cvel[c], w = d.cw[c];
+__device__ __forceinline__ void load_kin(const Dev& d, int2 cm, Body<R>& b) {
+    const double4 r = ld32(d.kin + cm.y), v = ld32(d.cvel + cm.x), w = ld32(d.cw + cm.x);
     b.arm = v3(r.x, r.y, r.z);
     b.m = r.w;
     b.v = v3(v.x, v.y, v.z);
@@ -2030,7 +1890,8 @@ __device__ __forceinline__ void boundary_contact(const Law<R>& L, const Body<R>&
 // [2q + 1] (one 32-byte record in FP32), Dr.z as a scalar after the 2*cap R4s
 template <typename R>
 __device__ __forceinline__ void hist_read(const R4<R>* H, size_t cap, size_t q, V3<R>& hs, V3<R>& ht, V3<R>& hr) {
-    R4<R> a = H[2 * q], b = H[2 * q + 1];
+    R4<R> a, b;
+    ld_pair(H + 2 * q, a, b);
     const R c = ((const R*)(H + 2 * cap))[q];
     hs = v3<R>(a.x, a.y, a.z);
     ht = v3<R>(b.x, b.y, b.z);
@@ -2038,8 +1899,7 @@ __device__ __forceinline__ void hist_read(const R4<R>* H, size_t cap, size_t q, 
 }
 template <typename R>
 __device__ __forceinline__ void hist_write(R4<R>* H, size_t cap, size_t q, V3<R> hs, V3<R> ht, V3<R> hr) {
-    H[2 * q] = pack<R>(hs, hr.x);
-    H[2 * q + 1] = pack<R>(ht, hr.y);
+    st_pair(H + 2 * q, pack<R>(hs, hr.x), pack<R>(ht, hr.y));
     ((R*)(H + 2 * cap))[q] = hr.z;
 }
 
@@ -2224,7 +2084,7 @@ __device__ __forceinline__ void boundary_one(const Dev& d, int i, int s) {
         if (!on) continue;
         if (!have_kin) {
             me.p = pp;
-            load_kin<R>(d, i, d.clump_id[i], me);
+            load_kin<R>(d, d.cm[i], me);
             have_kin = true;
         }
         if (is_intr) Mij = P.intr_motion == 1 ? me.m * P.intr_mass / (me.m + P.intr_mass) : me.m;
@@ -2319,16 +2179,16 @@ __device__ __forceinline__ bool overlaps(double4 a, double4 b) {
 }
 
 // The law of one touching near pair (front entry ef of scene s, pair slot p,
-// owner i of clump ci, partner jr of clump cj, near back entry eb; a.p and b.p
-// loaded): kinematics and spring history in, new history, touch flag and the
+// owner i and partner jr with their clumps and member slots ci and cj, near
+// back entry eb; a.p and b.p loaded): kinematics and spring history in, new history, touch flag and the
 // four contact slots out (and the export record).
 template <typename R, bool EXPORT>
-__device__ __forceinline__ void pair_law(const Dev& d, int s, int ef, int p, int i, int jr, int ci, int cj, int eb,
+__device__ __forceinline__ void pair_law(const Dev& d, int s, int ef, int p, int i, int jr, int2 ci, int2 cj, int eb,
                                          Body<R>& a, Body<R>& b) {
     const int hg = *d.hgen;
     const size_t cap = (size_t)d.cap;
-    load_kin<R>(d, i, ci, a);
-    load_kin<R>(d, jr, cj, b);
+    load_kin<R>(d, ci, a);
+    load_kin<R>(d, cj, b);
     V3<R> hs = v3<R>(0, 0, 0), ht = hs, hr = hs;
     if (d.touch[hg & 1][p]) hist_read<R>((const R4<R>*)d.H[hg & 1], cap, p, hs, ht, hr);
     const ScenePar& P = d.par[s];
@@ -2344,10 +2204,8 @@ __device__ __forceinline__ void pair_law(const Dev& d, int s, int ef, int p, int
     d.touch[(hg + 1) & 1][p] = 1;
     R4<R>* fs = (R4<R>*)d.nfs;
     R4<R>* bs = (R4<R>*)d.nbs;
-    fs[2 * (size_t)ef] = pack<R>(fa, R(0));
-    fs[2 * (size_t)ef + 1] = pack<R>(ta, R(0));
-    bs[2 * (size_t)eb] = pack<R>(-fa, R(0));
-    bs[2 * (size_t)eb + 1] = pack<R>(tb, R(0));
+    st_pair(fs + 2 * (size_t)ef, pack<R>(fa, R(0)), pack<R>(ta, R(0)));
+    st_pair(bs + 2 * (size_t)eb, pack<R>(-fa, R(0)), pack<R>(tb, R(0)));
     if (EXPORT) {
         R4<R>* xf = (R4<R>*)d.xfcn;
         double4* xc = (double4*)d.xcpt;
@@ -2384,7 +2242,7 @@ __global__ void __launch_bounds__(PR_THREADS, NBC_PAIR_MINB) k_pairs(const Dev* 
     const int np = npre[S];
     const int4* __restrict__ nfr = d.nfr;
     const double4* __restrict__ posr = d.posr;
-    const int* __restrict__ cid = d.clump_id;
+    const int2* __restrict__ cm = d.cm;
     uint8_t* __restrict__ to = d.touch[(hg + 1) & 1];
     R4<R>* __restrict__ fs = (R4<R>*)d.nfs;
     R4<R>* __restrict__ bs = (R4<R>*)d.nbs;
@@ -2413,20 +2271,18 @@ __global__ void __launch_bounds__(PR_THREADS, NBC_PAIR_MINB) k_pairs(const Dev* 
         const int p = rec.x, jr = rec.y, i = rec.z, eb = rec.w;
         Body<R> a, b;
         bool on = jr >= 0;   // pairs inside one clump have no force (src/dem_force_clump.cu:18-19)
-        int ci = 0, cj = 0;
+        int2 ci = make_int2(0, 0), cj = ci;
         if (on) {
-            a.p = posr[i];
-            b.p = posr[jr];
-            ci = cid[i];      // with the positions, for the kinematics of a touching pair
-            cj = cid[jr];
+            a.p = ld32(posr + i);
+            b.p = ld32(posr + jr);
+            ci = cm[i];       // with the positions, for the kinematics of a touching pair
+            cj = cm[jr];
             on = overlaps(a.p, b.p);
         }
         if (!on) {
             to[p] = 0;
-            fs[2 * (size_t)ef] = zero;
-            fs[2 * (size_t)ef + 1] = zero;
-            bs[2 * (size_t)eb] = zero;
-            bs[2 * (size_t)eb + 1] = zero;
+            st_pair(fs + 2 * (size_t)ef, zero, zero);
+            st_pair(bs + 2 * (size_t)eb, zero, zero);
             continue;
         }
         pair_law<R, EXPORT>(d, s, ef, p, i, jr, ci, cj, eb, a, b);
@@ -2442,7 +2298,7 @@ __device__ __forceinline__ void contact_sum(const Dev& d, int i, int s, V3<R>& F
                                             V3<R>* pairT = nullptr) {
     const size_t N = (size_t)d.N;
     const int2 ra = d.nrb[i + s], rb = d.nrb[i + s + 1];
-    slot_sum<R>((const R4<R>*)d.nfs, (const R4<R>*)d.nbs, (size_t)d.cap, ra.x, rb.x, ra.y, rb.y, F, T);
+    slot_sum<R>((const R4<R>*)d.nfs, (const R4<R>*)d.nbs, ra.x, rb.x, ra.y, rb.y, F, T);
     if (pairF) { *pairF = F; *pairT = T; }
     if (d.bbits[i]) {
         const R4<R>* fb = (const R4<R>*)d.fbnd;

@@ -122,14 +122,10 @@ struct Dev {
     // alternates and writes them back once the new list is complete, so
     // nothing changes if it stops early.
     double4* posr;    double4* posr2;    // x y z r
-    double4* lom;     double4* lom2;     // local offset (body frame) xyz, mass
-    double4* cum;     double4* cum2;     // displacement since the last rebuild
-    int* clump_id;    int* clump_id2;
+    int2* cm;         int2* cm2;         // clump, member slot
     int* part_fix;    int* part_fix2;    // original index (ParticleID)
     int* level;       int* level2;       // hgrid level (0 = coarsest)
     int* key;         int* key2;         // global cell key at the last rebuild (sorted)
-    void* kin;        void* kin2;        // double4 [N]: world arm, mass (the velocities are the
-                                         // clump's; see Body in kernels.cuh)
     void* bhist;      void* bhist2;      // Real4 [NB_SLOTS][N][3] boundary histories (Dv, Dt, Dr adjacent)
     uint16_t* bbits;  uint16_t* bbits2;  // [N] boundary slots in contact at the last step
     void* fsum;       // Real4 [2][N]: force and torque on each subsphere (pairs + walls + intruder),
@@ -137,20 +133,29 @@ struct Dev {
     void* fbnd;       // Real4 [2][N]: wall + intruder force and torque, valid where bbits != 0
     void* fint;       // Real4 [2][N]: intruder force and torque alone, valid where the intruder bit of
                       // bbits is set, in SPH_KIN scenes (null when there are none)
-    // clumps
+    // clumps, in the order of their first grid cell at creation (the host maps to the caller's order)
     double4* cpos;    // xyz
     double4* cvel;
     double4* cw;
     double4* cq;      // x y z w
     double4* cprop;   // Ixx Iyy Izz M
-    int* mem_cl;      // [N] clump of each member slot (fixed: members stay in their clump's range)
+    // member slots [N]: clump k owns the slots [mem_start[k], mem_start[k + 1]), a member keeps its slot for
+    // the engine's life, and what only the clump pass touches lies in slot order, so the pass streams it
+    double4* lom;     // local offset (body frame) xyz, mass
+    double4* cum;     // displacement since the last rebuild
+    double4* kin;     // world arm, mass (the velocities are the clump's; see Body in kernels.cuh)
+    int4* ltab;       // [32 W] lanes of the clump pass: entry of mo (-1: none), clump (-1: idle lane),
+                      // the clump's members << 5 | its first lane, scene
+    int W;            // warps of that table
     double4* cinv;    // 1/Ixx 1/Iyy 1/Izz 1/M (correctly rounded divisions, computed once)
     int* kind;        // [K] body kind of the split driver (0 free, 1 prescribed velocity, 2 fixed),
                       // read in SPH_KINDS scenes only (null when there are none)
+    int* cold;        // [K] the caller's number of each clump (counted over all scenes)
+    double4* stage;   // [K] clump records on their way from and to the caller's order
     double4* cF;      // force on clump from the last force pass
     double4* cT;
     int* mem_start;   // [K+1]
-    int* mem_idx;     // [N] member subspheres of each clump, ascending
+    int2* mo;         // [N] members of each clump, ascending by subsphere: subsphere, member slot
     int* post_pending;// device flag: a force pass has run whose half-kick is pending
     // broad phase scratch
     int* kA; int* vA; int* kB; int* vB;   // radix sort ping-pong

@@ -40,33 +40,71 @@ template <typename R> __device__ __forceinline__ R4<R> pack(V3<R> a, R w) {
     R4<R> o; o.x = a.x; o.y = a.y; o.z = a.z; o.w = w; return o;
 }
 
+// 32-byte records in one access (sm_100 loads and stores 256 bits a lane): a
+// gather of 32 scattered records costs the L1 one tag lookup per lane instead
+// of two.  p is 32-byte aligned.  The asm is volatile so that it keeps its
+// place between barriers; nothing written by the same kernel is read this way
+// unless a barrier lies between.
+__device__ __forceinline__ double4 ld32(const double4* p) {
+    double4 v;
+    asm volatile("ld.global.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(v.x), "=d"(v.y), "=d"(v.z), "=d"(v.w) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ void st32(double4* p, double4 v) {
+    asm volatile("st.global.v4.f64 [%0], {%1, %2, %3, %4};" ::"l"(p), "d"(v.x), "d"(v.y), "d"(v.z), "d"(v.w) : "memory");
+}
+// two adjacent Real4 (a contact slot, a spring record): 32 bytes in FP32,
+// two 32-byte halves in FP64
+__device__ __forceinline__ void ld_pair(const float4* p, float4& a, float4& b) {
+    asm volatile("ld.global.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w)
+                 : "l"(p));
+}
+__device__ __forceinline__ void ld_pair(const double4* p, double4& a, double4& b) {
+    a = ld32(p);
+    b = ld32(p + 1);
+}
+__device__ __forceinline__ void st_pair(float4* p, float4 a, float4 b) {
+    asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "f"(a.x), "f"(a.y), "f"(a.z),
+                 "f"(a.w), "f"(b.x), "f"(b.y), "f"(b.z), "f"(b.w)
+                 : "memory");
+}
+__device__ __forceinline__ void st_pair(double4* p, double4 a, double4 b) {
+    st32(p, a);
+    st32(p + 1, b);
+}
+
+// The integrator's sums of products with their rounding written out: which
+// product of a sum is fused is otherwise the compiler's choice, and changes
+// with the code around it; a bed's trajectory should not change with it.
+__device__ __forceinline__ double fma2(double a, double b, double c, double d) {   // a b + c d
+    return __fma_rn(a, b, __dmul_rn(c, d));
+}
+__device__ __forceinline__ double fma3(double a, double b, double c, double d, double e, double f) {   // a b + c d + e f
+    return __fma_rn(e, f, fma2(a, b, c, d));
+}
+
 // body->world rotation (Quat2IvDCM, src/type.h:238-250) applied to u
-__host__ __device__ __forceinline__ V3<double> rot_b2w(double4 q, V3<double> u) {
-    double m00 = q.x * q.x - q.y * q.y - q.z * q.z + q.w * q.w;
-    double m10 = 2.0 * (q.x * q.y + q.z * q.w);
-    double m20 = 2.0 * (q.x * q.z - q.y * q.w);
-    double m01 = 2.0 * (q.x * q.y - q.z * q.w);
-    double m11 = -q.x * q.x + q.y * q.y - q.z * q.z + q.w * q.w;
-    double m21 = 2.0 * (q.y * q.z + q.x * q.w);
-    double m02 = 2.0 * (q.x * q.z + q.y * q.w);
-    double m12 = 2.0 * (q.y * q.z - q.x * q.w);
-    double m22 = -q.x * q.x - q.y * q.y + q.z * q.z + q.w * q.w;
-    return {m00 * u.x + m01 * u.y + m02 * u.z, m10 * u.x + m11 * u.y + m12 * u.z,
-            m20 * u.x + m21 * u.y + m22 * u.z};
+__device__ __forceinline__ V3<double> rot_b2w(double4 q, V3<double> u) {
+    const double m00 = __fma_rn(q.w, q.w, fma3(q.x, q.x, -q.y, q.y, -q.z, q.z));
+    const double m11 = __fma_rn(q.w, q.w, fma3(-q.x, q.x, q.y, q.y, -q.z, q.z));
+    const double m22 = __fma_rn(q.w, q.w, fma3(-q.x, q.x, -q.y, q.y, q.z, q.z));
+    const double m10 = 2.0 * fma2(q.x, q.y, q.z, q.w), m01 = 2.0 * fma2(q.x, q.y, -q.z, q.w);
+    const double m20 = 2.0 * fma2(q.x, q.z, -q.y, q.w), m02 = 2.0 * fma2(q.x, q.z, q.y, q.w);
+    const double m21 = 2.0 * fma2(q.y, q.z, q.x, q.w), m12 = 2.0 * fma2(q.y, q.z, -q.x, q.w);
+    return {fma3(m00, u.x, m01, u.y, m02, u.z), fma3(m11, u.y, m10, u.x, m12, u.z),
+            fma3(m20, u.x, m21, u.y, m22, u.z)};
 }
 // world->body rotation (Quat2DCM, src/type.h:223-236) applied to u
-__host__ __device__ __forceinline__ V3<double> rot_w2b(double4 q, V3<double> u) {
-    double m00 = q.x * q.x - q.y * q.y - q.z * q.z + q.w * q.w;
-    double m10 = 2.0 * (q.x * q.y - q.z * q.w);
-    double m20 = 2.0 * (q.x * q.z + q.y * q.w);
-    double m01 = 2.0 * (q.x * q.y + q.z * q.w);
-    double m11 = -q.x * q.x + q.y * q.y - q.z * q.z + q.w * q.w;
-    double m21 = 2.0 * (q.y * q.z - q.x * q.w);
-    double m02 = 2.0 * (q.x * q.z - q.y * q.w);
-    double m12 = 2.0 * (q.y * q.z + q.x * q.w);
-    double m22 = -q.x * q.x - q.y * q.y + q.z * q.z + q.w * q.w;
-    return {m00 * u.x + m01 * u.y + m02 * u.z, m10 * u.x + m11 * u.y + m12 * u.z,
-            m20 * u.x + m21 * u.y + m22 * u.z};
+__device__ __forceinline__ V3<double> rot_w2b(double4 q, V3<double> u) {
+    const double m00 = __fma_rn(q.w, q.w, fma3(q.x, q.x, -q.y, q.y, -q.z, q.z));
+    const double m11 = __fma_rn(q.w, q.w, fma3(-q.x, q.x, q.y, q.y, -q.z, q.z));
+    const double m22 = __fma_rn(q.w, q.w, fma3(-q.x, q.x, -q.y, q.y, q.z, q.z));
+    const double m10 = 2.0 * fma2(q.x, q.y, -q.z, q.w), m01 = 2.0 * fma2(q.x, q.y, q.z, q.w);
+    const double m20 = 2.0 * fma2(q.x, q.z, q.y, q.w), m02 = 2.0 * fma2(q.x, q.z, -q.y, q.w);
+    const double m21 = 2.0 * fma2(q.y, q.z, -q.x, q.w), m12 = 2.0 * fma2(q.y, q.z, q.x, q.w);
+    return {fma3(m00, u.x, m01, u.y, m02, u.z), fma3(m10, u.x, m11, u.y, m12, u.z),
+            fma3(m20, u.x, m21, u.y, m22, u.z)};
 }
 
 }  // namespace nbc
