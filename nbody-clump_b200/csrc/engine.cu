@@ -291,16 +291,12 @@ class EngineT final : public EngineBase {
     // those of them that touched at the last contact pass, over all scenes
     void contact_counts(long long* nnear, long long* ntouch) override {
         refresh_dev();
-        const int hg = read_int(h_.hgen);
         std::vector<SceneDyn> y = read_dyn_all();
-        std::vector<uint8_t> t(h_.cap);
-        copy_(t.data(), h_.touch[(hg + 1) & 1], (size_t)h_.cap, cudaMemcpyDeviceToHost);
         long long n = 0, c = 0;
         for (int s = 0; s < S_; s++) {
-            std::vector<int4> rec(y[s].nnear);
-            if (y[s].nnear)
-                copy_(rec.data(), h_.nfr + y[s].pair_off, (size_t)y[s].nnear * sizeof(int4), cudaMemcpyDeviceToHost);
-            for (const int4& e : rec) c += t[e.x] != 0;
+            std::vector<uint8_t> t(y[s].nnear);
+            copy_(t.data(), h_.touch[0] + y[s].pair_off, t.size(), cudaMemcpyDeviceToHost);
+            for (uint8_t v : t) c += v != 0;
             n += y[s].nnear;
         }
         if (nnear) *nnear = n;
@@ -425,8 +421,10 @@ class EngineT final : public EngineBase {
         SceneDyn y = read_dyn(s);
         std::vector<R4<R>> xf(y.npairs);
         std::vector<double4> xc(y.npairs);
-        copy_(xf.data(), (R4<R>*)h_.xfcn + y.pair_off, y.npairs * sizeof(R4<R>), cudaMemcpyDeviceToHost);
-        copy_(xc.data(), (double4*)h_.xcpt + y.pair_off, y.npairs * sizeof(double4), cudaMemcpyDeviceToHost);
+        if (h_.xfcn) {   // zeros where no export step has run
+            copy_(xf.data(), (R4<R>*)h_.xfcn + y.pair_off, y.npairs * sizeof(R4<R>), cudaMemcpyDeviceToHost);
+            copy_(xc.data(), (double4*)h_.xcpt + y.pair_off, y.npairs * sizeof(double4), cudaMemcpyDeviceToHost);
+        }
         std::fill(fcn, fcn + (size_t)n * bl * 3, 0.0);
         std::fill(cpt, cpt + (size_t)n * bl * 3, 0.0);
         const int p0 = rd.row[0];
@@ -461,7 +459,7 @@ class EngineT final : public EngineBase {
         if (!fcn) return;
         if (cap_in < y.npairs) throw ArgError("pair buffer too small");
         std::vector<R4<R>> xf(y.npairs);
-        copy_(xf.data(), (R4<R>*)h_.xfcn + y.pair_off, y.npairs * sizeof(R4<R>), cudaMemcpyDeviceToHost);
+        if (h_.xfcn) copy_(xf.data(), (R4<R>*)h_.xfcn + y.pair_off, y.npairs * sizeof(R4<R>), cudaMemcpyDeviceToHost);
         for (int p = 0; p < y.npairs; p++) {
             fcn[3 * p] = xf[p].x; fcn[3 * p + 1] = xf[p].y; fcn[3 * p + 2] = xf[p].z;
         }
@@ -737,32 +735,143 @@ class EngineT final : public EngineBase {
         // rows and work-item prefixes
         blk(h_.L[0].row, (N + S_) * sizeof(int));
         blk(h_.L[0].brow, (N + S_) * sizeof(int));
-        blk(h_.nrb, (N + S_) * sizeof(int2));
+        // near rows in the file: offsets of each subsphere's near front and
+        // near back entries, the contact slots in that order
+        std::vector<int2> nrb(N + S_);
+        std::vector<int> nro(N + S_);
+        std::vector<int2> nsl(N);
+        if (!src) {
+            copy_(nro.data(), h_.nro[0], (N + S_) * sizeof(int), cudaMemcpyDeviceToHost);
+            copy_(nsl.data(), h_.nsl, N * sizeof(int2), cudaMemcpyDeviceToHost);
+            for (int s = 0; s < S_; s++) {
+                int back = y[s].pair_off;
+                const int e = hpar_[s].sub_off + hpar_[s].nsub;
+                for (int i = hpar_[s].sub_off; i < e; i++) {
+                    nrb[i + s] = make_int2(nro[i + s], back);
+                    back += nsl[cm[i].y].y - (nro[i + s + 1] - nro[i + s]);
+                }
+                nrb[e + s] = make_int2(nro[e + s], back);
+            }
+        }
+        hblk(nrb.data(), (N + S_) * sizeof(int2));
+        if (src) {
+            for (int s = 0; s < S_; s++) {
+                int at = 2 * y[s].pair_off;
+                const int o = hpar_[s].sub_off, e = o + hpar_[s].nsub;
+                for (int i = o; i <= e; i++) nro[i + s] = nrb[i + s].x;
+                std::vector<int> row(hpar_[s].nsub);   // subsphere of each member slot
+                for (int i = o; i < e; i++) row[cm[i].y - o] = i;
+                for (int m = o; m < e; m++) {
+                    const int2 a = nrb[row[m - o] + s], b = nrb[row[m - o] + s + 1];
+                    nsl[m] = make_int2(at, (b.x - a.x) + (b.y - a.y));
+                    at += nsl[m].y;
+                    if (nsl[m].y < 0 || at > 2 * (y[s].pair_off + y[s].pcap)) throw ArgError("checkpoint of different scenes");
+                }
+            }
+            copy_(h_.nro[0], nro.data(), (N + S_) * sizeof(int), cudaMemcpyHostToDevice);
+            copy_(h_.nsl, nsl.data(), N * sizeof(int2), cudaMemcpyHostToDevice);
+            std::vector<int4> lr(2 * 32 * (size_t)h_.W);
+            copy_(lr.data(), h_.lrec, lr.size() * sizeof(int4), cudaMemcpyDeviceToHost);
+            std::vector<int2> mo(N);
+            copy_(mo.data(), h_.mo, N * sizeof(int2), cudaMemcpyDeviceToHost);
+            for (int k = 0; k < K_; k++)
+                for (int m = mstart_[k]; m < std::min(mstart_[k + 1], mstart_[k] + 32); m++) {
+                    int4* r = &lr[2 * (size_t)(clane_[k] + m - mstart_[k])];
+                    r[0].x = mo[m].x; r[0].y = mo[m].y;
+                    r[1].y = nsl[mo[m].y].x; r[1].z = nsl[mo[m].y].y;
+                }
+            copy_(h_.lrec, lr.data(), lr.size() * sizeof(int4), cudaMemcpyHostToDevice);
+        }
         blk(h_.nprefix, (S_ + 1) * sizeof(int));
         blk(h_.bprefix, (S_ + 1) * sizeof(int));
         blk(h_.ring, (size_t)S_ * ring_len_ * 6 * sizeof(double));
-        // each scene's pair region: the history generation the next contact
-        // pass reads is (hgen + 1) & 1 (k_clump advances hgen first)
-        const int g = (hd.hgen + 1) & 1;
+        // each scene's pair region; springs, touch and near flags per listed
+        // pair in the file, per near pair here
         const size_t cap = h_.cap;
         for (int s = 0; s < S_; s++) {
             const size_t o = y[s].pair_off, np = y[s].npairs, nn = y[s].nnear;
+            if (src && (np > (size_t)y[s].pcap || nn > np || o + np > cap)) throw ArgError("checkpoint of different scenes");
             blk(h_.L[0].nbr + o, np * sizeof(int));
             blk(h_.L[0].own + o, np * sizeof(int));
             blk(h_.L[0].bnbr + o, np * sizeof(int));
             blk(h_.L[0].bpair + o, np * sizeof(int));
-            R4<R>* H = (R4<R>*)h_.H[g];
-            blk(H + 2 * o, 2 * np * sizeof(R4<R>));
-            blk((R*)(H + 2 * cap) + o, np * sizeof(R));
-            blk(h_.touch[g] + o, np);
-            blk(h_.nearf + o, np);
-            blk(h_.nbpos + o, np * sizeof(int));
-            blk(h_.nfr + o, nn * sizeof(int4));
-            blk(h_.nbq + o, nn * sizeof(int));
-            R4<R>* fs = (R4<R>*)h_.nfs;
-            R4<R>* bs = (R4<R>*)h_.nbs;
-            blk(fs + 2 * o, 2 * nn * sizeof(R4<R>));
-            blk(bs + 2 * o, 2 * nn * sizeof(R4<R>));
+            std::vector<R4<R>> hf(2 * np), hn(2 * nn), fs(2 * nn), bs(2 * nn), sl(4 * nn);
+            std::vector<R> zf(np), zn(nn);
+            std::vector<uint8_t> tf(np), tn(nn), nf(np);
+            std::vector<int> pos(np, -1), nbq(nn), pr(nn);
+            std::vector<int4> nfr(nn), rec(2 * nn);
+            R4<R>* H = (R4<R>*)h_.H[0];
+            R4<R>* S = (R4<R>*)h_.slots;
+            if (!src) {
+                std::vector<int> brow(hpar_[s].nsub + 1), bpair(np);
+                copy_(hn.data(), H + 2 * o, 2 * nn * sizeof(R4<R>), cudaMemcpyDeviceToHost);
+                copy_(zn.data(), (R*)(H + 2 * cap) + o, nn * sizeof(R), cudaMemcpyDeviceToHost);
+                copy_(tn.data(), h_.touch[0] + o, nn, cudaMemcpyDeviceToHost);
+                copy_(pr.data(), h_.np[0] + o, nn * sizeof(int), cudaMemcpyDeviceToHost);
+                copy_(rec.data(), h_.rec[0] + 2 * o, 2 * nn * sizeof(int4), cudaMemcpyDeviceToHost);
+                copy_(sl.data(), S + 4 * o, 4 * nn * sizeof(R4<R>), cudaMemcpyDeviceToHost);
+                copy_(brow.data(), h_.L[0].brow + hpar_[s].sub_off + s, brow.size() * sizeof(int), cudaMemcpyDeviceToHost);
+                copy_(bpair.data(), h_.L[0].bpair + o, np * sizeof(int), cudaMemcpyDeviceToHost);
+                for (size_t w = 0; w < nn; w++) nf[pr[w] - o] = 1;
+                size_t e = 0;
+                for (int k = brow.front(); k < brow.back(); k++) {
+                    const int q = bpair[k - o];
+                    if (q < 0 || !nf[q - o] || e >= nn) continue;
+                    pos[q - o] = (int)(o + e);
+                    nbq[e++] = q;
+                }
+                for (size_t w = 0; w < nn; w++) {
+                    const size_t p = pr[w] - o;
+                    const int4 a = rec[2 * w], b = rec[2 * w + 1];
+                    nfr[w] = make_int4(pr[w], a.y, a.x, pos[p]);
+                    tf[p] = tn[w];
+                    if (tn[w]) { hf[2 * p] = hn[2 * w]; hf[2 * p + 1] = hn[2 * w + 1]; zf[p] = zn[w]; }
+                    for (int c = 0; c < 2; c++) {
+                        fs[2 * w + c] = sl[2 * (b.z - 2 * o) + c];
+                        if (pos[p] >= 0) bs[2 * (pos[p] - o) + c] = sl[2 * (b.w - 2 * o) + c];
+                    }
+                }
+            }
+            hblk(hf.data(), 2 * np * sizeof(R4<R>));
+            hblk(zf.data(), np * sizeof(R));
+            hblk(tf.data(), np);
+            hblk(nf.data(), np);
+            hblk(pos.data(), np * sizeof(int));
+            hblk(nfr.data(), nn * sizeof(int4));
+            hblk(nbq.data(), nn * sizeof(int));
+            hblk(fs.data(), 2 * nn * sizeof(R4<R>));
+            hblk(bs.data(), 2 * nn * sizeof(R4<R>));
+            if (src) {
+                const int lo = hpar_[s].sub_off, hi = lo + hpar_[s].nsub;
+                for (size_t w = 0; w < nn; w++) {
+                    const int4 v = nfr[w];
+                    const size_t p = (size_t)((long long)v.x - (long long)o);
+                    if (p >= np || v.y < lo || v.y >= hi || v.z < lo || v.z >= hi) throw ArgError("checkpoint of different scenes");
+                    const int2 ci = cm[v.z], cj = cm[v.y];
+                    const int2 ri = nrb[v.z + s], rj = nrb[v.y + s], rj1 = nrb[v.y + s + 1];
+                    const int sf = nsl[ci.y].x + (int)(o + w) - ri.x;
+                    // the partner's near back entry, behind its near front entries (-1: it has none)
+                    const int e = v.w, own = e >= rj.y && e < rj1.y && nbq[e - o] == v.x;
+                    const int sb = own ? nsl[cj.y].x + (rj1.x - rj.x) + (e - rj.y) : -1;
+                    if (sf < 2 * (int)o || sf >= 2 * (int)(o + nn) || sb >= 2 * (int)(o + nn))
+                        throw ArgError("checkpoint of different scenes");
+                    rec[2 * w] = make_int4(v.z, v.y, ci.y, cj.y);
+                    rec[2 * w + 1] = make_int4(ci.x, cj.x, sf, sb);
+                    pr[w] = v.x;
+                    tn[w] = tf[p];
+                    hn[2 * w] = hf[2 * p]; hn[2 * w + 1] = hf[2 * p + 1]; zn[w] = zf[p];
+                    for (int c = 0; c < 2; c++) {
+                        sl[2 * (sf - 2 * o) + c] = fs[2 * w + c];
+                        if (sb >= 0) sl[2 * (sb - 2 * o) + c] = bs[2 * (e - o) + c];
+                    }
+                }
+                copy_(H + 2 * o, hn.data(), 2 * nn * sizeof(R4<R>), cudaMemcpyHostToDevice);
+                copy_((R*)(H + 2 * cap) + o, zn.data(), nn * sizeof(R), cudaMemcpyHostToDevice);
+                copy_(h_.touch[0] + o, tn.data(), nn, cudaMemcpyHostToDevice);
+                copy_(h_.np[0] + o, pr.data(), nn * sizeof(int), cudaMemcpyHostToDevice);
+                copy_(h_.rec[0] + 2 * o, rec.data(), 2 * nn * sizeof(int4), cudaMemcpyHostToDevice);
+                copy_(S + 4 * o, sl.data(), 4 * nn * sizeof(R4<R>), cudaMemcpyHostToDevice);
+            }
         }
         if (src && off != src->size()) throw ArgError("checkpoint has trailing bytes");
     }
@@ -786,6 +895,8 @@ class EngineT final : public EngineBase {
     char* pslab_ = nullptr;  // the pair buffers' slab
     int4* relmap_ = nullptr; // [S] region moves of a re-layout
     size_t pslab_bytes_ = 0;
+    char* xslab_ = nullptr;  // the export step's per-pair buffers (null until one runs)
+    size_t xslab_bytes_ = 0;
     cudaStream_t stream_ = nullptr;
     cudaStream_t stream2_ = nullptr;   // second branch of a step: k_boundary beside k_pairs
     cudaEvent_t ev_fork_ = nullptr, ev_join_ = nullptr;
@@ -797,7 +908,7 @@ class EngineT final : public EngineBase {
     bool sphere_kin_ = false;   // some scene runs the sphere drivers' kinematics (Dev::fint)
     bool has_kinds_ = false;    // some scene has split-driver body kinds (Dev::kind)
     bool first_list_ = true;
-    int search_lanes_ = 8;
+    int search_lanes_ = 8;   // as given; the search has its own (SEARCH_G)
     int clump_batch_ = 1;    // as given; the clump pass has one member per lane whatever it says
     int pair_bps_ = 12;      // blocks per SM of the pair kernel's grid
     int sm_count_ = 148;
@@ -807,7 +918,7 @@ class EngineT final : public EngineBase {
     // the engine's clump order (see clump_order): the caller's number within
     // its scene of each clump, the first member slot and the clump of each
     // member slot, and the member slot of each of the caller's subspheres
-    std::vector<int> cold_, mstart_, mcl_, mrow_;
+    std::vector<int> cold_, mstart_, mcl_, mrow_, clane_;   // clane_: first lane in Dev::lrec
     int* hflag_ = nullptr;  // pinned
     int steps_done_ = 0;
     int pend_ = 0, pend_eager_ = 0, pend_before_ = 0;  // steps enqueued and not yet waited for
@@ -849,11 +960,10 @@ class EngineT final : public EngineBase {
         return n;
     }
     // kernels one rebuild launches (launch_rebuild)
-    // kernels of one rebuild in a graph (the eager path adds a k_check_cap):
-    // plan, hash, the cell counts' scan, scatter, per-cell order and table,
-    // reorder, search, scan, check, compact, (hgrid: xsort), backref, carry,
-    // write-back, 2 near-row passes and their scan, the finishing pass
-    int rebuild_launches() const { return 17 + (hgrid_ ? 1 : 0); }
+    // kernels of one rebuild in a graph (the eager path adds a k_need): plan,
+    // hash, the cell counts' scan, scatter, order, search, the rows' scan,
+    // fill, rows, commit
+    int rebuild_launches() const { return 10; }
     cudaEvent_t* next_record() {
         if ((size_t)(NMARK * (ev_used_ + 1)) > ev_.size()) {
             for (int k = 0; k < 64 * NMARK; k++) {
@@ -979,6 +1089,7 @@ class EngineT final : public EngineBase {
                 P.box_lo[a] = D.box_lo[a];
                 P.box_hi[a] = D.box_hi[a];
             }
+            P.lrmax[0] = (float)rmax * 1.000001f;
             P.levels = D.levels > 1 ? D.levels : 1;
             if (P.levels > 1) hgrid_ = true;
             if (P.levels > MAX_LEVELS) throw ArgError("too many grid levels");
@@ -988,6 +1099,11 @@ class EngineT final : public EngineBase {
                 int off = 0;
                 for (int l = 0; l < P.levels; l++) {
                     P.lcell[l] = D.level_cell[l];
+                    P.licell[l] = 1.0 / P.lcell[l];
+                    double rl = 0;
+                    for (int i = 0; i < D.n_sub; i++)
+                        if (D.level[i] == l) rl = std::max(rl, D.radius[i]);
+                    P.lrmax[l] = (float)rl * 1.000001f;
                     for (int a = 0; a < 3; a++)
                         P.ldim[l][a] = (int)std::ceil((D.world_size[a] + 2 * mesh) / P.lcell[l]);
                     P.loff[l] = off;
@@ -1078,7 +1194,7 @@ class EngineT final : public EngineBase {
         // host arrays: subspheres in the input order, clumps in the engine's
         std::vector<double4> posr(N_), lom(N_);
         std::vector<int> fix(N_), lev(N_, 0), sid(N_), csid(K_);
-        std::vector<int2> cm(N_), mo(N_);
+        std::vector<int2> cm(N_);
         std::vector<double4> cpos(K_), cvel(K_), cw(K_), cq(K_), cprop(K_);
         std::vector<int> kind(has_kinds_ ? K_ : 0, 0);
         cold_.resize(K_);
@@ -1129,7 +1245,6 @@ class EngineT final : public EngineBase {
                 for (int i = 0; i < D.n_sub; i++) {
                     const int g = hpar_[s].sub_off + i, k = cm[g].x, m = cur[k]++;
                     cm[g].y = m;
-                    mo[m] = make_int2(g, m);
                     mcl_[m] = k;
                     mrow_[g] = m;
                 }
@@ -1139,19 +1254,16 @@ class EngineT final : public EngineBase {
         // the clump pass's lanes: whole clumps packed into warps, a lane per
         // member (a clump of more than 32 has a warp of its own, one without
         // members a lane)
-        std::vector<int4> ltab;
-        ltab.reserve((size_t)N_ + N_ / 4 + 32);
-        for (int s = 0; s < S_; s++)
-            for (int k = hpar_[s].clump_off; k < hpar_[s].clump_off + hpar_[s].nclump; k++) {
-                const int nm = mstart_[k + 1] - mstart_[k], lanes = std::min(std::max(nm, 1), 32);
-                while (ltab.size() % 32 + lanes > 32) ltab.push_back(make_int4(-1, -1, 0, 0));
-                const int head = (int)(ltab.size() % 32);
-                for (int q = 0; q < lanes; q++)
-                    ltab.push_back(make_int4(nm ? mstart_[k] + q : -1, k, nm << 5 | head, s));
-                while (nm > 32 && ltab.size() % 32) ltab.push_back(make_int4(-1, -1, 0, 0));
-            }
-        while (ltab.size() % 32) ltab.push_back(make_int4(-1, -1, 0, 0));
-        h_.W = (int)(ltab.size() / 32);
+        clane_.resize(K_);
+        size_t lanes = 0;
+        for (int k = 0; k < K_; k++) {
+            const int nm = mstart_[k + 1] - mstart_[k], n = std::min(std::max(nm, 1), 32);
+            if (lanes % 32 + n > 32) lanes = (lanes + 31) / 32 * 32;
+            clane_[k] = (int)lanes;
+            lanes += n;
+            if (nm > 32) lanes = (lanes + 31) / 32 * 32;
+        }
+        h_.W = cdiv(lanes, 32);
 
         // device allocation: the per-subsphere and per-clump buffers in one
         // slab, the pair buffers (which grow) in another
@@ -1176,7 +1288,7 @@ class EngineT final : public EngineBase {
             h_.cpos = m.take<double4>(K_); h_.cvel = m.take<double4>(K_); h_.cw = m.take<double4>(K_);
             h_.cq = m.take<double4>(K_); h_.cprop = m.take<double4>(K_);
             h_.cinv = m.take<double4>(K_);
-            h_.ltab = m.take<int4>(ltab.size());
+            h_.lrec = m.take<int4>(2 * 32 * (size_t)h_.W); h_.clane = m.take<int>(K_);
             h_.cold = m.take<int>(K_); h_.stage = m.take<double4>(K_);
             h_.cF = m.take<double4>(K_); h_.cT = m.take<double4>(K_);
             h_.mem_start = m.take<int>(K_ + 1);
@@ -1192,35 +1304,35 @@ class EngineT final : public EngineBase {
             h_.lstep = flags + 7;
             h_.loop_left = flags + 8;
             h_.scan_fail = flags + 9;
-            h_.kA = m.take<int>(N); h_.vA = m.take<int>(N); h_.kB = m.take<int>(N); h_.vB = m.take<int>(N);
+            h_.kA = m.take<int>(N); h_.vA = m.take<int>(N); h_.vB = m.take<int>(N);
+            h_.posf = m.take<float4>(N);
             h_.ccnt = m.take<int>((size_t)cells + S_ + 1);
-            h_.ccur = m.take<int>((size_t)cells + S_ + 1);
             h_.perm = m.take<int>(N);
             h_.inv = m.take<int>(N);
             h_.cstart = m.take<int>(cells + 1);
-            h_.scr = m.take<int>((size_t)N * 2 * SCR_CAP);
-            h_.cnt_f = m.take<int>(N + 1);
-            h_.nrb = m.take<int2>(N + S_);
+            h_.scr = m.take<int>((size_t)N * SCR_CAP);
+            h_.rlong = m.take<uint8_t>(N);
+            h_.cnt_f = m.take<int>(N + 1); h_.cnt_b = m.take<int>(N + 1); h_.cnt_nf = m.take<int>(N + 1);
+            h_.cnt_ns = m.take<int>(N + 1); h_.xcnt = m.take<int>(N + 1);
+            h_.fcur = m.take<int>(N);
+            h_.nsl = m.take<int2>(N);
             h_.nprefix = m.take<int>(S_ + 1);
             h_.bidx = m.take<int>(N);
             h_.bprefix = m.take<int>(S_ + 1);
-            h_.cnt_b = m.take<int>(N + 1);
-            h_.sfc = m.take<int>(N);
-            h_.xcnt = m.take<int>(N + 1);
             const long long scan_tiles = std::max(cdiv(N + 1, SC_TILE), cdiv((long long)cells + S_ + 1, SC_TILE));
             h_.scan_tmp = m.take<int>(scan_tiles + 1);
-            h_.scan_st = m.take<unsigned long long>(3 * scan_tiles + 3);
+            h_.scan_st = m.take<unsigned long long>(5 * scan_tiles + 5);
             h_.scan_ctl = m.take<int>(2);
             for (int l = 0; l < 2; l++) {
                 h_.L[l].row = m.take<int>(N + S_);
                 h_.L[l].brow = m.take<int>(N + S_);
+                h_.nro[l] = m.take<int>(N + S_);
             }
             h_.plan = m.take<int>(PL_SIZE);
             h_.pscene = m.take<int>(S_);
             h_.psub = m.take<int>(S_ + 1);
             h_.pcell = m.take<int>(S_ + 1);
             h_.pclump = m.take<int>(S_ + 1);
-            h_.ppair = m.take<int>(S_ + 1);
             h_.need = m.take<int>(S_);
             relmap_ = m.take<int4>(S_);
             h_.xparts = m.take<R4<R>>(6 * N);
@@ -1270,14 +1382,17 @@ class EngineT final : public EngineBase {
             for (int k = 0; k < K_; k++)
                 cinv[k] = make_double4(1.0 / cprop[k].x, 1.0 / cprop[k].y, 1.0 / cprop[k].z, 1.0 / cprop[k].w);
             clumps_in(cinv, h_.cinv);
-            copy_(h_.ltab, ltab.data(), ltab.size() * sizeof(int4), cudaMemcpyHostToDevice);
         }
+        copy_(h_.clane, clane_.data(), K_ * sizeof(int), cudaMemcpyHostToDevice);
         copy_(h_.mem_start, mstart_.data(), (K_ + 1) * sizeof(int), cudaMemcpyHostToDevice);
-        copy_(h_.mo, mo.data(), N * sizeof(int2), cudaMemcpyHostToDevice);
         // the first list is empty: rows of zeros (the slab is zeroed)
         int one = 1;
         copy_(h_.any_rebuild, &one, sizeof(int), cudaMemcpyHostToDevice);
         push_dev();
+        const int g = std::min(cdiv(std::max(N_, 32 * h_.W), 256), sm_count_ * 8);
+        k_members_init<<<g, 256, 0, stream_>>>(d_);
+        k_lanes_init<<<g, 256, 0, stream_>>>(d_);
+        CK(cudaGetLastError());
     }
 
     void alloc_pairs(long long cap) {
@@ -1291,16 +1406,17 @@ class EngineT final : public EngineBase {
                 h_.L[l].bpair = m.take<int>(cap);
                 h_.H[l] = m.take<char>(hist_bytes(cap));
                 h_.touch[l] = m.take<uint8_t>(cap);
+                h_.rec[l] = m.take<int4>(2 * cap);
+                h_.np[l] = m.take<int>(cap);
             }
-            h_.nfs = m.take<R4<R>>(2 * cap);
-            h_.nbs = m.take<R4<R>>(2 * cap);
-            h_.nbpos = m.take<int>(cap);
-            h_.nfr = m.take<int4>(cap);
-            h_.nbq = m.take<int>(cap);
-            h_.nearf = m.take<uint8_t>(cap);
-            h_.xfcn = m.take<R4<R>>(cap);
-            h_.xcpt = m.take<double4>(cap);
+            h_.slots = m.take<R4<R>>(4 * cap);
+            h_.tmp = m.take<int2>(cap);
+            h_.bslot = m.take<int>(cap);
         };
+        // the export step's pair buffers are made when one runs
+        if (xslab_) mem_.release(xslab_, xslab_bytes_);
+        xslab_ = nullptr;
+        h_.xfcn = h_.xcpt = nullptr;
         Carver sz;
         layout(sz);
         pslab_bytes_ = sz.off;
@@ -1308,13 +1424,28 @@ class EngineT final : public EngineBase {
         Carver m{(uintptr_t)pslab_};
         layout(m);
     }
+    void alloc_export() {
+        if (xslab_) return;
+        refresh_dev();
+        auto layout = [&](Carver& m) {
+            h_.xfcn = m.take<R4<R>>(h_.cap);
+            h_.xcpt = m.take<double4>(h_.cap);
+        };
+        Carver sz;
+        layout(sz);
+        xslab_bytes_ = sz.off;
+        xslab_ = mem_.alloc<char>(xslab_bytes_);
+        Carver m{(uintptr_t)xslab_};
+        layout(m);
+        push_dev();
+    }
     static size_t hist_bytes(long long cap) { return (size_t)cap * (2 * sizeof(R4<R>) + sizeof(R)); }
 
     double slack() const { return opt_.pair_slack >= 1.0 ? opt_.pair_slack : 1.6; }
     // Bytes of the pair buffers per pair slot.
     static double bytes_per_pair() {
-        return 2.0 * (4 * sizeof(int) + (double)hist_bytes(1) + 1) + 5 * sizeof(R4<R>) + sizeof(double4) +
-               2 * sizeof(int) + sizeof(int4) + 1;
+        return 2.0 * (5 * sizeof(int) + (double)hist_bytes(1) + 1 + 2 * sizeof(int4)) + 4 * sizeof(R4<R>) +
+               sizeof(int2) + sizeof(int);
     }
     // Region capacities for the first lists: slack x each scene's pairs; with
     // the default slack at least the reference's own list capacity, n_sub x
@@ -1357,10 +1488,9 @@ class EngineT final : public EngineBase {
         return y;
     }
     // New pair regions of the given capacities: the pair buffers are
-    // re-allocated and every scene's current list, the history generation
-    // the next contact pass reads, touch and near flags move to its new
-    // region (rows shifted).  The build list and the other generation need
-    // nothing: a rebuild writes them before reading.
+    // re-allocated and every scene's current list, work records, histories
+    // and touch flags move to its new region (rows shifted).  The build
+    // buffers need nothing: a rebuild writes them before reading.
     void layout_pairs(const std::vector<long long>& pcap) {
         refresh_dev();
         std::vector<SceneDyn> y = read_dyn_all();
@@ -1378,7 +1508,6 @@ class EngineT final : public EngineBase {
             total += pcap[s];
             if (total > 2000000000LL) throw CudaError("pair capacity above 2^31");
         }
-        const int hg = read_int(h_.hgen);
         Dev old = h_;
         char* old_slab = pslab_;
         const size_t old_bytes = pslab_bytes_;
@@ -1388,9 +1517,7 @@ class EngineT final : public EngineBase {
         push_dev();
         const int B = 256;
         if (moved > 0)
-            k_relayout<R><<<std::min(148 * 8, cdiv(moved, B)), B, 0, stream_>>>(
-                d_, old.L[0], old.H[hg & 1], old.touch[hg & 1], old.nearf, old.nfr, old.nbq, old.nbpos, old.cap,
-                relmap_, moved);
+            k_relayout<R><<<std::min(148 * 8, cdiv(moved, B)), B, 0, stream_>>>(d_, old, relmap_, moved);
         k_shift_rows<<<std::min(148 * 8, cdiv((long long)N_ + S_, B)), B, 0, stream_>>>(d_, relmap_);
         CK(cudaGetLastError());
         CK(cudaStreamSynchronize(stream_));
@@ -1482,6 +1609,7 @@ class EngineT final : public EngineBase {
     // captured), then k_sum
     void launch_contact(bool exp) {
         if (exp) {
+            alloc_export();
             CK(cudaMemsetAsync(h_.xfcn, 0, (size_t)h_.cap * sizeof(R4<R>), stream_));
             CK(cudaMemsetAsync(h_.xcpt, 0, (size_t)h_.cap * sizeof(double4), stream_));
             // wall and intruder parts: k_boundary writes its candidates only
@@ -1523,14 +1651,16 @@ class EngineT final : public EngineBase {
         else k_sum<R, false><<<cdiv(N_, CT_THREADS), CT_THREADS, 0, stream_>>>(d_);
         CK(cudaGetLastError());
     }
-    // exclusive scans of a0 (and a1, a2, of the same length) over [0, n), or
-    // over [0, *dn) when dn is given (n then bounds it), in one launch
-    void scan(int* a0, int* a1, int* a2, int n, const int* dn = nullptr) {
+    // exclusive scans of arrays of the same length over [0, n), or over
+    // [0, *dn) when dn is given (n then bounds it), in one launch
+    void scan(std::initializer_list<int*> arrays, int n, const int* dn = nullptr) {
+        ScanArrays a{};
+        for (int* p : arrays) a.a[a.n++] = p;
         // a grid of at most a few blocks per SM takes the tiles; a grid sized
         // for the largest length would start tens of thousands of blocks that
         // find nothing to do when few scenes are rebuilt
-        const int nb = std::min(std::max(1, cdiv(n, SC_TILE)) * (a2 ? 3 : (a1 ? 2 : 1)), sm_count_ * 4);
-        k_scan1<<<nb, SC_THREADS, 0, stream_>>>(a0, a1, a2, n, dn, h_.scan_st, h_.scan_ctl, h_.halt, h_.scan_fail);
+        const int nb = std::min(std::max(1, cdiv(n, SC_TILE)) * a.n, sm_count_ * 4);
+        k_scan1<<<nb, SC_THREADS, 0, stream_>>>(a, n, dn, h_.scan_st, h_.scan_ctl, h_.halt, h_.scan_fail);
     }
     // The rebuild block of src/dem_simulation_clump.cu:124-176, over the
     // scenes whose rebuild flag is set: every kernel but the near rows walks
@@ -1538,26 +1668,20 @@ class EngineT final : public EngineBase {
     // device), so a batch pays for the scenes it rebuilds.
     void launch_rebuild(bool eager) {
         const int B = 128;
-        const int gN = std::min(cdiv(N_, B), 148 * 16);         // grid-stride grids
-        const int sl = search_lanes_;
-        const int gS = std::min(cdiv(N_, SEARCH_THREADS / sl), 148 * 16);
+        const int gN = std::min(cdiv(N_ + 1, B), sm_count_ * 16);         // grid-stride grids
         const int* pl = h_.plan;
         k_plan<<<1, SC_THREADS, 0, stream_>>>(d_);
         k_hash<<<gN, B, 0, stream_>>>(d_);
-        // counting sort by cell: the counts' scan, the scatter, each cell's
-        // range in subsphere order with the permutation and the cell table
-        scan(h_.ccnt, nullptr, nullptr, h_.cells + S_ + 1, pl + PL_TC1);
+        scan({h_.ccnt}, h_.cells + S_ + 1, pl + PL_TC1);
         k_cscatter<<<gN, B, 0, stream_>>>(d_);
-        k_cellfix<<<std::min(cdiv(h_.cells + S_, 256), 148 * 16), 256, 0, stream_>>>(d_);
-        k_reorder<R><<<gN, B, 0, stream_>>>(d_);
-        if (sl == 16) k_search<16><<<gS, SEARCH_THREADS, 0, stream_>>>(d_);
-        else if (sl == 32) k_search<32><<<gS, SEARCH_THREADS, 0, stream_>>>(d_);
-        else k_search<8><<<gS, SEARCH_THREADS, 0, stream_>>>(d_);
-        scan(h_.cnt_f, h_.cnt_b, nullptr, N_ + 1, pl + PL_T1);
+        k_order<R><<<gN, B, 0, stream_>>>(d_);
+        const int gS = std::min(cdiv((long long)N_ * SEARCH_G, SEARCH_THREADS), sm_count_ * 16);
+        k_search<<<gS, SEARCH_THREADS, 0, stream_>>>(d_);
+        scan({h_.cnt_f, h_.cnt_b, h_.cnt_nf, h_.cnt_ns, h_.xcnt}, N_ + 1, pl + PL_T1);
         CK(cudaGetLastError());
         if (eager) {
             // size the regions to the first lists, or grow the ones that overflow
-            k_check_cap<<<1, 256, 0, stream_>>>(d_, 0);
+            k_need<<<1, 256, 0, stream_>>>(d_);
             CK(cudaStreamSynchronize(stream_));
             check_scan();
             std::vector<int> need(S_);
@@ -1574,23 +1698,9 @@ class EngineT final : public EngineBase {
                 if (grow) layout_pairs(grown_capacities(need, y));
             }
         }
-        k_check_cap<<<1, 256, 0, stream_>>>(d_, 1);
-        if (sl == 16) k_compact<16><<<gS, SEARCH_THREADS, 0, stream_>>>(d_);
-        else if (sl == 32) k_compact<32><<<gS, SEARCH_THREADS, 0, stream_>>>(d_);
-        else k_compact<8><<<gS, SEARCH_THREADS, 0, stream_>>>(d_);
-        if (hgrid_) k_xsort<<<gN, B, 0, stream_>>>(d_);
-        k_backref<<<gN, B, 0, stream_>>>(d_);
-        const int gP = std::min(148 * 8, cdiv(8LL * N_, 256));
-        k_carry<R><<<gP, 256, 0, stream_>>>(d_);
-        k_writeback<R><<<gP, 256, 0, stream_>>>(d_);
-        // near rows and boundary candidates of the rebuilt scenes (counts and
-        // flags, their scans, rows and list with the rebuild's bookkeeping),
-        // then the work-item prefixes over the scenes
-        const int gNr = std::min(cdiv(N_, SEARCH_THREADS / 4), 148 * 16);
-        k_near<false, 4><<<gNr, SEARCH_THREADS, 0, stream_>>>(d_);
-        scan(h_.cnt_f, h_.cnt_b, h_.xcnt, N_ + 1, pl + PL_T1);
-        k_near<true, 4><<<gNr, SEARCH_THREADS, 0, stream_>>>(d_);
-        k_near_finish<<<std::min(cdiv(N_, SC_THREADS), 148 * 8), SC_THREADS, 0, stream_>>>(d_);
+        k_fill<<<gS, SEARCH_THREADS, 0, stream_>>>(d_);
+        k_rows<R><<<std::min(cdiv(8LL * N_, SEARCH_THREADS), sm_count_ * 16), SEARCH_THREADS, 0, stream_>>>(d_);
+        k_commit<R><<<S_ == 1 ? 1 : std::min(sm_count_ * 4, cdiv(8LL * N_, SC_THREADS)), SC_THREADS, 0, stream_>>>(d_);
         CK(cudaGetLastError());
     }
 

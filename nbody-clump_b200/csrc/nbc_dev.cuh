@@ -49,7 +49,8 @@ struct ScenePar {
     int cellnum;    // cells of this scene incl. the out-of-box bucket
     int cell_off;   // first global cell id of this scene
     int levels;     // 1 = single level grid
-    double lcell[MAX_LEVELS];
+    double lcell[MAX_LEVELS], licell[MAX_LEVELS];
+    float lrmax[MAX_LEVELS];                    // largest radius on each level
     int ldim[MAX_LEVELS][3];
     int loff[MAX_LEVELS];
     // ranges
@@ -77,8 +78,8 @@ struct SceneDyn {
     int npairs;                    // pairs in the current list
     int pair_off;                  // first pair slot of this scene's region of the pair buffers
     int pcap;                      // pair slots of that region (set by the host, grown on overflow)
-    int nnear;                     // near pairs of the current list (see k_near)
-    int nbound;                    // boundary candidates of the current list (see k_bflag)
+    int nnear;                     // near pairs of the current list (see k_rows)
+    int nbound;                    // boundary candidates of the current list (see bound_candidate)
     int stop;                      // steps the scene takes before it stands still (0: no limit)
     int frozen;                    // the scene took no step at the last k_clump (its stop was reached)
     long long ifix[6];             // fixed-point sums of intruder force (2^-40 N) and torque (2^-44 N m)
@@ -103,10 +104,8 @@ constexpr int PL_T = 1;      // their subspheres
 constexpr int PL_TC = 2;     // their cell-table entries
 constexpr int PL_T1 = 3;     // PL_T + 1 (scan length of the counts)
 constexpr int PL_TK = 4;     // their clumps
-constexpr int PL_CS = 5;     // work counter of k_search (subspheres claimed)
-constexpr int PL_CC = 6;     // work counter of k_compact
-constexpr int PL_TC1 = 7;    // PL_TC + 1 (scan length of the cell counts)
-constexpr int PL_SIZE = 8;
+constexpr int PL_TC1 = 5;    // PL_TC + 1 (scan length of the cell counts)
+constexpr int PL_SIZE = 6;
 
 struct Dev {
     int S, N, K;
@@ -144,9 +143,10 @@ struct Dev {
     double4* lom;     // local offset (body frame) xyz, mass
     double4* cum;     // displacement since the last rebuild
     double4* kin;     // world arm, mass (the velocities are the clump's; see Body in kernels.cuh)
-    int4* ltab;       // [32 W] lanes of the clump pass: entry of mo (-1: none), clump (-1: idle lane),
-                      // the clump's members << 5 | its first lane, scene
-    int W;            // warps of that table
+    int4* lrec;       // [32 W][2] lanes of the clump pass: subsphere (-1: none), member slot, clump (-1: idle
+                      // lane), the clump's members << 5 | its first lane; scene, first contact slot, slots
+    int* clane;       // [K] first lane of each clump in that table
+    int W;            // warps of it
     double4* cinv;    // 1/Ixx 1/Iyy 1/Izz 1/M (correctly rounded divisions, computed once)
     int* kind;        // [K] body kind of the split driver (0 free, 1 prescribed velocity, 2 fixed),
                       // read in SPH_KINDS scenes only (null when there are none)
@@ -158,14 +158,18 @@ struct Dev {
     int2* mo;         // [N] members of each clump, ascending by subsphere: subsphere, member slot
     int* post_pending;// device flag: a force pass has run whose half-kick is pending
     // broad phase scratch
-    int* kA; int* vA; int* kB; int* vB;   // radix sort ping-pong
+    int* kA; int* vA; int* vB;            // cell and arrival of each element, elements by cell (see k_hash)
+    float4* posf;     // [N] FP32 position from the scene's origin, widened cutoff (the search)
     int* perm;        // [N] old index of new slot i (part_idx_pre)
     int* inv;         // [N] new slot of old index
     int* cstart;                          // [cells+1] first sorted slot of each cell
-    int* scr;                             // [N][2][SCR_CAP] front / back scratch rows of the fused search
-    int* cnt_f; int* cnt_b;               // [N+1] counts, scanned in place
-    int* sfc;                             // [N] same-level front count (hierarchical grid)
-    int* xcnt;                            // [N] cross-level entries placed so far (hierarchical grid)
+    int* scr;                             // [N][SCR_CAP] scratch back rows of the search
+    uint8_t* rlong;                       // [N] the row is not in the scratch (see k_search)
+    // counts, scanned in place [N+1]: front and back rows, near front rows,
+    // contact slots by member slot, boundary candidates; then the front rows'
+    // fill cursors [N]
+    int* cnt_f; int* cnt_b; int* cnt_nf; int* cnt_ns; int* xcnt;
+    int* fcur;
     int* scan_tmp;                        // block sums
     unsigned long long* scan_st;          // single-launch scan: tile states (zero between scans)
     int* scan_ctl;                        // single-launch scan: ticket and finished-block counters
@@ -176,38 +180,36 @@ struct Dev {
     // concatenation of the rebuilt scenes only
     int* plan;        // [PL_SIZE] counts, see PL_*
     int* ccnt;        // [cells + S + 1] subspheres per cell of the rebuilt scenes (the sort's counts; zero at rest)
-    int* ccur;        // [cells + S + 1] fill cursors of the sort's scatter (zero at rest)
     int* pscene;      // [S] rebuilt scenes
     int* psub;        // [S+1] prefix of their subsphere counts
     int* pcell;       // [S+1] prefix of their cell-table entries (cellnum + 1)
     int* pclump;      // [S+1] prefix of their clump counts
-    int* ppair;       // [S+1] prefix of the pairs of their new lists
     int* need;        // [S] pairs of the new list of each rebuilt scene, -1 for the others
     int* halt;                            // device flag: pair capacity exceeded, kernels stand still
-    // pair lists: the current one and the one a rebuild builds (written
-    // back into the current one), histories ping-pong between steps
+    // pair lists: the current one and the one a rebuild builds (which becomes
+    // the current one, see k_commit); so too what follows for the near pairs
+    // (those that can touch before the next rebuild), in each scene's pair
+    // region in the order of the near front rows
     PairList L[2];
     int* lcur;        // index of the current list (0)
-    void* H[2];       // per pair: Real4 (Dv.xyz, Dr.x), Real4 (Dt.xyz, Dr.y) adjacent, [2*cap] Real4, then Real Dr.z [cap]
-    uint8_t* touch[2];// [cap] pair in contact at the step that wrote H
-    // contact slots, one per near row entry (see k_near), written by every
-    // contact pass (zero for a pair that does not touch) and summed by the
-    // next clump pass in row order: front entries hold the force and torque
-    // on the row's subsphere as owner, back entries as partner
-    void* nfs;        // Real4 [cap][2]: force and torque (adjacent) per near front entry
-    void* nbs;        // Real4 [cap][2]: force and torque (adjacent) per near back entry
-    int* nbpos;       // [cap] the near back entry of each near pair
-    // near rows (the entries that can touch before the next rebuild)
-    // (kept in each scene's pair region like the list: rows [N+S] with
-    // absolute slots, one row array per scene with its end entry)
-    int2* nrb;        // [N+S] near row offsets (front, back), one record per subsphere
-    int4* nfr;        // [cap] near front entries: pair slot, partner, owner, near back entry
-    int* nbq;         // [cap] near back entries: pair slot
+    int2* tmp;        // [cap] front entries being built: partner with flags, back entry
+    int* bslot;       // [cap] contact slot of each near back entry, being built
+    int* nro[2];      // [N+S] near front row offsets (absolute; one row array per scene with its end entry)
+    int4* rec[2];     // [cap][2] work records: owner, partner, their member slots; their clumps, contact slots
+                      // (partner slot -1: a front-only pair, which the partner does not list)
+    int* np[2];       // [cap] the pair slot of each near pair
+    void* H[2];       // per near pair: Real4 (Dv.xyz, Dr.x), Real4 (Dt.xyz, Dr.y) adjacent, [2*cap] Real4, then Real Dr.z [cap]
+    uint8_t* touch[2];// [cap] near pair in contact at the last step
+    // contact slots: force and torque (Real4 each) per near entry of each
+    // subsphere, in member-slot order within the scene's region [2 pair_off,
+    // 2 (pair_off + pcap)): a member's near front entries, then its near back
+    // entries; zero for a pair that does not touch
+    void* slots;      // Real4 [2 cap][2]
+    int2* nsl;        // [N] first contact slot and slots of each member slot
     int* nprefix;     // [S+1] prefix over the scenes of their near pairs (the contact pass's work items)
-    int* bidx;        // [N] boundary candidates of scene s at [sub_off, sub_off + nbound) (see k_bflag)
+    int* bidx;        // [N] boundary candidates of scene s at [sub_off, sub_off + nbound)
     int* bprefix;     // [S+1] prefix over the scenes of their boundary candidates (k_boundary's work items)
-    uint8_t* nearf;   // [cap] pair can touch before the next rebuild
-    int* hgen;        // history generation: read H[hgen&1], write H[(hgen+1)&1]
+    int* hgen;        // steps whose springs have been written (checkpoint files carry it)
     int* gstep;       // steps started by k_clump (counts steps across graph launches)
     int* kc_done;     // blocks of k_clump finished (last-block detection)
     int* lstep;       // steps started by k_clump, counted by its last block (per-scene stops)

@@ -74,6 +74,13 @@ __device__ __forceinline__ void st_pair(double4* p, double4 a, double4 b) {
     st32(p + 1, b);
 }
 
+// a 32-byte record of eight integers
+__device__ __forceinline__ void ld_rec(const int4* p, int4& a, int4& b) {
+    asm volatile("ld.global.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=r"(a.x), "=r"(a.y), "=r"(a.z), "=r"(a.w), "=r"(b.x), "=r"(b.y), "=r"(b.z), "=r"(b.w)
+                 : "l"(p));
+}
+
 // The integrator's sums of products with their rounding written out: which
 // product of a sum is fused is otherwise the compiler's choice, and changes
 // with the code around it; a bed's trajectory should not change with it.

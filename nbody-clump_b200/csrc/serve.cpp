@@ -143,7 +143,7 @@ struct Cohort {
 double estimate_bytes(const nbc_scene_desc& s, const nbc_options& o) {
     const double r = o.precision == NBC_PREC_F64 ? 8.0 : 4.0;
     const double per_sub = 1100.0 + 3 * 2 * 4 * r * 7;       // state, alternates, boundary histories
-    const double per_pair = 2 * (16 + 2 * 4 * r + r + 1) + 5 * 4 * r + 32 + 9;
+    const double per_pair = 2 * (20 + 9 * r + 1 + 32) + 16 * r + 12;
     const double cells = 2.0 * (double)s.n_sub * 4.0;          // grid table, a few ints per subsphere
     return (double)s.n_sub * per_sub + 12.0 * (double)s.n_sub * per_pair * 1.6 + cells;
 }
