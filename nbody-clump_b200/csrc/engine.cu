@@ -172,7 +172,8 @@ static void validate_scene(const nbc_scene_desc& D, int s) {
 template <typename R>
 class EngineT final : public EngineBase {
    public:
-    EngineT(const std::vector<const nbc_scene_desc*>& sc, const nbc_options& opt) : opt_(opt) { setup(sc); }
+    EngineT(const std::vector<const nbc_scene_desc*>& sc, const nbc_options& opt, bool shared_gpu)
+        : opt_(opt), shared_gpu_(shared_gpu) { setup(sc); }
     ~EngineT() override {
         for (int t = 0; t < 3; t++) {
             if (gexec_[t]) cudaGraphExecDestroy(gexec_[t]);
@@ -228,6 +229,8 @@ class EngineT final : public EngineBase {
         if (timing_ == 0 && !loop_tried_) capture_loop();
         pend_before_ = read_gstep();
         if (timing_ == 0 && gexec_loop_) {
+            n = std::min(n, ST_MAX_STEPS);
+            runs_before_ = read_int(h_.step_runs);
             launch_loop(n);
         } else {
             if (!gexec_[timing_]) capture(timing_);
@@ -241,7 +244,11 @@ class EngineT final : public EngineBase {
         if (pend_ > 0) {
             CK(cudaStreamSynchronize(stream_));
             const int started = read_gstep() - pend_before_;
-            launches_ += (1LL + CONTACT_LAUNCHES) * started + (timing_ == 0 && gexec_loop_ ? 1 : 0);
+            if (timing_ == 0 && gexec_loop_) {
+                launches_ += 1 + read_int(h_.step_runs) - runs_before_;   // k_loop_init, k_steps
+            } else {
+                launches_ += (1LL + CONTACT_LAUNCHES) * started;
+            }
             if (read_int(h_.halt)) {
                 check_scan();
                 // the last step started stopped at its rebuild: finish it on the host path
@@ -891,6 +898,7 @@ class EngineT final : public EngineBase {
 
    private:
     nbc_options opt_;
+    bool shared_gpu_;        // other engines step beside this one (see step_grid)
     DevMem mem_;
     char* pslab_ = nullptr;  // the pair buffers' slab
     int4* relmap_ = nullptr; // [S] region moves of a re-layout
@@ -921,6 +929,7 @@ class EngineT final : public EngineBase {
     std::vector<int> cold_, mstart_, mcl_, mrow_, clane_;   // clane_: first lane in Dev::lrec
     int* hflag_ = nullptr;  // pinned
     int steps_done_ = 0;
+    int runs_before_ = 0;    // launches of k_steps before the ones enqueued
     int pend_ = 0, pend_eager_ = 0, pend_before_ = 0;  // steps enqueued and not yet waited for
     bool post_done_ = false;
     double last_ms_ = 0;
@@ -1304,6 +1313,9 @@ class EngineT final : public EngineBase {
             h_.lstep = flags + 7;
             h_.loop_left = flags + 8;
             h_.scan_fail = flags + 9;
+            h_.step_phase = flags + 10;
+            h_.step_runs = flags + 11;
+            h_.step_bar = (unsigned long long*)(flags + 12);
             h_.kA = m.take<int>(N); h_.vA = m.take<int>(N); h_.vB = m.take<int>(N);
             h_.posf = m.take<float4>(N);
             h_.ccnt = m.take<int>((size_t)cells + S_ + 1);
@@ -1595,11 +1607,10 @@ class EngineT final : public EngineBase {
     }
 
     // ---- launches -------------------------------------------------------------
-    void launch_clump(int do_pre, cudaGraphConditionalHandle cond = 0, int use_cond = 0,
-                      cudaGraphConditionalHandle loop = 0, int use_loop = 0) {
+    void launch_clump(int do_pre, cudaGraphConditionalHandle cond = 0, int use_cond = 0) {
         const int g = cdiv(h_.W + cdiv(S_, 32), CL_WARPS);
-        if (sphere_any_) k_clump<R, true><<<g, CL_THREADS, 0, stream_>>>(d_, do_pre, cond, use_cond, loop, use_loop);
-        else k_clump<R, false><<<g, CL_THREADS, 0, stream_>>>(d_, do_pre, cond, use_cond, loop, use_loop);
+        if (sphere_any_) k_clump<R, true><<<g, CL_THREADS, 0, stream_>>>(d_, do_pre, cond, use_cond);
+        else k_clump<R, false><<<g, CL_THREADS, 0, stream_>>>(d_, do_pre, cond, use_cond);
         CK(cudaGetLastError());
         if (!capturing_) launches_ += 1;
     }
@@ -1781,15 +1792,15 @@ class EngineT final : public EngineBase {
         CK(cudaGraphLaunch(gexec_[timing_], stream_));
     }
 
-    // Many steps in one graph launch: a while node whose body is one step
-    // (k_clump, the rebuild under an if node, the contact pass).  The step
-    // count goes to the kernel node ahead of the loop; the last block of each
-    // step's k_clump counts it down and ends the loop at zero, or at once
-    // when a rebuild has run out of pair capacity (the host then finishes
-    // that step, as after a per-step graph).  Step graphs with timing event
-    // nodes stay one step per launch (an event node in a loop body would be
-    // overwritten by every iteration).  If the loop graph cannot be built the
-    // engine keeps launching one step per graph.
+    // Many steps in one graph launch: a while node whose body is k_steps (as
+    // many steps as go without a rebuild) and the rebuild under an if node.
+    // The step count goes to the kernel node ahead of the loop; k_steps ends
+    // the loop when it has taken them, or at once when a rebuild has run out
+    // of pair capacity (the host then finishes that step, as after a per-step
+    // graph).  Step graphs with timing event nodes stay one step per launch
+    // (an event node in a loop body would be overwritten by every iteration).
+    // If the loop graph cannot be built the engine keeps launching one step
+    // per graph.
     void capture_loop() {
         loop_tried_ = true;
         capturing_ = true;
@@ -1800,7 +1811,7 @@ class EngineT final : public EngineBase {
             CK(cudaGraphConditionalHandleCreate(&hw, graph_loop_, 1, cudaGraphCondAssignDefault));
             CK(cudaStreamBeginCaptureToGraph(stream_, graph_loop_, nullptr, nullptr, 0,
                                              cudaStreamCaptureModeThreadLocal));
-            k_loop_init<<<1, 1, 0, stream_>>>(h_.loop_left, 1);
+            k_loop_init<<<1, 1, 0, stream_>>>(h_.loop_left, h_.step_phase, h_.step_bar, 1);
             CK(cudaGetLastError());
             loop_init_node_ = last_captured_node(stream_);
             cudaGraph_t body = add_conditional(graph_loop_, hw, cudaGraphCondTypeWhile);
@@ -1809,9 +1820,8 @@ class EngineT final : public EngineBase {
             cudaGraphConditionalHandle hif;
             CK(cudaGraphConditionalHandleCreate(&hif, body, 0, cudaGraphCondAssignDefault));
             CK(cudaStreamBeginCaptureToGraph(stream_, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
-            launch_clump(1, hif, 1, hw, 1);
+            launch_steps(hif, hw);
             cudaGraph_t rbody = add_conditional(body, hif, cudaGraphCondTypeIf);
-            launch_contact(false);
             CK(cudaStreamEndCapture(stream_, &g2));
             CK(cudaStreamBeginCaptureToGraph(stream_, rbody, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
             launch_rebuild(false);
@@ -1832,6 +1842,34 @@ class EngineT final : public EngineBase {
         }
         capturing_ = false;
     }
+    // Blocks of k_steps: one per SM at most; a smaller scene gets blocks for
+    // its warps (clump pass, or about two near pairs per subsphere) at two busy
+    // warps each, so that its work spreads over the SMs (2,000 spheres in FP64,
+    // us a step: 2 warps 12.8, 8 warps 15.2, 16 warps 20.7).  Launches of
+    // engines that run beside each other have to fit the GPU together: an engine
+    // of a request server takes a block per 16 warps (8 requests of 400 to
+    // 5,000 clumps: 2 warps 47.5 ms, 16 warps 32.4, 32 warps 32.9, 64 warps 38.6).
+    int step_grid() const {
+        int per_sm = 0;
+        const void* f = sphere_any_ ? (const void*)k_steps<R, true> : (const void*)k_steps<R, false>;
+        CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, f, ST_THREADS, 0));
+        const int warps = std::max(h_.W + cdiv(S_, 32), cdiv(2LL * N_, 32));
+        return std::max(1, std::min(per_sm * sm_count_, cdiv(warps, shared_gpu_ ? 16 : 2)));
+    }
+    void launch_steps(cudaGraphConditionalHandle hif, cudaGraphConditionalHandle hw) {
+        cudaLaunchConfig_t c = {};
+        c.gridDim = dim3(step_grid());
+        c.blockDim = dim3(ST_THREADS);
+        c.stream = stream_;
+        cudaLaunchAttribute at[1];
+        at[0].id = cudaLaunchAttributeCooperative;   // the blocks wait for one another
+        at[0].val.cooperative = 1;
+        c.attrs = at;
+        c.numAttrs = 1;
+        const Dev* dp = d_;
+        if (sphere_any_) CK(cudaLaunchKernelEx(&c, k_steps<R, true>, dp, hif, hw));
+        else CK(cudaLaunchKernelEx(&c, k_steps<R, false>, dp, hif, hw));
+    }
     // a conditional node after the capture's current dependencies; returns its body
     cudaGraph_t add_conditional(cudaGraph_t graph, cudaGraphConditionalHandle h, cudaGraphConditionalNodeType type) {
         cudaStreamCaptureStatus st;
@@ -1848,8 +1886,7 @@ class EngineT final : public EngineBase {
         return cp.conditional.phGraph_out[0];
     }
     void launch_loop(int n) {
-        int* left = h_.loop_left;
-        void* args[] = {&left, &n};
+        void* args[] = {&h_.loop_left, &h_.step_phase, &h_.step_bar, &n};
         cudaKernelNodeParams kp = {};
         kp.func = (void*)k_loop_init;
         kp.gridDim = dim3(1);
@@ -1879,9 +1916,9 @@ class EngineT final : public EngineBase {
     }
 };
 
-EngineBase* make_engine(const std::vector<const nbc_scene_desc*>& sc, const nbc_options& opt) {
-    if (opt.precision == NBC_PREC_F64) return new EngineT<double>(sc, opt);
-    return new EngineT<float>(sc, opt);
+EngineBase* make_engine(const std::vector<const nbc_scene_desc*>& sc, const nbc_options& opt, bool shared_gpu) {
+    if (opt.precision == NBC_PREC_F64) return new EngineT<double>(sc, opt, shared_gpu);
+    return new EngineT<float>(sc, opt, shared_gpu);
 }
 
 }  // namespace nbc

@@ -56,6 +56,8 @@ class EngineBase {
     virtual void checkpoint_load(const char* data, size_t bytes) = 0;
 };
 
-EngineBase* make_engine(const std::vector<const nbc_scene_desc*>& scenes, const nbc_options& opt);
+// shared_gpu: other engines step at the same time (a request server's)
+EngineBase* make_engine(const std::vector<const nbc_scene_desc*>& scenes, const nbc_options& opt,
+                        bool shared_gpu = false);
 
 }  // namespace nbc

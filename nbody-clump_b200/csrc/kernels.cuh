@@ -132,14 +132,18 @@ __device__ __forceinline__ V3<double> shfl3(V3<double> v, int src) {
     return v3(__shfl_sync(0xffffffffu, v.x, src), __shfl_sync(0xffffffffu, v.y, src), __shfl_sync(0xffffffffu, v.z, src));
 }
 
-// The work of warp w of the lane table (see above); every lane of the warp
-// calls it.  SPH: the build for batches with a sphere-driver scene
+// The work of one warp of the lane table (see above); every lane of the warp
+// calls it with its record (ta: subsphere (-1: none), member slot, clump,
+// members << 5 | first lane; tb: scene, first contact slot, slots) and the
+// scene's parameters.  Returns whether the lane's subsphere has moved past its
+// rebuild threshold.  SPH: the build for batches with a sphere-driver scene
 // (ScenePar::sphere); the clump path's build carries none of that code.
-template <typename R, bool SPH>
-__device__ __forceinline__ void clump_warp(const Dev& d, int w, int do_pre, int post, int L) {
+// EARLY: the pose's records are loaded with the first ones (where registers
+// allow).
+template <typename R, bool SPH, bool EARLY>
+__device__ __forceinline__ bool clump_warp(const Dev& d, const ScenePar& P, int4 ta, int4 tb, int do_pre, int post,
+                                           int L) {
     const int lane = threadIdx.x & 31;
-    int4 ta, tb;   // subsphere (-1: none), member slot, clump, members << 5 | first lane; scene, first contact slot, slots
-    ld_rec(d.lrec + 2 * (size_t)(w * 32 + lane), ta, tb);
     const bool isc = ta.z >= 0;
     const int k = isc ? ta.z : 0, sc = tb.x;
     const int head = ta.w & 31, nm = ta.w >> 5;
@@ -147,12 +151,16 @@ __device__ __forceinline__ void clump_warp(const Dev& d, int w, int do_pre, int 
     const bool pre_k = isc && (stops ? scene_pre(d.dyn[sc], do_pre, L) : do_pre != 0);
     const bool post_k = isc && (stops ? scene_post(d.dyn[sc], post, L) : post != 0);
     // a warp whose clumps all belong to scenes standing still has no work
-    if (stops && !__any_sync(0xffffffffu, pre_k || post_k)) return;
+    if (stops && !__any_sync(0xffffffffu, pre_k || post_k)) return false;
     int2 im = make_int2(ta.x, ta.y), sl = make_int2(tb.y, tb.z);
     double4 cp = ld32(d.cpos + k), cv = ld32(d.cvel + k), cw = ld32(d.cw + k), cq = ld32(d.cq + k);
     const double4 pr = ld32(d.cinv + k);            // the reciprocals 1/I, 1/M
-    const ScenePar& P = d.par[sc];
     const double Dt = P.dt, grav = P.gravity;
+    double4 lo = make_double4(0, 0, 0, 0), c = lo;
+    if (EARLY && im.x >= 0) {
+        lo = ld32(d.lom + im.y);
+        c = ld32(d.cum + im.y);
+    }
     const int most = __reduce_max_sync(0xffffffffu, nm);   // members of the warp's largest clump
     double4 ps = make_double4(0, 0, 0, 0);
     V3<double> F = v3(0.0, 0.0, 0.0), T = F;
@@ -166,7 +174,7 @@ __device__ __forceinline__ void clump_warp(const Dev& d, int w, int do_pre, int 
                 V3<R> fr, tr;
                 slot_sum<R>((const R4<R>*)d.slots + 2 * (size_t)sl.x, sl.y, fr, tr);
                 if (bb) {
-                    const R4<R>* __restrict__ fbd = (const R4<R>*)d.fbnd;
+                    const R4<R>* fbd = (const R4<R>*)d.fbnd;
                     fr = fr + xyz<R>(fbd[i]);
                     tr = tr + xyz<R>(fbd[(size_t)d.N + i]);
                 }
@@ -223,13 +231,13 @@ __device__ __forceinline__ void clump_warp(const Dev& d, int w, int do_pre, int 
         st32(d.cvel + k, cv);
         st32(d.cw + k, cw);
     }
-    if (!pre_k) return;
+    if (!pre_k) return false;
     if (SPH && (P.sphere & SPH_KIN) && nm > 0) {
         // the sphere drivers' first half-kick and attitude leave the
         // intruder out (src/dem_integrate.cu:20-21,72); one member
         const int i = im.x;
         if ((d.bbits[i] >> SLOT_INTR) & 1) {
-            const R4<R>* __restrict__ fi = (const R4<R>*)d.fint;
+            const R4<R>* fi = (const R4<R>*)d.fint;
             const R4<R> a = fi[i], b = fi[(size_t)d.N + i];
             F = F - v3((double)a.x, (double)a.y, (double)a.z);
             T = T - v3((double)b.x, (double)b.y, (double)b.z);
@@ -276,13 +284,17 @@ __device__ __forceinline__ void clump_warp(const Dev& d, int w, int do_pre, int 
     }
     // ---- the member's pose
     double thr = P.thresh;
+    bool moved = false;
     for (int c0 = 0; c0 < nm; c0 += 32) {
         if (nm > 32) {   // a warp of its own: the members once more
             if (c0 + lane >= nm) break;
             im = d.mo[d.mem_start[k] + c0 + lane];
             ps = ld32(d.posr + im.x);
         }
-        const double4 lo = ld32(d.lom + im.y), c = ld32(d.cum + im.y);
+        if (!EARLY || nm > 32) {
+            lo = ld32(d.lom + im.y);
+            c = ld32(d.cum + im.y);
+        }
         const V3<double> arm = rot_b2w(q, v3(lo.x, lo.y, lo.z));
         const V3<double> p = v3(__dadd_rn(cp.x, arm.x), __dadd_rn(cp.y, arm.y), __dadd_rn(cp.z, arm.z));
         const V3<double> cn = v3((c.x + p.x) - ps.x, (c.y + p.y) - ps.y, (c.z + p.z) - ps.z);
@@ -295,8 +307,10 @@ __device__ __forceinline__ void clump_warp(const Dev& d, int w, int do_pre, int 
             SceneDyn& y = d.dyn[sc];
             if (!*(volatile int*)&y.rebuild) atomicExch(&y.rebuild, 1);
             if (!*(volatile int*)d.any_rebuild) atomicExch(d.any_rebuild, 1);
+            moved = true;
         }
     }
+    return moved;
 }
 
 // the intruder and the step count of scene s (one thread)
@@ -345,15 +359,9 @@ __device__ __forceinline__ void scene_step(const Dev& d, int s, int do_pre, int 
 
 template <typename R, bool SPH>
 __global__ void __launch_bounds__(CL_THREADS, NBC_CLUMP_MINB) k_clump(const Dev* __restrict__ dp, int do_pre,
-                                                                      cudaGraphConditionalHandle cond, int use_cond,
-                                                                      cudaGraphConditionalHandle loop, int use_loop) {
+                                                                      cudaGraphConditionalHandle cond, int use_cond) {
     const Dev& d = *dp;
-    if (*d.halt) {
-        // a rebuild ran out of pair capacity: the host finishes that step, so
-        // a device-side step loop ends here
-        if (use_loop && blockIdx.x == 0 && threadIdx.x == 0) cudaGraphSetConditional(loop, 0u);
-        return;
-    }
+    if (*d.halt) return;   // a rebuild ran out of pair capacity: the host finishes that step
     const int post = *d.post_pending;
     const int L = *d.lstep;   // written only by the last block, after every block has read it
     if (do_pre && blockIdx.x == 0 && threadIdx.x == 0) {
@@ -362,7 +370,9 @@ __global__ void __launch_bounds__(CL_THREADS, NBC_CLUMP_MINB) k_clump(const Dev*
     }
     const int w = blockIdx.x * CL_WARPS + (threadIdx.x >> 5);
     if (w < d.W) {
-        clump_warp<R, SPH>(d, w, do_pre, post, L);
+        int4 ta, tb;
+        ld_rec(d.lrec + 2 * (size_t)(w * 32 + (threadIdx.x & 31)), ta, tb);
+        clump_warp<R, SPH, false>(d, d.par[tb.x], ta, tb, do_pre, post, L);
     } else {
         const int s = (w - d.W) * 32 + (threadIdx.x & 31);
         if (s < d.S) scene_step(d, s, do_pre, post, L);
@@ -374,11 +384,6 @@ __global__ void __launch_bounds__(CL_THREADS, NBC_CLUMP_MINB) k_clump(const Dev*
             *d.kc_done = 0;
             if (do_pre) *d.lstep = L + 1;
             if (use_cond) cudaGraphSetConditional(cond, atomicAdd(d.any_rebuild, 0) ? 1u : 0u);
-            if (use_loop) {
-                const int left = *d.loop_left - 1;
-                *d.loop_left = left;
-                cudaGraphSetConditional(loop, left > 0 ? 1u : 0u);
-            }
         }
     }
 }
@@ -434,10 +439,6 @@ static __global__ void k_lanes_init(const Dev* __restrict__ dp) {
         }
     }
 }
-
-// The steps a graph launch with a device-side step loop takes (the first
-// node of that graph; its argument is set before each launch).
-static __global__ void k_loop_init(int* __restrict__ left, int n) { *left = n; }
 
 // ===========================================================================
 // broad phase
@@ -1531,7 +1532,10 @@ __global__ void __launch_bounds__(SC_THREADS) k_commit(Dev* __restrict__ dp) {
             y.nrebuild++;
             y.rebuild = 0;
         }
-        if (threadIdx.x == 0) *d.any_rebuild = 0;
+        if (threadIdx.x == 0) {
+            *d.any_rebuild = 0;
+            *d.step_bar = 0ull;
+        }
         __syncthreads();
         int run = 0, brun = 0;
         for (int b = 0; b < d.S; b += SC_THREADS) {
@@ -1728,7 +1732,7 @@ template <typename R> struct LawOut {
 // FP32 would leave that contact's force with an error of 1e-4 of itself.  The
 // tangential, rolling and twisting parts, the histories and everything after
 // run in R.  With R = double every operation is the reference's, in its order.
-template <typename R>
+template <typename R, bool WALL>
 __device__ __forceinline__ void hm_law(const Law<R>& L, V3<double> nd, double Dn, V3<double> Vtot, V3<R> Dth,
                                        double Rij, double Mij, R cs_mult, V3<R> H, V3<R> Mr, V3<R> Mt,
                                        LawOut<R>& o) {
@@ -1745,12 +1749,12 @@ __device__ __forceinline__ void hm_law(const Law<R>& L, V3<double> nd, double Dn
     const double ERR = dot(nd, Vtot);
     const V3<double> Vnor = ERR * nd;
     const V3<R> Vtan = cvt<R>(Vtot - Vnor);
-    const V3<double> Fn = (Kn * Dn) * nd + Cn * Vnor;
+    const V3<double> Fn = fma2(mul_rn(Kn, Dn), nd, Cn, Vnor);
     const V3<R> n = cvt<R>(nd);
     o.Fn = cvt<R>(Fn);
     o.FnL = (R)len_floor(Fn);
-    V3<R> Ft = (-Ks) * (L.dt * Vtan) + Cs * Vtan + H;
-    const R FtL = len_floor(Ft);
+    V3<R> Ft = fma2(-Ks, L.dt * Vtan, Cs, Vtan) + H;
+    const R FtL = WALL && sizeof(R) == 8 ? len_floor_yx(Ft) : len_floor(Ft);
     if (FtL > o.FnL * L.mu) {
         Ft = (L.mu * o.FnL * (R(1) / FtL)) * Ft;
         o.hs = Ft;
@@ -1761,25 +1765,25 @@ __device__ __forceinline__ void hm_law(const Law<R>& L, V3<double> nd, double Dn
     const R DthL = dot(Dth, n);
     const V3<R> DthT = DthL * n;
     const V3<R> DthR = Dth - DthT;
-    V3<R> rm = Kr * DthR + Mr;
-    const R rmL = len_floor(rm);
+    V3<R> rm = fma1(Kr, DthR, Mr);
+    const R rmL = WALL ? len_floor_yx(rm) : len_floor(rm);
     const R rcap = R(0.525) * L.beta * (R)Rij * o.FnL;
     if (rmL > rcap) {
         rm = (rcap * (R(1) / rmL)) * rm;
         o.hr = rm;
     } else {
         o.hr = rm;
-        rm = rm - (Cr * (R(1) / L.dt)) * DthR;
+        rm = fma1(-(Cr * (R(1) / L.dt)), DthR, rm);
     }
-    V3<R> tm = Kt * DthT + Mt;
-    const R tmL = len_floor(tm);
+    V3<R> tm = fma1(Kt, DthT, Mt);
+    const R tmL = WALL ? len_floor_yx(tm) : len_floor(tm);
     const R tcap = R(0.65) * L.mu * L.beta * (R)Rij * o.FnL;
     if (tmL > tcap) {
         tm = (tcap * (R(1) / tmL)) * tm;
         o.ht = tm;
     } else {
         o.ht = tm;
-        tm = tm - (Ct * (R(1) / L.dt)) * DthT;
+        tm = fma1(-(Ct * (R(1) / L.dt)), DthT, tm);
     }
     o.Mr = rm;
     o.Mt = tm;
@@ -1821,28 +1825,29 @@ __device__ __forceinline__ bool pair_contact2(const Law<R>& L, R cohesion, const
                                               V3<R> H, V3<R> Mr, V3<R> Mt, V3<R>& fa, V3<R>& ta, V3<R>& tb,
                                               LawOut<R>& o, double& Ap_out, V3<double>& n_out) {
     const double dx = b.p.x - a.p.x, dy = b.p.y - a.p.y, dz = b.p.z - a.p.z;
-    const double DistS = dx * dx + dy * dy + dz * dz;
+    const double DistS = fma3(dx, dx, dy, dy, dz, dz);
     const double DistL = sqrt(DistS);
     const double Dn = a.p.w + b.p.w - DistL;
     if (!(Dn > 0.0)) return false;
     const double DistR = 1.0 / DistL;
     const V3<double> nd = v3(DistR * dx, DistR * dy, DistR * dz);
-    const double Ap = 0.50 * (a.p.w * a.p.w - b.p.w * b.p.w + DistS) * DistR;
-    const double An = DistL - Ap;
-    const double Ab = 0.50 * (b.p.w * b.p.w - a.p.w * a.p.w + DistS) * DistR;
+    const double bb = mul_rn(b.p.w, b.p.w);
+    const double Ap = mul_rn(0.50 * add_rn(fma_rn(a.p.w, a.p.w, -bb), DistS), DistR);
+    const double An = sub_rn(DistL, Ap);
+    const double Ab = mul_rn(0.50 * add_rn(fma_rn(-a.p.w, a.p.w, bb), DistS), DistR);
     const double Rij = a.p.w * b.p.w / (a.p.w + b.p.w);
     const double Mij = a.m * b.m / (a.m + b.m);
-    const V3<double> ARMa = a.arm + Ap * nd;
-    const V3<double> ARMb = b.arm - An * nd;
+    const V3<double> ARMa = fma1(Ap, nd, a.arm);
+    const V3<double> ARMb = fma1(-An, nd, b.arm);
     const V3<double> Vtot = (b.v - a.v) + (cross(b.w, ARMb) - cross(a.w, ARMa));
     const V3<R> Dth = L.dt * cvt<R>(a.w - b.w);
-    hm_law<R>(L, nd, Dn, Vtot, Dth, Rij, Mij, R(1), H, Mr, Mt, o);
+    hm_law<R, false>(L, nd, Dn, Vtot, Dth, Rij, Mij, R(1), H, Mr, Mt, o);
     const V3<R> n = cvt<R>(nd);
     const R br = L.beta * (R)Rij;
-    fa = (-o.Fn - o.Ft) + (cohesion * br * br) * n;
+    fa = fma1(cohesion * br * br, n, -o.Fn - o.Ft);
     const V3<R> nxF = cross(n, o.Ft);
-    ta = ((-(R)Ap) * nxF - o.Mr) - o.Mt;
-    tb = ((-(R)Ab) * nxF + o.Mr) + o.Mt;
+    ta = fma1(-(R)Ap, nxF, -o.Mr) - o.Mt;
+    tb = fma1(-(R)Ab, nxF, o.Mr) + o.Mt;
     Ap_out = Ap;
     n_out = nd;
     return true;
@@ -1856,14 +1861,14 @@ __device__ __forceinline__ void boundary_contact(const Law<R>& L, const Body<R>&
                                                  double Dn, V3<double> RVo, V3<double> wv, V3<double> ww,
                                                  double Rij, double Mij, R cs_mult, V3<R> H, V3<R> Mr, V3<R> Mt,
                                                  V3<R>& f, V3<R>& t, LawOut<R>& o, V3<R>& arm_out) {
-    const V3<double> Arm = (-a.arm) + Ap * nd;
+    const V3<double> Arm = fma1(Ap, nd, -a.arm);
     const V3<double> Vwall = cross(ww, RVo);
     const V3<double> Vtot = (a.v - wv) + (cross(Arm, a.w) - Vwall);
     const V3<R> Dth = L.dt * cvt<R>(a.w - ww);
-    hm_law<R>(L, nd, Dn, Vtot, Dth, Rij, Mij, cs_mult, H, Mr, Mt, o);
+    hm_law<R, true>(L, nd, Dn, Vtot, Dth, Rij, Mij, cs_mult, H, Mr, Mt, o);
     const V3<R> n = cvt<R>(nd);
     f = o.Fn + o.Ft;
-    t = ((-(R)Ap) * cross(n, o.Ft) - o.Mr) - o.Mt;
+    t = fma1(-(R)Ap, cross(n, o.Ft), -o.Mr) - o.Mt;
     arm_out = cvt<R>(Arm);
 }
 
@@ -1898,7 +1903,7 @@ constexpr int BD_THREADS = 128;
 // the build for batches with a sphere-driver scene (ScenePar::sphere); the
 // clump path's build carries none of that code.
 template <typename R, bool EXPORT, bool SPH>
-__device__ __forceinline__ void boundary_one(const Dev& d, int i, int s);
+__device__ __forceinline__ void boundary_one(const Dev& d, const ScenePar& P, int i, int s);
 
 template <typename R, bool EXPORT, bool SPH>
 __global__ void __launch_bounds__(BD_THREADS) k_boundary(const Dev* __restrict__ dp) {
@@ -1910,20 +1915,18 @@ __global__ void __launch_bounds__(BD_THREADS) k_boundary(const Dev* __restrict__
     for (int w = blockIdx.x * BD_THREADS + threadIdx.x; w < nb; w += gridDim.x * BD_THREADS) {
         // work item w: boundary candidate w - bprefix[s] of scene s
         const int s = S == 1 ? 0 : plan_find(bpre, S, w);
-        const int i = d.bidx[d.par[s].sub_off + (w - bpre[s])];
-        boundary_one<R, EXPORT, SPH>(d, i, s);
+        const ScenePar& P = d.par[s];
+        boundary_one<R, EXPORT, SPH>(d, P, d.bidx[P.sub_off + (w - bpre[s])], s);
     }
 }
 
 template <typename R, bool EXPORT, bool SPH>
-__device__ __forceinline__ void boundary_one(const Dev& d, int i, int s) {
-    const double4 pp = d.posr[i];   // issued before the scene's flag is known
+__device__ __forceinline__ void boundary_one(const Dev& d, const ScenePar& P, int i, int s) {
+    const double4 pp = ld32(d.posr + i);   // issued before the scene's flag is known
     const uint16_t bb_old = d.bbits[i];
     if (d.has_stops && d.dyn[s].frozen) return;   // a scene past its stop stands still
-    const ScenePar& P = d.par[s];
     const size_t N = (size_t)d.N;
     const double r = pp.w;
-    const int nwall = P.wall == WALL_CUBE ? 6 : (P.wall == WALL_CYL ? 3 : 0);
     {
         // conservative early-out: clearly inside every wall and outside the
         // intruder's bounding sphere (margins of 1e-9 relative cover rounding)
@@ -1972,14 +1975,32 @@ __device__ __forceinline__ void boundary_one(const Dev& d, int i, int s) {
     if (P.wall == WALL_CYL) {
         axv = v3(P.cyl_axis[0], P.cyl_axis[1], P.cyl_axis[2]);
         ERRc = dot(RV, axv);
-        RVbc = RV - ERRc * axv;
+        RVbc = fma1(-ERRc, axv, RV);
         RVtc = ERRc * axv;
         nrmc = len_floor(RVbc);
     }
-    for (int slot = 0; slot < NB_SLOTS; slot++) {
-        const bool is_wall = slot < nwall;
-        const bool is_intr = slot == SLOT_INTR && P.has_intr;
-        if (!is_wall && !is_intr) continue;
+    // the slots that may be in contact, then the law slot by slot of the lane's
+    // own: lanes on different walls share one evaluation (taking every wall in
+    // turn made it three or six)
+    unsigned slots = P.has_intr ? 1u << SLOT_INTR : 0u;
+    if (P.wall == WALL_CUBE) {
+        const double e[3] = {RV.x, RV.y, RV.z};
+#pragma unroll
+        for (int ax = 0; ax < 3; ax++) {
+            const double h = P.w_half[ax];
+            if (e[ax] > 0 && e[ax] + r - h > 0) slots |= 1u << (2 * ax);
+            if (e[ax] < 0 && e[ax] - r + h < 0) slots |= 2u << (2 * ax);
+        }
+    } else if (P.wall == WALL_CYL) {
+        const double d_cap = fabs(ERRc) - P.cyl_H + r, d_side = nrmc - P.cyl_R + r;
+        if (d_cap >= 1e-14 && ERRc < 0) slots |= 1u;
+        if (d_cap >= 1e-14 && ERRc > 0) slots |= 2u;
+        if (d_side >= 1e-14) slots |= 4u;
+    }
+#pragma unroll 1
+    for (; slots; slots &= slots - 1) {
+        const int slot = __ffs(slots) - 1;
+        const bool is_intr = slot == SLOT_INTR, is_wall = !is_intr;
         double Apd = 0, Dnd = 0;
         V3<double> nd = v3(0.0, 0.0, 0.0), RVo = nd;
         bool on = false;
@@ -1991,33 +2012,23 @@ __device__ __forceinline__ void boundary_one(const Dev& d, int i, int s) {
             const int ax = slot >> 1;
             const bool up = (slot & 1) == 0;
             const double e = (ax == 0 ? RV.x : (ax == 1 ? RV.y : RV.z)), h = P.w_half[ax];
-            on = up ? (e > 0 && e + r - h > 0) : (e < 0 && e - r + h < 0);
-            if (on) {
-                const double o = (h / fabs(e)) * e;
-                RVo = RV;
-                if (ax == 0) RVo.x = o; else if (ax == 1) RVo.y = o; else RVo.z = o;
-                const double sgn = up ? -1.0 : 1.0;
-                if (ax == 0) nd.x = sgn; else if (ax == 1) nd.y = sgn; else nd.z = sgn;
-                Apd = dot(RV - RVo, nd);
-                Dnd = r - Apd;
-                on = Dnd > 0.0;
-            }
+            const double o = (h / fabs(e)) * e;
+            RVo = RV;
+            if (ax == 0) RVo.x = o; else if (ax == 1) RVo.y = o; else RVo.z = o;
+            const double sgn = up ? -1.0 : 1.0;
+            if (ax == 0) nd.x = sgn; else if (ax == 1) nd.y = sgn; else nd.z = sgn;
+            Apd = dot(RV - RVo, nd);
+            Dnd = r - Apd;
+            on = Dnd > 0.0;
         } else if (is_wall) {
-            const double d_cap = fabs(ERRc) - P.cyl_H + r;
-            const double d_side = nrmc - P.cyl_R + r;
-            if (slot == 0) on = d_cap >= 1e-14 && ERRc < 0;
-            else if (slot == 1) on = d_cap >= 1e-14 && ERRc > 0;
-            else on = d_side >= 1e-14;
+            RVo = slot < 2 ? fma1(P.cyl_H / fabs(ERRc), RVtc, RVbc) : fma1(P.cyl_R / nrmc, RVbc, RVtc);
+            const V3<double> RVn = RV - RVo;
+            Dnd = r - len_floor_yx(RVn);
+            on = Dnd > 0.0;
             if (on) {
-                RVo = slot < 2 ? (P.cyl_H / fabs(ERRc)) * RVtc + RVbc : (P.cyl_R / nrmc) * RVbc + RVtc;
-                const V3<double> RVn = RV - RVo;
-                Dnd = r - len_floor(RVn);
-                on = Dnd > 0.0;
-                if (on) {
-                    const double DistL = sqrt(RVn.x * RVn.x + RVn.y * RVn.y + RVn.z * RVn.z);
-                    nd = (1.0 / DistL) * RVn;
-                    Apd = DistL;
-                }
+                const double DistL = sqrt(len2_yx(RVn));
+                nd = (1.0 / DistL) * RVn;
+                Apd = DistL;
             }
         } else {
             const SceneDyn& y = d.dyn[s];
@@ -2045,15 +2056,15 @@ __device__ __forceinline__ void boundary_one(const Dev& d, int i, int s) {
                 const V3<double> pv = v3(P.intr_axis[0], P.intr_axis[1], P.intr_axis[2]);
                 const double ERR = dot(RI, pv);
                 if (fabs(ERR) < (P.intr_H + 0.80 * LatDx)) {
-                    const V3<double> RVb = RI - ERR * pv;
+                    const V3<double> RVb = fma1(-ERR, pv, RI);
                     const double nrm = len_floor(RVb);
                     if (nrm < (P.intr_R + 0.80 * LatDx)) {
                         const V3<double> RVt = ERR * pv;
-                        if (fabs(ERR) < P.intr_H) RVo = ((1.0 / nrm) * P.intr_R) * RVb + RVt;
-                        else if (nrm < P.intr_R) RVo = ((1.0 / fabs(ERR)) * P.intr_H) * RVt + RVb;
-                        else RVo = ((1.0 / nrm) * P.intr_R) * RVb + ((1.0 / fabs(ERR)) * P.intr_H) * RVt;
+                        if (fabs(ERR) < P.intr_H) RVo = fma1((1.0 / nrm) * P.intr_R, RVb, RVt);
+                        else if (nrm < P.intr_R) RVo = fma1((1.0 / fabs(ERR)) * P.intr_H, RVt, RVb);
+                        else RVo = fma2((1.0 / nrm) * P.intr_R, RVb, (1.0 / fabs(ERR)) * P.intr_H, RVt);
                         const V3<double> RVn = RI - RVo;
-                        const double DistL = sqrt(RVn.x * RVn.x + RVn.y * RVn.y + RVn.z * RVn.z);
+                        const double DistL = sqrt(dot(RVn, RVn));
                         Dnd = r - DistL;
                         on = Dnd > 0.0;
                         if (on) { nd = (1.0 / DistL) * RVn; Apd = DistL; }
@@ -2182,6 +2193,59 @@ constexpr int PR_THREADS = 256;
 #define NBC_PAIR_MINB 2
 #endif
 constexpr int CONTACT_LAUNCHES = 2;   // k_pairs and k_boundary
+
+// near pair q with its work record (ra: owner, partner, their member slots; rb:
+// their clumps, the slots of the two) and whether it touched a step ago;
+// returns whether it touches now
+template <typename R, bool EXPORT>
+__device__ __forceinline__ uint8_t pair_item(const Dev& d, const ScenePar& P, int4 ra, int4 rb, size_t q, uint8_t was) {
+    R4<R>* slots = (R4<R>*)d.slots;
+    R4<R>* H = (R4<R>*)d.H[0];
+    const size_t cap = (size_t)d.cap;
+    Body<R> a, b;
+    V3<R> hs = v3<R>(0, 0, 0), ht = hs, hr = hs;
+    a.p = ld32(d.posr + ra.x);
+    b.p = ld32(d.posr + ra.y);
+    // (in FP64 the springs' registers leave no room for that)
+    const bool early = sizeof(R) == 4 && was;
+    if (early) {
+        load_kin<R>(d, make_int2(rb.x, ra.z), a);
+        load_kin<R>(d, make_int2(rb.y, ra.w), b);
+        hist_read<R>(H, cap, q, hs, ht, hr);
+    }
+    if (!overlaps(a.p, b.p)) {
+        if (was) {
+            const R4<R> zero = pack<R>(v3<R>(0, 0, 0), R(0));
+            st_pair(slots + 2 * (size_t)rb.z, zero, zero);
+            if (rb.w >= 0) st_pair(slots + 2 * (size_t)rb.w, zero, zero);
+        }
+        return 0;
+    }
+    if (!early) {
+        load_kin<R>(d, make_int2(rb.x, ra.z), a);
+        load_kin<R>(d, make_int2(rb.y, ra.w), b);
+        if (sizeof(R) == 8 && was) hist_read<R>(H, cap, q, hs, ht, hr);
+    }
+    Law<R> L;
+    L.kn_fac = P.kn_fac; L.ks_fac = P.ks_fac; L.damping = P.damping;
+    L.beta = (R)P.beta; L.mu = (R)P.mu; L.dt = (R)P.dt;
+    V3<R> fa, ta, tb;
+    LawOut<R> o;
+    double Ap;
+    V3<double> nd;
+    pair_contact2<R>(L, (R)P.cohesion, a, b, hs, hr, ht, fa, ta, tb, o, Ap, nd);
+    hist_write<R>(H, cap, q, o.hs, o.ht, o.hr);
+    st_pair(slots + 2 * (size_t)rb.z, pack<R>(fa, R(0)), pack<R>(ta, R(0)));
+    if (rb.w >= 0) st_pair(slots + 2 * (size_t)rb.w, pack<R>(-fa, R(0)), pack<R>(tb, R(0)));
+    if (EXPORT) {
+        const int p = d.np[0][q];
+        R4<R>* xf = (R4<R>*)d.xfcn;
+        double4* xc = (double4*)d.xcpt;
+        xf[p] = pack<R>(-o.Fn, R(0));
+        xc[p] = make_double4(a.p.x + Ap * nd.x, a.p.y + Ap * nd.y, a.p.z + Ap * nd.z, 0.0);
+    }
+    return 1;
+}
 template <typename R, bool EXPORT>
 __global__ void __launch_bounds__(PR_THREADS, NBC_PAIR_MINB) k_pairs(const Dev* __restrict__ dp) {
     const Dev& d = *dp;
@@ -2191,12 +2255,7 @@ __global__ void __launch_bounds__(PR_THREADS, NBC_PAIR_MINB) k_pairs(const Dev* 
     const int* __restrict__ npre = d.nprefix;
     const int np = npre[S];
     const int4* __restrict__ recs = d.rec[0];
-    const double4* __restrict__ posr = d.posr;
-    uint8_t* __restrict__ touch = d.touch[0];
-    R4<R>* __restrict__ slots = (R4<R>*)d.slots;
-    R4<R>* __restrict__ H = (R4<R>*)d.H[0];
-    const size_t cap = (size_t)d.cap;
-    const R4<R> zero = pack<R>(v3<R>(0, 0, 0), R(0));
+    uint8_t* touch = d.touch[0];
     // work item w: near pair w - nprefix[s] of scene s
     auto fetch = [&](int w, int4& ra, int4& rb, int& s, size_t& q, uint8_t& was) {
         if (w >= np) return false;
@@ -2215,57 +2274,15 @@ __global__ void __launch_bounds__(PR_THREADS, NBC_PAIR_MINB) k_pairs(const Dev* 
     uint8_t wasn = 0;
     bool liven = fetch(blockIdx.x * blockDim.x + threadIdx.x, ran, rbn, sn, qn, wasn);
     for (int w = blockIdx.x * blockDim.x + threadIdx.x; w < np; w += stride) {
-        const int4 ra = ran, rb = rbn;   // owner, partner, their member slots; their clumps, slots of the two
+        const int4 ra = ran, rb = rbn;
         const int s = sn;
         const size_t q = qn;
         const uint8_t was = wasn;
         const bool live = liven;
         liven = fetch(w + stride, ran, rbn, sn, qn, wasn);
         if (!live) continue;
-        Body<R> a, b;
-        V3<R> hs = v3<R>(0, 0, 0), ht = hs, hr = hs;
-        a.p = ld32(posr + ra.x);
-        b.p = ld32(posr + ra.y);
-        // (in FP64 the springs' registers leave no room for that)
-        const bool early = sizeof(R) == 4 && was;
-        if (early) {
-            load_kin<R>(d, make_int2(rb.x, ra.z), a);
-            load_kin<R>(d, make_int2(rb.y, ra.w), b);
-            hist_read<R>(H, cap, q, hs, ht, hr);
-        }
-        if (!overlaps(a.p, b.p)) {
-            if (was) {
-                touch[q] = 0;
-                st_pair(slots + 2 * (size_t)rb.z, zero, zero);
-                if (rb.w >= 0) st_pair(slots + 2 * (size_t)rb.w, zero, zero);
-            }
-            continue;
-        }
-        if (!early) {
-            load_kin<R>(d, make_int2(rb.x, ra.z), a);
-            load_kin<R>(d, make_int2(rb.y, ra.w), b);
-            if (sizeof(R) == 8 && was) hist_read<R>(H, cap, q, hs, ht, hr);
-            touch[q] = 1;
-        }
-        const ScenePar& P = d.par[s];
-        Law<R> L;
-        L.kn_fac = P.kn_fac; L.ks_fac = P.ks_fac; L.damping = P.damping;
-        L.beta = (R)P.beta; L.mu = (R)P.mu; L.dt = (R)P.dt;
-        V3<R> fa, ta, tb;
-        LawOut<R> o;
-        double Ap;
-        V3<double> nd;
-        pair_contact2<R>(L, (R)P.cohesion, a, b, hs, hr, ht, fa, ta, tb, o, Ap, nd);
-        hist_write<R>(H, cap, q, o.hs, o.ht, o.hr);
-        st_pair(slots + 2 * (size_t)rb.z, pack<R>(fa, R(0)), pack<R>(ta, R(0)));
-        if (rb.w >= 0) st_pair(slots + 2 * (size_t)rb.w, pack<R>(-fa, R(0)), pack<R>(tb, R(0)));
-        if (EXPORT) {
-            const int p = d.np[0][q];
-            R4<R>* xf = (R4<R>*)d.xfcn;
-            double4* xc = (double4*)d.xcpt;
-            xf[p] = pack<R>(-o.Fn, R(0));
-            xc[p] = make_double4(a.p.x + Ap * nd.x, a.p.y + Ap * nd.y, a.p.z + Ap * nd.z, 0.0);
-        }
+        const uint8_t on = pair_item<R, EXPORT>(d, d.par[s], ra, rb, q, was);
+        if (on != was) touch[q] = on;
     }
 }
 
@@ -2308,6 +2325,216 @@ __global__ void __launch_bounds__(CT_THREADS) k_sum(const Dev* __restrict__ dp) 
     R4<R>* fo = (R4<R>*)d.fsum;
     fo[i] = pack<R>(F, R(0));
     fo[N + i] = pack<R>(T, R(0));
+}
+
+// ===========================================================================
+// many steps in one launch
+// ===========================================================================
+
+// A grid barrier that also tells whether any block raised `flag`: one 64-bit
+// counter, arrivals below, raised flags above, zeroed between launches.  The
+// wait is bounded (ST_SPIN polls, some seconds); a block that gives up sets
+// *fail and *halt and every block leaves at its own limit.  The launch is
+// cooperative, so all blocks run at the same time.  Returns 0 or 1, or -1 when
+// it gave up; s_out is shared.
+constexpr int ST_THREADS = 256;
+constexpr int ST_WARPS = ST_THREADS / 32;
+constexpr int ST_SCENES = 512;          // scenes whose prefixes fit shared memory
+constexpr int ST_SPIN = 1 << 23;
+constexpr int ST_MAX_STEPS = 1 << 20;   // steps per launch: the arrivals stay below 2^32
+
+__device__ __forceinline__ int step_barrier(const Dev& d, unsigned target, int flag, int* s_out) {
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        unsigned long long* bar = d.step_bar;
+        const unsigned long long add = 1ull | (flag ? 1ull << 32 : 0ull);
+        asm volatile("red.release.gpu.global.add.u64 [%0], %1;" ::"l"(bar), "l"(add) : "memory");
+        unsigned long long v = 0;
+        int polls = 0;
+        for (;;) {
+            asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(bar) : "memory");
+            if ((unsigned)v >= target) break;
+            if (++polls > ST_SPIN) {
+                atomicExch(d.scan_fail, 1);
+                atomicExch(d.halt, 1);
+                break;
+            }
+        }
+        *s_out = polls > ST_SPIN ? -1 : (int)((v >> 32) != 0);
+    }
+    __syncthreads();
+    return *s_out;
+}
+
+// Steps until *loop_left are done or some scene needs a rebuild: per step the
+// clump pass, a grid barrier, pairs and boundary candidates, a grid barrier.
+// A step that needs a rebuild leaves the launch after its clump pass (the
+// graph's if node runs the rebuild) and the next launch takes up its contact
+// pass (*step_phase = 1).  The pointer table and, in a single scene, its
+// parameters are kept in shared memory, and so are the work records of a
+// warp's first items, which change at rebuilds only: a pass then starts with
+// the one load that brings positions, kinematics, springs and slots.
+//
+// Work items go to the warps block by block (warp w of block b: item
+// w gridDim + b), so that a small scene's few warps spread over the SMs.
+//
+// Bound by latency: at 500 clumps a step is 7,300 cycles of clump pass, 5,400
+// of contacts and two barriers of 2,200.  One block of 8 warps per SM with 255
+// registers a thread beats 16 warps with 128 and 570 bytes of spilled stack
+// (us a step, rebuilds included: 500 clumps 12.9 -> 11.5, 50,000 100 -> 83,
+// 250,000 469 -> 432), and one launch per pass (three kernel nodes, fork and
+// join, an if and a while node a step: 23.4, 94 and 454 us, 25.8 against 12.4
+// for 2,000 spheres in FP64).
+template <typename R, bool SPH>
+__device__ __noinline__ void boundary_call(const Dev& d, const ScenePar& P, int i, int s) {
+    boundary_one<R, false, SPH>(d, P, i, s);
+}
+
+template <typename R, bool SPH>
+__global__ void __launch_bounds__(ST_THREADS, 1) k_steps(const Dev* __restrict__ dp, cudaGraphConditionalHandle cond,
+                                                         cudaGraphConditionalHandle loop) {
+    __shared__ Dev s_dev;
+    __shared__ ScenePar s_par;
+    __shared__ int4 s_lane[ST_THREADS][2], s_pair[ST_THREADS][2];
+    __shared__ int s_npre[ST_SCENES + 1], s_bpre[ST_SCENES + 1], s_off[ST_SCENES];
+    __shared__ int s_out, s_moved;
+    for (int k = threadIdx.x; k < (int)(sizeof(Dev) / sizeof(int)); k += ST_THREADS)
+        ((int*)&s_dev)[k] = ((const int*)dp)[k];
+    if (threadIdx.x == 0) s_moved = 0;
+    __syncthreads();
+    const Dev& d = s_dev;
+    const bool lead = blockIdx.x == 0 && threadIdx.x == 0;
+    if (lead) *d.step_runs += 1;
+    if (*d.halt) {
+        // a rebuild ran out of pair capacity: the host finishes that step
+        if (lead) {
+            *d.step_phase = 0;
+            cudaGraphSetConditional(cond, 0u);
+            cudaGraphSetConditional(loop, 0u);
+        }
+        return;
+    }
+    const int S = d.S, W = d.W, sw = (S + 31) / 32;
+    for (int k = threadIdx.x; S == 1 && k < (int)(sizeof(ScenePar) / sizeof(int)); k += ST_THREADS)
+        ((int*)&s_par)[k] = ((const int*)d.par)[k];
+    const int lane = threadIdx.x & 31;
+    const int gw = (threadIdx.x >> 5) * gridDim.x + blockIdx.x, nw = gridDim.x * ST_WARPS;
+    int L = *d.lstep, post = *d.post_pending, left = *d.loop_left, started = 0;
+    bool contact = *d.step_phase != 0;
+    const int np = d.nprefix[S], nb = d.bprefix[S];
+    const int wp = (np + 31) / 32, wb = (nb + 31) / 32;
+    // the warp's first items
+    int4 ta = make_int4(-1, 0, -1, 0), tb = make_int4(0, 0, 0, 0);
+    if (gw < W) ld_rec(d.lrec + 2 * (size_t)(gw * 32 + lane), ta, tb);
+    s_lane[threadIdx.x][0] = ta;
+    s_lane[threadIdx.x][1] = tb;
+    // the scenes' work items: prefixes, and the first pair slot less the prefix
+    const bool tab = S <= ST_SCENES;
+    for (int k = threadIdx.x; tab && k <= S; k += ST_THREADS) {
+        const int p = d.nprefix[k];
+        s_npre[k] = p;
+        s_bpre[k] = d.bprefix[k];
+        if (k < S) s_off[k] = d.dyn[k].pair_off - p;
+    }
+    __syncthreads();
+    const int* npre = tab ? s_npre : d.nprefix;
+    const int* bpre = tab ? s_bpre : d.bprefix;
+    // work item w of the contact pass: pair w - nprefix[s] of scene s
+    auto pair_of = [&](int w, int& s) {
+        s = S == 1 ? 0 : plan_find(npre, S, w);
+        return (size_t)((tab ? s_off[s] : d.dyn[s].pair_off - npre[s]) + w);
+    };
+    int ps = 0;
+    size_t pq = 0;
+    uint8_t was = 0;
+    const bool own = gw * 32 + lane < np;
+    if (own) {
+        int4 ra, rb;
+        pq = pair_of(gw * 32 + lane, ps);
+        ld_rec(d.rec[0] + 2 * pq, ra, rb);
+        was = d.touch[0][pq];
+        s_pair[threadIdx.x][0] = ra;
+        s_pair[threadIdx.x][1] = rb;
+    }
+    const uint8_t was0 = was;
+    __syncthreads();
+    const ScenePar* par = S == 1 ? &s_par : nullptr;
+    unsigned target = 0;
+    int out = 0;
+    for (;;) {
+        if (!contact) {
+            bool moved = false;
+            int4 xa = s_lane[threadIdx.x][0], xb = s_lane[threadIdx.x][1];
+            for (int w = gw; w < W + sw; w += nw) {
+                const int4 ya = xa, yb = xb;
+                if (w + nw < W) ld_rec(d.lrec + 2 * (size_t)((w + nw) * 32 + lane), xa, xb);   // the next item's
+                if (w < W) moved |= clump_warp<R, SPH, true>(d, par ? *par : d.par[yb.x], ya, yb, 1, post, L);
+                else if ((w - W) * 32 + lane < S) scene_step(d, (w - W) * 32 + lane, 1, post, L);
+            }
+            if (moved) s_moved = 1;
+            L++;
+            started++;
+            target += gridDim.x;
+            __syncthreads();
+            out = step_barrier(d, target, s_moved, &s_out);
+            if (out) break;
+        }
+        contact = false;
+        int4 xa = s_pair[threadIdx.x][0], xb = s_pair[threadIdx.x][1];
+        int xs = ps;
+        size_t xq = pq;
+        uint8_t xt = was;
+        for (int w = gw; w < wp + wb; w += nw) {
+            const int4 ra = xa, rb = xb;
+            const int s = xs;
+            const size_t q = xq;
+            const uint8_t t0 = xt;
+            if (w + nw < wp && (w + nw) * 32 + lane < np) {   // the next item's
+                xq = pair_of((w + nw) * 32 + lane, xs);
+                ld_rec(d.rec[0] + 2 * xq, xa, xb);
+                xt = d.touch[0][xq];
+            }
+            if (w < wp) {
+                if (w * 32 + lane >= np) continue;
+                if (d.has_stops && d.dyn[s].frozen) continue;
+                const uint8_t on = pair_item<R, false>(d, par ? *par : d.par[s], ra, rb, q, t0);
+                if (w == gw) was = on;   // its flag goes to memory when the launch ends
+                else if (on != t0) d.touch[0][q] = on;
+            } else {
+                const int x = (w - wp) * 32 + lane;
+                if (x >= nb) continue;
+                const int b = S == 1 ? 0 : plan_find(bpre, S, x);
+                const ScenePar& P = par ? *par : d.par[b];
+                boundary_call<R, SPH>(d, P, d.bidx[P.sub_off + (x - bpre[b])], b);
+            }
+        }
+        post = 1;
+        target += gridDim.x;
+        // a raised flag seen here is another block's next clump pass: not yet ours
+        out = min(step_barrier(d, target, 0, &s_out), 0);
+        left--;
+        if (out || left <= 0) break;
+    }
+    if (own && was != was0) d.touch[0][pq] = was;
+    if (lead) {
+        const int reb = out == 1;
+        *d.lstep = L;
+        *d.hgen += started;
+        *d.gstep += started;
+        *d.post_pending = post;
+        *d.loop_left = left;
+        *d.step_phase = reb;
+        cudaGraphSetConditional(cond, reb ? 1u : 0u);
+        cudaGraphSetConditional(loop, reb ? 1u : 0u);
+    }
+}
+
+// The steps a graph launch takes (the first node of its graph; the count is
+// set before each launch) and the barrier's start.
+static __global__ void k_loop_init(int* left, int* phase, unsigned long long* bar, int n) {
+    *left = n;
+    *phase = 0;
+    *bar = 0ull;
 }
 
 }  // namespace nbc

@@ -213,7 +213,12 @@ struct Dev {
     int* gstep;       // steps started by k_clump (counts steps across graph launches)
     int* kc_done;     // blocks of k_clump finished (last-block detection)
     int* lstep;       // steps started by k_clump, counted by its last block (per-scene stops)
-    int* loop_left;   // steps left in a graph launch with a device-side step loop
+    // a graph launch of many steps (k_steps): steps left, whether the next
+    // launch starts with a contact pass, launches so far, the grid barrier
+    int* loop_left;
+    int* step_phase;
+    int* step_runs;
+    unsigned long long* step_bar;
     // export (per pair), written by the export variant of the contact kernel
     void* xfcn;       // Real4 [cap] normal force on the owner (CacheFcn)
     void* xcpt;       // double4 [cap] contact point (CacheCpt)

@@ -12,16 +12,54 @@ namespace nbc {
 template <typename R> struct V3 { R x, y, z; };
 
 template <typename R> __host__ __device__ __forceinline__ V3<R> v3(R x, R y, R z) { return {x, y, z}; }
-template <typename R> __host__ __device__ __forceinline__ V3<R> operator+(V3<R> a, V3<R> b) { return {a.x + b.x, a.y + b.y, a.z + b.z}; }
-template <typename R> __host__ __device__ __forceinline__ V3<R> operator-(V3<R> a, V3<R> b) { return {a.x - b.x, a.y - b.y, a.z - b.z}; }
-template <typename R> __host__ __device__ __forceinline__ V3<R> operator-(V3<R> a) { return {-a.x, -a.y, -a.z}; }
-template <typename R> __host__ __device__ __forceinline__ V3<R> operator*(R s, V3<R> a) { return {s * a.x, s * a.y, s * a.z}; }
-template <typename R> __host__ __device__ __forceinline__ R dot(V3<R> a, V3<R> b) { return a.x * b.x + a.y * b.y + a.z * b.z; }
-template <typename R> __host__ __device__ __forceinline__ V3<R> cross(V3<R> a, V3<R> b) {
-    return {a.y * b.z - a.z * b.y, a.z * b.x - a.x * b.z, a.x * b.y - a.y * b.x};
+
+// Sums and products with their rounding written out: which product of a sum is
+// fused is otherwise the compiler's choice, and changes with the code around
+// it; the step's results should not change with the kernel it runs in.  Sums
+// of vectors are not fused with anything; what is fused says so (fma1: a s +
+// c; fma2: a b + c d, the first product fused; fma3; dot, cross, len_floor).
+__device__ __forceinline__ double add_rn(double a, double b) { return __dadd_rn(a, b); }
+__device__ __forceinline__ float add_rn(float a, float b) { return __fadd_rn(a, b); }
+__device__ __forceinline__ double sub_rn(double a, double b) { return __dsub_rn(a, b); }
+__device__ __forceinline__ float sub_rn(float a, float b) { return __fsub_rn(a, b); }
+__device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(a, b); }
+__device__ __forceinline__ float mul_rn(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ double fma_rn(double a, double b, double c) { return __fma_rn(a, b, c); }
+__device__ __forceinline__ float fma_rn(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+template <typename R> __device__ __forceinline__ R fma2(R a, R b, R c, R d) {   // a b + c d
+    return fma_rn(a, b, mul_rn(c, d));
 }
-template <typename R> __host__ __device__ __forceinline__ R len_floor(V3<R> a) {
-    R t = a.x * a.x + a.y * a.y + a.z * a.z;
+template <typename R> __device__ __forceinline__ R fma3(R a, R b, R c, R d, R e, R f) {   // a b + c d + e f
+    return fma_rn(e, f, fma2(a, b, c, d));
+}
+template <typename R> __device__ __forceinline__ V3<R> operator+(V3<R> a, V3<R> b) {
+    return {add_rn(a.x, b.x), add_rn(a.y, b.y), add_rn(a.z, b.z)};
+}
+template <typename R> __device__ __forceinline__ V3<R> operator-(V3<R> a, V3<R> b) {
+    return {sub_rn(a.x, b.x), sub_rn(a.y, b.y), sub_rn(a.z, b.z)};
+}
+template <typename R> __device__ __forceinline__ V3<R> operator-(V3<R> a) { return {-a.x, -a.y, -a.z}; }
+template <typename R> __device__ __forceinline__ V3<R> operator*(R s, V3<R> a) {
+    return {mul_rn(s, a.x), mul_rn(s, a.y), mul_rn(s, a.z)};
+}
+template <typename R> __device__ __forceinline__ V3<R> fma1(R s, V3<R> a, V3<R> c) {   // s a + c
+    return {fma_rn(s, a.x, c.x), fma_rn(s, a.y, c.y), fma_rn(s, a.z, c.z)};
+}
+template <typename R> __device__ __forceinline__ V3<R> fma2(R s, V3<R> a, R t, V3<R> b) {   // s a + t b
+    return {fma2(s, a.x, t, b.x), fma2(s, a.y, t, b.y), fma2(s, a.z, t, b.z)};
+}
+template <typename R> __device__ __forceinline__ R dot(V3<R> a, V3<R> b) { return fma3(a.x, b.x, a.y, b.y, a.z, b.z); }
+template <typename R> __device__ __forceinline__ V3<R> cross(V3<R> a, V3<R> b) {
+    return {fma2(a.y, b.z, -a.z, b.y), fma2(a.z, b.x, -a.x, b.z), fma2(a.x, b.y, -a.y, b.x)};
+}
+template <typename R> __device__ __forceinline__ R len_floor(V3<R> a) {
+    const R t = dot(a, a);
+    return t > R(1e-32) ? sqrt(t) : R(0);
+}
+// the same with the y product fused first (the boundary laws' lengths)
+template <typename R> __device__ __forceinline__ R len2_yx(V3<R> a) { return fma3(a.y, a.y, a.x, a.x, a.z, a.z); }
+template <typename R> __device__ __forceinline__ R len_floor_yx(V3<R> a) {
+    const R t = len2_yx(a);
     return t > R(1e-32) ? sqrt(t) : R(0);
 }
 template <typename R, typename S> __host__ __device__ __forceinline__ V3<R> cvt(V3<S> a) {
@@ -79,16 +117,6 @@ __device__ __forceinline__ void ld_rec(const int4* p, int4& a, int4& b) {
     asm volatile("ld.global.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
                  : "=r"(a.x), "=r"(a.y), "=r"(a.z), "=r"(a.w), "=r"(b.x), "=r"(b.y), "=r"(b.z), "=r"(b.w)
                  : "l"(p));
-}
-
-// The integrator's sums of products with their rounding written out: which
-// product of a sum is fused is otherwise the compiler's choice, and changes
-// with the code around it; a bed's trajectory should not change with it.
-__device__ __forceinline__ double fma2(double a, double b, double c, double d) {   // a b + c d
-    return __fma_rn(a, b, __dmul_rn(c, d));
-}
-__device__ __forceinline__ double fma3(double a, double b, double c, double d, double e, double f) {   // a b + c d + e f
-    return __fma_rn(e, f, fma2(a, b, c, d));
 }
 
 // body->world rotation (Quat2IvDCM, src/type.h:238-250) applied to u

@@ -253,7 +253,7 @@ nbc_status nbc_server_advance(nbc_server* s, int chunk, int* n_active, int* n_qu
             try {
                 c.eng.reset(new nbc_engine());
                 c.eng->opt = s->opt;
-                c.eng->eng.reset(nbc::make_engine(v, s->opt));
+                c.eng->eng.reset(nbc::make_engine(v, s->opt, s->max_active > 1));
                 for (size_t k = 0; k < adm.size(); k++) {
                     Request& r = *s->req[adm[k]];
                     c.eng->eng->set_stop((int)k, r.nsteps);
