@@ -122,7 +122,8 @@ typedef struct {
     int device;         /* CUDA device ordinal */
     double pair_slack;  /* pair capacity = slack * pairs of the first list; 0 = 1.6 and at least
                            the reference's own n_sub * BranchLmtLen/2 as far as 30% of free memory allows */
-    int search_lanes;   /* lanes per subsphere in the neighbour search: 8, 16 or 32 (0 = 8) */
+    int search_lanes;   /* kept for callers and reported back (8, 16 or 32; 0 = 8): the neighbour search has
+                           8 lanes a subsphere */
     int clump_batch;    /* kept for callers and reported back (1, 2 or 4; 0 = 1): the clump pass gives each
                            member a lane of its own */
     int pair_blocks;    /* blocks per SM of the pair kernel's grid: 2 .. 16 (0 = 12) */

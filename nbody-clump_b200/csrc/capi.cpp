@@ -499,13 +499,7 @@ nbc_status nbc_autotune(const nbc_scene_desc* const* scenes, int n, nbc_options*
         best.pair_blocks = 12;
         best.use_graph = 1;
         double tb = trial(best);
-        const int lanes[] = {16, 32}, blocks[] = {4, 8, 16};
-        for (int x : lanes) {
-            nbc_options o = best;
-            o.search_lanes = x;
-            const double t = trial(o);
-            if (t < 0.97 * tb) { best = o; tb = t; }
-        }
+        const int blocks[] = {4, 8, 16};
         for (int x : blocks) {
             nbc_options o = best;
             o.pair_blocks = x;

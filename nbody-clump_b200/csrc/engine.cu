@@ -1344,7 +1344,7 @@ class EngineT final : public EngineBase {
             h_.pscene = m.take<int>(S_);
             h_.psub = m.take<int>(S_ + 1);
             h_.pcell = m.take<int>(S_ + 1);
-            h_.pclump = m.take<int>(S_ + 1);
+            h_.pwarp = m.take<int>(S_ + 1);
             h_.need = m.take<int>(S_);
             relmap_ = m.take<int4>(S_);
             h_.xparts = m.take<R4<R>>(6 * N);

@@ -666,7 +666,7 @@ static __global__ void __launch_bounds__(SC_THREADS) k_plan(const Dev* __restric
     __shared__ int sh[SC_THREADS / 32];
     const Dev& d = *dp;
     if (*d.halt) return;
-    int ns = 0, nsub = 0, ncell = 0, nclump = 0;
+    int ns = 0, nsub = 0, ncell = 0, nwarp = 0;
     for (int b = 0; b < d.S; b += SC_THREADS) {
         const int s = b + threadIdx.x;
         const bool f = s < d.S && d.dyn[s].rebuild;
@@ -675,7 +675,9 @@ static __global__ void __launch_bounds__(SC_THREADS) k_plan(const Dev* __restric
             const ScenePar& P = d.par[s];
             a1 = P.nsub;
             a2 = P.cellnum + 1;
-            a3 = P.nclump;
+            // warps of the clump pass's table that hold lanes of the scene
+            const int c0 = P.clump_off, c1 = c0 + P.nclump - 1, n1 = d.mem_start[c1 + 1] - d.mem_start[c1];
+            a3 = (d.clane[c1] + min(max(n1, 1), 32) - 1) / 32 - d.clane[c0] / 32 + 1;
         }
         if (s < d.S) d.need[s] = -1;
         int t0, t1, t2, t3;
@@ -687,22 +689,22 @@ static __global__ void __launch_bounds__(SC_THREADS) k_plan(const Dev* __restric
             d.pscene[ns + e0] = s;
             d.psub[ns + e0] = nsub + e1;
             d.pcell[ns + e0] = ncell + e2;
-            d.pclump[ns + e0] = nclump + e3;
+            d.pwarp[ns + e0] = nwarp + e3;
         }
         ns += t0;
         nsub += t1;
         ncell += t2;
-        nclump += t3;
+        nwarp += t3;
     }
     if (threadIdx.x == 0) {
         d.psub[ns] = nsub;
         d.pcell[ns] = ncell;
-        d.pclump[ns] = nclump;
+        d.pwarp[ns] = nwarp;
         d.plan[PL_NS] = ns;
         d.plan[PL_T] = nsub;
         d.plan[PL_TC] = ncell;
         d.plan[PL_T1] = nsub + 1;
-        d.plan[PL_TK] = nclump;
+        d.plan[PL_TW] = nwarp;
         d.plan[PL_TC1] = ncell + 1;
     }
 }
@@ -954,17 +956,19 @@ static __global__ void __launch_bounds__(RS_THREADS) k_rs_scatter(const int* __r
 // range of the sorted order.  G lanes share a subsphere: they resolve its rows
 // (passing over rows and end cells that the largest cutoff on their level,
 // 1.5 (ri + largest radius), cannot reach, but never at the grid's border, whose
-// cells also hold what lies beyond them), take equal contiguous parts of the
-// rows' concatenation, and keep what passes an FP32 test (a 16-byte copy of
+// cells also hold what lies beyond them), walk the rows' concatenation G
+// candidates at a time, and keep what passes an FP32 test (a 16-byte copy of
 // the position, a cutoff widened by the rounding) in a list in shared memory;
-// then the list is tested in FP64, G entries at a time, and appended to the
-// back row through ballots.  So the candidate loop is a dozen instructions with
+// the list is tested in FP64, G entries at a time, and appended to the back row
+// through ballots.  So the candidate loop is some thirty instructions with
 // every lane busy, and the FP64 test, the flags and the counters run on full
 // groups for the one candidate in eight that needs them.  50,000 clumps on five
-// levels, 1.7 M pairs: 132 us (both directions with FP64 tests on 8 lanes took
+// levels, 1.7 M pairs: 115 us (both directions with FP64 tests on 8 lanes took
 // 241, and compaction, cross-level sort, reverse map, history carry and near
-// rows another 250 in eight launches where k_fill and k_rows take 64 + 65);
-// 64 registers (8 blocks per SM) against 80 and 94: 132, 143 and 156 us.
+// rows another 250 in eight launches where k_fill and k_rows take 52 + 56).
+// Half of it is the rows, a third the FP32 tests; votes with a mask per group
+// instead of the whole warp's: 167 us, every lane finding its rows' levels for
+// itself: 125 us, 80 or 94 registers a thread: 9 and 18% more than with 64.
 //
 // A subsphere in a single-level scene's last cell, where out-of-box ones are
 // put, does not search; those whose stencil holds that cell list its members
@@ -973,14 +977,22 @@ constexpr int SEARCH_THREADS = 128;
 constexpr int SEARCH_G = 8;                   // lanes per subsphere
 constexpr int SEARCH_GROUPS = SEARCH_THREADS / SEARCH_G;
 constexpr int SCR_CAP = 64;                   // scratch entries per back row
-constexpr int LANE_CAP = 16;                  // FP32 hits per lane
+constexpr int LIST_CAP = 32;                  // FP32 hits held before they are tested in FP64
 constexpr int MAX_ROWS = 5 + 9 * (MAX_LEVELS - 1);
 constexpr int NEAR = 0x40000000;              // scratch: the pair can touch before the next rebuild
 constexpr int SUB_MASK = 0x3fffffff;
 
+// per row that has candidates: the end of its range in the rows' concatenation,
+// and the sorted index of a candidate less its place in the concatenation
 struct SearchRows {
-    int rs[SEARCH_GROUPS][MAX_ROWS];        // first sorted index of each row that has candidates
-    int pre[SEARCH_GROUPS][MAX_ROWS + 1];   // exclusive prefix of their lengths
+    int2 row[SEARCH_GROUPS][MAX_ROWS];
+    // where the subsphere sits on each level it searches, one lane a level:
+    // squared distance to the neighbour cells' faces (0 where a cell is never
+    // passed over, INF where there is none), the squared reach; the centre cell,
+    // the strides of the grid, the range of x neighbours
+    float4 dist[SEARCH_GROUPS][MAX_LEVELS][2];   // z-, z0, z+, reach; y-, y0, y+, x-
+    float xp[SEARCH_GROUPS][MAX_LEVELS];
+    int4 cell[SEARCH_GROUPS][MAX_LEVELS];        // centre, stride y, stride z, (x range)
 };
 
 // FP64 test of a candidate that passed the FP32 one: 0 no pair, 1 a pair, 2 a
@@ -997,63 +1009,74 @@ __device__ __forceinline__ int pair_test(double4 a, double4 b, double margin) {
 // 2 Thresh cannot touch before the next one.
 __device__ __forceinline__ double near_margin(const ScenePar& P) { return 2.0 * P.thresh * (1.0 + 1e-6) + 1e-12; }
 
-// The stencil rows of subsphere i by the G lanes of its group (g of them, lane
-// mask gm): candidates j < i as ranges in rs / pre, in back-row order; the
-// number of candidates.
-__device__ __forceinline__ int group_rows(const Dev& d, const ScenePar& P, int i, double4 pi, int g, unsigned gm,
-                                          int* __restrict__ rs, int* __restrict__ pre) {
+// The stencil rows of subsphere i by the G lanes of its group (g of them):
+// candidates j < i as ranges in back-row order; the number of candidates.
+// Every lane of the warp calls it; `on`: the group has a subsphere.  (The
+// warp's groups run in step, votes and shuffles over the whole warp: with a
+// mask per group the compiler takes the groups through them one by one.)
+__device__ __forceinline__ int group_rows(const Dev& d, const ScenePar& P, bool on, int i, double4 pi, int g,
+                                          SearchRows& sh, int grp) {
     constexpr int G = SEARCH_G, MAXC = (MAX_ROWS + G - 1) / G;
     const int* __restrict__ cstart = d.cstart;
     const bool hg = P.levels > 1;
-    const int my = hg ? d.level2[i] : 0;
-    const double x0 = pi.x - P.origin[0], y0 = pi.y - P.origin[1], z0 = pi.z - P.origin[2];
-    const int nrows = 5 + 9 * my, r0 = nrows * g / G, r1 = nrows * (g + 1) / G;
-    int ca[MAXC], cb[MAXC];
-    int lc = -1, gx = 0, gy = 0, gz = 0, base = 0, cx = 0, cy = 0, cz = 0;
-    float clx = 0, cly = 0, clz = 0, fx = 0, fy = 0, fz = 0, cut2 = 0;   // cell size, distance to the lower face, reach^2
+    const int my = hg && on ? d.level2[i] : 0;
+    const int nrows = on ? 5 + 9 * my : 0, r0 = nrows * g / G, r1 = nrows * (g + 1) / G;
+    int2* rows = sh.row[grp];
+    __syncwarp();   // the previous rows and levels are no longer read
+    if (on && g <= my) {
+        const int l = my - g;
+        double c0, c1, c2, i0, i1, i2;
+        int gx, gy, gz, base;
+        if (hg) {
+            gx = P.ldim[l][0]; gy = P.ldim[l][1]; gz = P.ldim[l][2];
+            base = P.cell_off + P.loff[l];
+            c0 = c1 = c2 = P.lcell[l];
+            i0 = i1 = i2 = P.licell[l];
+        } else {
+            gx = P.gdim[0]; gy = P.gdim[1]; gz = P.gdim[2];
+            base = P.cell_off;
+            c0 = P.cell[0]; c1 = P.cell[1]; c2 = P.cell[2];
+            i0 = P.icell[0]; i1 = P.icell[1]; i2 = P.icell[2];
+        }
+        const double x0 = pi.x - P.origin[0], y0 = pi.y - P.origin[1], z0 = pi.z - P.origin[2];
+        const int cx = (int)floor(x0 * i0), cy = (int)floor(y0 * i1), cz = (int)floor(z0 * i2);
+        const float fx = (float)(x0 - cx * c0), fy = (float)(y0 - cy * c1), fz = (float)(z0 - cz * c2);
+        const float ux = (float)c0 - fx, uy = (float)c1 - fy, uz = (float)c2 - fz;
+        const float cut = 1.5f * ((float)pi.w + P.lrmax[l]) * 1.0001f + 1e-4f * (float)c0;
+        // a neighbour at c of g cells, h away
+        auto far2 = [](int c, int g, float h) {
+            return c < 0 || c >= g ? INFINITY : (c == 0 || c == g - 1 ? 0.0f : h * h);
+        };
+        const int xa = max(cx - 1, 0), xb = min(cx + 1, gx - 1);
+        sh.dist[grp][g][0] = make_float4(far2(cz - 1, gz, fz), cz < 0 || cz >= gz ? INFINITY : 0.0f,
+                                         far2(cz + 1, gz, uz), cut * cut);
+        sh.dist[grp][g][1] = make_float4(far2(cy - 1, gy, fy), cy < 0 || cy >= gy ? INFINITY : 0.0f,
+                                         far2(cy + 1, gy, uy), xa > 0 && xa < cx ? fx * fx : -1.0f);
+        sh.xp[grp][g] = xb < gx - 1 && xb > cx ? ux * ux : -1.0f;
+        sh.cell[grp][g] = make_int4(base + (cz * gy + cy) * gx + cx, gx, gx * gy,
+                                    xa > xb ? 0 : (1 << 16 | (xa - cx + 64) << 8 | (xb - cx + 64)));
+    }
+    __syncwarp();
     // the cells of the lane's rows first, then all their cstart loads at once
+    int ca[MAXC], cb[MAXC];
 #pragma unroll
     for (int k = 0; k < MAXC; k++) {
         const int r = r0 + k;
         ca[k] = -1;
         cb[k] = -1;
         if (r >= r1) continue;
-        const int l = r < 5 ? my : my - 1 - (r - 5) / 9, rr = r < 5 ? r : (r - 5) % 9;
-        if (l != lc) {
-            lc = l;
-            double c0, c1, c2, i0, i1, i2;
-            if (hg) {
-                gx = P.ldim[l][0]; gy = P.ldim[l][1]; gz = P.ldim[l][2];
-                base = P.cell_off + P.loff[l];
-                c0 = c1 = c2 = P.lcell[l];
-                i0 = i1 = i2 = P.licell[l];
-            } else {
-                gx = P.gdim[0]; gy = P.gdim[1]; gz = P.gdim[2];
-                base = P.cell_off;
-                c0 = P.cell[0]; c1 = P.cell[1]; c2 = P.cell[2];
-                i0 = P.icell[0]; i1 = P.icell[1]; i2 = P.icell[2];
-            }
-            cx = (int)floor(x0 * i0);
-            cy = (int)floor(y0 * i1);
-            cz = (int)floor(z0 * i2);
-            fx = (float)(x0 - cx * c0); fy = (float)(y0 - cy * c1); fz = (float)(z0 - cz * c2);
-            clx = (float)c0; cly = (float)c1; clz = (float)c2;
-            const float cut = 1.5f * ((float)pi.w + P.lrmax[l]) * 1.0001f + 1e-4f * clx;
-            cut2 = cut * cut;
-        }
+        const int q = r < 5 ? 0 : 1 + (r - 5) / 9, rr = r < 5 ? r : (r - 5) % 9;
         const int sz = rr / 3 - 1, sy = rr % 3 - 1;
-        const int z = cz + sz, y = cy + sy;
-        if (z < 0 || z >= gz || y < 0 || y >= gy) continue;
-        float rem = cut2;
-        if (sz != 0 && z != 0 && z != gz - 1) { const float h = sz < 0 ? fz : clz - fz; rem -= h * h; }
-        if (sy != 0 && y != 0 && y != gy - 1) { const float h = sy < 0 ? fy : cly - fy; rem -= h * h; }
-        int xa = max(cx - 1, 0), xb = min(cx + 1, gx - 1);
-        if (xa > 0 && xa < cx && fx * fx > rem) xa = cx;
-        if (xb < gx - 1 && xb > cx && (clx - fx) * (clx - fx) > rem) xb = cx;
-        if (rem < 0 || xa > xb) continue;
-        const int c = base + (z * gy + y) * gx;
-        ca[k] = c + xa;
-        cb[k] = c + xb + 1;
+        const float4 fz = sh.dist[grp][q][0], fy = sh.dist[grp][q][1];
+        const int4 c = sh.cell[grp][q];
+        const float rem = fz.w - (sz < 0 ? fz.x : (sz ? fz.z : fz.y)) - (sy < 0 ? fy.x : (sy ? fy.z : fy.y));
+        int lo = ((c.w >> 8) & 255) - 64, hi = (c.w & 255) - 64;
+        if (fy.w > rem) lo = 0;
+        if (sh.xp[grp][q] > rem) hi = 0;
+        if (!(rem >= 0) || c.w == 0 || lo > hi) continue;
+        const int m = c.x + sz * c.z + sy * c.y;
+        ca[k] = m + lo;
+        cb[k] = m + hi + 1;
     }
 #pragma unroll
     for (int k = 0; k < MAXC; k++) {
@@ -1069,23 +1092,20 @@ __device__ __forceinline__ int group_rows(const Dev& d, const ScenePar& P, int i
     unsigned inc = acc;
 #pragma unroll
     for (int o = 1; o < G; o <<= 1) {
-        const unsigned v = __shfl_up_sync(gm, inc, o, G);
+        const unsigned v = __shfl_up_sync(0xffffffffu, inc, o, G);
         if (g >= o) inc += v;
     }
-    const unsigned all = __shfl_sync(gm, inc, G - 1, G);
+    const unsigned all = __shfl_sync(0xffffffffu, inc, G - 1, G);
     unsigned at = inc - acc;
-    __syncwarp(gm);   // the group's previous rows are no longer read
 #pragma unroll
     for (int k = 0; k < MAXC; k++)
         if (ca[k] >= 0 && cb[k] > ca[k]) {
-            rs[at >> 24] = ca[k];
-            pre[at >> 24] = (int)(at & 0xffffffu);
+            const int c = (int)(at & 0xffffffu);
+            rows[at >> 24] = make_int2(c + cb[k] - ca[k], ca[k] - c);
             at += (1u << 24) + (unsigned)(cb[k] - ca[k]);
         }
-    const int total = (int)(all & 0xffffffu);
-    if (g == 0) pre[all >> 24] = total;
-    __syncwarp(gm);
-    return total;
+    __syncwarp();
+    return (int)(all & 0xffffffu);
 }
 
 // the members of a single-level scene's last cell when subsphere i's stencil
@@ -1121,13 +1141,14 @@ __device__ __forceinline__ bool searches(const Dev& d, const ScenePar& P, int i)
 static __global__ void __launch_bounds__(SEARCH_THREADS, 8) k_search(const Dev* __restrict__ dp) {
     constexpr int G = SEARCH_G;
     __shared__ SearchRows sh;
-    __shared__ int s_buf[SEARCH_GROUPS][G * LANE_CAP];
+    __shared__ int s_buf[SEARCH_GROUPS][LIST_CAP];
     const Dev& d = *dp;
     if (*d.halt) return;
     const int T = d.plan[PL_T], ns = d.plan[PL_NS], TC1 = d.plan[PL_TC1];
     const int g = threadIdx.x % G, grp = threadIdx.x / G;
     const int gshift = (threadIdx.x & 31) & ~(G - 1);
-    const unsigned gm = ((1u << G) - 1u) << gshift, lt = (1u << g) - 1u;
+    constexpr unsigned GM = (1u << G) - 1u;
+    const unsigned lt = (1u << g) - 1u;
     NBC_GRID_STRIDE(u, TC1) d.ccnt[u] = 0;   // the sort's cell counts back to zero for the next rebuild
     const double4* __restrict__ posr = d.posr2;
     const float4* __restrict__ posf = d.posf;
@@ -1135,104 +1156,76 @@ static __global__ void __launch_bounds__(SEARCH_THREADS, 8) k_search(const Dev* 
     int* __restrict__ cnt_f = d.cnt_f;
     int* __restrict__ cnt_nf = d.cnt_nf;
     int* __restrict__ cnt_ns = d.cnt_ns;
-    int* rs = sh.rs[grp];
-    int* pre = sh.pre[grp];
+    int2* rows = sh.row[grp];
     int* buf = s_buf[grp];
-    for (int t = blockIdx.x * SEARCH_GROUPS + grp; t < T; t += gridDim.x * SEARCH_GROUPS) {
-        const PlanItem it = plan_item(d, ns, t);
-        const int i = it.i, tb = t - i;
+    constexpr unsigned FULL = 0xffffffffu;
+    for (int b0 = blockIdx.x * SEARCH_GROUPS + (grp & ~3); b0 < T; b0 += gridDim.x * SEARCH_GROUPS) {
+        const int t = b0 + (grp & 3);
+        const PlanItem it = plan_item(d, ns, min(t, T - 1));
+        const int i = it.i, tb = min(t, T - 1) - i;
         const ScenePar& P = d.par[it.s];
-        int nb = 0, near = 0;
-        bool isl = false;
-        if (searches(d, P, i)) {
-            const double4 pi = ld32(posr + i);
-            const float4 pf = posf[i];
-            const int2 ci = cm[i];
-            const int total = group_rows(d, P, i, pi, g, gm, rs, pre);
-            // the lane's part of the candidates
-            const int f0 = (int)((long long)total * g / G), f1 = (int)((long long)total * (g + 1) / G);
-            int n = 0, f = f0;
-            if (f < f1) {
-                int r = 0;
-                while (pre[r + 1] <= f) r++;
-                int j = rs[r] + (f - pre[r]), end = pre[r + 1];
-                constexpr int U = 4;   // candidates in flight
-                while (f < f1) {
-                    int jj[U];
-                    float4 q[U];
-#pragma unroll
-                    for (int u = 0; u < U; u++) {
-                        jj[u] = j;
-                        q[u] = posf[j];
-                        f++;
-                        j++;
-                        if (f == end && f < f1) { r++; j = rs[r]; end = pre[r + 1]; }
-                        else if (f >= f1) j = jj[u];   // past the lane's part: the last candidate again
-                    }
-                    const int m = f1 - (f - U);   // candidates of this batch
-#pragma unroll
-                    for (int u = 0; u < U; u++) {
-                        const float dx = pf.x - q[u].x, dy = pf.y - q[u].y, dz = pf.z - q[u].z, w = pf.w + q[u].w;
-                        if (u < m && !(dx * dx + dy * dy + dz * dz > w * w)) {
-                            if (n < LANE_CAP) buf[g * LANE_CAP + n] = jj[u];
-                            n++;
-                        }
-                    }
+        const bool on = t < T && searches(d, P, i);
+        const double4 pi = ld32(posr + i);
+        const float4 pf = posf[i];
+        const int2 ci = cm[i];
+        const int total = group_rows(d, P, on, i, pi, g, sh, grp);
+        const int most = __reduce_max_sync(FULL, total);
+        // the candidates in order, G at a time (the next ones' positions in
+        // flight): what passes goes to the list through a vote, and a list that
+        // cannot take another G is tested in FP64 and emptied
+        const double margin = near_margin(P);
+        int* __restrict__ scr = d.scr + (size_t)i * SCR_CAP;
+        int nb = 0, near = 0, n = 0, r = 0, jn = -1;
+        float4 qn = make_float4(0, 0, 0, 0);
+        auto next = [&](int f) {
+            jn = -1;
+            if (f < total) {
+                int2 x = rows[r];
+                while (x.x <= f) x = rows[++r];
+                jn = f + x.y;
+                qn = posf[jn];
+            }
+        };
+        next(g);
+        for (int f0 = 0; f0 < most; f0 += G) {
+            const int j = jn;
+            const float dx = pf.x - qn.x, dy = pf.y - qn.y, dz = pf.z - qn.z, w = pf.w + qn.w;
+            next(f0 + G + g);
+            const bool pass = j >= 0 && !(dx * dx + dy * dy + dz * dz > w * w);
+            const unsigned pm = (__ballot_sync(FULL, pass) >> gshift) & GM;
+            if (pass) buf[n + __popc(pm & lt)] = j;
+            n += __popc(pm);
+            if (f0 + G < most && !__any_sync(FULL, n > LIST_CAP - G)) continue;
+            __syncwarp();
+            const int list = __reduce_max_sync(FULL, n);
+            for (int k0 = 0; k0 < list; k0 += G) {
+                int hit = 0, k = 0;
+                int2 ck = make_int2(0, 0);
+                if (k0 + g < n) {
+                    k = buf[k0 + g];
+                    ck = cm[k];
+                    hit = pair_test(ld32(posr + k), pi, margin);
                 }
-            }
-            // the lanes' hits one after the other
-            const bool over = __any_sync(gm, n > LANE_CAP);
-            int at = n;
-#pragma unroll
-            for (int o = 1; o < G; o <<= 1) {
-                const int v = __shfl_up_sync(gm, at, o, G);
-                if (g >= o) at += v;
-            }
-            const int hits = __shfl_sync(gm, at, G - 1, G);
-            const double margin = near_margin(P);
-            if (!over) {
-                int tmp[LANE_CAP];
-                at -= n;
-#pragma unroll
-                for (int k = 0; k < LANE_CAP; k++) tmp[k] = k < n ? buf[g * LANE_CAP + k] : 0;
-                __syncwarp(gm);
-#pragma unroll
-                for (int k = 0; k < LANE_CAP; k++)
-                    if (k < n) buf[at + k] = tmp[k];
-                __syncwarp(gm);
-            }
-            // FP64 test in order: the list, or (too many FP32 hits for it) every candidate
-            const int cand = over ? total : hits;
-            int* __restrict__ scr = d.scr + (size_t)i * SCR_CAP;
-            int r = 0;
-            for (int k0 = 0; k0 < cand; k0 += G) {
-                const int k = k0 + g;
-                int hit = 0, j = 0;
-                int2 cj = make_int2(0, 0);
-                if (k < cand) {
-                    if (over) {
-                        while (pre[r + 1] <= k) r++;
-                        j = rs[r] + (k - pre[r]);
-                    } else j = buf[k];
-                    cj = cm[j];
-                    hit = pair_test(ld32(posr + j), pi, margin);
-                }
-                const bool nr = hit == 2 && cj.x != ci.x;
-                const unsigned hm = __ballot_sync(gm, hit != 0) >> gshift;
-                const unsigned nm = __ballot_sync(gm, nr) >> gshift;
+                const bool nr = hit == 2 && ck.x != ci.x;
+                const unsigned hm = (__ballot_sync(FULL, hit != 0) >> gshift) & GM;
+                const unsigned nm = (__ballot_sync(FULL, nr) >> gshift) & GM;
                 if (hit) {
                     const int q = nb + __popc(hm & lt);
-                    if (q < SCR_CAP) scr[q] = j | (cj.x == ci.x ? INTRA : 0) | (nr ? NEAR : 0);
-                    atomicAdd(&cnt_f[j + tb], 1);
+                    if (q < SCR_CAP) scr[q] = k | (ck.x == ci.x ? INTRA : 0) | (nr ? NEAR : 0);
+                    atomicAdd(&cnt_f[k + tb], 1);
                     if (nr) {
-                        atomicAdd(&cnt_nf[j + tb], 1);
-                        atomicAdd(&cnt_ns[cj.y + tb], 1);
+                        atomicAdd(&cnt_nf[k + tb], 1);
+                        atomicAdd(&cnt_ns[ck.y + tb], 1);
                     }
                 }
                 nb += __popc(hm);
                 near += __popc(nm);
             }
-            isl = nb > SCR_CAP;
+            n = 0;
+            __syncwarp();
+        }
+        bool isl = nb > SCR_CAP;
+        if (on) {
             const int2 lcell = last_cell(d, P, pi);
             int nx = 0, nxn = 0;
             for (int j = lcell.x + g; j < lcell.y; j += G) {
@@ -1240,9 +1233,9 @@ static __global__ void __launch_bounds__(SEARCH_THREADS, 8) k_search(const Dev* 
                 nx += hit != 0;
                 nxn += hit == 2 && cm[j].x != ci.x;
             }
-            if (__any_sync(gm, nx)) {
+            if (nx) {
                 isl = true;
-                if (nx) atomicAdd(&cnt_f[t], nx);
+                atomicAdd(&cnt_f[t], nx);
                 if (nxn) {
                     atomicAdd(&cnt_nf[t], nxn);
                     atomicAdd(&cnt_ns[ci.y + tb], nxn);
@@ -1250,9 +1243,10 @@ static __global__ void __launch_bounds__(SEARCH_THREADS, 8) k_search(const Dev* 
             }
             if (g == 0 && near) atomicAdd(&cnt_ns[ci.y + tb], near);
         }
-        if (g == 0) {
+        const unsigned il = (__ballot_sync(FULL, isl) >> gshift) & GM;
+        if (g == 0 && t < T) {
             d.cnt_b[t] = nb;
-            d.rlong[t] = isl;
+            d.rlong[t] = il != 0;
         }
     }
 }
@@ -1287,7 +1281,7 @@ static __global__ void __launch_bounds__(SEARCH_THREADS, 8) k_fill(const Dev* __
     __shared__ SearchRows sh;
     const Dev& d = *dp;
     if (*d.halt) return;
-    const int T = d.plan[PL_T], ns = d.plan[PL_NS], TK = d.plan[PL_TK];
+    const int T = d.plan[PL_T], ns = d.plan[PL_NS], TW = d.plan[PL_TW];
     int over = 0;
     for (int k = threadIdx.x; k < ns; k += SEARCH_THREADS) {
         const int s = d.pscene[k], need = list_need(d, k);
@@ -1303,7 +1297,8 @@ static __global__ void __launch_bounds__(SEARCH_THREADS, 8) k_fill(const Dev* __
     }
     const int g = threadIdx.x % G, grp = threadIdx.x / G;
     const int gshift = (threadIdx.x & 31) & ~(G - 1);
-    const unsigned gm = ((1u << G) - 1u) << gshift, lt = (1u << g) - 1u;
+    constexpr unsigned FULL = 0xffffffffu, GM = (1u << G) - 1u;
+    const unsigned lt = (1u << g) - 1u;
     const PairList& Nw = d.L[1];
     const int* __restrict__ cnt_f = d.cnt_f;
     const int* __restrict__ cnt_b = d.cnt_b;
@@ -1311,7 +1306,9 @@ static __global__ void __launch_bounds__(SEARCH_THREADS, 8) k_fill(const Dev* __
     const int* __restrict__ cnt_ns = d.cnt_ns;
     int* __restrict__ fcur = d.fcur;
     int2* __restrict__ tmp = d.tmp;
-    for (int t = blockIdx.x * SEARCH_GROUPS + grp; t < T; t += gridDim.x * SEARCH_GROUPS) {
+    for (int b0 = blockIdx.x * SEARCH_GROUPS + (grp & ~3); b0 < T; b0 += gridDim.x * SEARCH_GROUPS) {
+        const bool has = b0 + (grp & 3) < T;
+        const int t = min(b0 + (grp & 3), T - 1);
         const PlanItem it = plan_item(d, ns, t);
         const int i = it.i, s = it.s, tb = t - i, t0 = d.psub[it.k];
         const ScenePar& P = d.par[s];
@@ -1321,8 +1318,8 @@ static __global__ void __launch_bounds__(SEARCH_THREADS, 8) k_fill(const Dev* __
         const int nr = base + cnt_nf[t] - cnt_nf[t0], nnf = cnt_nf[t + 1] - cnt_nf[t];
         const int2 ci = d.cm2[i];
         const int s0 = 2 * base + cnt_ns[ci.y + tb] - cnt_ns[t0];
-        const bool isl = d.rlong[t];
-        if (g == 0) {
+        const bool isl = has && d.rlong[t];
+        if (has && g == 0) {
             Nw.row[i + s] = rf;
             Nw.brow[i + s] = rb;
             d.nro[1][i + s] = nr;
@@ -1338,14 +1335,16 @@ static __global__ void __launch_bounds__(SEARCH_THREADS, 8) k_fill(const Dev* __
         // a row that is not in the scratch: its candidates once more
         double4 pi = make_double4(0, 0, 0, 0);
         double margin = 0;
-        int cand = nb, r = 0, kb = s0 + nnf, kr = rb;
+        int cand = has ? nb : 0, r = 0, kb = s0 + nnf, kr = rb;
         const int* __restrict__ scr = d.scr + (size_t)i * SCR_CAP;
-        if (isl) {
+        if (__any_sync(FULL, isl)) {
             pi = ld32(d.posr2 + i);
             margin = near_margin(P);
-            cand = searches(d, P, i) ? group_rows(d, P, i, pi, g, gm, sh.rs[grp], sh.pre[grp]) : 0;
+            const int c = group_rows(d, P, isl && searches(d, P, i), i, pi, g, sh, grp);
+            if (isl) cand = c;
         }
-        for (int k0 = 0; k0 < cand; k0 += G) {
+        const int most = __reduce_max_sync(FULL, cand);
+        for (int k0 = 0; k0 < most; k0 += G) {
             const int k = k0 + g;
             bool hit = k < cand, near = false;
             int v = 0;
@@ -1353,16 +1352,16 @@ static __global__ void __launch_bounds__(SEARCH_THREADS, 8) k_fill(const Dev* __
                 v = scr[k];
                 near = v & NEAR;
             } else if (hit) {
-                while (sh.pre[grp][r + 1] <= k) r++;
-                const int j = sh.rs[grp][r] + (k - sh.pre[grp][r]);
+                while (sh.row[grp][r].x <= k) r++;
+                const int j = k + sh.row[grp][r].y;
                 const int h = pair_test(ld32(d.posr2 + j), pi, margin);
                 const bool intra = d.cm2[j].x == ci.x;
                 hit = h != 0;
                 near = h == 2 && !intra;
                 v = j | (intra ? INTRA : 0) | (near ? NEAR : 0);
             }
-            const unsigned hm = __ballot_sync(gm, hit) >> gshift;
-            const unsigned nm = __ballot_sync(gm, near) >> gshift;
+            const unsigned hm = (__ballot_sync(FULL, hit) >> gshift) & GM;
+            const unsigned nm = (__ballot_sync(FULL, near) >> gshift) & GM;
             if (hit) {
                 const int j = v & SUB_MASK, q = kr + __popc(hm & lt);
                 Nw.bnbr[q] = v & ~NEAR;
@@ -1383,33 +1382,54 @@ static __global__ void __launch_bounds__(SEARCH_THREADS, 8) k_fill(const Dev* __
             }
         }
     }
-    NBC_GRID_STRIDE(u, TK) {
-        const int k = plan_find(d.pclump, ns, u);
+    // the clump pass's lanes of the rebuilt scenes, a warp per warp of the
+    // table: a clump's members change places among its lanes (a thread per
+    // clump and a sort in memory: 64 us for the kernel, so 52)
+    const int nw = gridDim.x * (SEARCH_THREADS / 32), ln = threadIdx.x & 31;
+    for (int u = (blockIdx.x * SEARCH_THREADS + threadIdx.x) / 32; u < TW; u += nw) {
+        const int k = plan_find(d.pwarp, ns, u);
         const int s = d.pscene[k];
         const ScenePar& P = d.par[s];
-        const int c = P.clump_off + (u - d.pclump[k]);
         const int t0 = d.psub[k], tb = t0 - P.sub_off, base = 2 * d.dyn[s].pair_off - cnt_ns[t0];
-        const int mb = d.mem_start[c], me = d.mem_start[c + 1];
-        int2* __restrict__ mo = d.mo;
-        for (int m = mb; m < me; m++) {
+        const int l = (d.clane[P.clump_off] / 32 + (u - d.pwarp[k])) * 32 + ln;
+        int4 ra, rb;
+        ld_rec(d.lrec + 2 * (size_t)l, ra, rb);
+        const int head = ra.w & 31, nm = ra.w >> 5, c = ra.z;
+        const bool mine = c >= 0 && rb.x == s && nm > 0;
+        const bool lanes = mine && nm <= 32;
+        const int x = lanes ? d.inv[ra.x] : 0;
+        int rank = 0;
+        const int most = __reduce_max_sync(0xffffffffu, lanes ? nm : 0);
+        for (int q = 0; q < most; q++) {
+            const int y = __shfl_sync(0xffffffffu, x, head + q);
+            if (lanes && q < nm) rank += y < x;
+        }
+        if (lanes) {
+            const int z = cnt_ns[ra.y + tb];
+            int4* r = d.lrec + 2 * (size_t)(l - ln + head + rank);   // all lanes have read theirs
+            r[0] = make_int4(x, ra.y, c, ra.w);
+            r[1] = make_int4(s, base + z, cnt_ns[ra.y + tb + 1] - z, 0);
+            d.mo[d.mem_start[c] + rank] = make_int2(x, ra.y);
             // the displacement restarts at zero (src/dem_simulation_clump.cu:172)
-            st32(d.cum + m, make_double4(0, 0, 0, 0));
-            mo[m].x = d.inv[mo[m].x];
-        }
-        for (int m = mb + 1; m < me; m++) {
-            const int2 v = mo[m];
-            int q = m - 1;
-            while (q >= mb && mo[q].x > v.x) { mo[q + 1] = mo[q]; q--; }
-            mo[q + 1] = v;
-        }
-        if (mb == me) continue;
-        const int l0 = d.clane[c];
-        for (int m = mb; m < min(me, mb + 32); m++) {
-            const int2 v = mo[m];
-            d.lrec[2 * (l0 + m - mb)].x = v.x;
-            d.lrec[2 * (l0 + m - mb)].y = v.y;
-            const int z = cnt_ns[v.y + tb];
-            d.lrec[2 * (l0 + m - mb) + 1] = make_int4(s, base + z, cnt_ns[v.y + tb + 1] - z, 0);
+            st32(d.cum + ra.y, make_double4(0, 0, 0, 0));
+        } else if (mine && ln == 0) {
+            // a clump of more than 32 members has the warp to itself
+            int2* mo = d.mo;
+            const int mb = d.mem_start[c], me = mb + nm;
+            for (int m = mb; m < me; m++) {
+                st32(d.cum + m, make_double4(0, 0, 0, 0));
+                int2 v = mo[m];
+                v.x = d.inv[v.x];
+                int q = m - 1;
+                while (q >= mb && mo[q].x > v.x) { mo[q + 1] = mo[q]; q--; }
+                mo[q + 1] = v;
+            }
+            for (int q = 0; q < 32; q++) {
+                const int2 v = mo[mb + q];
+                const int z = cnt_ns[v.y + tb];
+                d.lrec[2 * (l + q)] = make_int4(v.x, v.y, c, ra.w);
+                d.lrec[2 * (l + q) + 1] = make_int4(s, base + z, cnt_ns[v.y + tb + 1] - z, 0);
+            }
         }
     }
 }
@@ -1423,91 +1443,150 @@ static __global__ void __launch_bounds__(SEARCH_THREADS, 8) k_fill(const Dev* __
 // changed; pairs absent from it start from zero).  Only near pairs can touch
 // before the next rebuild, so only they have a history, a touch flag and
 // contact slots, and the contact pass visits only them.
+//
+// A warp takes four rows at a time, 8 lanes each; the near entries, one in
+// eight, are put in a queue in shared memory and worked off 32 at a time (done
+// in place they ran on two or three lanes of every warp: 65 us at 50,000
+// clumps, the queue 56; what is left waits on the scattered tmp and records).
+constexpr int ROWS_QUEUE = 64;
+template <typename R>
+__device__ __forceinline__ void near_record(const Dev& d, int i, int s, int4 e) {
+    // e: partner, near pair, listed pair, slot of the back entry (-1: none)
+    const int j = e.x, w = e.y;
+    const size_t cap = (size_t)d.cap;
+    const int* nro = d.nro[0];
+    const int2 ci = d.cm2[i], cj = d.cm2[j];
+    const int io = d.perm[i], jo = d.perm[j];
+    const int oo = min(io, jo), op = max(io, jo);
+    const int sf = d.nsl[ci.y].x + (w - d.nro[1][i + s]), sb = e.w;
+    const int q0 = nro[oo + s], q1 = nro[oo + s + 1];
+    d.rec[1][2 * (size_t)w] = make_int4(i, j, ci.y, cj.y);
+    d.rec[1][2 * (size_t)w + 1] = make_int4(ci.x, cj.x, sf, sb);
+    d.np[1][w] = e.z;
+    // both slots zero until the pair touches
+    R4<R>* slots = (R4<R>*)d.slots;
+    const R4<R> zero = pack<R>(v3<R>(0, 0, 0), R(0));
+    st_pair(slots + 2 * (size_t)sf, zero, zero);
+    if (sb >= 0) st_pair(slots + 2 * (size_t)sb, zero, zero);
+    uint8_t on = 0;
+    // DEMmain::RunSimulation and _Split exchange the history pointers
+    // once more after the list build has carried the histories and
+    // cleared the other buffer (src/dem_simulation_cylind.cu:141,
+    // src/dem_grid.cu:687-749): after a rebuild every pair starts from zero
+    if (!(d.par[s].sphere & SPH_RESET)) {
+        const R4<R>* Hi = (const R4<R>*)d.H[0];
+        R4<R>* Ho = (R4<R>*)d.H[1];
+        const int4* orec = d.rec[0];
+        const R sign = oo == io ? R(1) : R(-1);
+        for (int q = q0; q < q1; q++) {
+            if (orec[2 * (size_t)q].y != op) continue;
+            if (d.touch[0][q]) {
+                R4<R> a, b;
+                ld_pair(Hi + 2 * (size_t)q, a, b);
+                a.x *= sign; a.y *= sign; a.z *= sign; a.w *= sign;
+                b.x *= sign; b.y *= sign; b.z *= sign; b.w *= sign;
+                st_pair(Ho + 2 * (size_t)w, a, b);
+                ((R*)(Ho + 2 * cap))[w] = sign * ((const R*)(Hi + 2 * cap))[q];
+                on = 1;
+            }
+            break;
+        }
+    }
+    d.touch[1][w] = on;
+}
+
 template <typename R>
 __global__ void __launch_bounds__(SEARCH_THREADS) k_rows(const Dev* __restrict__ dp) {
     constexpr int SL = 8;
+    __shared__ int4 s_q[SEARCH_THREADS / 32][ROWS_QUEUE];
+    __shared__ int2 s_own[SEARCH_THREADS / 32][ROWS_QUEUE];   // owner, scene
     const Dev& d = *dp;
     if (*d.halt) return;
     const int T = d.plan[PL_T], ns = d.plan[PL_NS];
-    const int lane = threadIdx.x % SL;
+    const int g = threadIdx.x % SL, ln = threadIdx.x & 31, wp = threadIdx.x / 32;
+    const unsigned lt = (1u << ln) - 1u;
     const PairList& Nw = d.L[1];
     const int2* __restrict__ tmp = d.tmp;
-    const int* __restrict__ nro = d.nro[0];
-    const int4* __restrict__ orec = d.rec[0];
-    const uint8_t* __restrict__ ot = d.touch[0];
-    const R4<R>* __restrict__ Hi = (const R4<R>*)d.H[0];
-    R4<R>* __restrict__ Ho = (R4<R>*)d.H[1];
-    R4<R>* __restrict__ slots = (R4<R>*)d.slots;
-    const size_t cap = (size_t)d.cap;
-    const R4<R> zero = pack<R>(v3<R>(0, 0, 0), R(0));
-    for (int t = (blockIdx.x * SEARCH_THREADS + threadIdx.x) / SL; t < T; t += gridDim.x * (SEARCH_THREADS / SL)) {
-        const PlanItem it = plan_item(d, ns, t);
-        const int i = it.i, s = it.s;
-        const int rf = Nw.row[i + s], n = d.cnt_f[t + 1] - d.cnt_f[t];
-        const int hb = d.par[s].bl / 2;
-        if (lane == 0 && (n > hb || d.cnt_b[t + 1] - d.cnt_b[t] > hb)) {
-            // the reference's row capacity: back rows, and front rows on one level
-            const ScenePar& P = d.par[s];
-            int same = n;
-            if (P.levels > 1) {
-                const int lv = d.level2[i];
-                const int end = d.cstart[P.cell_off + (lv + 1 < P.levels ? P.loff[lv + 1] : P.cellnum - 1)];
-                same = 0;
-                for (int e = 0; e < n; e++) same += (tmp[rf + e].x & SUB_MASK) < end;
+    int4* qe = s_q[wp];
+    int2* qo = s_own[wp];
+    int nq = 0;   // queued entries of the warp
+    auto flush = [&](int from) {
+        __syncwarp();
+        if (from + ln < nq) near_record<R>(d, qo[from + ln].x, qo[from + ln].y, qe[from + ln]);
+        __syncwarp();
+    };
+    // (every lane of a warp takes part in each round: rows past the end are empty)
+    const int rpb = SEARCH_THREADS / SL;
+    for (int b0 = blockIdx.x * rpb + wp * 4; b0 < T; b0 += gridDim.x * rpb) {
+        const int t = b0 + ln / SL;
+        int i = 0, s = 0, rf = 0, n = 0, wn = 0;
+        if (t < T) {
+            const PlanItem it = plan_item(d, ns, t);
+            i = it.i;
+            s = it.s;
+            rf = Nw.row[i + s];
+            wn = d.nro[1][i + s];
+            n = d.cnt_f[t + 1] - d.cnt_f[t];
+            const int hb = d.par[s].bl / 2, nb = d.cnt_b[t + 1] - d.cnt_b[t];
+            if (g == 0 && (n > hb || nb > hb)) {
+                // the reference's row capacity: back rows, and front rows on one level
+                const ScenePar& P = d.par[s];
+                int same = n;
+                if (P.levels > 1) {
+                    const int lv = d.level2[i];
+                    const int end = d.cstart[P.cell_off + (lv + 1 < P.levels ? P.loff[lv + 1] : P.cellnum - 1)];
+                    same = 0;
+                    for (int e = 0; e < n; e++) same += (tmp[rf + e].x & SUB_MASK) < end;
+                }
+                if (same > hb || nb > hb) atomicOr(&d.dyn[s].err, ERR_ROW_OVERFLOW);
             }
-            if (same > hb || d.cnt_b[t + 1] - d.cnt_b[t] > hb) atomicOr(&d.dyn[s].err, ERR_ROW_OVERFLOW);
         }
-        for (int e = lane; e < n; e += SL) {
-            const int2 v = tmp[rf + e];
+        const int most = __reduce_max_sync(0xffffffffu, n);
+        for (int e0 = 0; e0 < most; e0 += SL) {
+            const int e = e0 + g;
+            const bool has = e < n;
+            const int2 v = has ? tmp[rf + e] : make_int2(0, -1);
             const int j = v.x & SUB_MASK;
             int rank = 0, nrank = 0;
-            for (int y = 0; y < n; y++) {
-                const int w = tmp[rf + y].x;
-                if ((w & SUB_MASK) < j) {
-                    rank++;
-                    nrank += (w & NEAR) != 0;
+            if (most <= SL) {   // the row's entries are in the group's lanes
+#pragma unroll
+                for (int y = 0; y < SL; y++) {
+                    const int w = __shfl_sync(0xffffffffu, v.x, y, SL);
+                    if (y < n && (w & SUB_MASK) < j) {
+                        rank++;
+                        nrank += (w & NEAR) != 0;
+                    }
+                }
+            } else if (has) {
+                for (int y = 0; y < n; y++) {
+                    const int w = tmp[rf + y].x;
+                    if ((w & SUB_MASK) < j) {
+                        rank++;
+                        nrank += (w & NEAR) != 0;
+                    }
                 }
             }
             const int p = rf + rank;
-            Nw.nbr[p] = v.x & ~NEAR;
-            Nw.own[p] = i;
-            if (v.y >= 0) Nw.bpair[v.y] = p;
-            if (!(v.x & NEAR)) continue;
-            const int w = d.nro[1][i + s] + nrank;
-            const int2 ci = d.cm2[i], cj = d.cm2[j];
-            const int sf = d.nsl[ci.y].x + nrank, sb = v.y >= 0 ? d.bslot[v.y] : -1;
-            d.rec[1][2 * (size_t)w] = make_int4(i, j, ci.y, cj.y);
-            d.rec[1][2 * (size_t)w + 1] = make_int4(ci.x, cj.x, sf, sb);
-            d.np[1][w] = p;
-            // both slots zero until the pair touches
-            st_pair(slots + 2 * (size_t)sf, zero, zero);
-            if (sb >= 0) st_pair(slots + 2 * (size_t)sb, zero, zero);
-            uint8_t on = 0;
-            // DEMmain::RunSimulation and _Split exchange the history pointers
-            // once more after the list build has carried the histories and
-            // cleared the other buffer (src/dem_simulation_cylind.cu:141,
-            // src/dem_grid.cu:687-749): after a rebuild every pair starts from zero
-            if (!(d.par[s].sphere & SPH_RESET)) {
-                const int io = d.perm[i], jo = d.perm[j];
-                const int oo = min(io, jo), op = max(io, jo);
-                const R sign = oo == io ? R(1) : R(-1);
-                for (int q = nro[oo + s]; q < nro[oo + s + 1]; q++) {
-                    if (orec[2 * (size_t)q].y != op) continue;
-                    if (ot[q]) {
-                        R4<R> a, b;
-                        ld_pair(Hi + 2 * (size_t)q, a, b);
-                        a.x *= sign; a.y *= sign; a.z *= sign; a.w *= sign;
-                        b.x *= sign; b.y *= sign; b.z *= sign; b.w *= sign;
-                        st_pair(Ho + 2 * (size_t)w, a, b);
-                        ((R*)(Ho + 2 * cap))[w] = sign * ((const R*)(Hi + 2 * cap))[q];
-                        on = 1;
-                    }
-                    break;
-                }
+            if (has) {
+                Nw.nbr[p] = v.x & ~NEAR;
+                Nw.own[p] = i;
+                if (v.y >= 0) Nw.bpair[v.y] = p;
             }
-            d.touch[1][w] = on;
+            const bool near = has && (v.x & NEAR);
+            const unsigned nm = __ballot_sync(0xffffffffu, near);
+            if (near) {
+                const int q = nq + __popc(nm & lt);
+                qe[q] = make_int4(j, wn + nrank, p, v.y >= 0 ? d.bslot[v.y] : -1);
+                qo[q] = make_int2(i, s);
+            }
+            nq += __popc(nm);
+            if (nq > ROWS_QUEUE - 32) {
+                flush(nq - 32);
+                nq -= 32;
+            }
         }
     }
+    if (nq > 0) flush(0);
 }
 
 // Commits a rebuild.  When every scene was rebuilt (always for a single
@@ -2467,7 +2546,9 @@ __global__ void __launch_bounds__(ST_THREADS, 1) k_steps(const Dev* __restrict__
             int4 xa = s_lane[threadIdx.x][0], xb = s_lane[threadIdx.x][1];
             for (int w = gw; w < W + sw; w += nw) {
                 const int4 ya = xa, yb = xb;
-                if (w + nw < W) ld_rec(d.lrec + 2 * (size_t)((w + nw) * 32 + lane), xa, xb);   // the next item's
+                if (w + nw < W) {   // the next item's
+                    ld_rec(d.lrec + 2 * (size_t)((w + nw) * 32 + lane), xa, xb);
+                }
                 if (w < W) moved |= clump_warp<R, SPH, true>(d, par ? *par : d.par[yb.x], ya, yb, 1, post, L);
                 else if ((w - W) * 32 + lane < S) scene_step(d, (w - W) * 32 + lane, 1, post, L);
             }

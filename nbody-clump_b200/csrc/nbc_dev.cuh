@@ -103,7 +103,7 @@ constexpr int PL_NS = 0;     // rebuilt scenes
 constexpr int PL_T = 1;      // their subspheres
 constexpr int PL_TC = 2;     // their cell-table entries
 constexpr int PL_T1 = 3;     // PL_T + 1 (scan length of the counts)
-constexpr int PL_TK = 4;     // their clumps
+constexpr int PL_TW = 4;     // warps of the clump pass's table with lanes of theirs
 constexpr int PL_TC1 = 5;    // PL_TC + 1 (scan length of the cell counts)
 constexpr int PL_SIZE = 6;
 
@@ -183,7 +183,7 @@ struct Dev {
     int* pscene;      // [S] rebuilt scenes
     int* psub;        // [S+1] prefix of their subsphere counts
     int* pcell;       // [S+1] prefix of their cell-table entries (cellnum + 1)
-    int* pclump;      // [S+1] prefix of their clump counts
+    int* pwarp;       // [S+1] prefix of the clump pass's warps that hold lanes of theirs
     int* need;        // [S] pairs of the new list of each rebuilt scene, -1 for the others
     int* halt;                            // device flag: pair capacity exceeded, kernels stand still
     // pair lists: the current one and the one a rebuild builds (which becomes
