@@ -347,7 +347,7 @@ nbc_status nbc_union_mass(const double* centres, const double* radii, const int*
  * list rebuild plus a stable radix sort by cell (the order of the engine's
  * sort), with the caller's
  * buffers and one scratch array compiled into the library (NBC_NOALLOC_MAX_N
- * elements, about 2.2 MB per GPU that loads the library, kept until exit).
+ * elements, about 2.5 MB per GPU that loads the library, kept until exit).
  *   pos_dev   device array [n][3] of positions (caller-owned)
  *   grid      the padded grid: origin, cell size, dims, the box whose
  *             outside goes to the last cell (as the engine's hash)

@@ -1332,7 +1332,6 @@ class EngineT final : public EngineBase {
             h_.bidx = m.take<int>(N);
             h_.bprefix = m.take<int>(S_ + 1);
             const long long scan_tiles = std::max(cdiv(N + 1, SC_TILE), cdiv((long long)cells + S_ + 1, SC_TILE));
-            h_.scan_tmp = m.take<int>(scan_tiles + 1);
             h_.scan_st = m.take<unsigned long long>(5 * scan_tiles + 5);
             h_.scan_ctl = m.take<int>(2);
             for (int l = 0; l < 2; l++) {

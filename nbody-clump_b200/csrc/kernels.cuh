@@ -465,10 +465,7 @@ __device__ __forceinline__ int plan_find(const int* __restrict__ pre, int n, int
     return lo;
 }
 
-// --- exclusive scan of ints (three passes) --------------------------------
-// The length is n, or *dn when dn is given (a count computed on the device);
-// the kernels walk the tiles with grid-stride loops, so a fixed grid serves
-// any length.
+// --- exclusive scan of ints -----------------------------------------------
 constexpr int SC_THREADS = 256, SC_ITEMS = 8, SC_TILE = SC_THREADS * SC_ITEMS;
 
 // Exclusive scan over a block of NT threads (every thread calls it); sh:
@@ -498,51 +495,6 @@ __device__ __forceinline__ int block_excl_scan(int v, int* sh, int& total) {
     total = sh[NW - 1];
     __syncthreads();
     return warp_base + x - v;
-}
-
-static __global__ void __launch_bounds__(SC_THREADS) k_scan_tiles(int* __restrict__ a, int n, int* __restrict__ sums,
-                                                           const int* __restrict__ dn) {
-    __shared__ int sh[SC_THREADS / 32];
-    const int nn = dn ? *dn : n;
-    const int tiles = (nn + SC_TILE - 1) / SC_TILE;
-    for (int b = blockIdx.x; b < tiles; b += gridDim.x) {
-        const int base = b * SC_TILE + threadIdx.x * SC_ITEMS;
-        int v[SC_ITEMS], s = 0;
-        for (int j = 0; j < SC_ITEMS; j++) { v[j] = base + j < nn ? a[base + j] : 0; s += v[j]; }
-        int total;
-        int ex = block_excl_scan(s, sh, total);
-        for (int j = 0; j < SC_ITEMS; j++) {
-            if (base + j < nn) a[base + j] = ex;
-            ex += v[j];
-        }
-        if (threadIdx.x == 0) sums[b] = total;
-    }
-}
-
-static __global__ void __launch_bounds__(SC_THREADS) k_scan_sums(int* __restrict__ sums, int nb, const int* __restrict__ dn) {
-    __shared__ int sh[SC_THREADS / 32];
-    if (dn) nb = (*dn + SC_TILE - 1) / SC_TILE;
-    int carry = 0;
-    for (int off = 0; off < nb; off += SC_THREADS) {
-        int i = off + threadIdx.x;
-        int v = i < nb ? sums[i] : 0;
-        int total;
-        int ex = block_excl_scan(v, sh, total);
-        if (i < nb) sums[i] = carry + ex;
-        carry += total;
-    }
-}
-
-static __global__ void __launch_bounds__(SC_THREADS) k_scan_add(int* __restrict__ a, int n, const int* __restrict__ sums,
-                                                         const int* __restrict__ dn) {
-    const int nn = dn ? *dn : n;
-    const int tiles = (nn + SC_TILE - 1) / SC_TILE;
-    for (int b = blockIdx.x; b < tiles; b += gridDim.x) {
-        const int base = b * SC_TILE + threadIdx.x * SC_ITEMS;
-        const int add = sums[b];
-        for (int j = 0; j < SC_ITEMS; j++)
-            if (base + j < nn) a[base + j] += add;
-    }
 }
 
 // --- exclusive scan of ints in one launch (decoupled look-back) ----------
@@ -652,11 +604,6 @@ static __global__ void __launch_bounds__(SC_THREADS) k_scan1(ScanArrays arrs, in
         }
     }
 }
-
-// --- LSD radix sort, 8-bit digits, stable (the reference sorts with CUB's
-// stable DeviceRadixSort, src/dem_grid.cu:278-305); the allocation-free
-// sort (noalloc.cu) uses it, the engine's rebuild sorts by counting --------
-constexpr int RS_THREADS = 256, RS_ITEMS = 8, RS_TILE = RS_THREADS * RS_ITEMS;
 
 // The plan of a rebuild (one block).  Rebuilt scenes are listed in ascending
 // order; their cell keys (cell_off + local cell) ascend with the scene, so
@@ -869,64 +816,6 @@ __global__ void k_order(const Dev* __restrict__ dp) {
         const int k = plan_find(d.pcell, ns, u);
         const ScenePar& P = d.par[d.pscene[k]];
         d.cstart[P.cell_off + (u - d.pcell[k])] = P.sub_off - d.psub[k] + d.ccnt[u];
-    }
-}
-
-// Tiles of RS_TILE keys, n keys (or *dn); the histogram of tile b, digit v
-// sits at hist[v * tiles + b].  Grid-stride over the tiles.
-static __global__ void __launch_bounds__(RS_THREADS) k_rs_hist(const int* __restrict__ keys, int n, int shift,
-                                                        int* __restrict__ hist, const int* __restrict__ dn) {
-    __shared__ int h[256];
-    const int tid = threadIdx.x;
-    const int nn = dn ? *dn : n;
-    const int tiles = (nn + RS_TILE - 1) / RS_TILE;
-    for (int blk = blockIdx.x; blk < tiles; blk += gridDim.x) {
-        h[tid] = 0;
-        __syncthreads();
-        for (int it = 0; it < RS_ITEMS; it++) {
-            const int idx = blk * RS_TILE + it * RS_THREADS + tid;
-            if (idx < nn) atomicAdd(&h[(keys[idx] >> shift) & 255], 1);
-        }
-        __syncthreads();
-        hist[tid * tiles + blk] = h[tid];
-        __syncthreads();
-    }
-}
-
-static __global__ void __launch_bounds__(RS_THREADS) k_rs_scatter(const int* __restrict__ kin, const int* __restrict__ vin,
-                                                           int* __restrict__ kout, int* __restrict__ vout, int n,
-                                                           int shift, const int* __restrict__ hist,
-                                                           const int* __restrict__ dn) {
-    __shared__ int base[256];
-    __shared__ int wcnt[RS_THREADS / 32][257];
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int nn = dn ? *dn : n;
-    const int tiles = (nn + RS_TILE - 1) / RS_TILE;
-    for (int blk = blockIdx.x; blk < tiles; blk += gridDim.x) {
-        base[tid] = hist[tid * tiles + blk];
-        for (int it = 0; it < RS_ITEMS; it++) {
-            for (int w = 0; w < RS_THREADS / 32; w++) wcnt[w][tid] = 0;
-            __syncthreads();
-            const int idx = blk * RS_TILE + it * RS_THREADS + tid;
-            const bool valid = idx < nn;
-            const int k = valid ? kin[idx] : 0;
-            const int dig = valid ? ((k >> shift) & 255) : 256;
-            const unsigned peers = __match_any_sync(0xffffffffu, dig);
-            const int rank = __popc(peers & ((1u << lane) - 1u));
-            if (valid && lane == __ffs(peers) - 1) wcnt[warp][dig] = __popc(peers);
-            __syncthreads();
-            if (valid) {
-                int off = base[dig] + rank;
-                for (int w = 0; w < warp; w++) off += wcnt[w][dig];
-                kout[off] = k;
-                vout[off] = vin[idx];
-            }
-            __syncthreads();
-            int add = 0;
-            for (int w = 0; w < RS_THREADS / 32; w++) add += wcnt[w][tid];
-            base[tid] += add;
-            __syncthreads();
-        }
     }
 }
 

@@ -170,7 +170,6 @@ struct Dev {
     // fill cursors [N]
     int* cnt_f; int* cnt_b; int* cnt_nf; int* cnt_ns; int* xcnt;
     int* fcur;
-    int* scan_tmp;                        // block sums
     unsigned long long* scan_st;          // single-launch scan: tile states (zero between scans)
     int* scan_ctl;                        // single-launch scan: ticket and finished-block counters
     int* scan_fail;                       // a single-launch scan gave up a wait (the step halted)
