@@ -972,7 +972,7 @@ class EngineT final : public EngineBase {
     // kernels of one rebuild in a graph (the eager path adds a k_need): plan,
     // hash, the cell counts' scan, scatter, order, search, the rows' scan,
     // fill, rows, commit
-    int rebuild_launches() const { return 10; }
+    int rebuild_launches() const { return S_ == 1 ? 8 : 10; }
     cudaEvent_t* next_record() {
         if ((size_t)(NMARK * (ev_used_ + 1)) > ev_.size()) {
             for (int k = 0; k < 64 * NMARK; k++) {
@@ -1680,7 +1680,7 @@ class EngineT final : public EngineBase {
         const int B = 128;
         const int gN = std::min(cdiv(N_ + 1, B), sm_count_ * 16);         // grid-stride grids
         const int* pl = h_.plan;
-        k_plan<<<1, SC_THREADS, 0, stream_>>>(d_);
+        if (S_ > 1) k_plan<<<1, SC_THREADS, 0, stream_>>>(d_);
         k_hash<<<gN, B, 0, stream_>>>(d_);
         scan({h_.ccnt}, h_.cells + S_ + 1, pl + PL_TC1);
         k_cscatter<<<gN, B, 0, stream_>>>(d_);
@@ -1709,8 +1709,9 @@ class EngineT final : public EngineBase {
             }
         }
         k_fill<<<gS, SEARCH_THREADS, 0, stream_>>>(d_);
-        k_rows<R><<<std::min(cdiv(8LL * N_, SEARCH_THREADS), sm_count_ * 16), SEARCH_THREADS, 0, stream_>>>(d_);
-        k_commit<R><<<S_ == 1 ? 1 : std::min(sm_count_ * 4, cdiv(8LL * N_, SC_THREADS)), SC_THREADS, 0, stream_>>>(d_);
+        k_rows<R><<<std::min(cdiv(8LL * N_, SEARCH_THREADS), sm_count_ * 16), SEARCH_THREADS, 0, stream_>>>(d_, d_);
+        if (S_ > 1)
+            k_commit<R><<<std::min(sm_count_ * 4, cdiv(8LL * N_, SC_THREADS)), SC_THREADS, 0, stream_>>>(d_);
         CK(cudaGetLastError());
     }
 

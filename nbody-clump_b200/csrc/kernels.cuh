@@ -171,12 +171,16 @@ __device__ __forceinline__ bool clump_warp(const Dev& d, const ScenePar& P, int4
             if (i >= 0) {
                 const uint16_t bb = d.bbits[i];
                 ps = ld32(d.posr + i);
-                V3<R> fr, tr;
-                slot_sum<R>((const R4<R>*)d.slots + 2 * (size_t)sl.x, sl.y, fr, tr);
+                V3<R> fr, tr, fw, tw;   // the boundary's share is on its way while the slots are summed
                 if (bb) {
                     const R4<R>* fbd = (const R4<R>*)d.fbnd;
-                    fr = fr + xyz<R>(fbd[i]);
-                    tr = tr + xyz<R>(fbd[(size_t)d.N + i]);
+                    fw = xyz<R>(fbd[i]);
+                    tw = xyz<R>(fbd[(size_t)d.N + i]);
+                }
+                slot_sum<R>((const R4<R>*)d.slots + 2 * (size_t)sl.x, sl.y, fr, tr);
+                if (bb) {
+                    fr = fr + fw;
+                    tr = tr + tw;
                 }
                 const V3<double> r = v3(ps.x - cp.x, ps.y - cp.y, ps.z - cp.z);
                 f = v3((double)fr.x, (double)fr.y, (double)fr.z);
@@ -520,7 +524,7 @@ struct ScanArrays {
     int* a[5];
     int n;
 };
-static __global__ void __launch_bounds__(SC_THREADS) k_scan1(ScanArrays arrs, int n, const int* __restrict__ dn,
+static __global__ void __launch_bounds__(SC_THREADS) k_scan1(ScanArrays arrs, int n, const int* dn,
                                                             unsigned long long* __restrict__ st, int* __restrict__ ctl,
                                                             int* __restrict__ halt, int* __restrict__ fail) {
     __shared__ int sh[SC_THREADS / 32];
@@ -605,7 +609,24 @@ static __global__ void __launch_bounds__(SC_THREADS) k_scan1(ScanArrays arrs, in
     }
 }
 
-// The plan of a rebuild (one block).  Rebuilt scenes are listed in ascending
+// warps of the clump pass's table that hold lanes of a scene
+__device__ __forceinline__ int table_warps(const Dev& d, const ScenePar& P) {
+    const int c0 = P.clump_off, c1 = c0 + P.nclump - 1, n1 = d.mem_start[c1 + 1] - d.mem_start[c1];
+    return (d.clane[c1] + min(max(n1, 1), 32) - 1) / 32 - d.clane[c0] / 32 + 1;
+}
+__device__ __forceinline__ void plan_totals(const Dev& d, int ns, int nsub, int ncell, int nwarp) {
+    d.psub[ns] = nsub;
+    d.pcell[ns] = ncell;
+    d.pwarp[ns] = nwarp;
+    d.plan[PL_NS] = ns;
+    d.plan[PL_T] = nsub;
+    d.plan[PL_TC] = ncell;
+    d.plan[PL_T1] = nsub + 1;
+    d.plan[PL_TW] = nwarp;
+    d.plan[PL_TC1] = ncell + 1;
+}
+
+// The plan of a rebuild (one block; a single scene's is made by k_hash).  Rebuilt scenes are listed in ascending
 // order; their cell keys (cell_off + local cell) ascend with the scene, so
 // sorting the concatenation of their subspheres keeps every scene in its own
 // range.
@@ -622,9 +643,7 @@ static __global__ void __launch_bounds__(SC_THREADS) k_plan(const Dev* __restric
             const ScenePar& P = d.par[s];
             a1 = P.nsub;
             a2 = P.cellnum + 1;
-            // warps of the clump pass's table that hold lanes of the scene
-            const int c0 = P.clump_off, c1 = c0 + P.nclump - 1, n1 = d.mem_start[c1 + 1] - d.mem_start[c1];
-            a3 = (d.clane[c1] + min(max(n1, 1), 32) - 1) / 32 - d.clane[c0] / 32 + 1;
+            a3 = table_warps(d, P);
         }
         if (s < d.S) d.need[s] = -1;
         int t0, t1, t2, t3;
@@ -643,17 +662,7 @@ static __global__ void __launch_bounds__(SC_THREADS) k_plan(const Dev* __restric
         ncell += t2;
         nwarp += t3;
     }
-    if (threadIdx.x == 0) {
-        d.psub[ns] = nsub;
-        d.pcell[ns] = ncell;
-        d.pwarp[ns] = nwarp;
-        d.plan[PL_NS] = ns;
-        d.plan[PL_T] = nsub;
-        d.plan[PL_TC] = ncell;
-        d.plan[PL_T1] = nsub + 1;
-        d.plan[PL_TW] = nwarp;
-        d.plan[PL_TC1] = ncell + 1;
-    }
+    if (threadIdx.x == 0) plan_totals(d, ns, nsub, ncell, nwarp);
 }
 
 #define NBC_GRID_STRIDE(t, n) for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < (n); t += gridDim.x * blockDim.x)
@@ -671,14 +680,26 @@ static __global__ void __launch_bounds__(SC_THREADS) k_plan(const Dev* __restric
 // cell's range, and k_order finds each element's place among the cell's
 // elements by counting the smaller ones -- the order a stable sort keeps --
 // and moves the element there.
+//
+// A single scene's plan is known to every block and written for the later
+// kernels by the first one: a launch less, and with the commit in k_rows two of
+// ten (53,000 subspheres in FP64: 35.9 -> 35.3 us a step, 1,000,000: 425 -> 416).
 static __global__ void k_hash(const Dev* __restrict__ dp) {
     const Dev& d = *dp;
     if (*d.halt) return;
-    const int T = d.plan[PL_T], ns = d.plan[PL_NS];
+    const bool one = d.S == 1, all = one && d.dyn[0].rebuild;
+    const int T = one ? (all ? d.par[0].nsub : 0) : d.plan[PL_T], ns = one ? 1 : d.plan[PL_NS];
+    if (one && blockIdx.x == 0 && threadIdx.x == 0) {
+        const ScenePar& P = d.par[0];
+        d.need[0] = -1;
+        d.pscene[0] = d.psub[0] = d.pcell[0] = d.pwarp[0] = 0;
+        if (all) plan_totals(d, 1, P.nsub, P.cellnum + 1, table_warps(d, P));
+        else plan_totals(d, 0, 0, 0, 0);
+    }
     NBC_GRID_STRIDE(t, T) {
-        const int k = plan_find(d.psub, ns, t);
-        const ScenePar& P = d.par[d.pscene[k]];
-        const int i = P.sub_off + (t - d.psub[k]);
+        const int k = one ? 0 : plan_find(d.psub, ns, t);
+        const ScenePar& P = d.par[one ? 0 : d.pscene[k]];
+        const int i = P.sub_off + (one ? t : t - d.psub[k]);
         const double4 p = ld32(d.posr + i);
         int local;
         if (P.levels <= 1) {
@@ -708,7 +729,7 @@ static __global__ void k_hash(const Dev* __restrict__ dp) {
                 local = P.loff[lv] + (cz * P.ldim[lv][1] * P.ldim[lv][0] + cy * P.ldim[lv][0] + cx);
             }
         }
-        const int u = d.pcell[k] + local;
+        const int u = (one ? 0 : d.pcell[k]) + local;
         d.kA[t] = u;
         d.vA[t] = atomicAdd(&d.ccnt[u], 1);
     }
@@ -854,7 +875,7 @@ __global__ void k_order(const Dev* __restrict__ dp) {
 // groups for the one candidate in eight that needs them.  50,000 clumps on five
 // levels, 1.7 M pairs: 115 us (both directions with FP64 tests on 8 lanes took
 // 241, and compaction, cross-level sort, reverse map, history carry and near
-// rows another 250 in eight launches where k_fill and k_rows take 52 + 56).
+// rows another 250 in eight launches where k_fill and k_rows take 52 + 50).
 // Half of it is the rows, a third the FP32 tests; votes with a mask per group
 // instead of the whole warp's: 167 us, every lane finding its rows' levels for
 // itself: 125 us, 80 or 94 registers a thread: 9 and 18% more than with 64.
@@ -1336,8 +1357,11 @@ static __global__ void __launch_bounds__(SEARCH_THREADS, 8) k_fill(const Dev* __
 // A warp takes four rows at a time, 8 lanes each; the near entries, one in
 // eight, are put in a queue in shared memory and worked off 32 at a time (done
 // in place they ran on two or three lanes of every warp: 65 us at 50,000
-// clumps, the queue 56; what is left waits on the scattered tmp and records).
+// clumps, the queue 57; a row of up to 32 entries in the group's registers,
+// its keys compared as they go round, instead of read again for each entry: 50;
+// what is left waits on the scattered tmp and records).
 constexpr int ROWS_QUEUE = 64;
+constexpr int ROWS_HELD = 4;   // entries of a row that a lane of its group holds
 template <typename R>
 __device__ __forceinline__ void near_record(const Dev& d, int i, int s, int4 e) {
     // e: partner, near pair, listed pair, slot of the back entry (-1: none)
@@ -1384,11 +1408,24 @@ __device__ __forceinline__ void near_record(const Dev& d, int i, int s, int4 e) 
     d.touch[1][w] = on;
 }
 
+// what the rebuild of every scene built becomes current
+static __device__ __noinline__ void commit_pointers(Dev& w) {
+#define NBC_SWAP(a, b) { auto tmp_ = w.a; w.a = w.b; w.b = tmp_; }
+    NBC_SWAP(posr, posr2) NBC_SWAP(cm, cm2)
+    NBC_SWAP(part_fix, part_fix2) NBC_SWAP(level, level2) NBC_SWAP(key, key2)
+    NBC_SWAP(bhist, bhist2) NBC_SWAP(bbits, bbits2)
+    NBC_SWAP(L[0], L[1]) NBC_SWAP(H[0], H[1]) NBC_SWAP(touch[0], touch[1])
+    NBC_SWAP(nro[0], nro[1]) NBC_SWAP(rec[0], rec[1]) NBC_SWAP(np[0], np[1])
+#undef NBC_SWAP
+}
+
+// (now: the table once more, which the last block of a single scene changes)
 template <typename R>
-__global__ void __launch_bounds__(SEARCH_THREADS) k_rows(const Dev* __restrict__ dp) {
+__global__ void __launch_bounds__(SEARCH_THREADS) k_rows(const Dev* __restrict__ dp, Dev* now) {
     constexpr int SL = 8;
     __shared__ int4 s_q[SEARCH_THREADS / 32][ROWS_QUEUE];
     __shared__ int2 s_own[SEARCH_THREADS / 32][ROWS_QUEUE];   // owner, scene
+    __shared__ int s_last;
     const Dev& d = *dp;
     if (*d.halt) return;
     const int T = d.plan[PL_T], ns = d.plan[PL_NS];
@@ -1431,30 +1468,8 @@ __global__ void __launch_bounds__(SEARCH_THREADS) k_rows(const Dev* __restrict__
             }
         }
         const int most = __reduce_max_sync(0xffffffffu, n);
-        for (int e0 = 0; e0 < most; e0 += SL) {
-            const int e = e0 + g;
-            const bool has = e < n;
-            const int2 v = has ? tmp[rf + e] : make_int2(0, -1);
-            const int j = v.x & SUB_MASK;
-            int rank = 0, nrank = 0;
-            if (most <= SL) {   // the row's entries are in the group's lanes
-#pragma unroll
-                for (int y = 0; y < SL; y++) {
-                    const int w = __shfl_sync(0xffffffffu, v.x, y, SL);
-                    if (y < n && (w & SUB_MASK) < j) {
-                        rank++;
-                        nrank += (w & NEAR) != 0;
-                    }
-                }
-            } else if (has) {
-                for (int y = 0; y < n; y++) {
-                    const int w = tmp[rf + y].x;
-                    if ((w & SUB_MASK) < j) {
-                        rank++;
-                        nrank += (w & NEAR) != 0;
-                    }
-                }
-            }
+        // an entry at its place; near entries to the queue
+        auto place = [&](bool has, int2 v, int rank, int nrank) {
             const int p = rf + rank;
             if (has) {
                 Nw.nbr[p] = v.x & ~NEAR;
@@ -1465,7 +1480,7 @@ __global__ void __launch_bounds__(SEARCH_THREADS) k_rows(const Dev* __restrict__
             const unsigned nm = __ballot_sync(0xffffffffu, near);
             if (near) {
                 const int q = nq + __popc(nm & lt);
-                qe[q] = make_int4(j, wn + nrank, p, v.y >= 0 ? d.bslot[v.y] : -1);
+                qe[q] = make_int4(v.x & SUB_MASK, wn + nrank, p, v.y >= 0 ? d.bslot[v.y] : -1);
                 qo[q] = make_int2(i, s);
             }
             nq += __popc(nm);
@@ -1473,13 +1488,87 @@ __global__ void __launch_bounds__(SEARCH_THREADS) k_rows(const Dev* __restrict__
                 flush(nq - 32);
                 nq -= 32;
             }
+        };
+        if (most <= SL * ROWS_HELD) {
+            // the row in the group's registers: each entry's key (partner, near
+            // flag) goes round once and is compared with all of them
+            int2 v[ROWS_HELD];
+            unsigned key[ROWS_HELD];
+            int rank[ROWS_HELD];   // near entries << 16 | entries before
+#pragma unroll
+            for (int c = 0; c < ROWS_HELD; c++) {
+                const bool has = c * SL + g < n;
+                v[c] = has ? tmp[rf + c * SL + g] : make_int2(0, -1);
+                key[c] = has ? (unsigned)v[c].x << 2 | (v[c].x & NEAR ? 1u : 0u) : 0xffffffffu;
+                rank[c] = 0;
+            }
+#pragma unroll
+            for (int b = 0; b < ROWS_HELD; b++) {
+                if (b * SL >= most) break;
+#pragma unroll
+                for (int y = 0; y < SL; y++) {
+                    const unsigned w = __shfl_sync(0xffffffffu, key[b], y, SL);
+                    const int inc = 1 + (int)((w & 1u) << 16);
+#pragma unroll
+                    for (int c = 0; c < ROWS_HELD; c++)
+                        if (w < key[c]) rank[c] += inc;
+                }
+            }
+#pragma unroll
+            for (int c = 0; c < ROWS_HELD; c++)
+                if (c * SL < most) place(c * SL + g < n, v[c], rank[c] & 0xffff, rank[c] >> 16);
+            continue;
+        }
+        for (int e0 = 0; e0 < most; e0 += SL) {
+            const int e = e0 + g;
+            const bool has = e < n;
+            const int2 v = has ? tmp[rf + e] : make_int2(0, -1);
+            const int j = v.x & SUB_MASK;
+            int rank = 0, nrank = 0;
+            if (has) {
+                for (int y = 0; y < n; y++) {
+                    const int w = tmp[rf + y].x;
+                    if ((w & SUB_MASK) < j) {
+                        rank++;
+                        nrank += (w & NEAR) != 0;
+                    }
+                }
+            }
+            place(has, v, rank, nrank);
         }
     }
     if (nq > 0) flush(0);
+    if (d.S > 1) return;   // k_commit follows
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        s_last = atomicAdd(d.kc_done, 1) == (int)gridDim.x - 1;
+    }
+    __syncthreads();
+    if (!s_last) return;
+    // every block is done with the table
+    if (threadIdx.x == 0) {
+        if (ns) commit_pointers(*now);
+    } else if (threadIdx.x == 32) {
+        *d.kc_done = 0;
+        *d.any_rebuild = 0;
+        *d.step_bar = 0ull;
+    } else if (threadIdx.x == 64 && ns) {
+        SceneDyn& y = d.dyn[0];
+        const int np = d.cnt_f[T], nn = d.cnt_nf[T], nb = y.nbound;
+        y.npairs = np;
+        y.nnear = nn;
+        y.nrebuild++;
+        y.rebuild = 0;
+        d.nprefix[0] = d.bprefix[0] = 0;
+        d.nprefix[1] = nn;
+        d.bprefix[1] = nb;
+    }
 }
 
-// Commits a rebuild.  When every scene was rebuilt (always for a single
-// scene) the gathered buffers, the build list, work records and histories
+// Commits a rebuild of several scenes' engine (a single scene's is committed
+// by the last block of k_rows).  When every scene was
+// rebuilt the gathered buffers, the build list, work records and histories
 // become the current ones by exchanging pointers in the table (one thread).
 // Otherwise the rebuilt scenes' gathered per-subsphere state, rows, list
 // entries, records and histories are copied into the current buffers.  Block 0
@@ -1522,16 +1611,7 @@ __global__ void __launch_bounds__(SC_THREADS) k_commit(Dev* __restrict__ dp) {
         }
     }
     if (ns == d.S) {
-        if (blockIdx.x == 0 && threadIdx.x == 0) {
-            Dev& w = *dp;
-#define NBC_SWAP(a, b) { auto tmp_ = w.a; w.a = w.b; w.b = tmp_; }
-            NBC_SWAP(posr, posr2) NBC_SWAP(cm, cm2)
-            NBC_SWAP(part_fix, part_fix2) NBC_SWAP(level, level2) NBC_SWAP(key, key2)
-            NBC_SWAP(bhist, bhist2) NBC_SWAP(bbits, bbits2)
-            NBC_SWAP(L[0], L[1]) NBC_SWAP(H[0], H[1]) NBC_SWAP(touch[0], touch[1])
-            NBC_SWAP(nro[0], nro[1]) NBC_SWAP(rec[0], rec[1]) NBC_SWAP(np[0], np[1])
-#undef NBC_SWAP
-        }
+        if (blockIdx.x == 0 && threadIdx.x == 0) commit_pointers(*dp);
         return;
     }
     const int T = d.plan[PL_T];
