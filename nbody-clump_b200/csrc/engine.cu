@@ -1847,14 +1847,15 @@ class EngineT final : public EngineBase {
     // warps each, so that its work spreads over the SMs (2,000 spheres in FP64,
     // us a step: 2 warps 12.8, 8 warps 15.2, 16 warps 20.7).  Launches of
     // engines that run beside each other have to fit the GPU together: an engine
-    // of a request server takes a block per 16 warps (8 requests of 400 to
-    // 5,000 clumps: 2 warps 47.5 ms, 16 warps 32.4, 32 warps 32.9, 64 warps 38.6).
+    // of a request server takes a block per 32 warps (8 requests of 400 to
+    // 5,000 clumps: 2 warps 47.5 ms, 16 warps 32 and in one process of five 44,
+    // 32 warps 32 to 34, 64 warps 38.6).
     int step_grid() const {
         int per_sm = 0;
         const void* f = sphere_any_ ? (const void*)k_steps<R, true> : (const void*)k_steps<R, false>;
         CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, f, ST_THREADS, 0));
         const int warps = std::max(h_.W + cdiv(S_, 32), cdiv(2LL * N_, 32));
-        return std::max(1, std::min(per_sm * sm_count_, cdiv(warps, shared_gpu_ ? 16 : 2)));
+        return std::max(1, std::min(per_sm * sm_count_, cdiv(warps, shared_gpu_ ? 32 : 2)));
     }
     void launch_steps(cudaGraphConditionalHandle hif, cudaGraphConditionalHandle hw) {
         cudaLaunchConfig_t c = {};

@@ -545,9 +545,22 @@ static __global__ void __launch_bounds__(SC_THREADS) k_scan1(ScanArrays arrs, in
         int* __restrict__ a = arrs.a[arr];
         unsigned long long* __restrict__ sa = st + (size_t)arr * tiles;
         const int base = b * SC_TILE + threadIdx.x * SC_ITEMS;
+        // eight items a thread in one access (the arrays start on 256 bytes;
+        // one by one: 12.8 us instead of 8.8 for five arrays of 200,000)
+        static_assert(SC_ITEMS == 8, "a 32-byte access per thread");
+        const bool whole = base + SC_ITEMS <= nn;
         int v[SC_ITEMS], sum = 0;
+        if (whole) {
+            int4 p, q;
+            ld_rec((const int4*)(a + base), p, q);
+            v[0] = p.x; v[1] = p.y; v[2] = p.z; v[3] = p.w;
+            v[4] = q.x; v[5] = q.y; v[6] = q.z; v[7] = q.w;
+        } else {
 #pragma unroll
-        for (int j = 0; j < SC_ITEMS; j++) { v[j] = base + j < nn ? a[base + j] : 0; sum += v[j]; }
+            for (int j = 0; j < SC_ITEMS; j++) v[j] = base + j < nn ? a[base + j] : 0;
+        }
+#pragma unroll
+        for (int j = 0; j < SC_ITEMS; j++) sum += v[j];
         int total;
         int ex = block_excl_scan(sum, sh, total);
         if (threadIdx.x < 32) {
@@ -588,8 +601,16 @@ static __global__ void __launch_bounds__(SC_THREADS) k_scan1(ScanArrays arrs, in
         ex += s_excl;
 #pragma unroll
         for (int j = 0; j < SC_ITEMS; j++) {
-            if (base + j < nn) a[base + j] = ex;
-            ex += v[j];
+            const int x = v[j];
+            v[j] = ex;
+            ex += x;
+        }
+        if (whole) {
+            st_rec((int4*)(a + base), make_int4(v[0], v[1], v[2], v[3]), make_int4(v[4], v[5], v[6], v[7]));
+        } else {
+#pragma unroll
+            for (int j = 0; j < SC_ITEMS; j++)
+                if (base + j < nn) a[base + j] = v[j];
         }
     }
     // every block has taken its ticket and is done with the tile states

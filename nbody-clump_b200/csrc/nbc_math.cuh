@@ -118,6 +118,11 @@ __device__ __forceinline__ void ld_rec(const int4* p, int4& a, int4& b) {
                  : "=r"(a.x), "=r"(a.y), "=r"(a.z), "=r"(a.w), "=r"(b.x), "=r"(b.y), "=r"(b.z), "=r"(b.w)
                  : "l"(p));
 }
+__device__ __forceinline__ void st_rec(int4* p, int4 a, int4 b) {
+    asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "r"(a.x), "r"(a.y), "r"(a.z),
+                 "r"(a.w), "r"(b.x), "r"(b.y), "r"(b.z), "r"(b.w)
+                 : "memory");
+}
 
 // body->world rotation (Quat2IvDCM, src/type.h:238-250) applied to u
 __device__ __forceinline__ V3<double> rot_b2w(double4 q, V3<double> u) {
