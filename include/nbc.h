@@ -225,8 +225,8 @@ nbc_status nbc_timing_read(nbc_engine* e, double* contact_ms, int* contact_launc
                            int* rebuilds);
 /* (timing level 2) mean CUDA-event time per timed step, in ms, of its
  * phases: [0] k_clump, [1] the rebuild node (its condition evaluated, the
- * rebuild when taken), [2] k_boundary, [3] k_contact, [4] the whole step from
- * its first kernel to its last (k_boundary runs beside k_contact); no
+ * rebuild when taken), [2] k_boundary, [3] k_pairs, [4] the whole step from
+ * its first kernel to its last (k_boundary runs beside k_pairs); no
  * reference counterpart */
 nbc_status nbc_timing_phases(nbc_engine* e, double* phase_ms);
 /* the launch shapes an engine uses (see nbc_options) and whether its
@@ -310,8 +310,8 @@ nbc_status nbc_server_set_cohort(nbc_server* s, int max_requests);
 
 /* Autotuner (no reference counterpart): times trial_steps steps (after a
  * short warm-up) of engines made from these scenes with candidate launch
- * shapes -- lanes per subsphere of the neighbour search, blocks per SM of
- * the pair kernel -- by coordinate descent from the defaults, a candidate replacing the incumbent only when
+ * shapes -- blocks per SM of the pair kernel, which steps outside the
+ * device-side loop use -- by coordinate descent from the defaults, a candidate replacing the incumbent only when
  * it is at least 3% faster, and writes the fastest into opt (other fields
  * untouched).  The shapes change no result: every candidate computes the
  * same lists and forces bit for bit.  The choice is cached in the process
