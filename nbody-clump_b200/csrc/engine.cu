@@ -1201,10 +1201,8 @@ class EngineT final : public EngineBase {
         h_.cells = cells;
 
         // host arrays: subspheres in the input order, clumps in the engine's
-        std::vector<double4> posr(N_), lom(N_);
         std::vector<int> fix(N_), lev(N_, 0), sid(N_), csid(K_);
         std::vector<int2> cm(N_);
-        std::vector<double4> cpos(K_), cvel(K_), cw(K_), cq(K_), cprop(K_);
         std::vector<int> kind(has_kinds_ ? K_ : 0, 0);
         cold_.resize(K_);
         mstart_.assign(K_ + 1, 0);
@@ -1225,20 +1223,8 @@ class EngineT final : public EngineBase {
                 // any larger index; see k_clump)
                 if (has_kinds_ && D.body_kind) kind[g] = D.body_kind[k] | (std::min(k, 3) << 2);
             }
-            // clump records and body offsets go up in the caller's order and are
-            // put in place on the device
-            for (int k = 0; k < D.n_clump; k++) {
-                const int g = P.clump_off + k;
-                cpos[g] = make_double4(D.clump_pos[3 * k], D.clump_pos[3 * k + 1], D.clump_pos[3 * k + 2], 0);
-                cvel[g] = make_double4(D.clump_vel[3 * k], D.clump_vel[3 * k + 1], D.clump_vel[3 * k + 2], 0);
-                cw[g] = make_double4(D.clump_angvel[3 * k], D.clump_angvel[3 * k + 1], D.clump_angvel[3 * k + 2], 0);
-                cq[g] = make_double4(D.clump_quat[4 * k], D.clump_quat[4 * k + 1], D.clump_quat[4 * k + 2], D.clump_quat[4 * k + 3]);
-                cprop[g] = make_double4(D.clump_prop[4 * k], D.clump_prop[4 * k + 1], D.clump_prop[4 * k + 2], D.clump_prop[4 * k + 3]);
-            }
             for (int i = 0; i < D.n_sub; i++) {
                 int g = P.sub_off + i;
-                lom[g] = make_double4(D.local[3 * i], D.local[3 * i + 1], D.local[3 * i + 2], D.mass[i]);
-                posr[g] = make_double4(D.pos[3 * i], D.pos[3 * i + 1], D.pos[3 * i + 2], D.radius[i]);
                 cm[g].x = now[D.clump_id[i]];
                 fix[g] = i;
                 sid[g] = s;
@@ -1363,12 +1349,34 @@ class EngineT final : public EngineBase {
         copy_(h_.dyn, hdyn.data(), S_ * sizeof(SceneDyn), cudaMemcpyHostToDevice);
         copy_(h_.sid, sid.data(), N * sizeof(int), cudaMemcpyHostToDevice);
         copy_(h_.csid, csid.data(), K_ * sizeof(int), cudaMemcpyHostToDevice);
-        copy_(h_.posr, posr.data(), N * sizeof(double4), cudaMemcpyHostToDevice);
         copy_(h_.cm, cm.data(), N * sizeof(int2), cudaMemcpyHostToDevice);
         copy_(h_.part_fix, fix.data(), N * sizeof(int), cudaMemcpyHostToDevice);
         copy_(h_.level, lev.data(), N * sizeof(int), cudaMemcpyHostToDevice);
-        copy_(h_.posr2, lom.data(), N * sizeof(double4), cudaMemcpyHostToDevice);
-        k_members_in<<<std::min(cdiv(N_, 256), sm_count_ * 8), 256, 0, stream_>>>(h_.posr2, h_.cm, N_, h_.lom);
+        // the caller's arrays go up as they are (several scenes': one after the
+        // other) and are packed into records and put in place on the device
+        std::vector<double> joined;
+        auto upload = [&](double* dst, const double* nbc_scene_desc::*field, bool members, int width) {
+            const size_t total = (size_t)width * (members ? N_ : K_);
+            const double* src = sc[0]->*field;
+            if (S_ > 1) {
+                joined.resize(total);
+                for (int s = 0; s < S_; s++) {
+                    const ScenePar& P = hpar_[s];
+                    memcpy(&joined[(size_t)width * (members ? P.sub_off : P.clump_off)], sc[s]->*field,
+                           sizeof(double) * width * (members ? P.nsub : P.nclump));
+                }
+                src = joined.data();
+            }
+            copy_(dst, src, total * sizeof(double), cudaMemcpyHostToDevice);
+        };
+        double *so = (double*)h_.posr2, *sp = (double*)h_.kin;   // 4 N doubles each, not in use yet
+        upload(so, &nbc_scene_desc::local, true, 3);
+        upload(so + 3 * N, &nbc_scene_desc::mass, true, 1);
+        upload(sp, &nbc_scene_desc::pos, true, 3);
+        upload(sp + 3 * N, &nbc_scene_desc::radius, true, 1);
+        k_members_up<<<std::min(cdiv(N_, 256), sm_count_ * 8), 256, 0, stream_>>>(so, sp, h_.cm, N_, h_.lom, h_.posr);
+        CK(cudaGetLastError());
+        CK(cudaMemsetAsync(h_.kin, 0, N * sizeof(double4), stream_));
         {
             std::vector<int> abs(K_);
             for (int s = 0; s < S_; s++)
@@ -1376,24 +1384,21 @@ class EngineT final : public EngineBase {
                     abs[c] = hpar_[s].clump_off + cold_[c];
             copy_(h_.cold, abs.data(), K_ * sizeof(int), cudaMemcpyHostToDevice);
         }
-        auto clumps_in = [&](const std::vector<double4>& src, double4* dst) {
-            copy_(h_.stage, src.data(), K_ * sizeof(double4), cudaMemcpyHostToDevice);
-            k_clumps_in<<<std::min(cdiv(K_, 256), sm_count_ * 8), 256, 0, stream_>>>(h_.stage, h_.cold, K_, dst);
-            CK(cudaGetLastError());
+        const int gc = std::min(cdiv(K_, 256), sm_count_ * 8);
+        double* st = (double*)h_.stage;
+        auto clumps_up = [&](const double* nbc_scene_desc::*field, double4* dst) {
+            upload(st, field, false, 3);
+            k_clumps_up<3><<<gc, 256, 0, stream_>>>(st, h_.cold, K_, dst, nullptr);
         };
-        clumps_in(cpos, h_.cpos);
-        clumps_in(cvel, h_.cvel);
-        clumps_in(cw, h_.cw);
-        clumps_in(cq, h_.cq);
-        clumps_in(cprop, h_.cprop);
+        clumps_up(&nbc_scene_desc::clump_pos, h_.cpos);
+        clumps_up(&nbc_scene_desc::clump_vel, h_.cvel);
+        clumps_up(&nbc_scene_desc::clump_angvel, h_.cw);
+        upload(st, &nbc_scene_desc::clump_quat, false, 4);
+        k_clumps_up<4><<<gc, 256, 0, stream_>>>(st, h_.cold, K_, h_.cq, nullptr);
+        upload(st, &nbc_scene_desc::clump_prop, false, 4);
+        k_clumps_up<4><<<gc, 256, 0, stream_>>>(st, h_.cold, K_, h_.cprop, h_.cinv);
+        CK(cudaGetLastError());
         if (h_.kind) copy_(h_.kind, kind.data(), K_ * sizeof(int), cudaMemcpyHostToDevice);
-        {
-            // the clump pass's reciprocals: IEEE divisions, bitwise those it formed each step
-            std::vector<double4> cinv(K_);
-            for (int k = 0; k < K_; k++)
-                cinv[k] = make_double4(1.0 / cprop[k].x, 1.0 / cprop[k].y, 1.0 / cprop[k].z, 1.0 / cprop[k].w);
-            clumps_in(cinv, h_.cinv);
-        }
         copy_(h_.clane, clane_.data(), K_ * sizeof(int), cudaMemcpyHostToDevice);
         copy_(h_.mem_start, mstart_.data(), (K_ + 1) * sizeof(int), cudaMemcpyHostToDevice);
         // the first list is empty: rows of zeros (the slab is zeroed)

@@ -392,10 +392,9 @@ __global__ void __launch_bounds__(CL_THREADS, NBC_CLUMP_MINB) k_clump(const Dev*
     }
 }
 
-// Clump records between the engine's order and the caller's (old: the
-// caller's number of each): the n clumps from `first` on, a scene's, out of the
-// engine as W packed doubles per clump, ready to be copied to the caller's
-// array; all of them into it as whole records.
+// Clump records (old: the caller's number of each): the n clumps from `first`
+// on, a scene's, out of the engine as W packed doubles per clump, ready to be
+// copied to the caller's array.
 template <int W>
 static __global__ void k_clumps_out(const double4* __restrict__ src, const int* __restrict__ old, int first, int n,
                                     double* __restrict__ dst) {
@@ -406,18 +405,30 @@ static __global__ void k_clumps_out(const double4* __restrict__ src, const int* 
         if (W == 4) o[3] = v.w;
     }
 }
-static __global__ void k_clumps_in(const double4* __restrict__ src, const int* __restrict__ old, int n,
-                                   double4* __restrict__ dst) {
-    for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < n; c += gridDim.x * blockDim.x)
-        st32(dst + c, ld32(src + old[c]));
+// the caller's arrays of W doubles per clump into records in the engine's
+// order; inv: the reciprocals as well (IEEE divisions)
+template <int W>
+static __global__ void k_clumps_up(const double* __restrict__ src, const int* __restrict__ old, int n,
+                                   double4* __restrict__ dst, double4* __restrict__ inv) {
+    for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < n; c += gridDim.x * blockDim.x) {
+        const double* p = src + (size_t)W * old[c];
+        const double4 v = make_double4(p[0], p[1], p[2], W == 4 ? p[W - 1] : 0.0);
+        st32(dst + c, v);
+        if (inv)
+            st32(inv + c, make_double4(__ddiv_rn(1.0, v.x), __ddiv_rn(1.0, v.y), __ddiv_rn(1.0, v.z), __ddiv_rn(1.0, v.w)));
+    }
 }
-// member records from the caller's subsphere order into their slots
-static __global__ void k_members_in(const double4* __restrict__ src, const int2* __restrict__ cm, int n,
-                                    double4* __restrict__ dst) {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-        st32(dst + cm[i].y, ld32(src + i));
+// body offset and mass (so) into the member's slot, position and radius (sp)
+// into the subsphere's record: of both 3 n doubles, then n
+static __global__ void k_members_up(const double* __restrict__ so, const double* __restrict__ sp,
+                                    const int2* __restrict__ cm, int n, double4* __restrict__ lom,
+                                    double4* __restrict__ posr) {
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        const size_t q = 3 * (size_t)i, w = 3 * (size_t)n + i;
+        st32(lom + cm[i].y, make_double4(so[q], so[q + 1], so[q + 2], so[w]));
+        st32(posr + i, make_double4(sp[q], sp[q + 1], sp[q + 2], sp[w]));
+    }
 }
-
 // the member lists in subsphere order, and the clump pass's lanes (idle ones,
 // then those of every clump: see Dev::lrec)
 static __global__ void k_members_init(const Dev* __restrict__ dp) {
