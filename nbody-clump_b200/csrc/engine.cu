@@ -968,11 +968,10 @@ class EngineT final : public EngineBase {
         for (auto& v : y) n = std::max(n, v.nrebuild);
         return n;
     }
-    // kernels one rebuild launches (launch_rebuild)
-    // kernels of one rebuild in a graph (the eager path adds a k_need): plan,
-    // hash, the cell counts' scan, scatter, order, search, the rows' scan,
-    // fill, rows, commit
-    int rebuild_launches() const { return S_ == 1 ? 8 : 10; }
+    // kernels of one rebuild in a graph (launch_rebuild; the eager path adds a
+    // k_need): plan, hash, the cell counts' scan, scatter, order, the two
+    // searches, the rows' scan, fill, rows, commit
+    int rebuild_launches() const { return S_ == 1 ? 9 : 11; }
     cudaEvent_t* next_record() {
         if ((size_t)(NMARK * (ev_used_ + 1)) > ev_.size()) {
             for (int k = 0; k < 64 * NMARK; k++) {
@@ -1119,7 +1118,16 @@ class EngineT final : public EngineBase {
                     off += P.ldim[l][0] * P.ldim[l][1] * P.ldim[l][2];
                 }
                 P.cellnum = off + 1;
+                for (int l = 0; l < P.levels; l++)
+                    for (int f = l + 1; f < P.levels; f++)
+                        if (1.5 * ((double)P.lrmax[l] + P.lrmax[f]) >= P.lcell[l]) P.tight = 1;
             }
+            P.inside = 1;
+            for (int l = 0; l < P.levels; l++)
+                for (int a = 0; a < 3; a++) {
+                    const double ext = P.levels > 1 ? P.ldim[l][a] * P.lcell[l] : P.gdim[a] * P.cell[a];
+                    if (!(P.box_lo[a] >= P.origin[a] && P.box_hi[a] - P.origin[a] <= ext * (1.0 - 1e-9))) P.inside = 0;
+                }
             P.cell_off = cells;
             cells += P.cellnum;
             P.sub_off = N_;
@@ -1692,6 +1700,7 @@ class EngineT final : public EngineBase {
         k_order<R><<<gN, B, 0, stream_>>>(d_);
         const int gS = std::min(cdiv((long long)N_ * SEARCH_G, SEARCH_THREADS), sm_count_ * 16);
         k_search<<<gS, SEARCH_THREADS, 0, stream_>>>(d_);
+        k_search_faces<<<std::min(gS, sm_count_ * 4), SEARCH_THREADS, 0, stream_>>>(d_);
         scan({h_.cnt_f, h_.cnt_b, h_.cnt_nf, h_.cnt_ns, h_.xcnt}, N_ + 1, pl + PL_T1);
         CK(cudaGetLastError());
         if (eager) {

@@ -699,6 +699,25 @@ static __global__ void __launch_bounds__(SC_THREADS) k_plan(const Dev* __restric
 
 #define NBC_GRID_STRIDE(t, n) for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < (n); t += gridDim.x * blockDim.x)
 
+// Cells on faces.  The reference sorts by floor((x - origin) / cell) and, on a
+// single-level grid, centres its search on floor((x - origin) * (1 / cell))
+// (src/dem_grid.cu:155-202,466-552); its hierarchical search divides.  For a
+// coordinate on a cell's face, or within rounding of it, the two can differ;
+// lattices at rest with round radii are full of such coordinates, a settled bed
+// has none.  k_search finds cells by a product and takes the rows before a
+// subsphere's own cell as sorted before it, so it needs them equal.  k_hash
+// compares them: a rebuild in which some differ (or were clamped into the grid)
+// sets plan[PL_FACE] and is searched by k_search_faces.  On coarser levels than
+// a subsphere's own it compares them where the cells are no larger than the
+// reach (ScenePar::tight); in larger ones both find every pair.
+__device__ __forceinline__ int cell_coord(double x, double c) { return (int)floor(x / c); }
+// whether the product with inv = 1 / c gives another cell than the quotient (it
+// is off by less than 2^-50 of itself, 2^-19 at 2^31 cells)
+__device__ __forceinline__ bool cells_differ(double x, double c, double inv) {
+    const double t = x * inv;
+    return !(fabs(t - rint(t)) > 1e-5) && (int)floor(t) != cell_coord(x, c);
+}
+
 // GetParticleCellIndex_cuk (src/dem_grid.cu:155-202); hierarchical variant
 // GetParticleCellIndex_hGrid_cuk (src/dem_hgrid.cu:205-242) with the
 // out-of-box bucket kept inside the scene's cell range.  Element t of the
@@ -714,8 +733,8 @@ static __global__ void __launch_bounds__(SC_THREADS) k_plan(const Dev* __restric
 // and moves the element there.
 //
 // A single scene's plan is known to every block and written for the later
-// kernels by the first one: a launch less, and with the commit in k_rows two of
-// ten (53,000 subspheres in FP64: 35.9 -> 35.3 us a step, 1,000,000: 425 -> 416).
+// kernels by the first one: a launch less, and with the commit in k_rows two
+// (53,000 subspheres in FP64: 35.9 -> 35.3 us a step, 1,000,000: 425 -> 416).
 static __global__ void k_hash(const Dev* __restrict__ dp) {
     const Dev& d = *dp;
     if (*d.halt) return;
@@ -733,18 +752,19 @@ static __global__ void k_hash(const Dev* __restrict__ dp) {
         const ScenePar& P = d.par[one ? 0 : d.pscene[k]];
         const int i = P.sub_off + (one ? t : t - d.psub[k]);
         const double4 p = ld32(d.posr + i);
+        const double x = p.x - P.origin[0], y = p.y - P.origin[1], z = p.z - P.origin[2];
         int local;
+        bool face = false;
         if (P.levels <= 1) {
             if (p.z >= P.box_hi[2] || p.y >= P.box_hi[1] || p.x >= P.box_hi[0] ||
                 p.z < P.box_lo[2] || p.y < P.box_lo[1] || p.x < P.box_lo[0]) {
                 local = P.cellnum - 1;
             } else {
-                int cx = (int)floor((p.x - P.origin[0]) / P.cell[0]);
-                int cy = (int)floor((p.y - P.origin[1]) / P.cell[1]);
-                int cz = (int)floor((p.z - P.origin[2]) / P.cell[2]);
-                cx = clampi(cx, 0, P.gdim[0] - 1);
-                cy = clampi(cy, 0, P.gdim[1] - 1);
-                cz = clampi(cz, 0, P.gdim[2] - 1);
+                const int cx = clampi(cell_coord(x, P.cell[0]), 0, P.gdim[0] - 1);
+                const int cy = clampi(cell_coord(y, P.cell[1]), 0, P.gdim[1] - 1);
+                const int cz = clampi(cell_coord(z, P.cell[2]), 0, P.gdim[2] - 1);
+                face = cx != (int)floor(x * P.icell[0]) || cy != (int)floor(y * P.icell[1]) ||
+                       cz != (int)floor(z * P.icell[2]);
                 local = cz * P.gdim[1] * P.gdim[0] + cy * P.gdim[0] + cx;
                 local = clampi(local, 0, P.cellnum - 1);
             }
@@ -754,13 +774,19 @@ static __global__ void k_hash(const Dev* __restrict__ dp) {
                 local = P.cellnum - 1;
             } else {
                 const int lv = d.level[i];
-                const double c = P.lcell[lv];
-                const int cx = clampi((int)floor((p.x - P.origin[0]) / c), 0, P.ldim[lv][0] - 1);
-                const int cy = clampi((int)floor((p.y - P.origin[1]) / c), 0, P.ldim[lv][1] - 1);
-                const int cz = clampi((int)floor((p.z - P.origin[2]) / c), 0, P.ldim[lv][2] - 1);
+                const double c = P.lcell[lv], in = P.licell[lv];
+                const int cx = clampi(cell_coord(x, c), 0, P.ldim[lv][0] - 1);
+                const int cy = clampi(cell_coord(y, c), 0, P.ldim[lv][1] - 1);
+                const int cz = clampi(cell_coord(z, c), 0, P.ldim[lv][2] - 1);
+                face = cx != (int)floor(x * in) || cy != (int)floor(y * in) || cz != (int)floor(z * in);
+                if (P.tight)   // the coarser levels it searches
+                    for (int l = 0; l < lv; l++)
+                        face |= cells_differ(x, P.lcell[l], P.licell[l]) | cells_differ(y, P.lcell[l], P.licell[l]) |
+                                cells_differ(z, P.lcell[l], P.licell[l]);
                 local = P.loff[lv] + (cz * P.ldim[lv][1] * P.ldim[lv][0] + cy * P.ldim[lv][0] + cx);
             }
         }
+        if (face) d.plan[PL_FACE] = 1;
         const int u = (one ? 0 : d.pcell[k]) + local;
         d.kA[t] = u;
         d.vA[t] = atomicAdd(&d.ccnt[u], 1);
@@ -919,6 +945,7 @@ constexpr int SEARCH_THREADS = 128;
 constexpr int SEARCH_G = 8;                   // lanes per subsphere
 constexpr int SEARCH_GROUPS = SEARCH_THREADS / SEARCH_G;
 constexpr int SCR_CAP = 64;                   // scratch entries per back row
+constexpr int ROW_LONG = 1, ROW_FACES = 2;     // Dev::rlong: the row is not in the scratch; made by fill_faces
 constexpr int LIST_CAP = 32;                  // FP32 hits held before they are tested in FP64
 constexpr int MAX_ROWS = 5 + 9 * (MAX_LEVELS - 1);
 constexpr int NEAR = 0x40000000;              // scratch: the pair can touch before the next rebuild
@@ -951,18 +978,78 @@ __device__ __forceinline__ int pair_test(double4 a, double4 b, double margin) {
 // 2 Thresh cannot touch before the next one.
 __device__ __forceinline__ double near_margin(const ScenePar& P) { return 2.0 * P.thresh * (1.0 + 1e-6) + 1e-12; }
 
+// FACES (k_search_faces, and fill_faces' rows): own cells as
+// the sort has them, and the reference's stencils.  A pair belongs to the list
+// when the owner's stencil holds the partner's cell, and has a back entry when
+// the partner's holds the owner's; across levels the finer one's stencil decides
+// both.  The two disagree only on pairs about a cell apart on a single level,
+// where an owner whose product lies in the next cell may list partners two cells
+// on, and on subspheres outside the grid.  Where the partner alone would list
+// the other there is no pair to refer to, and no entry.
+//
+// The rows on a single level then: two cells to each side, as far as the reach
+// goes (r of 13, the last one the subsphere's own).
+constexpr int FACE_ROWS = 13;
+__device__ __forceinline__ bool face_row(const ScenePar& P, double4 pi, int r, int& ca, int& cb) {
+    const double x = pi.x - P.origin[0], y = pi.y - P.origin[1], z = pi.z - P.origin[2], c = P.cell[0];   // cells are cubes
+    const int gx = P.gdim[0], gy = P.gdim[1], gz = P.gdim[2];
+    const int cx = clampi(cell_coord(x, c), 0, gx - 1), cy = clampi(cell_coord(y, c), 0, gy - 1);
+    const int cz = clampi(cell_coord(z, c), 0, gz - 1);
+    const int sz = r / 5 - 2, sy = r % 5 - 2;
+    if (cz + sz < 0 || cy + sy < 0 || cy + sy >= gy) return false;
+    const float cf = (float)c, cut = 1.5f * ((float)pi.w + P.lrmax[0]) * 1.0001f + 1e-4f * cf;
+    // squared distance to the cells s away along an axis, f from the own cell's lower face
+    auto dist2 = [&](int q, int n, int s, float f) {
+        const float h = s < 0 ? f - (float)(s + 1) * cf : (float)s * cf - f;
+        return s == 0 || q + s == 0 || q + s == n - 1 ? 0.0f : h * h;
+    };
+    const float rem = cut * cut - dist2(cz, gz, sz, (float)(z - cz * c)) - dist2(cy, gy, sy, (float)(y - cy * c));
+    if (!(rem >= 0)) return false;
+    const float fx = (float)(x - cx * c);
+    int lo = max(-2, -cx), hi = min(2, gx - 1 - cx);
+    while (lo < 0 && dist2(cx, gx, lo, fx) > rem) lo++;
+    while (hi > 0 && dist2(cx, gx, hi, fx) > rem) hi--;
+    const int m = P.cell_off + ((cz + sz) * gy + cy + sy) * gx + cx;
+    ca = m + lo;
+    cb = m + hi + 1;
+    return true;
+}
+// Whose stencil holds the other's cell, of a pair j < i: 1 the owner's, 2 that
+// of i.  Both when they are less than a cell apart on every axis (the cells'
+// rounding is 2^-50 of a coordinate) in a box inside the grid.
+__device__ __forceinline__ int face_sides(const Dev& d, const ScenePar& P, int j, double4 pj, int i, double4 pi) {
+    const bool hg = P.levels > 1;
+    const int l = hg ? d.level2[i] : 0;
+    if (hg && d.level2[j] != l) return 3;
+    const double c = hg ? P.lcell[l] : P.cell[0];
+    if (P.inside && fmax(fmax(fabs(pi.x - pj.x), fabs(pi.y - pj.y)), fabs(pi.z - pj.z)) < c * (1.0 - 1e-6)) return 3;
+    int sides = 3;
+#pragma unroll 1
+    for (int a = 0; a < 3; a++) {
+        const double xj = (a == 0 ? pj.x : (a == 1 ? pj.y : pj.z)) - P.origin[a];
+        const double xi = (a == 0 ? pi.x : (a == 1 ? pi.y : pi.z)) - P.origin[a];
+        const int top = (hg ? P.ldim[l][a] : P.gdim[a]) - 1, uj = cell_coord(xj, c), ui = cell_coord(xi, c);
+        const int mj = hg ? uj : (int)floor(xj * P.icell[a]), mi = hg ? ui : (int)floor(xi * P.icell[a]);
+        if ((unsigned)clampi(ui, 0, top) - (unsigned)mj + 1u > 2u) sides &= ~1;
+        if ((unsigned)clampi(uj, 0, top) - (unsigned)mi + 1u > 2u) sides &= ~2;
+    }
+    return sides;
+}
+
 // The stencil rows of subsphere i by the G lanes of its group (g of them):
 // candidates j < i as ranges in back-row order; the number of candidates.
 // Every lane of the warp calls it; `on`: the group has a subsphere.  (The
 // warp's groups run in step, votes and shuffles over the whole warp: with a
 // mask per group the compiler takes the groups through them one by one.)
+template <bool FACES>
 __device__ __forceinline__ int group_rows(const Dev& d, const ScenePar& P, bool on, int i, double4 pi, int g,
                                           SearchRows& sh, int grp) {
     constexpr int G = SEARCH_G, MAXC = (MAX_ROWS + G - 1) / G;
     const int* __restrict__ cstart = d.cstart;
     const bool hg = P.levels > 1;
     const int my = hg && on ? d.level2[i] : 0;
-    const int nrows = on ? 5 + 9 * my : 0, r0 = nrows * g / G, r1 = nrows * (g + 1) / G;
+    const bool wide = FACES && !hg;
+    const int nrows = on ? (wide ? FACE_ROWS : 5 + 9 * my) : 0, r0 = nrows * g / G, r1 = nrows * (g + 1) / G;
     int2* rows = sh.row[grp];
     __syncwarp();   // the previous rows and levels are no longer read
     if (on && g <= my) {
@@ -981,7 +1068,14 @@ __device__ __forceinline__ int group_rows(const Dev& d, const ScenePar& P, bool 
             i0 = P.icell[0]; i1 = P.icell[1]; i2 = P.icell[2];
         }
         const double x0 = pi.x - P.origin[0], y0 = pi.y - P.origin[1], z0 = pi.z - P.origin[2];
-        const int cx = (int)floor(x0 * i0), cy = (int)floor(y0 * i1), cz = (int)floor(z0 * i2);
+        int cx = FACES ? cell_coord(x0, c0) : (int)floor(x0 * i0);
+        int cy = FACES ? cell_coord(y0, c1) : (int)floor(y0 * i1);
+        int cz = FACES ? cell_coord(z0, c2) : (int)floor(z0 * i2);
+        if (FACES && g == 0) {   // on its own level
+            cx = clampi(cx, 0, gx - 1);
+            cy = clampi(cy, 0, gy - 1);
+            cz = clampi(cz, 0, gz - 1);
+        }
         const float fx = (float)(x0 - cx * c0), fy = (float)(y0 - cy * c1), fz = (float)(z0 - cz * c2);
         const float ux = (float)c0 - fx, uy = (float)c1 - fy, uz = (float)c2 - fz;
         const float cut = 1.5f * ((float)pi.w + P.lrmax[l]) * 1.0001f + 1e-4f * (float)c0;
@@ -1007,6 +1101,10 @@ __device__ __forceinline__ int group_rows(const Dev& d, const ScenePar& P, bool 
         ca[k] = -1;
         cb[k] = -1;
         if (r >= r1) continue;
+        if (wide) {
+            face_row(P, pi, r, ca[k], cb[k]);
+            continue;
+        }
         const int q = r < 5 ? 0 : 1 + (r - 5) / 9, rr = r < 5 ? r : (r - 5) % 9;
         const int sz = rr / 3 - 1, sy = rr % 3 - 1;
         const float4 fz = sh.dist[grp][q][0], fy = sh.dist[grp][q][1];
@@ -1024,7 +1122,7 @@ __device__ __forceinline__ int group_rows(const Dev& d, const ScenePar& P, bool 
     for (int k = 0; k < MAXC; k++) {
         if (ca[k] < 0) continue;
         ca[k] = cstart[ca[k]];
-        cb[k] = r0 + k == 4 ? i : cstart[cb[k]];
+        cb[k] = r0 + k == (wide ? FACE_ROWS - 1 : 4) ? i : cstart[cb[k]];
     }
     // rows with candidates, packed: (rows << 24 | candidates) summed over the lanes
     unsigned acc = 0;
@@ -1080,18 +1178,14 @@ __device__ __forceinline__ bool searches(const Dev& d, const ScenePar& P, int i)
 // there are front-only partners), their lengths (cnt_b), those of
 // the front rows (cnt_f) and of the near front rows (cnt_nf), and the contact
 // slots of each member slot (cnt_ns: near entries of both rows).
-static __global__ void __launch_bounds__(SEARCH_THREADS, 8) k_search(const Dev* __restrict__ dp) {
+template <bool FACES>
+__device__ __forceinline__ void search_rows(const Dev& d, SearchRows& sh, int (*s_buf)[LIST_CAP]) {
     constexpr int G = SEARCH_G;
-    __shared__ SearchRows sh;
-    __shared__ int s_buf[SEARCH_GROUPS][LIST_CAP];
-    const Dev& d = *dp;
-    if (*d.halt) return;
-    const int T = d.plan[PL_T], ns = d.plan[PL_NS], TC1 = d.plan[PL_TC1];
+    const int T = d.plan[PL_T], ns = d.plan[PL_NS];
     const int g = threadIdx.x % G, grp = threadIdx.x / G;
     const int gshift = (threadIdx.x & 31) & ~(G - 1);
     constexpr unsigned GM = (1u << G) - 1u;
     const unsigned lt = (1u << g) - 1u;
-    NBC_GRID_STRIDE(u, TC1) d.ccnt[u] = 0;   // the sort's cell counts back to zero for the next rebuild
     const double4* __restrict__ posr = d.posr2;
     const float4* __restrict__ posf = d.posf;
     const int2* __restrict__ cm = d.cm2;
@@ -1110,7 +1204,7 @@ static __global__ void __launch_bounds__(SEARCH_THREADS, 8) k_search(const Dev* 
         const double4 pi = ld32(posr + i);
         const float4 pf = posf[i];
         const int2 ci = cm[i];
-        const int total = group_rows(d, P, on, i, pi, g, sh, grp);
+        const int total = group_rows<FACES>(d, P, on, i, pi, g, sh, grp);
         const int most = __reduce_max_sync(FULL, total);
         // the candidates in order, G at a time (the next ones' positions in
         // flight): what passes goes to the list through a vote, and a list that
@@ -1118,6 +1212,7 @@ static __global__ void __launch_bounds__(SEARCH_THREADS, 8) k_search(const Dev* 
         const double margin = near_margin(P);
         int* __restrict__ scr = d.scr + (size_t)i * SCR_CAP;
         int nb = 0, near = 0, n = 0, r = 0, jn = -1;
+        bool alone = false;   // (FACES) some entry without a back entry: the row is made by k_fill
         float4 qn = make_float4(0, 0, 0, 0);
         auto next = [&](int f) {
             jn = -1;
@@ -1148,12 +1243,18 @@ static __global__ void __launch_bounds__(SEARCH_THREADS, 8) k_search(const Dev* 
                     ck = cm[k];
                     hit = pair_test(ld32(posr + k), pi, margin);
                 }
+                int sides = 3;
+                if (FACES && hit) {
+                    sides = face_sides(d, P, k, ld32(posr + k), i, pi);
+                    if (!(sides & 1)) hit = 0;
+                    if (sides == 1) alone = true;
+                }
                 const bool nr = hit == 2 && ck.x != ci.x;
-                const unsigned hm = (__ballot_sync(FULL, hit != 0) >> gshift) & GM;
-                const unsigned nm = (__ballot_sync(FULL, nr) >> gshift) & GM;
+                const unsigned hm = (__ballot_sync(FULL, hit != 0 && sides == 3) >> gshift) & GM;
+                const unsigned nm = (__ballot_sync(FULL, nr && sides == 3) >> gshift) & GM;
                 if (hit) {
                     const int q = nb + __popc(hm & lt);
-                    if (q < SCR_CAP) scr[q] = k | (ck.x == ci.x ? INTRA : 0) | (nr ? NEAR : 0);
+                    if (q < SCR_CAP && sides == 3) scr[q] = k | (ck.x == ci.x ? INTRA : 0) | (nr ? NEAR : 0);
                     atomicAdd(&cnt_f[k + tb], 1);
                     if (nr) {
                         atomicAdd(&cnt_nf[k + tb], 1);
@@ -1166,7 +1267,7 @@ static __global__ void __launch_bounds__(SEARCH_THREADS, 8) k_search(const Dev* 
             n = 0;
             __syncwarp();
         }
-        bool isl = nb > SCR_CAP;
+        bool isl = nb > SCR_CAP || alone;
         if (on) {
             const int2 lcell = last_cell(d, P, pi);
             int nx = 0, nxn = 0;
@@ -1188,9 +1289,30 @@ static __global__ void __launch_bounds__(SEARCH_THREADS, 8) k_search(const Dev* 
         const unsigned il = (__ballot_sync(FULL, isl) >> gshift) & GM;
         if (g == 0 && t < T) {
             d.cnt_b[t] = nb;
-            d.rlong[t] = il != 0;
+            d.rlong[t] = il ? (FACES ? ROW_FACES : ROW_LONG) : 0;
         }
     }
+}
+static __global__ void __launch_bounds__(SEARCH_THREADS, 8) k_search(const Dev* __restrict__ dp) {
+    __shared__ SearchRows sh;
+    __shared__ int s_buf[SEARCH_GROUPS][LIST_CAP];
+    const Dev& d = *dp;
+    if (*d.halt) return;
+    const int TC1 = d.plan[PL_TC1];
+    NBC_GRID_STRIDE(u, TC1) d.ccnt[u] = 0;   // the sort's cell counts back to zero for the next rebuild
+    if (!d.plan[PL_FACE]) search_rows<false>(d, sh, s_buf);
+}
+// The same for a rebuild with cells on faces (see cell_coord); in any other it
+// returns at once, 3 us by itself and under 1% of a step in the graph.  A launch of
+// its own: in k_search the second build costs the first 10% (registers), and
+// dividing there for every subsphere 2 to 3%.  A lattice of 195,112 spheres at
+// rest: 168 us, on three levels 118.
+static __global__ void __launch_bounds__(SEARCH_THREADS) k_search_faces(const Dev* __restrict__ dp) {
+    __shared__ SearchRows sh;
+    __shared__ int s_buf[SEARCH_GROUPS][LIST_CAP];
+    const Dev& d = *dp;
+    if (*d.halt || !d.plan[PL_FACE]) return;
+    search_rows<true>(d, sh, s_buf);
 }
 
 // the pairs of rebuilt scene k's new list (after the scans; a pair has one
@@ -1204,6 +1326,70 @@ static __global__ void k_need(const Dev* __restrict__ dp) {
     const Dev& d = *dp;
     if (*d.halt) return;
     for (int k = threadIdx.x; k < d.plan[PL_NS]; k += blockDim.x) d.need[d.pscene[k]] = list_need(d, k);
+}
+
+// The rows of k_search_faces that are not in the scratch (long ones, and those
+// with an entry without a back entry), a thread each: their candidates once more.
+static __device__ __forceinline__ void fill_faces(const Dev& d) {
+    const int T = d.plan[PL_T], ns = d.plan[PL_NS];
+    NBC_GRID_STRIDE(t, T) {
+        if (d.rlong[t] != ROW_FACES) continue;
+        const PlanItem it = plan_item(d, ns, t);
+        const int i = it.i, tb = t - i, t0 = d.psub[it.k];
+        const ScenePar& P = d.par[it.s];
+        const double4 pi = ld32(d.posr2 + i);
+        const int2 ci = d.cm2[i];
+        const bool hg = P.levels > 1;
+        const int my = hg ? d.level2[i] : 0, w = hg ? 1 : 2;
+        const int base = d.dyn[it.s].pair_off, poff = base - d.cnt_f[t0];
+        int kr = base + d.cnt_b[t] - d.cnt_b[t0];
+        int kb = 2 * base + d.cnt_ns[ci.y + tb] - d.cnt_ns[t0] + d.cnt_nf[t + 1] - d.cnt_nf[t];
+        const double margin = near_margin(P);
+        auto put = [&](int at, int a, int b, int h, int back) {   // b into the front row of a
+            const bool intra = d.cm2[a].x == d.cm2[b].x;
+            const int v = intra ? INTRA : (h == 2 ? NEAR : 0);
+            d.tmp[d.cnt_f[at] + poff + atomicAdd(&d.fcur[at], 1)] = make_int2(b | v, back);
+            return v;
+        };
+#pragma unroll 1
+        for (int l = my; l >= 0; l--) {
+            const bool own = l == my;
+            const double c = hg ? P.lcell[l] : P.cell[0];
+            const int gx = hg ? P.ldim[l][0] : P.gdim[0], gy = hg ? P.ldim[l][1] : P.gdim[1];
+            const int gz = hg ? P.ldim[l][2] : P.gdim[2], c0 = P.cell_off + (hg ? P.loff[l] : 0);
+            int cx = cell_coord(pi.x - P.origin[0], c), cy = cell_coord(pi.y - P.origin[1], c);
+            int cz = cell_coord(pi.z - P.origin[2], c);
+            if (own) {
+                cx = clampi(cx, 0, gx - 1);
+                cy = clampi(cy, 0, gy - 1);
+                cz = clampi(cz, 0, gz - 1);
+            }
+            const int xa = max(cx - w, 0), xb = min(cx + w, gx - 1);
+#pragma unroll 1
+            for (int r = 0; r < (2 * w + 1) * (2 * w + 1) && xa <= xb; r++) {
+                const int sz = r / (2 * w + 1) - w, sy = r % (2 * w + 1) - w, z = cz + sz, y = cy + sy;
+                if (own && (sz > 0 || (sz == 0 && sy > 0))) break;   // sorted behind i
+                if (z < 0 || z >= gz || y < 0 || y >= gy) continue;
+                const int m = c0 + (z * gy + y) * gx, e = min(d.cstart[m + xb + 1], i);
+#pragma unroll 1
+                for (int j = d.cstart[m + xa]; j < e; j++) {
+                    const double4 pj = ld32(d.posr2 + j);
+                    const int h = pair_test(pj, pi, margin), sides = h ? face_sides(d, P, j, pj, i, pi) : 0;
+                    if (!(sides & 1)) continue;
+                    const int v = put(j + tb, j, i, h, sides == 3 ? kr : -1);
+                    if (sides != 3) continue;
+                    d.L[1].bnbr[kr] = j | (v & ~NEAR);
+                    if (v & NEAR) d.bslot[kr] = kb++;
+                    kr++;
+                }
+            }
+        }
+        const int2 lcell = last_cell(d, P, pi);
+        for (int j = lcell.x; j < lcell.y; j++) {
+            const int h = pair_test(pi, ld32(d.posr2 + j), margin);
+            if (h) put(t, i, j, h, -1);
+        }
+    }
 }
 
 // From the scanned counts: row offsets, back rows, every back entry's pair
@@ -1260,7 +1446,8 @@ static __global__ void __launch_bounds__(SEARCH_THREADS, 8) k_fill(const Dev* __
         const int nr = base + cnt_nf[t] - cnt_nf[t0], nnf = cnt_nf[t + 1] - cnt_nf[t];
         const int2 ci = d.cm2[i];
         const int s0 = 2 * base + cnt_ns[ci.y + tb] - cnt_ns[t0];
-        const bool isl = has && d.rlong[t];
+        const int rl = d.rlong[t];
+        const bool isl = has && rl == ROW_LONG;
         if (has && g == 0) {
             Nw.row[i + s] = rf;
             Nw.brow[i + s] = rb;
@@ -1277,12 +1464,12 @@ static __global__ void __launch_bounds__(SEARCH_THREADS, 8) k_fill(const Dev* __
         // a row that is not in the scratch: its candidates once more
         double4 pi = make_double4(0, 0, 0, 0);
         double margin = 0;
-        int cand = has ? nb : 0, r = 0, kb = s0 + nnf, kr = rb;
+        int cand = has && rl != ROW_FACES ? nb : 0, r = 0, kb = s0 + nnf, kr = rb;
         const int* __restrict__ scr = d.scr + (size_t)i * SCR_CAP;
         if (__any_sync(FULL, isl)) {
             pi = ld32(d.posr2 + i);
             margin = near_margin(P);
-            const int c = group_rows(d, P, isl && searches(d, P, i), i, pi, g, sh, grp);
+            const int c = group_rows<false>(d, P, isl && searches(d, P, i), i, pi, g, sh, grp);
             if (isl) cand = c;
         }
         const int most = __reduce_max_sync(FULL, cand);
@@ -1324,6 +1511,7 @@ static __global__ void __launch_bounds__(SEARCH_THREADS, 8) k_fill(const Dev* __
             }
         }
     }
+    if (d.plan[PL_FACE]) fill_faces(d);
     // the clump pass's lanes of the rebuilt scenes, a warp per warp of the
     // table: a clump's members change places among its lanes (a thread per
     // clump and a sort in memory: 64 us for the kernel, so 52)
@@ -1585,6 +1773,7 @@ __global__ void __launch_bounds__(SEARCH_THREADS) k_rows(const Dev* __restrict__
         *d.kc_done = 0;
         *d.any_rebuild = 0;
         *d.step_bar = 0ull;
+        d.plan[PL_FACE] = 0;
     } else if (threadIdx.x == 64 && ns) {
         SceneDyn& y = d.dyn[0];
         const int np = d.cnt_f[T], nn = d.cnt_nf[T], nb = y.nbound;
@@ -1624,6 +1813,7 @@ __global__ void __launch_bounds__(SC_THREADS) k_commit(Dev* __restrict__ dp) {
         if (threadIdx.x == 0) {
             *d.any_rebuild = 0;
             *d.step_bar = 0ull;
+            d.plan[PL_FACE] = 0;
         }
         __syncthreads();
         int run = 0, brun = 0;

@@ -51,6 +51,8 @@ struct ScenePar {
     int levels;     // 1 = single level grid
     double lcell[MAX_LEVELS], licell[MAX_LEVELS];
     float lrmax[MAX_LEVELS];                    // largest radius on each level
+    int inside;     // the box lies inside the grid (of every level)
+    int tight;      // some level's cells are no larger than the reach of a pair with a finer level
     int ldim[MAX_LEVELS][3];
     int loff[MAX_LEVELS];
     // ranges
@@ -105,7 +107,8 @@ constexpr int PL_TC = 2;     // their cell-table entries
 constexpr int PL_T1 = 3;     // PL_T + 1 (scan length of the counts)
 constexpr int PL_TW = 4;     // warps of the clump pass's table with lanes of theirs
 constexpr int PL_TC1 = 5;    // PL_TC + 1 (scan length of the cell counts)
-constexpr int PL_SIZE = 6;
+constexpr int PL_FACE = 6;   // some subsphere lies on a cell's face (see cell_coord); zero between rebuilds
+constexpr int PL_SIZE = 7;
 
 struct Dev {
     int S, N, K;
