@@ -1207,6 +1207,7 @@ class EngineT final : public EngineBase {
         if ((long long)N_ >= (1LL << 30)) throw ArgError("more than 2^30 subspheres in one engine");
         h_.S = S_; h_.N = N_; h_.K = K_;
         h_.cells = cells;
+        h_.turn = step_turn();
 
         // host arrays: subspheres in the input order, clumps in the engine's
         std::vector<int> fix(N_), lev(N_, 0), sid(N_), csid(K_);
@@ -1310,6 +1311,7 @@ class EngineT final : public EngineBase {
             h_.step_phase = flags + 10;
             h_.step_runs = flags + 11;
             h_.step_bar = (unsigned long long*)(flags + 12);
+            h_.step_base = flags + 14;
             h_.kA = m.take<int>(N); h_.vA = m.take<int>(N); h_.vB = m.take<int>(N);
             h_.posf = m.take<float4>(N);
             h_.ccnt = m.take<int>((size_t)cells + S_ + 1);
@@ -1825,7 +1827,7 @@ class EngineT final : public EngineBase {
             CK(cudaGraphConditionalHandleCreate(&hw, graph_loop_, 1, cudaGraphCondAssignDefault));
             CK(cudaStreamBeginCaptureToGraph(stream_, graph_loop_, nullptr, nullptr, 0,
                                              cudaStreamCaptureModeThreadLocal));
-            k_loop_init<<<1, 1, 0, stream_>>>(h_.loop_left, h_.step_phase, h_.step_bar, 1);
+            k_loop_init<<<1, 1, 0, stream_>>>(h_.loop_left, h_.step_phase, h_.step_bar, h_.step_base, 1);
             CK(cudaGetLastError());
             loop_init_node_ = last_captured_node(stream_);
             cudaGraph_t body = add_conditional(graph_loop_, hw, cudaGraphCondTypeWhile);
@@ -1856,6 +1858,14 @@ class EngineT final : public EngineBase {
         }
         capturing_ = false;
     }
+    // Steps of one launch of k_steps at most: about 2 ms' worth.  Its blocks fill
+    // an SM each, so what other streams of the process have waiting (copies and
+    // kernels of other libraries, other engines) runs between two launches; 9,000
+    // spheres at rest, a call of 20,000 steps: a small kernel on another stream
+    // waited 186 ms without this, and waits 1.3 with it.  A launch costs 8 us (500
+    // clumps, us a step: 11.5 without turns, 11.5 with 128 steps, 11.6 with 64,
+    // 11.9 with 16).
+    int step_turn() const { return std::max(4, std::min(128, (int)(2000.0 / (12.0 + N_ / 2500.0)))); }
     // Blocks of k_steps: one per SM at most; a smaller scene gets blocks for
     // its warps (clump pass, or about two near pairs per subsphere) at two busy
     // warps each, so that its work spreads over the SMs (2,000 spheres in FP64,
@@ -1901,7 +1911,7 @@ class EngineT final : public EngineBase {
         return cp.conditional.phGraph_out[0];
     }
     void launch_loop(int n) {
-        void* args[] = {&h_.loop_left, &h_.step_phase, &h_.step_bar, &n};
+        void* args[] = {&h_.loop_left, &h_.step_phase, &h_.step_bar, &h_.step_base, &n};
         cudaKernelNodeParams kp = {};
         kp.func = (void*)k_loop_init;
         kp.gridDim = dim3(1);

@@ -1773,6 +1773,7 @@ __global__ void __launch_bounds__(SEARCH_THREADS) k_rows(const Dev* __restrict__
         *d.kc_done = 0;
         *d.any_rebuild = 0;
         *d.step_bar = 0ull;
+        *d.step_base = 0;
         d.plan[PL_FACE] = 0;
     } else if (threadIdx.x == 64 && ns) {
         SceneDyn& y = d.dyn[0];
@@ -1813,6 +1814,7 @@ __global__ void __launch_bounds__(SC_THREADS) k_commit(Dev* __restrict__ dp) {
         if (threadIdx.x == 0) {
             *d.any_rebuild = 0;
             *d.step_bar = 0ull;
+            *d.step_base = 0;
             d.plan[PL_FACE] = 0;
         }
         __syncthreads();
@@ -2602,7 +2604,8 @@ __global__ void __launch_bounds__(CT_THREADS) k_sum(const Dev* __restrict__ dp) 
 // ===========================================================================
 
 // A grid barrier that also tells whether any block raised `flag`: one 64-bit
-// counter, arrivals below, raised flags above, zeroed between launches.  The
+// counter, arrivals below, raised flags above, zeroed when a rebuild or a graph
+// launch starts it anew (in between, Dev::step_base has the arrivals so far).  The
 // wait is bounded (ST_SPIN polls, some seconds); a block that gives up sets
 // *fail and *halt and every block leaves at its own limit.  The launch is
 // cooperative, so all blocks run at the same time.  Returns 0 or 1, or -1 when
@@ -2636,7 +2639,8 @@ __device__ __forceinline__ int step_barrier(const Dev& d, unsigned target, int f
     return *s_out;
 }
 
-// Steps until *loop_left are done or some scene needs a rebuild: per step the
+// Steps until *loop_left are done, some scene needs a rebuild, or Dev::turn steps
+// have been taken: per step the
 // clump pass, a grid barrier, pairs and boundary candidates, a grid barrier.
 // A step that needs a rebuild leaves the launch after its clump pass (the
 // graph's if node runs the rebuild) and the next launch takes up its contact
@@ -2690,6 +2694,7 @@ __global__ void __launch_bounds__(ST_THREADS, 1) k_steps(const Dev* __restrict__
     const int lane = threadIdx.x & 31;
     const int gw = (threadIdx.x >> 5) * gridDim.x + blockIdx.x, nw = gridDim.x * ST_WARPS;
     int L = *d.lstep, post = *d.post_pending, left = *d.loop_left, started = 0;
+    const int turn = d.turn;
     bool contact = *d.step_phase != 0;
     const int np = d.nprefix[S], nb = d.bprefix[S];
     const int wp = (np + 31) / 32, wb = (nb + 31) / 32;
@@ -2729,7 +2734,7 @@ __global__ void __launch_bounds__(ST_THREADS, 1) k_steps(const Dev* __restrict__
     const uint8_t was0 = was;
     __syncthreads();
     const ScenePar* par = S == 1 ? &s_par : nullptr;
-    unsigned target = 0;
+    unsigned target = *d.step_base;
     int out = 0;
     for (;;) {
         if (!contact) {
@@ -2785,7 +2790,7 @@ __global__ void __launch_bounds__(ST_THREADS, 1) k_steps(const Dev* __restrict__
         // a raised flag seen here is another block's next clump pass: not yet ours
         out = min(step_barrier(d, target, 0, &s_out), 0);
         left--;
-        if (out || left <= 0) break;
+        if (out || left <= 0 || started >= turn) break;
     }
     if (own && was != was0) d.touch[0][pq] = was;
     if (lead) {
@@ -2797,16 +2802,18 @@ __global__ void __launch_bounds__(ST_THREADS, 1) k_steps(const Dev* __restrict__
         *d.loop_left = left;
         *d.step_phase = reb;
         cudaGraphSetConditional(cond, reb ? 1u : 0u);
-        cudaGraphSetConditional(loop, reb ? 1u : 0u);
+        *d.step_base = (int)target;   // (a rebuild starts the barrier anew)
+        cudaGraphSetConditional(loop, reb || (out == 0 && left > 0) ? 1u : 0u);
     }
 }
 
 // The steps a graph launch takes (the first node of its graph; the count is
 // set before each launch) and the barrier's start.
-static __global__ void k_loop_init(int* left, int* phase, unsigned long long* bar, int n) {
+static __global__ void k_loop_init(int* left, int* phase, unsigned long long* bar, int* base, int n) {
     *left = n;
     *phase = 0;
     *bar = 0ull;
+    *base = 0;
 }
 
 }  // namespace nbc

@@ -216,11 +216,14 @@ struct Dev {
     int* kc_done;     // blocks of k_clump finished (last-block detection)
     int* lstep;       // steps started by k_clump, counted by its last block (per-scene stops)
     // a graph launch of many steps (k_steps): steps left, whether the next
-    // launch starts with a contact pass, launches so far, the grid barrier
+    // launch starts with a contact pass, launches so far, the grid barrier and
+    // its arrivals before the next launch
     int* loop_left;
     int* step_phase;
     int* step_runs;
     unsigned long long* step_bar;
+    int* step_base;
+    int turn;         // steps of one launch of k_steps at most
     // export (per pair), written by the export variant of the contact kernel
     void* xfcn;       // Real4 [cap] normal force on the owner (CacheFcn)
     void* xcpt;       // double4 [cap] contact point (CacheCpt)
