@@ -9,6 +9,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <chrono>
 #include <cmath>
 #include <cstdio>
@@ -169,6 +170,10 @@ static void validate_scene(const nbc_scene_desc& D, int s) {
             throw ArgError(at + "grid cell size not positive on level " + std::to_string(l));
 }
 
+// Engines of the process with step launches on their device that nobody has
+// waited for yet (see step_grid); one count per device.
+static std::atomic<int> g_stepping[64];
+
 template <typename R>
 class EngineT final : public EngineBase {
    public:
@@ -179,8 +184,11 @@ class EngineT final : public EngineBase {
             if (gexec_[t]) cudaGraphExecDestroy(gexec_[t]);
             if (graph_[t]) cudaGraphDestroy(graph_[t]);
         }
-        if (gexec_loop_) cudaGraphExecDestroy(gexec_loop_);
-        if (graph_loop_) cudaGraphDestroy(graph_loop_);
+        leave_stepping();
+        for (Loop& l : loop_) {
+            if (l.exec) cudaGraphExecDestroy(l.exec);
+            if (l.graph) cudaGraphDestroy(l.graph);
+        }
         for (cudaEvent_t e : ev_) cudaEventDestroy(e);
         for (auto& row : gev_)
             for (cudaEvent_t e : row) if (e) cudaEventDestroy(e);
@@ -226,9 +234,10 @@ class EngineT final : public EngineBase {
             n--;
         }
         if (n <= 0) return pend_eager_;
-        if (timing_ == 0 && !loop_tried_) capture_loop();
+        cur_ = &loop_[timing_ == 0 ? enter_stepping() : 0];
+        if (timing_ == 0 && !cur_->tried) capture_loop(*cur_);
         pend_before_ = read_gstep();
-        if (timing_ == 0 && gexec_loop_) {
+        if (timing_ == 0 && cur_->exec) {
             n = std::min(n, ST_MAX_STEPS);
             runs_before_ = read_int(h_.step_runs);
             launch_loop(n);
@@ -243,8 +252,9 @@ class EngineT final : public EngineBase {
         int done = pend_eager_;
         if (pend_ > 0) {
             CK(cudaStreamSynchronize(stream_));
+            leave_stepping();
             const int started = read_gstep() - pend_before_;
-            if (timing_ == 0 && gexec_loop_) {
+            if (timing_ == 0 && cur_->exec) {
                 launches_ += 1 + read_int(h_.step_runs) - runs_before_;   // k_loop_init, k_steps
             } else {
                 launches_ += (1LL + CONTACT_LAUNCHES) * started;
@@ -884,8 +894,8 @@ class EngineT final : public EngineBase {
     }
     void launch_info(int* step_loop, int* search_lanes, int* clump_batch, int* pair_blocks) override {
         if (step_loop) {
-            if (opt_.use_graph && !loop_tried_) capture_loop();
-            *step_loop = gexec_loop_ ? 1 : 0;
+            if (opt_.use_graph && !loop_[0].tried) capture_loop(loop_[0]);
+            *step_loop = loop_[0].exec ? 1 : 0;
         }
         if (search_lanes) *search_lanes = search_lanes_;
         if (clump_batch) *clump_batch = clump_batch_;
@@ -898,7 +908,7 @@ class EngineT final : public EngineBase {
 
    private:
     nbc_options opt_;
-    bool shared_gpu_;        // other engines step beside this one (see step_grid)
+    bool shared_gpu_;        // a request server's, which steps several side by side (see step_grid)
     DevMem mem_;
     char* pslab_ = nullptr;  // the pair buffers' slab
     int4* relmap_ = nullptr; // [S] region moves of a re-layout
@@ -937,12 +947,32 @@ class EngineT final : public EngineBase {
     // contact pass (k_pairs + k_sum), [2] event nodes at every mark
     cudaGraph_t graph_[3] = {nullptr, nullptr, nullptr};
     cudaGraphExec_t gexec_[3] = {nullptr, nullptr, nullptr};
-    // the untimed graph with a device-side step loop (capture_loop)
-    cudaGraph_t graph_loop_ = nullptr;
-    cudaGraphExec_t gexec_loop_ = nullptr;
-    cudaGraphNode_t loop_init_node_ = nullptr;
-    bool loop_tried_ = false;
-    std::string loop_error_;
+    // the untimed graph with a device-side step loop (capture_loop): [v] for an
+    // engine that is one of up to 2^v stepping on the device (see step_grid),
+    // made when needed
+    struct Loop {
+        cudaGraph_t graph = nullptr;
+        cudaGraphExec_t exec = nullptr;
+        cudaGraphNode_t init = nullptr;
+        bool tried = false;
+    };
+    static constexpr int SHARES = 6;
+    Loop loop_[SHARES];
+    Loop* cur_ = &loop_[0];   // the one of the steps enqueued
+    bool stepping_ = false;   // counted in g_stepping
+    // the engine counts as stepping; which of its loops to take
+    int enter_stepping() {
+        std::atomic<int>& n = g_stepping[opt_.device & 63];
+        const int all = stepping_ ? n.load() : n.fetch_add(1) + 1;
+        stepping_ = true;
+        int v = 0;
+        while (!shared_gpu_ && v + 1 < SHARES && (1 << v) < all) v++;
+        return v;
+    }
+    void leave_stepping() {
+        if (stepping_) g_stepping[opt_.device & 63].fetch_sub(1);
+        stepping_ = false;
+    }
     // kernel timing: one record of NMARK events per step, at the marks
     //   0 step start  1 after k_clump  2 after the rebuild node
     //   3/4 around k_boundary and 5 start of the contact pass (second branch)
@@ -1817,44 +1847,43 @@ class EngineT final : public EngineBase {
     // (an event node in a loop body would be overwritten by every iteration).
     // If the loop graph cannot be built the engine keeps launching one step
     // per graph.
-    void capture_loop() {
-        loop_tried_ = true;
+    void capture_loop(Loop& l) {
+        l.tried = true;
         capturing_ = true;
         capture_timed_ = 0;
         try {
-            CK(cudaGraphCreate(&graph_loop_, 0));
+            CK(cudaGraphCreate(&l.graph, 0));
             cudaGraphConditionalHandle hw;
-            CK(cudaGraphConditionalHandleCreate(&hw, graph_loop_, 1, cudaGraphCondAssignDefault));
-            CK(cudaStreamBeginCaptureToGraph(stream_, graph_loop_, nullptr, nullptr, 0,
+            CK(cudaGraphConditionalHandleCreate(&hw, l.graph, 1, cudaGraphCondAssignDefault));
+            CK(cudaStreamBeginCaptureToGraph(stream_, l.graph, nullptr, nullptr, 0,
                                              cudaStreamCaptureModeThreadLocal));
             k_loop_init<<<1, 1, 0, stream_>>>(h_.loop_left, h_.step_phase, h_.step_bar, h_.step_base, 1);
             CK(cudaGetLastError());
-            loop_init_node_ = last_captured_node(stream_);
-            cudaGraph_t body = add_conditional(graph_loop_, hw, cudaGraphCondTypeWhile);
+            l.init = last_captured_node(stream_);
+            cudaGraph_t body = add_conditional(l.graph, hw, cudaGraphCondTypeWhile);
             cudaGraph_t g2 = nullptr;
             CK(cudaStreamEndCapture(stream_, &g2));
             cudaGraphConditionalHandle hif;
             CK(cudaGraphConditionalHandleCreate(&hif, body, 0, cudaGraphCondAssignDefault));
             CK(cudaStreamBeginCaptureToGraph(stream_, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
-            launch_steps(hif, hw);
+            launch_steps(hif, hw, (int)(&l - loop_));
             cudaGraph_t rbody = add_conditional(body, hif, cudaGraphCondTypeIf);
             CK(cudaStreamEndCapture(stream_, &g2));
             CK(cudaStreamBeginCaptureToGraph(stream_, rbody, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
             launch_rebuild(false);
             CK(cudaStreamEndCapture(stream_, &g2));
-            CK(cudaGraphInstantiate(&gexec_loop_, graph_loop_, 0));
-        } catch (const CudaError& e) {
+            CK(cudaGraphInstantiate(&l.exec, l.graph, 0));
+        } catch (const CudaError&) {
             cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
             if (cudaStreamIsCapturing(stream_, &cs) == cudaSuccess && cs != cudaStreamCaptureStatusNone) {
                 cudaGraph_t g = nullptr;
                 cudaStreamEndCapture(stream_, &g);
             }
             (void)cudaGetLastError();
-            if (gexec_loop_) cudaGraphExecDestroy(gexec_loop_);
-            if (graph_loop_) cudaGraphDestroy(graph_loop_);
-            gexec_loop_ = nullptr;
-            graph_loop_ = nullptr;
-            loop_error_ = e.what();
+            if (l.exec) cudaGraphExecDestroy(l.exec);
+            if (l.graph) cudaGraphDestroy(l.graph);
+            l.exec = nullptr;
+            l.graph = nullptr;
         }
         capturing_ = false;
     }
@@ -1869,21 +1898,26 @@ class EngineT final : public EngineBase {
     // Blocks of k_steps: one per SM at most; a smaller scene gets blocks for
     // its warps (clump pass, or about two near pairs per subsphere) at two busy
     // warps each, so that its work spreads over the SMs (2,000 spheres in FP64,
-    // us a step: 2 warps 12.8, 8 warps 15.2, 16 warps 20.7).  Launches of
-    // engines that run beside each other have to fit the GPU together: an engine
-    // of a request server takes a block per 32 warps (8 requests of 400 to
-    // 5,000 clumps: 2 warps 47.5 ms, 16 warps 32 and in one process of five 44,
-    // 32 warps 32 to 34, 64 warps 38.6).
-    int step_grid() const {
+    // us a step: 2 warps 12.8, 8 warps 15.2, 16 warps 20.7).
+    //
+    // Launches of engines that run beside each other have to fit the GPU
+    // together, or they take turns.  One of up to 2^v engines that the process has
+    // stepping on the device takes 1/2^v of the SMs at most (us for a step of each
+    // of eight engines: 2,000 clumps 30, 5,000 57, 12,000 145; with one block per SM
+    // 80, 93, 165; separate kernels for every step 48, 66, 172).  The engines of a
+    // request server, which starts them all before it waits, take a block per 32
+    // warps (8 requests of 400 to 5,000 clumps: 2 warps 47.5 ms, 16 warps 32 and in
+    // one process of five 44, 32 warps 32 to 34, 64 warps 38.6).
+    int step_grid(int v) const {
         int per_sm = 0;
         const void* f = sphere_any_ ? (const void*)k_steps<R, true> : (const void*)k_steps<R, false>;
         CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, f, ST_THREADS, 0));
         const int warps = std::max(h_.W + cdiv(S_, 32), cdiv(2LL * N_, 32));
-        return std::max(1, std::min(per_sm * sm_count_, cdiv(warps, shared_gpu_ ? 32 : 2)));
+        return std::max(1, std::min(per_sm * sm_count_ >> v, cdiv(warps, shared_gpu_ ? 32 : 2)));
     }
-    void launch_steps(cudaGraphConditionalHandle hif, cudaGraphConditionalHandle hw) {
+    void launch_steps(cudaGraphConditionalHandle hif, cudaGraphConditionalHandle hw, int v) {
         cudaLaunchConfig_t c = {};
-        c.gridDim = dim3(step_grid());
+        c.gridDim = dim3(step_grid(v));
         c.blockDim = dim3(ST_THREADS);
         c.stream = stream_;
         cudaLaunchAttribute at[1];
@@ -1917,8 +1951,8 @@ class EngineT final : public EngineBase {
         kp.gridDim = dim3(1);
         kp.blockDim = dim3(1);
         kp.kernelParams = args;
-        CK(cudaGraphExecKernelNodeSetParams(gexec_loop_, loop_init_node_, &kp));
-        CK(cudaGraphLaunch(gexec_loop_, stream_));
+        CK(cudaGraphExecKernelNodeSetParams(cur_->exec, cur_->init, &kp));
+        CK(cudaGraphLaunch(cur_->exec, stream_));
     }
 
     // a graph launch stopped at a rebuild whose pairs did not fit: grow and
