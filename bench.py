@@ -185,9 +185,10 @@ def run_b200(args, world, rank, local):
     tuned = None
     if args.autotune:
         # launch shapes measured on this scene (results do not depend on them)
-        tuned = nbc.autotune([scene], precision=args.precision, device=local, trial_steps=200)
+        tuned = nbc.autotune([scene], precision=args.precision, device=local, trial_steps=200,
+                             use_graph=bool(args.graph))
     opts = dict(precision=args.precision, use_graph=args.graph, device=local, pair_slack=args.pair_slack,
-                search_lanes=args.search_lanes, tuned=tuned)
+                tuned=tuned)
 
     # ---- device-resident throughput -----------------------------------
     eng = nbc.Engine([scene], **opts)
@@ -594,11 +595,11 @@ def run_cfg2(args):
         # state in an eager engine (kernel nodes of a graph with a conditional
         # node are not profiled) and put the profiler range around --steps steps
         import torch
-        e = nbc.Engine([bed], precision=args.precision, search_lanes=args.search_lanes)
+        e = nbc.Engine([bed], precision=args.precision)
         e.step(args.profile_window)
         state = e.restart_scene(bed)
         e.close()
-        e = nbc.Engine([state], precision=args.precision, use_graph=False, search_lanes=args.search_lanes)
+        e = nbc.Engine([state], precision=args.precision, use_graph=False)
         e.step(3)
         e.sync()
         torch.cuda.synchronize()
@@ -612,7 +613,7 @@ def run_cfg2(args):
                           "rebuilds": st["rebuilds"], "pairs": st["npairs"]}), flush=True)
         e.close()
         return
-    e = nbc.Engine([bed], precision=args.precision, search_lanes=args.search_lanes)
+    e = nbc.Engine([bed], precision=args.precision)
     t0 = time.perf_counter()
     e.step(args.settle2)
     e.sync()
@@ -642,7 +643,7 @@ def run_cfg2(args):
     dt = float(sc["params"]["StepSize"])
     total = int(round(0.5 / dt))
     nchunk = 100
-    e = nbc.Engine([sc], precision=args.precision, search_lanes=args.search_lanes)
+    e = nbc.Engine([sc], precision=args.precision)
     z0 = float(sc["intruder"]["pos"][2])
     curve, done = [[0.0, 0.0, 0.0, 0.0]], 0
     t0 = time.perf_counter()
@@ -833,7 +834,6 @@ def main():
                     help="short run for profilers: warm-up + timed steps only, no e2e / CPU legs")
     ap.add_argument("--pair-slack", type=float, default=0.0,
                     help="pair buffer capacity over the first list (0 = engine default)")
-    ap.add_argument("--search-lanes", type=int, default=0, help="lanes per subsphere in the neighbour search")
     ap.add_argument("--scene", default=None, help="run this scene file instead of generating cfg1")
     ap.add_argument("--save-state", default=None, help="advance --advance steps, save the state to this file, exit")
     ap.add_argument("--advance", type=int, default=18000)

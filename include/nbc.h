@@ -122,11 +122,10 @@ typedef struct {
     int device;         /* CUDA device ordinal */
     double pair_slack;  /* pair capacity = slack * pairs of the first list; 0 = 1.6 and at least
                            the reference's own n_sub * BranchLmtLen/2 as far as 30% of free memory allows */
-    int search_lanes;   /* kept for callers and reported back (8, 16 or 32; 0 = 8): the neighbour search has
-                           8 lanes a subsphere */
-    int clump_batch;    /* kept for callers and reported back (1, 2 or 4; 0 = 1): the clump pass gives each
-                           member a lane of its own */
-    int pair_blocks;    /* blocks per SM of the pair kernel's grid: 2 .. 16 (0 = 12) */
+    int search_lanes;   /* kept for callers, selects nothing: the neighbour search has 8 lanes a subsphere */
+    int clump_batch;    /* kept for callers, selects nothing: the clump pass gives each member a lane of its own */
+    int pair_blocks;    /* blocks per SM of the pair kernel's grid: 2 .. 16 (0 = 12); untimed steps with
+                           use_graph do not launch it (see nbc_launch_info) */
 } nbc_options;
 
 typedef struct nbc_engine nbc_engine;
@@ -309,14 +308,15 @@ nbc_status nbc_server_destroy(nbc_server* s);
 nbc_status nbc_server_set_cohort(nbc_server* s, int max_requests);
 
 /* Autotuner (no reference counterpart): times trial_steps steps (after a
- * short warm-up) of engines made from these scenes with candidate launch
- * shapes -- blocks per SM of the pair kernel, which steps outside the
- * device-side loop use -- by coordinate descent from the defaults, a candidate replacing the incumbent only when
- * it is at least 3% faster, and writes the fastest into opt (other fields
- * untouched).  The shapes change no result: every candidate computes the
- * same lists and forces bit for bit.  The choice is cached in the process
- * by scene shape (scenes, subspheres, clumps, grid levels, precision) and
- * trial length; best_ms_per_step (may be NULL) receives its time. */
+ * short warm-up) of engines made from these scenes with these options and
+ * candidate blocks per SM of the pair kernel, a candidate replacing the
+ * incumbent only when it is at least 3% faster, and writes the launch shapes
+ * into opt (other fields untouched).  Where the steps run as a device-side loop
+ * (use_graph) they do not launch that kernel: one trial, and the default.  The
+ * shapes change no result: every candidate computes the same lists and forces
+ * bit for bit.  The choice is cached in the process by scene shape (scenes,
+ * subspheres, clumps, grid levels, precision), use_graph and trial length;
+ * best_ms_per_step (may be NULL) receives its time. */
 nbc_status nbc_autotune(const nbc_scene_desc* const* scenes, int n_scenes, nbc_options* opt, int trial_steps,
                         double* best_ms_per_step);
 

@@ -441,15 +441,16 @@ nbc_status nbc_checkpoint_read(nbc_engine* e, const char* path) {
 }
 
 // ---- autotuner ------------------------------------------------------------
-// Coordinate descent over the launch shapes from the defaults: each trial
-// makes an engine from the scenes, takes a short warm-up (the first list
-// build included) and times trial_steps steps on the host clock around a
-// synchronised nbc_step; a candidate replaces the incumbent only when it is
-// at least 3% faster, so timing noise between equal shapes keeps the
-// defaults.  Cached per process by scene shape.
+// The blocks per SM of the pair kernel, from the default: each trial makes an
+// engine from the scenes with the caller's options, takes a short warm-up (the
+// first list build included) and times trial_steps steps on the host clock around
+// a synchronised nbc_step; a candidate replaces the incumbent only when it is
+// at least 3% faster, so timing noise between equal shapes keeps the default.
+// Engines with the device-side step loop do not launch that kernel: their one
+// trial gives the time.  Cached per process by scene shape.
 namespace {
 struct Tuned {
-    int search_lanes, clump_batch, pair_blocks;
+    int pair_blocks;
     double ms;
 };
 std::map<std::string, Tuned> g_tuned;
@@ -470,48 +471,50 @@ nbc_status nbc_autotune(const nbc_scene_desc* const* scenes, int n, nbc_options*
     }
     const std::string key = std::to_string(n) + "|" + std::to_string(nsub) + "|" + std::to_string(ncl) + "|" +
                             std::to_string(lv) + "|" + std::to_string(opt->precision) + "|" +
-                            std::to_string(trial_steps) + "|" + std::to_string(opt->device);
+                            std::to_string(trial_steps) + "|" + std::to_string(opt->device) + "|" +
+                            std::to_string(opt->use_graph != 0);
+    auto write = [&](const Tuned& t) {
+        opt->search_lanes = 8;
+        opt->clump_batch = 1;
+        opt->pair_blocks = t.pair_blocks;
+        if (best_ms) *best_ms = t.ms;
+    };
     {
         std::lock_guard<std::mutex> lock(g_tuned_mu);
         auto it = g_tuned.find(key);
         if (it != g_tuned.end()) {
-            opt->search_lanes = it->second.search_lanes;
-            opt->clump_batch = it->second.clump_batch;
-            opt->pair_blocks = it->second.pair_blocks;
-            if (best_ms) *best_ms = it->second.ms;
+            write(it->second);
             return NBC_OK;
         }
     }
     return guard([&] {
         std::vector<const nbc_scene_desc*> v(scenes, scenes + n);
         const int warm = std::max(20, trial_steps / 5);
+        int loop = 0;   // the engine's steps ran as a device-side loop
         auto trial = [&](const nbc_options& o) {
             std::unique_ptr<nbc::EngineBase> e(nbc::make_engine(v, o));
             e->step(warm, false);
             const auto t0 = std::chrono::steady_clock::now();
             e->step(trial_steps, false);
             const auto t1 = std::chrono::steady_clock::now();
+            e->launch_info(&loop, nullptr, nullptr, nullptr);
             return std::chrono::duration<double, std::milli>(t1 - t0).count() / trial_steps;
         };
         nbc_options best = *opt;
-        best.search_lanes = 8;
-        best.clump_batch = 1;
         best.pair_blocks = 12;
-        best.use_graph = 1;
         double tb = trial(best);
         const int blocks[] = {4, 8, 16};
         for (int x : blocks) {
+            if (loop) break;
             nbc_options o = best;
             o.pair_blocks = x;
             const double t = trial(o);
             if (t < 0.97 * tb) { best = o; tb = t; }
         }
-        opt->search_lanes = best.search_lanes;
-        opt->clump_batch = best.clump_batch;
-        opt->pair_blocks = best.pair_blocks;
-        if (best_ms) *best_ms = tb;
+        const Tuned t{best.pair_blocks, tb};
+        write(t);
         std::lock_guard<std::mutex> lock(g_tuned_mu);
-        g_tuned[key] = Tuned{best.search_lanes, best.clump_batch, best.pair_blocks, tb};
+        g_tuned[key] = t;
     });
 }
 

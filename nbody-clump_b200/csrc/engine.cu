@@ -897,8 +897,8 @@ class EngineT final : public EngineBase {
             if (opt_.use_graph && !loop_[0].tried) capture_loop(loop_[0]);
             *step_loop = loop_[0].exec ? 1 : 0;
         }
-        if (search_lanes) *search_lanes = search_lanes_;
-        if (clump_batch) *clump_batch = clump_batch_;
+        if (search_lanes) *search_lanes = SEARCH_G;
+        if (clump_batch) *clump_batch = 1;   // members per lane
         if (pair_blocks) *pair_blocks = pair_bps_;
     }
     void info(double* bytes, double* ms) override {
@@ -926,8 +926,6 @@ class EngineT final : public EngineBase {
     bool sphere_kin_ = false;   // some scene runs the sphere drivers' kinematics (Dev::fint)
     bool has_kinds_ = false;    // some scene has split-driver body kinds (Dev::kind)
     bool first_list_ = true;
-    int search_lanes_ = 8;   // as given; the search has its own (SEARCH_G)
-    int clump_batch_ = 1;    // as given; the clump pass has one member per lane whatever it says
     int pair_bps_ = 12;      // blocks per SM of the pair kernel's grid
     int sm_count_ = 148;
     int ring_len_ = 1;
@@ -1091,8 +1089,6 @@ class EngineT final : public EngineBase {
         hflag_ = g_pinned.get();
         mem_.stream = stream_;
         DevMem::keep_pool(opt_.device);
-        search_lanes_ = opt_.search_lanes == 16 || opt_.search_lanes == 32 ? opt_.search_lanes : 8;
-        clump_batch_ = opt_.clump_batch == 2 || opt_.clump_batch == 4 ? opt_.clump_batch : 1;
         pair_bps_ = opt_.pair_blocks >= 2 && opt_.pair_blocks <= 16 ? opt_.pair_blocks : 12;
         CK(cudaDeviceGetAttribute(&sm_count_, cudaDevAttrMultiProcessorCount, opt_.device));
         S_ = (int)sc.size();

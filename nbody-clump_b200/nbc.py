@@ -480,15 +480,16 @@ def _options(precision="mixed", use_graph=True, device=0, pair_slack=0.0, search
     return o
 
 
-def autotune(scenes, precision="mixed", device=0, trial_steps=200, cache=None):
+def autotune(scenes, precision="mixed", device=0, trial_steps=200, cache=None, use_graph=True):
     """nbc_autotune: the fastest launch shapes for these scenes (a dict of
-    TUNED_KEYS plus ms_per_step).  `cache`, a JSON file, keeps the choice by
-    scene shape across processes, so a shape is measured once."""
+    TUNED_KEYS plus ms_per_step), for engines made with this `use_graph`.
+    `cache`, a JSON file, keeps the choice by scene shape across processes, so a
+    shape is measured once."""
     import json
     key = "|".join(str(x) for x in (len(scenes), sum(int(s["params"]["NumberBody"]) for s in scenes),
                                     sum(int(s["params"]["ClumpNum"]) for s in scenes),
                                     max(len(s["levels"]["cell"]) if s.get("levels") else 1 for s in scenes),
-                                    precision, trial_steps))
+                                    precision, trial_steps) + (() if use_graph else ("eager",)))
     book = {}
     if cache and os.path.exists(cache):
         with open(cache) as f:
@@ -497,7 +498,7 @@ def autotune(scenes, precision="mixed", device=0, trial_steps=200, cache=None):
             return dict(book[key], cached=True)
     descs = [scene_desc(s) for s in scenes]
     arr = (C.POINTER(SceneDesc) * len(scenes))(*[C.pointer(d) for d, _ in descs])
-    o = _options(precision, True, device)
+    o = _options(precision, use_graph, device)
     ms = C.c_double(0.0)
     _check(lib().nbc_autotune(arr, len(scenes), C.byref(o), int(trial_steps), C.byref(ms)))
     out = {k: int(getattr(o, k)) for k in TUNED_KEYS}
