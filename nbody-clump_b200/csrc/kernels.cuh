@@ -1124,11 +1124,15 @@ __device__ __forceinline__ int group_rows(const Dev& d, const ScenePar& P, bool 
         ca[k] = cstart[ca[k]];
         cb[k] = r0 + k == (wide ? FACE_ROWS - 1 : 4) ? i : cstart[cb[k]];
     }
-    // rows with candidates, packed: (rows << 24 | candidates) summed over the lanes
+    // rows with candidates, packed: (rows << 26 | candidates) summed over the lanes
+    // (2^26 subspheres are 100 GB of state, without their pairs)
+    constexpr int CBITS = 26;
+    constexpr unsigned CMASK = (1u << CBITS) - 1u;
+    static_assert(MAX_ROWS < 1 << (32 - CBITS) && FACE_ROWS <= MAX_ROWS, "the rows' count above the candidates");
     unsigned acc = 0;
 #pragma unroll
     for (int k = 0; k < MAXC; k++)
-        if (ca[k] >= 0 && cb[k] > ca[k]) acc += (1u << 24) + (unsigned)(cb[k] - ca[k]);
+        if (ca[k] >= 0 && cb[k] > ca[k]) acc += (1u << CBITS) + (unsigned)(cb[k] - ca[k]);
     unsigned inc = acc;
 #pragma unroll
     for (int o = 1; o < G; o <<= 1) {
@@ -1140,12 +1144,12 @@ __device__ __forceinline__ int group_rows(const Dev& d, const ScenePar& P, bool 
 #pragma unroll
     for (int k = 0; k < MAXC; k++)
         if (ca[k] >= 0 && cb[k] > ca[k]) {
-            const int c = (int)(at & 0xffffffu);
-            rows[at >> 24] = make_int2(c + cb[k] - ca[k], ca[k] - c);
-            at += (1u << 24) + (unsigned)(cb[k] - ca[k]);
+            const int c = (int)(at & CMASK);
+            rows[at >> CBITS] = make_int2(c + cb[k] - ca[k], ca[k] - c);
+            at += (1u << CBITS) + (unsigned)(cb[k] - ca[k]);
         }
     __syncwarp();
-    return (int)(all & 0xffffffu);
+    return (int)(all & CMASK);
 }
 
 // the members of a single-level scene's last cell when subsphere i's stencil
