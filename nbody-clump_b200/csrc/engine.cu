@@ -1636,7 +1636,9 @@ class EngineT final : public EngineBase {
     }
 
     void check_scan() {
-        if (read_int(h_.scan_fail)) throw CudaError("a list-rebuild scan gave up waiting on a tile (step halted)");
+        const int w = read_int(h_.scan_fail);
+        if (w == WAIT_BARRIER) throw CudaError("the step loop gave up waiting at its grid barrier (step halted)");
+        if (w) throw CudaError("a list-rebuild scan gave up waiting on a tile (step halted)");
     }
     void check_errors() {
         check_scan();

@@ -601,7 +601,7 @@ static __global__ void __launch_bounds__(SC_THREADS) k_scan1(ScanArrays arrs, in
                     if (inc) break;
                 }
                 if (!__all_sync(0xffffffffu, ok) && lane == 0) {
-                    atomicExch(fail, 1);
+                    atomicExch(fail, WAIT_SCAN);
                     atomicExch(halt, 1);
                 }
                 if (lane == 0) atomicExch(&sa[b], SCAN_INC | (unsigned)(excl + total));
@@ -2632,7 +2632,7 @@ __device__ __forceinline__ int step_barrier(const Dev& d, unsigned target, int f
             asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(bar) : "memory");
             if ((unsigned)v >= target) break;
             if (++polls > ST_SPIN) {
-                atomicExch(d.scan_fail, 1);
+                atomicExch(d.scan_fail, WAIT_BARRIER);
                 atomicExch(d.halt, 1);
                 break;
             }

@@ -31,6 +31,10 @@ constexpr int ERR_NONFINITE = 2;       // non-finite wall input/output (src/dem_
 constexpr int ERR_BAD_CLUMP = 4;       // clump id out of range
 constexpr int ERR_ROW_OVERFLOW = 8;    // a row exceeded BranchLmtLen/2 (reference semantics, export only)
 
+// Dev::scan_fail
+constexpr int WAIT_SCAN = 1;      // k_scan1 on a tile
+constexpr int WAIT_BARRIER = 2;   // k_steps at its grid barrier
+
 // ScenePar::sphere: the reference's sphere-only drivers where they differ
 // from the clump path (bits 1, 2, 4 are NBC_SPHERE_* of the C ABI)
 constexpr int SPH_KIN = 1;      // first half-kick and attitude without the intruder; penetrator cohesion
@@ -175,7 +179,7 @@ struct Dev {
     int* fcur;
     unsigned long long* scan_st;          // single-launch scan: tile states (zero between scans)
     int* scan_ctl;                        // single-launch scan: ticket and finished-block counters
-    int* scan_fail;                       // a single-launch scan gave up a wait (the step halted)
+    int* scan_fail;                       // a wait gave up and the step halted: WAIT_SCAN, WAIT_BARRIER
     int* any_rebuild;                     // device flag: some scene rebuilds this step
     // rebuild plan (k_plan): the scenes rebuilt at this step in ascending
     // order and prefix sums over them; every rebuild kernel runs over the
