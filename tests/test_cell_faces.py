@@ -159,3 +159,36 @@ def test_touching_lattice_forces(dims):
     a, b, c = dims
     assert e.contact_counts()[1] == (a - 1) * b * c + a * (b - 1) * c + a * b * (c - 1)
     e.close()
+
+
+def test_rebuilds_on_faces_inside_the_step_loop():
+    """Two lattices that approach along x, their y and z on faces: a rebuild at
+    every step, with lists that outgrow their region on the way."""
+    r = 1.5e-3
+    sc = _lattice(r, 2.0, (6, 3, 60))
+    x = sc["sub"]["pos"][:, 0]
+    right = x > 5 * r
+    for p in (sc["sub"]["pos"], sc["clump"]["pos"]):
+        p[right, 0] += 2.1 * r
+    sc["clump"]["vel"][right, 0] = -0.02 * r / sc["params"]["StepSize"]
+    for k in ("WorldSize_x", "BoxUpLmt_x"):
+        sc["params"][k] += 4 * r
+    assert _rounded_apart(sc).any()
+    a = nbc.Engine([sc], precision="f64", pair_slack=1.0)
+    b = nbc.Engine([sc], precision="f64", pair_slack=4.0, use_graph=False)
+    a.step(1)
+    first = a.info()["device_bytes"]
+    for n in (20, 40, 35):
+        a.step(n)
+    a.sync()
+    b.step(96)
+    b.sync()
+    assert a.info()["device_bytes"] > first, "the lists did not outgrow their region"
+    o = oracle.OracleScene(sc, threads=4)
+    o.step(96)
+    for e in (a, b):
+        (la, lb), (oa, ob) = e.pairs(), o.pairs()
+        assert np.array_equal(la, oa) and np.array_equal(lb, ob)
+        assert e.stats()["rebuilds"] == o.rebuilds
+    for k in ("pos", "vel", "quat", "angvel"):
+        assert np.array_equal(a.clumps()[k], b.clumps()[k])
