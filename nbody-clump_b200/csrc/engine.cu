@@ -403,8 +403,7 @@ class EngineT final : public EngineBase {
         *np = y.npairs;
         if (!lpa && !lpb) return;
         if (cap_in < y.npairs) throw ArgError("pair buffer too small");
-        int lc = read_int(h_.lcur);
-        const PairList& Lc = h_.L[lc & 1];
+        const PairList& Lc = h_.L[0];
         std::vector<int> own(y.npairs), nbr(y.npairs);
         copy_(own.data(), Lc.own + y.pair_off, y.npairs * sizeof(int), cudaMemcpyDeviceToHost);
         copy_(nbr.data(), Lc.nbr + y.pair_off, y.npairs * sizeof(int), cudaMemcpyDeviceToHost);
@@ -680,7 +679,6 @@ class EngineT final : public EngineBase {
             int zero = 0;
             copy_(h_.any_rebuild, &zero, sizeof(int), cudaMemcpyHostToDevice);
             copy_(h_.halt, &zero, sizeof(int), cudaMemcpyHostToDevice);
-            copy_(h_.lcur, &zero, sizeof(int), cudaMemcpyHostToDevice);
             copy_(h_.kc_done, &zero, sizeof(int), cudaMemcpyHostToDevice);
         }
         // subspheres, current sort order
@@ -911,7 +909,7 @@ class EngineT final : public EngineBase {
     bool shared_gpu_;        // a request server's, which steps several side by side (see step_grid)
     DevMem mem_;
     char* pslab_ = nullptr;  // the pair buffers' slab
-    int4* relmap_ = nullptr; // [S] region moves of a re-layout
+    int3* relmap_ = nullptr; // [S] region moves of a re-layout
     size_t pslab_bytes_ = 0;
     char* xslab_ = nullptr;  // the export step's per-pair buffers (null until one runs)
     size_t xslab_bytes_ = 0;
@@ -1327,7 +1325,6 @@ class EngineT final : public EngineBase {
             h_.post_pending = flags + 0;
             h_.any_rebuild = flags + 1;
             h_.halt = flags + 2;
-            h_.lcur = flags + 3;
             h_.hgen = flags + 4;
             h_.gstep = flags + 5;
             h_.kc_done = flags + 6;
@@ -1367,7 +1364,7 @@ class EngineT final : public EngineBase {
             h_.pcell = m.take<int>(S_ + 1);
             h_.pwarp = m.take<int>(S_ + 1);
             h_.need = m.take<int>(S_);
-            relmap_ = m.take<int4>(S_);
+            relmap_ = m.take<int3>(S_);
             h_.xparts = m.take<R4<R>>(6 * N);
             h_.xintr = m.take<R4<R>>(4 * N);
             h_.ring_len = ring_len_;
@@ -1546,14 +1543,13 @@ class EngineT final : public EngineBase {
     void layout_pairs(const std::vector<long long>& pcap) {
         refresh_dev();
         std::vector<SceneDyn> y = read_dyn_all();
-        std::vector<int4> map(S_);
+        std::vector<int3> map(S_);
         long long total = 0;
         int moved = 0;
         for (int s = 0; s < S_; s++) {
             map[s].x = y[s].pair_off;
             map[s].y = (int)total;
-            map[s].z = y[s].npairs;
-            map[s].w = moved;
+            map[s].z = moved;
             moved += y[s].npairs;
             y[s].pair_off = (int)total;
             y[s].pcap = (int)pcap[s];
@@ -1565,7 +1561,7 @@ class EngineT final : public EngineBase {
         const size_t old_bytes = pslab_bytes_;
         alloc_pairs(std::max<long long>(total, 1));
         copy_(h_.dyn, y.data(), S_ * sizeof(SceneDyn), cudaMemcpyHostToDevice);
-        copy_(relmap_, map.data(), S_ * sizeof(int4), cudaMemcpyHostToDevice);
+        copy_(relmap_, map.data(), S_ * sizeof(int3), cudaMemcpyHostToDevice);
         push_dev();
         const int B = 256;
         if (moved > 0)
@@ -1618,8 +1614,7 @@ class EngineT final : public EngineBase {
     RowData pull_rows(int s) {
         refresh_dev();
         const ScenePar& P = hpar_[s];
-        int lc = read_int(h_.lcur);
-        const PairList& Lc = h_.L[lc & 1];
+        const PairList& Lc = h_.L[0];
         RowData rd;
         rd.row.resize(P.nsub + 1);
         rd.brow.resize(P.nsub + 1);

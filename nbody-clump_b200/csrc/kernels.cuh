@@ -1,6 +1,8 @@
 // kernels.cuh -- sm_100a kernels of the B200 DEM engine.
 //
-// Step structure (one CUDA graph per step, see engine.cu):
+// Step structure.  k_steps takes many steps in a launch, the graph's loop puts the
+// rebuilds between its launches (engine.cu, capture_loop); timed, eager and
+// export steps launch the passes one by one:
 //   k_clump      per clump: member force/torque sum and second half-kick of
 //                the previous step, first half-kick, drift, attitude and the
 //                pose of every member subsphere (+ rebuild test); one extra
@@ -37,7 +39,7 @@ constexpr int INTRA = (int)0x80000000u;
 // (src/dem_clumpsphere.cu:86-151), IntegratePene_Before_cuk and
 // Integrate_After_cuk (src/dem_integrate_penetrator.cu:3-113).
 //
-// One member per lane.  The host packs whole clumps into warps (Dev::ltab, a
+// One member per lane.  The host packs whole clumps into warps (Dev::lrec, a
 // record per lane; members of a clump are consecutive lanes, a clump of more
 // than 32 members has a warp of its own that walks them 32 at a time, a clump
 // without members one lane).  A lane sums its member's contact slots, forms
@@ -1911,11 +1913,12 @@ __global__ void __launch_bounds__(SC_THREADS) k_commit(Dev* __restrict__ dp) {
 
 // Moves every scene's list to a new layout of the pair regions (the host
 // grows them): entries, back references, and the near pairs' records,
-// histories and touch flags (the contact slots are rewritten before they are
-// read).  map[s] = (old first slot, new first slot, pairs, prefix of the pairs
-// over the scenes); d holds the new buffers, o the old ones.
+// histories and touch flags.  The contact slots of touching pairs are rewritten
+// by the contact pass before they are read; those of the others, which it does
+// not write, are zeroed here.  map[s] = (old first slot, new first slot, prefix
+// of the pairs over the scenes); d holds the new buffers, o the old ones.
 template <typename R>
-__global__ void k_relayout(const Dev* __restrict__ dp, Dev o, const int4* __restrict__ map, int total) {
+__global__ void k_relayout(const Dev* __restrict__ dp, Dev o, const int3* __restrict__ map, int total) {
     const Dev& d = *dp;
     const size_t cap = (size_t)d.cap, oc = (size_t)o.cap;
     const R4<R>* Ho = (const R4<R>*)o.H[0];
@@ -1926,21 +1929,22 @@ __global__ void k_relayout(const Dev* __restrict__ dp, Dev o, const int4* __rest
         int lo = 0, hi = d.S - 1;
         while (lo < hi) {
             const int m = (lo + hi + 1) >> 1;
-            if (map[m].w <= u) lo = m;
+            if (map[m].z <= u) lo = m;
             else hi = m - 1;
         }
-        const int4 m = map[lo];
-        const size_t po = m.x + (u - m.w), pn = m.y + (u - m.w);
+        const int3 m = map[lo];
+        const size_t po = m.x + (u - m.z), pn = m.y + (u - m.z);
         const int delta = m.y - m.x;
         Lc.nbr[pn] = ol.nbr[po];
         Lc.own[pn] = ol.own[po];
         Lc.bnbr[pn] = ol.bnbr[po];
         const int bq = ol.bpair[po];
         Lc.bpair[pn] = bq >= 0 ? bq + delta : bq;
-        if (u - m.w >= d.dyn[lo].nnear) continue;
+        if (u - m.z >= d.dyn[lo].nnear) continue;
         const int4 a = o.rec[0][2 * po], b = o.rec[0][2 * po + 1];
         d.rec[0][2 * pn] = a;
-        d.rec[0][2 * pn + 1] = make_int4(b.x, b.y, b.z + 2 * delta, b.w >= 0 ? b.w + 2 * delta : b.w);
+        const int sf = b.z + 2 * delta, sb = b.w >= 0 ? b.w + 2 * delta : b.w;
+        d.rec[0][2 * pn + 1] = make_int4(b.x, b.y, sf, sb);
         d.np[0][pn] = o.np[0][po] + delta;
         const uint8_t f = o.touch[0][po];
         d.touch[0][pn] = f;
@@ -1948,6 +1952,11 @@ __global__ void k_relayout(const Dev* __restrict__ dp, Dev o, const int4* __rest
             Hn[2 * pn] = Ho[2 * po];
             Hn[2 * pn + 1] = Ho[2 * po + 1];
             ((R*)(Hn + 2 * cap))[pn] = ((const R*)(Ho + 2 * oc))[po];
+        } else {
+            R4<R>* slots = (R4<R>*)d.slots;
+            const R4<R> zero = pack<R>(v3<R>(0, 0, 0), R(0));
+            st_pair(slots + 2 * (size_t)sf, zero, zero);
+            if (sb >= 0) st_pair(slots + 2 * (size_t)sb, zero, zero);
         }
     }
 }
@@ -1955,7 +1964,7 @@ __global__ void k_relayout(const Dev* __restrict__ dp, Dev o, const int4* __rest
 // the current rows and near rows follow their scene's region: every offset of scene s
 // moves by its region's move (the subsphere threads take the row starts and
 // the contact slots, one thread per scene the end entry, then the clump pass's lanes)
-static __global__ void k_shift_rows(const Dev* __restrict__ dp, const int4* __restrict__ map) {
+static __global__ void k_shift_rows(const Dev* __restrict__ dp, const int3* __restrict__ map) {
     const Dev& d = *dp;
     const PairList& Lc = d.L[0];
     NBC_GRID_STRIDE(u, d.N + d.S) {

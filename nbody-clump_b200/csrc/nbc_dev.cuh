@@ -197,7 +197,6 @@ struct Dev {
     // (those that can touch before the next rebuild), in each scene's pair
     // region in the order of the near front rows
     PairList L[2];
-    int* lcur;        // index of the current list (0)
     int2* tmp;        // [cap] front entries being built: partner with flags, back entry
     int* bslot;       // [cap] contact slot of each near back entry, being built
     int* nro[2];      // [N+S] near front row offsets (absolute; one row array per scene with its end entry)
