@@ -203,18 +203,24 @@ class EngineT final : public EngineBase {
     void step(int n, bool exp) override {
         auto t0 = std::chrono::steady_clock::now();
         int left = n;
+        bool checked = false;   // wait_steps has looked for errors
         while (left > 0) {
             if (exp && left == 1) {
                 clear_post_done();
                 run_step_eager(true);
+                checked = false;
                 left -= 1;
                 continue;
             }
             enqueue(exp ? left - 1 : left);
             left -= wait_steps();
+            checked = true;
         }
-        CK(cudaStreamSynchronize(stream_));
-        check_errors();
+        if (!checked) {
+            CK(cudaStreamSynchronize(stream_));
+            check_wait(read_int(h_.scan_fail));
+            check_errors();
+        }
         last_ms_ = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
     }
 
@@ -236,10 +242,11 @@ class EngineT final : public EngineBase {
         if (n <= 0) return pend_eager_;
         cur_ = &loop_[timing_ == 0 ? enter_stepping() : 0];
         if (timing_ == 0 && !cur_->tried) capture_loop(*cur_);
-        pend_before_ = read_gstep();
+        const Flags f = read_flags();
+        pend_before_ = f.v[FL_GSTEP];
         if (timing_ == 0 && cur_->exec) {
             n = std::min(n, ST_MAX_STEPS);
-            runs_before_ = read_int(h_.step_runs);
+            runs_before_ = f.v[FL_STEP_RUNS];
             launch_loop(n);
         } else {
             if (!gexec_[timing_]) capture(timing_);
@@ -253,14 +260,15 @@ class EngineT final : public EngineBase {
         if (pend_ > 0) {
             CK(cudaStreamSynchronize(stream_));
             leave_stepping();
-            const int started = read_gstep() - pend_before_;
+            const Flags f = read_flags();
+            const int started = f.v[FL_GSTEP] - pend_before_;
             if (timing_ == 0 && cur_->exec) {
-                launches_ += 1 + read_int(h_.step_runs) - runs_before_;   // k_loop_init, k_steps
+                launches_ += 1 + f.v[FL_STEP_RUNS] - runs_before_;   // k_loop_init, k_steps
             } else {
                 launches_ += (1LL + CONTACT_LAUNCHES) * started;
             }
-            if (read_int(h_.halt)) {
-                check_scan();
+            check_wait(f.v[FL_SCAN_FAIL]);
+            if (f.v[FL_HALT]) {
                 // the last step started stopped at its rebuild: finish it on the host path
                 steps_done_ += started - 1;
                 recover_halt();
@@ -268,9 +276,11 @@ class EngineT final : public EngineBase {
                 steps_done_ += started;
             }
             done += started;
+        } else {
+            CK(cudaStreamSynchronize(stream_));
+            check_wait(read_int(h_.scan_fail));
         }
         pend_ = pend_eager_ = 0;
-        CK(cudaStreamSynchronize(stream_));
         check_errors();
         return done;
     }
@@ -1321,20 +1331,20 @@ class EngineT final : public EngineBase {
             h_.cF = m.take<double4>(K_); h_.cT = m.take<double4>(K_);
             h_.mem_start = m.take<int>(K_ + 1);
             h_.mo = m.take<int2>(N);
-            int* flags = m.take<int>(16);
-            h_.post_pending = flags + 0;
-            h_.any_rebuild = flags + 1;
-            h_.halt = flags + 2;
-            h_.hgen = flags + 4;
-            h_.gstep = flags + 5;
-            h_.kc_done = flags + 6;
-            h_.lstep = flags + 7;
-            h_.loop_left = flags + 8;
-            h_.scan_fail = flags + 9;
-            h_.step_phase = flags + 10;
-            h_.step_runs = flags + 11;
-            h_.step_bar = (unsigned long long*)(flags + 12);
-            h_.step_base = flags + 14;
+            int* flags = m.take<int>(FL_SIZE);
+            h_.post_pending = flags + FL_POST;
+            h_.any_rebuild = flags + FL_REBUILD;
+            h_.halt = flags + FL_HALT;
+            h_.step_base = flags + FL_BASE;
+            h_.hgen = flags + FL_HGEN;
+            h_.gstep = flags + FL_GSTEP;
+            h_.kc_done = flags + FL_KC_DONE;
+            h_.lstep = flags + FL_LSTEP;
+            h_.loop_left = flags + FL_LEFT;
+            h_.scan_fail = flags + FL_SCAN_FAIL;
+            h_.step_phase = flags + FL_PHASE;
+            h_.step_runs = flags + FL_STEP_RUNS;
+            h_.step_bar = (unsigned long long*)(flags + FL_BAR);
             h_.kA = m.take<int>(N); h_.vA = m.take<int>(N); h_.vB = m.take<int>(N);
             h_.posf = m.take<float4>(N);
             h_.ccnt = m.take<int>((size_t)cells + S_ + 1);
@@ -1598,7 +1608,18 @@ class EngineT final : public EngineBase {
         copy_(&v, p, sizeof(int), cudaMemcpyDeviceToHost);
         return v;
     }
-    int read_gstep() { return read_int(h_.gstep); }
+    // the device's words for the steps, one after the other, in one copy (a
+    // blocking copy is 10 us: five of them were a third of a call of one step)
+    enum { FL_POST, FL_REBUILD, FL_HALT, FL_BASE, FL_HGEN, FL_GSTEP, FL_KC_DONE, FL_LSTEP, FL_LEFT, FL_SCAN_FAIL,
+           FL_PHASE, FL_STEP_RUNS, FL_BAR, FL_SIZE = FL_BAR + 2 };
+    struct Flags {
+        int v[FL_SIZE];
+    };
+    Flags read_flags() {
+        Flags f;
+        copy_(&f, h_.post_pending, sizeof(f), cudaMemcpyDeviceToHost);
+        return f;
+    }
     SceneDyn read_dyn(int s) {
         CK(cudaStreamSynchronize(stream_));
         SceneDyn y;
@@ -1630,13 +1651,12 @@ class EngineT final : public EngineBase {
         return rd;
     }
 
-    void check_scan() {
-        const int w = read_int(h_.scan_fail);
+    // (w: Dev::scan_fail)
+    static void check_wait(int w) {
         if (w == WAIT_BARRIER) throw CudaError("the step loop gave up waiting at its grid barrier (step halted)");
         if (w) throw CudaError("a list-rebuild scan gave up waiting on a tile (step halted)");
     }
     void check_errors() {
-        check_scan();
         std::vector<SceneDyn> y(S_);
         copy_(y.data(), h_.dyn, S_ * sizeof(SceneDyn), cudaMemcpyDeviceToHost);
         for (int s = 0; s < S_; s++)
@@ -1732,7 +1752,7 @@ class EngineT final : public EngineBase {
             // size the regions to the first lists, or grow the ones that overflow
             k_need<<<1, 256, 0, stream_>>>(d_);
             CK(cudaStreamSynchronize(stream_));
-            check_scan();
+            check_wait(read_int(h_.scan_fail));
             std::vector<int> need(S_);
             copy_(need.data(), h_.need, S_ * sizeof(int), cudaMemcpyDeviceToHost);
             std::vector<SceneDyn> y = read_dyn_all();
