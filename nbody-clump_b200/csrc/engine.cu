@@ -337,9 +337,10 @@ class EngineT final : public EngineBase {
             copy_(fix, h_.part_fix + o, n * sizeof(int), cudaMemcpyDeviceToHost);
         }
         if (cid) {
-            std::vector<int2> cm(n);
-            copy_(cm.data(), h_.cm + o, n * sizeof(int2), cudaMemcpyDeviceToHost);
-            for (int i = 0; i < n; i++) cid[i] = cold_[cm[i].x];
+            k_clump_ids<<<std::min(cdiv(n, 256), sm_count_ * 8), 256, 0, stream_>>>(h_.cm + o, h_.cold, P.clump_off, n,
+                                                                                   h_.kA);   // a rebuild's scratch
+            CK(cudaGetLastError());
+            copy_(cid, h_.kA, n * sizeof(int), cudaMemcpyDeviceToHost);
         }
         if (pos || rad) {
             std::vector<double4> tmp(n);
@@ -363,28 +364,35 @@ class EngineT final : public EngineBase {
             if (mass) mass[i] = t.w;
         }
     }
-    void get_clump_prop(int s, double* prop) override {
-        const ScenePar& P = hpar_[s];
-        clumps_out<4>(h_.cprop, P, prop);
-    }
-    // clump records of one scene in the caller's order, W doubles each
-    template <int W>
-    void clumps_out(const double4* src, const ScenePar& P, double* dst) {
+    void get_clump_prop(int s, double* prop) override { clumps_out(hpar_[s], {{h_.cprop, prop, 4}}); }
+    // clump records of one scene in the caller's order, w doubles each
+    struct ClumpOut {
+        const double4* src;
+        double* dst;
+        int w;
+    };
+    void clumps_out(const ScenePar& P, std::initializer_list<ClumpOut> list) {
         const int n = P.nclump;
-        k_clumps_out<W><<<std::min(cdiv(n, 256), sm_count_ * 8), 256, 0, stream_>>>(src, h_.cold, P.clump_off, n,
-                                                                                   (double*)h_.stage);
+        ClumpArrays a{};
+        for (const ClumpOut& o : list)
+            if (o.dst) {
+                a.src[a.n] = o.src;
+                a.w[a.n++] = o.w;
+            }
+        k_clumps_out<<<std::min(cdiv(n, 256), sm_count_ * 8), 256, 0, stream_>>>(a, h_.cold, P.clump_off, n,
+                                                                                (double*)h_.stage);
         CK(cudaGetLastError());
-        copy_(dst, h_.stage, (size_t)n * W * sizeof(double), cudaMemcpyDeviceToHost);
+        const double* at = (const double*)h_.stage;
+        for (const ClumpOut& o : list)
+            if (o.dst) {
+                copy_(o.dst, at, (size_t)n * o.w * sizeof(double), cudaMemcpyDeviceToHost);
+                at += (size_t)n * o.w;
+            }
     }
     void get_clumps(int s, double* pos, double* vel, double* quat, double* w, double* f, double* t) override {
         refresh_dev();
-        const ScenePar& P = hpar_[s];
-        if (pos) clumps_out<3>(h_.cpos, P, pos);
-        if (vel) clumps_out<3>(h_.cvel, P, vel);
-        if (w) clumps_out<3>(h_.cw, P, w);
-        if (f) clumps_out<3>(h_.cF, P, f);
-        if (t) clumps_out<3>(h_.cT, P, t);
-        if (quat) clumps_out<4>(h_.cq, P, quat);
+        clumps_out(hpar_[s], {{h_.cpos, pos, 3}, {h_.cvel, vel, 3}, {h_.cw, w, 3}, {h_.cF, f, 3}, {h_.cT, t, 3},
+                              {h_.cq, quat, 4}});
     }
     void get_sub_forces(int s, double* f, double* t) override {
         refresh_dev();
@@ -1327,7 +1335,7 @@ class EngineT final : public EngineBase {
             h_.cq = m.take<double4>(K_); h_.cprop = m.take<double4>(K_);
             h_.cinv = m.take<double4>(K_);
             h_.lrec = m.take<int4>(2 * 32 * (size_t)h_.W); h_.clane = m.take<int>(K_);
-            h_.cold = m.take<int>(K_); h_.stage = m.take<double4>(K_);
+            h_.cold = m.take<int>(K_); h_.stage = m.take<double4>(5 * (size_t)K_);
             h_.cF = m.take<double4>(K_); h_.cT = m.take<double4>(K_);
             h_.mem_start = m.take<int>(K_ + 1);
             h_.mo = m.take<int2>(N);

@@ -395,17 +395,32 @@ __global__ void __launch_bounds__(CL_THREADS, NBC_CLUMP_MINB) k_clump(const Dev*
 }
 
 // Clump records (old: the caller's number of each): the n clumps from `first`
-// on, a scene's, out of the engine as W packed doubles per clump, ready to be
-// copied to the caller's array.
-template <int W>
-static __global__ void k_clumps_out(const double4* __restrict__ src, const int* __restrict__ old, int first, int n,
+// on, a scene's, out of the engine as packed doubles, ready to be copied to the
+// caller's arrays: for each src with a w, n times w doubles one after the other.
+struct ClumpArrays {
+    const double4* src[6];
+    int w[6];
+    int n;
+};
+static __global__ void k_clumps_out(ClumpArrays a, const int* __restrict__ old, int first, int n,
                                     double* __restrict__ dst) {
     for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < n; c += gridDim.x * blockDim.x) {
-        const double4 v = ld32(src + first + c);
-        double* o = dst + (size_t)W * (old[first + c] - first);
-        o[0] = v.x; o[1] = v.y; o[2] = v.z;
-        if (W == 4) o[3] = v.w;
+        const int k = old[first + c] - first;
+        double* o = dst;
+        for (int q = 0; q < a.n; q++) {
+            const double4 v = ld32(a.src[q] + first + c);
+            double* p = o + (size_t)a.w[q] * k;
+            p[0] = v.x; p[1] = v.y; p[2] = v.z;
+            if (a.w[q] == 4) p[3] = v.w;
+            o += (size_t)a.w[q] * n;
+        }
     }
+}
+// the caller's clump, within its scene, of n subspheres
+static __global__ void k_clump_ids(const int2* __restrict__ cm, const int* __restrict__ old, int first, int n,
+                                   int* __restrict__ dst) {
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+        dst[i] = old[cm[i].x] - first;
 }
 // the caller's arrays of W doubles per clump into records in the engine's
 // order; inv: the reciprocals as well (IEEE divisions)

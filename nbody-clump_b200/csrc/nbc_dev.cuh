@@ -158,7 +158,7 @@ struct Dev {
     int* kind;        // [K] body kind of the split driver (0 free, 1 prescribed velocity, 2 fixed),
                       // read in SPH_KINDS scenes only (null when there are none)
     int* cold;        // [K] the caller's number of each clump (counted over all scenes)
-    double4* stage;   // [K] clump records on their way from and to the caller's order
+    double4* stage;   // [5 K] clump records on their way from and to the caller's order (19 doubles a clump)
     double4* cF;      // force on clump from the last force pass
     double4* cT;
     int* mem_start;   // [K+1]
