@@ -1398,11 +1398,13 @@ class EngineT final : public EngineBase {
 
         copy_(h_.par, hpar_.data(), S_ * sizeof(ScenePar), cudaMemcpyHostToDevice);
         copy_(h_.dyn, hdyn.data(), S_ * sizeof(SceneDyn), cudaMemcpyHostToDevice);
-        copy_(h_.sid, sid.data(), N * sizeof(int), cudaMemcpyHostToDevice);
-        copy_(h_.csid, csid.data(), K_ * sizeof(int), cudaMemcpyHostToDevice);
+        if (S_ > 1) {   // (the slab is zeroed)
+            copy_(h_.sid, sid.data(), N * sizeof(int), cudaMemcpyHostToDevice);
+            copy_(h_.csid, csid.data(), K_ * sizeof(int), cudaMemcpyHostToDevice);
+        }
         copy_(h_.cm, cm.data(), N * sizeof(int2), cudaMemcpyHostToDevice);
         copy_(h_.part_fix, fix.data(), N * sizeof(int), cudaMemcpyHostToDevice);
-        copy_(h_.level, lev.data(), N * sizeof(int), cudaMemcpyHostToDevice);
+        if (hgrid_) copy_(h_.level, lev.data(), N * sizeof(int), cudaMemcpyHostToDevice);
         // the caller's arrays go up as they are (several scenes': one after the
         // other) and are packed into records and put in place on the device
         std::vector<double> joined;
@@ -1435,20 +1437,12 @@ class EngineT final : public EngineBase {
                     abs[c] = hpar_[s].clump_off + cold_[c];
             copy_(h_.cold, abs.data(), K_ * sizeof(int), cudaMemcpyHostToDevice);
         }
-        const int gc = std::min(cdiv(K_, 256), sm_count_ * 8);
         double* st = (double*)h_.stage;
-        auto clumps_up = [&](const double* nbc_scene_desc::*field, double4* dst) {
-            upload(st, field, false, 3);
-            k_clumps_up<3><<<gc, 256, 0, stream_>>>(st, h_.cold, K_, dst, nullptr);
-        };
-        clumps_up(&nbc_scene_desc::clump_pos, h_.cpos);
-        clumps_up(&nbc_scene_desc::clump_vel, h_.cvel);
-        clumps_up(&nbc_scene_desc::clump_angvel, h_.cw);
-        upload(st, &nbc_scene_desc::clump_quat, false, 4);
-        k_clumps_up<4><<<gc, 256, 0, stream_>>>(st, h_.cold, K_, h_.cq, nullptr);
-        upload(st, &nbc_scene_desc::clump_prop, false, 4);
-        k_clumps_up<4><<<gc, 256, 0, stream_>>>(st, h_.cold, K_, h_.cprop, h_.cinv);
-        CK(cudaGetLastError());
+        upload(st, &nbc_scene_desc::clump_pos, false, 3);
+        upload(st + 3 * (size_t)K_, &nbc_scene_desc::clump_vel, false, 3);
+        upload(st + 6 * (size_t)K_, &nbc_scene_desc::clump_angvel, false, 3);
+        upload(st + 9 * (size_t)K_, &nbc_scene_desc::clump_quat, false, 4);
+        upload(st + 13 * (size_t)K_, &nbc_scene_desc::clump_prop, false, 4);
         if (h_.kind) copy_(h_.kind, kind.data(), K_ * sizeof(int), cudaMemcpyHostToDevice);
         copy_(h_.clane, clane_.data(), K_ * sizeof(int), cudaMemcpyHostToDevice);
         copy_(h_.mem_start, mstart_.data(), (K_ + 1) * sizeof(int), cudaMemcpyHostToDevice);
@@ -1457,6 +1451,7 @@ class EngineT final : public EngineBase {
         copy_(h_.any_rebuild, &one, sizeof(int), cudaMemcpyHostToDevice);
         push_dev();
         const int g = std::min(cdiv(std::max(N_, 32 * h_.W), 256), sm_count_ * 8);
+        k_clumps_up<<<std::min(cdiv(K_, 256), sm_count_ * 8), 256, 0, stream_>>>(d_);
         k_members_init<<<g, 256, 0, stream_>>>(d_);
         k_lanes_init<<<g, 256, 0, stream_>>>(d_);
         CK(cudaGetLastError());

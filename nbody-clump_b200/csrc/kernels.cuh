@@ -422,17 +422,23 @@ static __global__ void k_clump_ids(const int2* __restrict__ cm, const int* __res
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
         dst[i] = old[cm[i].x] - first;
 }
-// the caller's arrays of W doubles per clump into records in the engine's
-// order; inv: the reciprocals as well (IEEE divisions)
-template <int W>
-static __global__ void k_clumps_up(const double* __restrict__ src, const int* __restrict__ old, int n,
-                                   double4* __restrict__ dst, double4* __restrict__ inv) {
-    for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < n; c += gridDim.x * blockDim.x) {
-        const double* p = src + (size_t)W * old[c];
-        const double4 v = make_double4(p[0], p[1], p[2], W == 4 ? p[W - 1] : 0.0);
-        st32(dst + c, v);
-        if (inv)
-            st32(inv + c, make_double4(__ddiv_rn(1.0, v.x), __ddiv_rn(1.0, v.y), __ddiv_rn(1.0, v.z), __ddiv_rn(1.0, v.w)));
+// the caller's arrays of clumps (st: position, velocity, angular velocity of 3 K
+// doubles each, attitude and properties of 4 K each) into records in the engine's
+// order, and the properties' reciprocals (IEEE divisions)
+static __global__ void k_clumps_up(const Dev* __restrict__ dp) {
+    const Dev& d = *dp;
+    const double* st = (const double*)d.stage;
+    const size_t K = (size_t)d.K;
+    for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < d.K; c += gridDim.x * blockDim.x) {
+        const size_t k = (size_t)d.cold[c];
+        const double *p = st + 3 * k, *v = p + 3 * K, *w = v + 3 * K, *q = st + 9 * K + 4 * k, *m = q + 4 * K;
+        st32(d.cpos + c, make_double4(p[0], p[1], p[2], 0.0));
+        st32(d.cvel + c, make_double4(v[0], v[1], v[2], 0.0));
+        st32(d.cw + c, make_double4(w[0], w[1], w[2], 0.0));
+        st32(d.cq + c, make_double4(q[0], q[1], q[2], q[3]));
+        st32(d.cprop + c, make_double4(m[0], m[1], m[2], m[3]));
+        st32(d.cinv + c,
+             make_double4(__ddiv_rn(1.0, m[0]), __ddiv_rn(1.0, m[1]), __ddiv_rn(1.0, m[2]), __ddiv_rn(1.0, m[3])));
     }
 }
 // body offset and mass (so) into the member's slot, position and radius (sp)
