@@ -595,8 +595,15 @@ class EngineT final : public EngineBase {
         hd.lstep = read_int(h_.lstep);
         hd.ring_len = ring_len_;
         hd.total_cap = h_.cap;
-        std::vector<char> out((const char*)&hd, (const char*)&hd + sizeof(hd));
-        ck_blocks(out, nullptr, 0, hd);
+        // what the file holds per subsphere, clump and pair, in one allocation
+        size_t pairs = 0, near = 0;
+        for (const SceneDyn& y : read_dyn_all()) { pairs += y.npairs; near += y.nnear; }
+        std::vector<char> out;
+        out.reserve(sizeof(hd) + S_ * (sizeof(SceneDyn) + (size_t)ring_len_ * 48 + 64) + (size_t)K_ * 264 +
+                    (size_t)N_ * (176 + (NB_SLOTS * 3 + 4) * sizeof(R4<R>)) + pairs * (26 + hist_bytes(1)) +
+                    near * (20 + 4 * sizeof(R4<R>)) + 4096);
+        out.assign((const char*)&hd, (const char*)&hd + sizeof(hd));
+        ck_blocks(out, nullptr, 0, 0, hd);
         return out;
     }
     void checkpoint_load(const char* data, size_t bytes) override {
@@ -614,8 +621,8 @@ class EngineT final : public EngineBase {
         mem_.release(pslab_, pslab_bytes_);
         alloc_pairs(std::max<long long>(hd.total_cap, 1));
         push_dev();
-        std::vector<char> in(data, data + bytes);
-        ck_blocks(in, &in, sizeof(hd), hd);
+        std::vector<char> none;
+        ck_blocks(none, data, bytes, sizeof(hd), hd);
         steps_done_ = hd.steps_done;
         first_list_ = false;
         post_done_ = false;
@@ -632,7 +639,7 @@ class EngineT final : public EngineBase {
     // off) the checkpoint's blocks in one fixed order.  The file holds clumps
     // in the caller's order and what the engine keeps per member slot in
     // subsphere order, so it does not depend on the engine's own order.
-    void ck_blocks(std::vector<char>& out, const std::vector<char>* src, size_t off, const CkHeader& hd) {
+    void ck_blocks(std::vector<char>& out, const char* src, size_t size, size_t off, const CkHeader& hd) {
         const size_t N = N_;
         auto blk = [&](void* dev, size_t n) {
             if (!n) return;
@@ -641,8 +648,8 @@ class EngineT final : public EngineBase {
                 out.resize(at + n);
                 copy_(out.data() + at, dev, n, cudaMemcpyDeviceToHost);
             } else {
-                if (off + n > src->size()) throw ArgError("checkpoint truncated");
-                copy_(dev, src->data() + off, n, cudaMemcpyHostToDevice);
+                if (off + n > size) throw ArgError("checkpoint truncated");
+                copy_(dev, src + off, n, cudaMemcpyHostToDevice);
                 off += n;
             }
         };
@@ -654,8 +661,8 @@ class EngineT final : public EngineBase {
                 out.resize(at + n);
                 memcpy(out.data() + at, host, n);
             } else {
-                if (off + n > src->size()) throw ArgError("checkpoint truncated");
-                memcpy(host, src->data() + off, n);
+                if (off + n > size) throw ArgError("checkpoint truncated");
+                memcpy(host, src + off, n);
                 off += n;
             }
         };
@@ -687,8 +694,8 @@ class EngineT final : public EngineBase {
             out.resize(at + sizeof(flags));
             memcpy(out.data() + at, flags, sizeof(flags));
         } else {
-            if (off + sizeof(flags) > src->size()) throw ArgError("checkpoint truncated");
-            memcpy(flags, src->data() + off, sizeof(flags));
+            if (off + sizeof(flags) > size) throw ArgError("checkpoint truncated");
+            memcpy(flags, src + off, sizeof(flags));
             off += sizeof(flags);
             copy_(h_.hgen, &flags[0], sizeof(int), cudaMemcpyHostToDevice);
             copy_(h_.gstep, &flags[1], sizeof(int), cudaMemcpyHostToDevice);
@@ -906,7 +913,7 @@ class EngineT final : public EngineBase {
                 copy_(S + 4 * o, sl.data(), 4 * nn * sizeof(R4<R>), cudaMemcpyHostToDevice);
             }
         }
-        if (src && off != src->size()) throw ArgError("checkpoint has trailing bytes");
+        if (src && off != size) throw ArgError("checkpoint has trailing bytes");
     }
     void launch_info(int* step_loop, int* search_lanes, int* clump_batch, int* pair_blocks) override {
         if (step_loop) {
