@@ -192,3 +192,34 @@ def test_rebuilds_on_faces_inside_the_step_loop():
         assert e.stats()["rebuilds"] == o.rebuilds
     for k in ("pos", "vel", "quat", "angvel"):
         assert np.array_equal(a.clumps()[k], b.clumps()[k])
+
+
+def test_batch_rebuilds_some_scenes_on_faces():
+    """Lattices that move along x at different speeds, so that most rebuilds are
+    of some of the scenes: each as it is alone, and as the oracle has it."""
+    scenes = []
+    for k, (r, spacing, dims) in enumerate([(1.5e-3, 2.0, (5, 3, 60)), (2.5e-3, 3.0, (4, 4, 60)), (0.05, 2.0, (4, 60, 3)),
+                                            (1.5e-3, 1.0, (4, 3, 40))]):
+        sc = _lattice(r, spacing, dims, fill=0.5001 if spacing == 1.0 else 1.0, levels=2 if k == 2 else 1)
+        sc["params"]["StepSize"] = 1e-9
+        sc["clump"]["vel"][:, 0] = (k + 1) * 0.17e-3 * r / sc["params"]["StepSize"] * np.linspace(1.0, 0.2, len(sc["clump"]["vel"]))
+        scenes.append(sc)
+    both = nbc.Engine(scenes, precision="f64", pair_slack=3.0)
+    both.step(50)
+    both.sync()
+    counts = set()
+    for s, sc in enumerate(scenes):
+        e = nbc.Engine([sc], precision="f64", pair_slack=3.0)
+        e.step(50)
+        e.sync()
+        o = oracle.OracleScene(sc, threads=4)
+        o.step(50)
+        for k in ("pos", "vel", "quat", "angvel", "force", "torque"):
+            assert np.array_equal(both.clumps(s)[k], e.clumps()[k]), (s, k)
+        assert both.stats(s) == e.stats() and e.stats()["rebuilds"] == o.rebuilds
+        counts.add(o.rebuilds)
+        for x, y in zip(both.rows(s, bl=2400), e.rows(bl=2400)):
+            assert np.array_equal(x, y)
+        (la, lb), (oa, ob) = both.pairs(s), o.pairs()
+        assert np.array_equal(la, oa) and np.array_equal(lb, ob)
+    assert len(counts) > 2
