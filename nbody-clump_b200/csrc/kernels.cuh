@@ -1110,8 +1110,9 @@ __device__ __forceinline__ int group_rows(const Dev& d, const ScenePar& P, bool 
         sh.dist[grp][g][0] = make_float4(far2(cz - 1, gz, fz), cz < 0 || cz >= gz ? INFINITY : 0.0f,
                                          far2(cz + 1, gz, uz), cut * cut);
         sh.dist[grp][g][1] = make_float4(far2(cy - 1, gy, fy), cy < 0 || cy >= gy ? INFINITY : 0.0f,
-                                         far2(cy + 1, gy, uy), xa > 0 && xa < cx ? fx * fx : -1.0f);
-        sh.xp[grp][g] = xb < gx - 1 && xb > cx ? ux * ux : -1.0f;
+                                         far2(cy + 1, gy, uy),
+                                         xa > 0 && xa < cx && xa < gx - 1 ? fx * fx : -1.0f);
+        sh.xp[grp][g] = xb < gx - 1 && xb > cx && xb > 0 ? ux * ux : -1.0f;
         sh.cell[grp][g] = make_int4(base + (cz * gy + cy) * gx + cx, gx, gx * gy,
                                     xa > xb ? 0 : (1 << 16 | (xa - cx + 64) << 8 | (xb - cx + 64)));
     }
@@ -1370,12 +1371,15 @@ static __device__ __forceinline__ void fill_faces(const Dev& d) {
         const int my = hg ? d.level2[i] : 0, w = hg ? 1 : 2;
         const int base = d.dyn[it.s].pair_off, poff = base - d.cnt_f[t0];
         int kr = base + d.cnt_b[t] - d.cnt_b[t0];
+        const int ke = base + d.cnt_b[t + 1] - d.cnt_b[t0];
         int kb = 2 * base + d.cnt_ns[ci.y + tb] - d.cnt_ns[t0] + d.cnt_nf[t + 1] - d.cnt_nf[t];
         const double margin = near_margin(P);
-        auto put = [&](int at, int a, int b, int h, int back) {   // b into the front row of a
+        // b into the front row of a (no row takes more than was counted)
+        auto put = [&](int at, int a, int b, int h, int back) {
             const bool intra = d.cm2[a].x == d.cm2[b].x;
             const int v = intra ? INTRA : (h == 2 ? NEAR : 0);
-            d.tmp[d.cnt_f[at] + poff + atomicAdd(&d.fcur[at], 1)] = make_int2(b | v, back);
+            const int q = d.cnt_f[at] + atomicAdd(&d.fcur[at], 1);
+            if (q < d.cnt_f[at + 1]) d.tmp[q + poff] = make_int2(b | v, back);
             return v;
         };
 #pragma unroll 1
@@ -1403,8 +1407,9 @@ static __device__ __forceinline__ void fill_faces(const Dev& d) {
                     const double4 pj = ld32(d.posr2 + j);
                     const int h = pair_test(pj, pi, margin), sides = h ? face_sides(d, P, j, pj, i, pi) : 0;
                     if (!(sides & 1)) continue;
-                    const int v = put(j + tb, j, i, h, sides == 3 ? kr : -1);
-                    if (sides != 3) continue;
+                    const bool back = sides == 3 && kr < ke;
+                    const int v = put(j + tb, j, i, h, back ? kr : -1);
+                    if (!back) continue;
                     d.L[1].bnbr[kr] = j | (v & ~NEAR);
                     if (v & NEAR) d.bslot[kr] = kb++;
                     kr++;

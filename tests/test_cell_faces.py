@@ -223,3 +223,22 @@ def test_batch_rebuilds_some_scenes_on_faces():
         (la, lb), (oa, ob) = both.pairs(s), o.pairs()
         assert np.array_equal(la, oa) and np.array_equal(lb, ob)
     assert len(counts) > 2
+
+
+@pytest.mark.parametrize("levels", [1, 2, 4])
+@pytest.mark.parametrize("axis", [0, 1, 2])
+@pytest.mark.parametrize("side", [-1, 1])
+def test_around_the_end_of_the_grid(levels, axis, side):
+    """A heap across the end of the grid in a box that goes on: members beyond it
+    are in the border cells however far they are, on every level."""
+    sc = _box(700, 5 + levels, levels, dense=0.5)
+    p, pos = sc["params"], sc["sub"]["pos"]
+    mesh = 3 * sc["sub"]["radius"].max()
+    a = "xyz"[axis]
+    end = p["WorldOrigin_" + a] - mesh if side < 0 else p["WorldOrigin_" + a] + p["WorldSize_" + a] + mesh
+    move = end - pos[:, axis].mean()
+    for q in (pos, sc["clump"]["pos"]):
+        q[:, axis] += move
+    p["BoxLowLmt_" + a] -= 1.0
+    p["BoxUpLmt_" + a] += 1.0
+    _list(sc)
